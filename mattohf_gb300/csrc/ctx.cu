@@ -94,13 +94,24 @@ struct mattohf_ctx {
   double2 *d_a = nullptr, *d_b = nullptr, *d_c = nullptr;
   size_t stage_cap = 0;
   // Fock partial sums
-  double2* d_scratch = nullptr;
-  size_t scratch_cap = 0;
   double* d_colbuf = nullptr;
   size_t colbuf_cap = 0;
   double2* d_sym = nullptr;   // symmetric-exchange tile partials
   size_t sym_cap = 0;
   double2* d_symF = nullptr;  // reduced symmetric exchange [NK*NBocc][NG]
+  // fixed-point exchange (k_fock_fx.cu)
+  int4* d_ufx = nullptr;      // occupied orbitals in limbs
+  int2* d_fx_sizes = nullptr;
+  int* d_fx_shift = nullptr;
+  double2* d_fx_fscale = nullptr;
+  int2* d_uscale = nullptr;
+  int4* d_wfx = nullptr;      // other functions in limbs and their scales
+  double2* d_wscale = nullptr;
+  unsigned long long *d_fx_acc = nullptr, *d_wacc = nullptr;  // exchange sums
+  size_t wfx_cap = 0;
+  int2* d_kern_fx = nullptr;  // kernel table in limbs, its scale, the twiddles
+  int2* d_kscale = nullptr;
+  int4* d_tw_fx = nullptr;
   float4* d_udf = nullptr;    // double-float copy of the occupied orbitals
   float2* d_kern_df = nullptr;
   float4* d_tw_df = nullptr;
@@ -201,31 +212,18 @@ int ensure_stage(mattohf_ctx* ctx, size_t elems) {
   return MATTOHF_OK;
 }
 
-// Pair chunking of the Fock kernel: enough items to fill the device's SMs
-// eight times over, each chunk a whole number of team rounds.
 void fock_split(const mattohf_ctx* c, int ncols, int* nchunks, int* chunk) {
-  const int npairs = c->NK * c->NBocc;
-  int nch = c->opt_chunks;
-  if (nch <= 0) {
-    const int target = std::max(1, c->nsm) * 8;
-    nch = (target + ncols - 1) / ncols;
-  }
-  nch = std::max(1, std::min(nch, npairs));
-  int ch = (npairs + nch - 1) / nch;
-  nch = (npairs + ch - 1) / ch;
-  *nchunks = nch;
-  *chunk = ch;
+  fx_rows_split(c->NG, ncols, c->NK * c->NBocc, c->nsm, c->opt_chunks, nchunks, chunk);
 }
 
 int ensure_scratch(mattohf_ctx* ctx, int ncols) {
-  int nch, ch;
-  fock_split(ctx, ncols, &nch, &ch);
-  const size_t need = (size_t)ncols * nch * ctx->NG;
-  if (need > ctx->scratch_cap) {
+  if ((size_t)ncols > ctx->wfx_cap) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
-    destroy_graph(ctx);  // the captured step holds the old pointer
-    CKR(dalloc(ctx, &ctx->d_scratch, need));
-    ctx->scratch_cap = need;
+    destroy_graph(ctx);  // the captured step holds the old pointers
+    CKR(dalloc(ctx, &ctx->d_wfx, (size_t)ncols * ctx->NG));
+    CKR(dalloc(ctx, &ctx->d_wacc, (size_t)ncols * 4 * ctx->NG));
+    CKR(dalloc(ctx, &ctx->d_wscale, (size_t)ncols));
+    ctx->wfx_cap = ncols;
   }
   const size_t cb = (size_t)ncols * 4;
   if (cb > ctx->colbuf_cap) {
@@ -254,7 +252,7 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr) {
   a.occ = ctx->occ;
   a.vCG = ctx->d_vCG;
   a.vion = ctx->d_vion;
-  a.tw = ctx->tw;
+  a.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
   a.dvcell = ctx->dvcell;
   a.rho = ctx->d_rho;
   a.vloc = ctx->d_vloc;
@@ -269,10 +267,9 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr) {
 
 // Which exchange partials a combine launch reads.
 struct FockPlan {
-  int nchunks = 1;            // chunked partials per column (bands >= b0)
-  int b0 = 0;                 // first band served by the chunked partials
-  const double2* sym = nullptr;
-  int S = 0, T = 0;
+  bool occ = false;           // occupied bands by the symmetric exchange
+  int b0 = 0;                 // first band of the others
+  bool rows = false;          // bands >= b0 by the exchange on rows
   bool any = false;           // exchange present at all
 };
 
@@ -317,19 +314,78 @@ int timed_end(mattohf_ctx* ctx) {
 // RK4 steps captured in one graph for mattohf_rk4_run (divides 256)
 constexpr int kGraphSteps = 8;
 
+// Tile of the fixed-point exchange.
+int fx_tile(const mattohf_ctx* ctx) {
+  return std::min(kFxMaxTile, ctx->opt_tile > 0 ? ctx->opt_tile : choose_sym_tile(ctx->NG, ctx->NK * ctx->NBocc, ctx->nsm));
+}
+
+// Tile of the adjoint's and the double-float exchange.
 int sym_tile(const mattohf_ctx* ctx) {
   return ctx->opt_tile > 0 ? ctx->opt_tile : choose_sym_tile(ctx->NG, ctx->NK * ctx->NBocc, ctx->nsm);
 }
 
 // Every buffer the RK4 step's exchange applies need, allocated up front so a
 // graph capture never has to grow one.
+int ensure_fx(mattohf_ctx* ctx) {
+  const size_t M = (size_t)ctx->NK * ctx->NBocc;
+  if (!ctx->d_symF) CKR(dalloc(ctx, &ctx->d_symF, M * ctx->NG));
+  if (!ctx->d_ufx) CKR(dalloc(ctx, &ctx->d_ufx, M * ctx->NG));
+  if (!ctx->d_fx_sizes) CKR(dalloc(ctx, &ctx->d_fx_sizes, M));
+  if (!ctx->d_fx_shift) CKR(dalloc(ctx, &ctx->d_fx_shift, M));
+  if (!ctx->d_fx_fscale) CKR(dalloc(ctx, &ctx->d_fx_fscale, M));
+  if (!ctx->d_uscale) CKR(dalloc(ctx, &ctx->d_uscale, 1));
+  if (!ctx->d_fx_acc) CKR(dalloc(ctx, &ctx->d_fx_acc, M * 4 * ctx->NG));
+  return MATTOHF_OK;
+}
+
+// The fixed-point exchange's arguments for the occupied orbitals of u at tile S.
+FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
+  FockFxArgs a;
+  a.u = u;
+  a.nk = ctx->NK;
+  a.nbocc = ctx->NBocc;
+  a.S = S;
+  a.T = (ctx->NK * ctx->NBocc + S - 1) / S;
+  a.sizes = ctx->d_fx_sizes;
+  a.ufx = reinterpret_cast<fx::lc*>(ctx->d_ufx);
+  a.shift = ctx->d_fx_shift;
+  a.fscale = ctx->d_fx_fscale;
+  a.uscale = ctx->d_uscale;
+  a.kern = ctx->d_kern_fx;
+  a.kscale = ctx->d_kscale;
+  a.tw = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
+  a.acc = ctx->d_fx_acc;
+  return a;
+}
+
+size_t sym_partials(int M, int S, int NG) {
+  const size_t T = (M + S - 1) / S;
+  return T * (T + 1) / 2 * 2 * S * NG;
+}
+
+// The exchange on columns w (k-points from k0 on) of the occupied orbitals of u,
+// which are already in fixed point.
+int enq_fock_rows(mattohf_ctx* ctx, Block u, Block w, int nk_w, int k0) {
+  const int ncols = nk_w * w.nb;
+  CKR(ensure_scratch(ctx, ncols));
+  FockFxArgs a = fx_args(ctx, u, 1);
+  a.kern += (size_t)k0 * ctx->NG;
+  FockFxRows r;
+  r.w = w;
+  r.ncols = ncols;
+  r.wfx = reinterpret_cast<fx::lc*>(ctx->d_wfx);
+  r.wscale = ctx->d_wscale;
+  r.acc = ctx->d_wacc;
+  fock_split(ctx, ncols, &r.nchunks, &r.chunk);
+  CK(launch_fock_fx(ctx->NG, a, r, ctx->st));
+  return MATTOHF_OK;
+}
+
 int ensure_fock_buffers(mattohf_ctx* ctx) {
   CKR(ensure_scratch(ctx, ctx->NK * ctx->NB));
   const int M = ctx->NK * ctx->NBocc;
-  const int S = sym_tile(ctx);
-  const int T = (M + S - 1) / S;
-  CKR(ensure_sym(ctx, (size_t)T * (T + 1) / 2 * 2 * S * ctx->NG));
-  if (!ctx->d_symF) CKR(dalloc(ctx, &ctx->d_symF, (size_t)M * ctx->NG));
+  if (ctx->opt_df) CKR(ensure_sym(ctx, sym_partials(M, sym_tile(ctx), ctx->NG)));
+  CKR(ensure_fx(ctx));
   if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * ctx->NG));
   return MATTOHF_OK;
 }
@@ -337,27 +393,17 @@ int ensure_fock_buffers(mattohf_ctx* ctx) {
 // Exchange partials of h[u] w.  When w is u itself (all RK4 stages, Ex,
 // Subspace_diag, eps) the occupied rows use the symmetric pair kernel and only
 // the unoccupied rows (if any) take the chunked kernel.
-int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan) {
+int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = false) {
   *plan = FockPlan();
   plan->any = true;
   const bool same = (w.p == u.p) && (w.kstride == u.kstride) && (w.nb == u.nb);
   const int NG = ctx->NG;
   if (same && ctx->opt_sym) {
     const int M = ctx->NK * ctx->NBocc;
-    const int S = sym_tile(ctx);
+    const int S = ctx->opt_df ? sym_tile(ctx) : fx_tile(ctx);
     const int T = (M + S - 1) / S;
-    CKR(ensure_sym(ctx, (size_t)T * (T + 1) / 2 * 2 * S * NG));
-    if (!ctx->d_symF) CKR(dalloc(ctx, &ctx->d_symF, (size_t)M * NG));
-    FockSymArgs a;
-    a.u = u;
-    a.nk = ctx->NK;
-    a.nbocc = ctx->NBocc;
-    a.S = S;
-    a.T = T;
-    a.kern = ctx->d_kern;
-    a.tw = ctx->tw;
-    a.scratch = ctx->d_sym;
-    a.F = ctx->d_symF;
+    if (ctx->opt_df) CKR(ensure_sym(ctx, sym_partials(M, S, NG)));
+    CKR(ensure_fx(ctx));
     CKR(timed_begin(ctx));
     if (ctx->opt_df) {
       if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * NG));
@@ -373,34 +419,29 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan) {
       d.F = ctx->d_symF;
       CK(launch_fock_sym_df(NG, d, u.p, u.kstride, ctx->d_udf, ctx->st));
     } else {
-      CK(launch_fock_sym(NG, a, ctx->st));
+      CK(launch_fx_orbitals(NG, fx_args(ctx, u, S), ctx->st));
+      CK(launch_fock_sym_fx(NG, fx_args(ctx, u, S), ctx->st));
     }
     CKR(timed_end(ctx));
-    plan->sym = ctx->d_symF;
-    plan->S = S;
-    plan->T = T;
+    plan->occ = true;
     plan->b0 = ctx->NBocc;
     if (w.nb == ctx->NBocc) return MATTOHF_OK;
   }
   Block wr = w;
   wr.p = w.p + (size_t)plan->b0 * NG;
   wr.nb = w.nb - plan->b0;
-  const int ncols = ctx->NK * wr.nb;
-  CKR(ensure_scratch(ctx, ncols));
-  FockArgs a;
-  a.u = u;
-  a.w = wr;
-  a.nk = ctx->NK;
-  a.nbocc = ctx->NBocc;
-  a.kern = ctx->d_kern;
-  a.tw = ctx->tw;
-  a.scratch = ctx->d_scratch;
-  fock_split(ctx, ncols, &a.nchunks, &a.chunk);
-  plan->nchunks = a.nchunks;
+  CKR(ensure_fx(ctx));
   CKR(timed_begin(ctx));
-  CK(launch_fock(ctx->NG, a, ncols, ctx->st));
+  if (!same_u && (!plan->occ || ctx->opt_df)) CK(launch_fx_orbitals(NG, fx_args(ctx, u, 1), ctx->st));
+  CKR(enq_fock_rows(ctx, u, wr, ctx->NK, 0));
+  plan->rows = true;
   CKR(timed_end(ctx));
   return MATTOHF_OK;
+}
+
+// The symmetric exchange's result, of the fixed-point or the double-float kernels.
+ExSource occ_source(const mattohf_ctx* ctx, bool df) {
+  return df ? ExSource{nullptr, nullptr, ctx->d_symF} : ExSource{ctx->d_fx_acc, ctx->d_fx_fscale, nullptr};
 }
 
 CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const FockPlan& fp) {
@@ -408,16 +449,13 @@ CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const F
   std::memset(&a, 0, sizeof(a));
   a.w = w;
   const bool ex = ctx->hf && mode != CM_T && fp.any;
-  a.scratch = ex ? ctx->d_scratch : nullptr;
-  a.sym = ex ? fp.sym : nullptr;
-  a.sym_S = fp.S;
-  a.sym_T = fp.T;
-  a.chunk_b0 = fp.b0;
-  a.nchunks = fp.nchunks;
+  if (ex && fp.occ) a.occ_ex = occ_source(ctx, ctx->opt_df);
+  if (ex && fp.rows) a.row_ex = ExSource{ctx->d_wacc, ctx->d_wscale, nullptr};
+  a.row_b0 = fp.b0;
   a.vloc = ctx->d_vloc;
   a.Gx = ctx->d_Gx;
   a.kx = ctx->d_kx;
-  a.tw = ctx->tw;
+  a.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
   a.af = af;
   a.mode = mode;
   a.nk = ctx->NK;
@@ -431,10 +469,12 @@ CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const F
 }
 
 // h[u] w -> out  (mode CM_H), or the exchange / kinetic term alone.
-int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mode) {
+// same_u: the previous enq_hpsi applied the operator of the same, unchanged u,
+// whose local potential and fixed-point orbitals still hold.
+int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mode, bool same_u = false) {
   FockPlan fp;
-  if (mode == CM_H) CKR(enq_density(ctx, u));
-  if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp));
+  if (mode == CM_H && !same_u) CKR(enq_density(ctx, u));
+  if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp, same_u));
   else if (mode == CM_F) {
     CK(cudaMemsetAsync(out.p, 0, sizeof(double2) * (size_t)ctx->NK * out.kstride, ctx->st));
     return MATTOHF_OK;
@@ -812,6 +852,12 @@ int compute_tables(mattohf_ctx* ctx) {
   return MATTOHF_OK;
 }
 
+std::vector<int4> fx_twiddles_host(int NG) {
+  std::vector<int4> t(fx_twiddle_table(NG, nullptr));
+  fx_twiddle_table(NG, t.data());
+  return t;
+}
+
 void compute_vion(mattohf_ctx* c) {
   const int NG = c->NG;
   c->vion.assign(NG, 0.0);
@@ -980,7 +1026,7 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
-    e = configure_kernels();
+    e = configure_fx_kernels();
     if (e == cudaSuccess) e = configure_adjoint_kernels();
     if (e == cudaSuccess) e = configure_df_kernels();
     if (e == cudaSuccess) e = configure_small_kernels();
@@ -1012,6 +1058,14 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
   k_twiddles<<<(NG + 127) / 128, 128, 0, ctx->st>>>(ctx->tw, NG);
   if (cudaGetLastError() != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
   if ((rc = compute_tables(ctx))) return bail(rc);
+  const std::vector<int4> twfx = fx_twiddles_host(NG);
+  if ((rc = dalloc(ctx, &ctx->d_kern_fx, (size_t)(2 * ctx->NK - 1) * NG)) || (rc = dalloc(ctx, &ctx->d_kscale, 1)) ||
+      (rc = dalloc(ctx, &ctx->d_tw_fx, twfx.size())))
+    return bail(rc);
+  if (cudaMemcpyAsync(ctx->d_tw_fx, twfx.data(), twfx.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st) !=
+          cudaSuccess ||
+      launch_fx_kern(ctx->d_kern, 2 * ctx->NK - 1, NG, ctx->d_kscale, ctx->d_kern_fx, ctx->st) != cudaSuccess)
+    return bail(MATTOHF_ERR_CUDA);
   if ((rc = dalloc(ctx, &ctx->d_kern_df, (size_t)(2 * ctx->NK - 1) * NG)) || (rc = dalloc(ctx, &ctx->d_tw_df, NG)))
     return bail(rc);
   if (launch_to_df_tables(ctx->d_kern, (2 * ctx->NK - 1) * NG, ctx->d_kern_df, ctx->tw, NG, ctx->d_tw_df, ctx->st) !=
@@ -1044,10 +1098,12 @@ int mattohf_destroy(mattohf_ctx* ctx) {
   void* ptrs[] = {ctx->tw, ctx->d_Gx, ctx->d_kx, ctx->d_vCG, ctx->d_vcq, ctx->d_kern, ctx->d_vion,
                   ctx->d_vloc, ctx->d_rho, ctx->d_scal, ctx->d_out, ctx->d_u, ctx->d_us, ctx->d_k[0],
                   ctx->d_k[1], ctx->d_k[2], ctx->d_k[3], ctx->d_a, ctx->d_b, ctx->d_c,
-                  ctx->d_scratch, ctx->d_colbuf, ctx->d_int, ctx->d_A, ctx->d_Aave, ctx->d_sE,
+                  ctx->d_colbuf, ctx->d_int, ctx->d_A, ctx->d_Aave, ctx->d_sE,
                   ctx->d_sJ, ctx->d_sN, ctx->d_work, ctx->d_hwork, ctx->d_M, ctx->d_V, ctx->d_evals,
                   ctx->d_eps, ctx->d_err, ctx->d_sym, ctx->d_symF, ctx->d_dpart,
-                  ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
+                  ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale,
+                  ctx->d_wfx, ctx->d_wscale, ctx->d_fx_acc, ctx->d_wacc, ctx->d_kern_fx, ctx->d_kscale,
+                  ctx->d_tw_fx, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
                   ctx->d_small_part, ctx->d_small_obs};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1265,18 +1321,11 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   CKR(ensure_scratch(ctx, ncols));
   FockPlan fp;
   if (ctx->hf && mode != CM_T) {
-    FockArgs a;
-    a.u = u;
-    a.w = w;
-    a.nk = ctx->NK;
-    a.nbocc = ctx->NBocc;
-    a.kern = ctx->d_kern + (size_t)k0 * NG;
-    a.tw = ctx->tw;
-    a.scratch = ctx->d_scratch;
-    fock_split(ctx, ncols, &a.nchunks, &a.chunk);
-    fp.nchunks = a.nchunks;
+    CKR(ensure_fx(ctx));
+    CK(launch_fx_orbitals(NG, fx_args(ctx, u, 1), ctx->st));
+    CKR(enq_fock_rows(ctx, u, w, nkl, k0));
     fp.any = true;
-    CK(launch_fock(NG, a, ncols, ctx->st));
+    fp.rows = true;
   } else if (mode == CM_F) {
     CK(cudaMemsetAsync(out.p, 0, sizeof(double2) * (size_t)nkl * out.kstride, ctx->st));
     return MATTOHF_OK;
@@ -1585,12 +1634,12 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
     return MATTOHF_OK;
   };
   // ---- exchange tile
-  int bestS = sym_tile(ctx);
+  int bestS = ctx->opt_df ? sym_tile(ctx) : fx_tile(ctx);
   double tS = 0.0;
   if (ctx->hf && ctx->opt_sym && ctx->NBocc > 0) {
     const int reps = std::max(2, std::min(steps, 20));
     double best = 1e300;
-    const int M = NK * ctx->NBocc, Smax = fock_sym_teams(NG);
+    const int M = NK * ctx->NBocc, Smax = ctx->opt_df ? fock_sym_teams(NG) : std::min(kFxMaxTile, fock_sym_teams(NG));
     for (int S = 1; S <= Smax; S <<= 1) {
       // tiles far beyond a few waves only add partial-sum traffic (and scratch)
       const long long T = (M + S - 1) / S;
@@ -1760,10 +1809,10 @@ int mattohf_gs_run(mattohf_ctx* ctx, int nscf, int ncg, double* Etot_iter, doubl
     for (int icg = 1; icg < ncg; ++icg) {
       Block wb = blk(ctx->d_work + (size_t)(icg - 1) * NB * NG, m, NG, NB);
       BlockOut ob = blko(ctx->d_work + (size_t)icg * NB * NG, m, NG, NB);
-      CKR(enq_hpsi(ctx, ub, wb, ob, aval(0.0), CM_H));
+      CKR(enq_hpsi(ctx, ub, wb, ob, aval(0.0), CM_H, icg > 1));
     }
     CK(launch_block_orth(NG, ctx->d_work, m * NG, m, ctx->dvcell, NK, ctx->d_int + 2, ctx->st));
-    CKR(enq_hpsi(ctx, ub, blk(ctx->d_work, m, NG, m), blko(ctx->d_hwork, m, NG, m), aval(0.0), CM_H));
+    CKR(enq_hpsi(ctx, ub, blk(ctx->d_work, m, NG, m), blko(ctx->d_hwork, m, NG, m), aval(0.0), CM_H, ncg > 1));
     CKR(enq_rayleigh_ritz(ctx, ctx->d_work, ctx->d_hwork, m, NB, ctx->d_u));
     CK(launch_gram_schmidt(NG, gsa, NK, ctx->st));
     // Subspace_diag (GS:197-237)
@@ -1947,7 +1996,7 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
     d.occ = ctx->occ;
     d.vCG = ctx->d_vCG;
     d.vion = ctx->d_vion;
-    d.tw = ctx->tw;
+    d.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
     d.dvcell = ctx->dvcell;
     d.rho = ctx->d_sig;
     d.vloc = ctx->d_psi;
@@ -2250,7 +2299,7 @@ static int enq_taylor(mattohf_ctx* ctx, double2* target, const double2* base, do
   double2* hw = ctx->d_k[3];
   CK(cudaMemcpyAsync(w, target, sizeof(double2) * n, cudaMemcpyDeviceToDevice, ctx->st));
   for (int iorder = 1; iorder <= 4; ++iorder) {
-    CKR(enq_hpsi(ctx, blk(base, NB, NG, NB), blk(w, NB, NG, NB), blko(hw, NB, NG, NB), aval(Aave), CM_H));
+    CKR(enq_hpsi(ctx, blk(base, NB, NG, NB), blk(w, NB, NG, NB), blko(hw, NB, NG, NB), aval(Aave), CM_H, iorder > 1));
     CK(launch_te_update(w, hw, nullptr, dt, (double)iorder, target, n, ctx->st));
   }
   return MATTOHF_OK;
@@ -2312,6 +2361,7 @@ struct mattohf_batch {
   DensArgs* d_dens[kVariants] = {};
   FockSymArgs* d_fsym[kVariants] = {};
   FockSymDfArgs* d_fsym_df[kVariants] = {};
+  FockFxArgs* d_fsym_fx[kVariants] = {};
   CombineArgs* d_comb[kVariants] = {};
   CombineArgs* d_comb_pre[4] = {};  // stages' kinetic + local-potential pass (beside the exchange)
   cudaStream_t st_side = nullptr;
@@ -2321,8 +2371,8 @@ struct mattohf_batch {
   ObsReduceArgs* d_obs = nullptr;
   ExArgs* d_ex = nullptr;
   ExArgs* d_exf = nullptr;
-  int *d_tile_pre = nullptr, *d_elem_pre = nullptr, *d_cta_pre = nullptr;
-  int total_tiles = 0, total_elems = 0, total_ctas = 0;
+  int *d_tile_pre = nullptr, *d_elem_pre = nullptr, *d_col_pre = nullptr;
+  int total_tiles = 0, total_elems = 0, total_cols = 0;
   cudaGraphExec_t exec = nullptr;
   int built_nt = -1;
   std::vector<double> dts;
@@ -2354,13 +2404,19 @@ int bupload(mattohf_batch* b, T** d, const std::vector<T>& h) {
   return MATTOHF_OK;
 }
 
-// Exchange partials of every run for argument variant v (FP64 or double-float).
+// Tile of every run's tile pairs.
+int batch_tile(const mattohf_batch* b) {
+  const int S = b->opt_tile > 0 ? b->opt_tile : fock_sym_teams(b->NG);
+  return b->opt_df ? S : std::min(S, kFxMaxTile);
+}
+
+// Exchange of every run for argument variant v (fixed point or double-float).
 cudaError_t batch_exchange(mattohf_batch* b, int v) {
   if (b->opt_df)
     return launch_fock_sym_df_batch(b->NG, b->d_fsym[v], b->d_fsym_df[v], b->d_tile_pre, b->R, b->total_tiles,
                                     b->d_elem_pre, b->total_elems, b->st);
-  return launch_fock_sym_batch(b->NG, b->d_fsym[v], b->d_tile_pre, b->R, b->total_tiles, b->d_elem_pre,
-                               b->total_elems, b->st);
+  return launch_fock_sym_fx_batch(b->NG, b->d_fsym_fx[v], b->d_tile_pre, b->R, batch_tile(b), b->total_tiles,
+                                  b->d_elem_pre, b->total_elems, b->st);
 }
 
 // (Re)build every per-run argument array for runs of `nt` steps.
@@ -2374,15 +2430,15 @@ int batch_prepare(mattohf_batch* b, int nt) {
   std::vector<DensArgs> dens[mattohf_batch::kVariants];
   std::vector<FockSymArgs> fsym[mattohf_batch::kVariants];
   std::vector<FockSymDfArgs> fsdf[mattohf_batch::kVariants];
+  std::vector<FockFxArgs> fsfx[mattohf_batch::kVariants];
   std::vector<CombineArgs> comb[mattohf_batch::kVariants];
   std::vector<CombineArgs> comb_pre[4];
   std::vector<ObsReduceArgs> obs(R);
   std::vector<ExArgs> ex(R), exf(R);
-  std::vector<int> tile_pre(R + 1, 0), elem_pre(R + 1, 0), cta_pre(R + 1, 0);
-  const int cpc = combine_cols_per_cta(NG);
+  std::vector<int> tile_pre(R + 1, 0), elem_pre(R + 1, 0), col_pre(R + 1, 0);
   // one launch shape (a CTA's teams) for every run; a smaller tile leaves
   // teams idle but gives small runs more CTAs
-  const int S = b->opt_tile > 0 ? b->opt_tile : fock_sym_teams(NG);
+  const int S = batch_tile(b);
   for (int r = 0; r < R; ++r) {
     mattohf_ctx* ctx = b->runs[r];
     int rc;
@@ -2390,12 +2446,12 @@ int batch_prepare(mattohf_batch* b, int nt) {
       return bfail(b, rc, ctx->err);
     const int M = ctx->NK * ctx->NBocc;
     const int T = (M + S - 1) / S;
-    if ((rc = ensure_sym(ctx, (size_t)T * (T + 1) / 2 * 2 * S * NG))) return bfail(b, rc, ctx->err);
-    if (!ctx->d_symF && (rc = dalloc(ctx, &ctx->d_symF, (size_t)M * NG))) return bfail(b, rc, ctx->err);
+    if (b->opt_df && (rc = ensure_sym(ctx, sym_partials(M, S, NG)))) return bfail(b, rc, ctx->err);
+    if ((rc = ensure_fx(ctx))) return bfail(b, rc, ctx->err);
     if (!ctx->d_udf && (rc = dalloc(ctx, &ctx->d_udf, (size_t)M * NG))) return bfail(b, rc, ctx->err);
     tile_pre[r + 1] = tile_pre[r] + T * (T + 1) / 2;
     elem_pre[r + 1] = elem_pre[r] + M * NG;
-    cta_pre[r + 1] = cta_pre[r] + (ctx->NK * ctx->NB + cpc - 1) / cpc;
+    col_pre[r + 1] = col_pre[r] + ctx->NK * ctx->NB;
     AField fld[4];
     for (int i = 0; i < 4; ++i) {
       fld[i].A = ctx->d_A;
@@ -2417,7 +2473,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
       d.occ = ctx->occ;
       d.vCG = ctx->d_vCG;
       d.vion = ctx->d_vion;
-      d.tw = ctx->tw;
+      d.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
       d.dvcell = ctx->dvcell;
       d.rho = ctx->d_rho;
       d.vloc = ctx->d_vloc;
@@ -2449,18 +2505,14 @@ int batch_prepare(mattohf_batch* b, int nt) {
       fd.scratch = reinterpret_cast<float4*>(ctx->d_sym);
       fd.F = ctx->d_symF;
       fsdf[v].push_back(fd);
+      fsfx[v].push_back(fx_args(ctx, ub, S));
       FockPlan fp;
       fp.any = (v != 4);
-      fp.sym = ctx->d_symF;
-      fp.S = S;
-      fp.T = T;
+      fp.occ = true;
       fp.b0 = ctx->NBocc;
       const AField af = v < 4 ? fld[v] : fld[3];
       CombineArgs c = combine_base(ctx, ub, af, v < 4 ? modes[v] : CM_OBS, fp);
-      if (v == 4) {
-        c.sym = nullptr;
-        c.scratch = nullptr;
-      }
+      if (v != 4 && ctx->hf) c.occ_ex = occ_source(ctx, b->opt_df);
       if (v == 5) c.af = aval(0.0);
       c.out = blko(ctx->d_us, ctx->NB, NG, ctx->NB);
       c.dt = b->dts[r];
@@ -2504,17 +2556,17 @@ int batch_prepare(mattohf_batch* b, int nt) {
   int rc;
   for (int v = 0; v < mattohf_batch::kVariants; ++v) {
     if ((rc = bupload(b, &b->d_dens[v], dens[v])) || (rc = bupload(b, &b->d_fsym[v], fsym[v])) ||
-        (rc = bupload(b, &b->d_fsym_df[v], fsdf[v])) || (rc = bupload(b, &b->d_comb[v], comb[v])))
+        (rc = bupload(b, &b->d_fsym_df[v], fsdf[v])) || (rc = bupload(b, &b->d_fsym_fx[v], fsfx[v])) || (rc = bupload(b, &b->d_comb[v], comb[v])))
       return rc;
     if (v < 4 && (rc = bupload(b, &b->d_comb_pre[v], comb_pre[v]))) return rc;
   }
   if ((rc = bupload(b, &b->d_obs, obs)) || (rc = bupload(b, &b->d_ex, ex)) || (rc = bupload(b, &b->d_exf, exf)) ||
       (rc = bupload(b, &b->d_tile_pre, tile_pre)) || (rc = bupload(b, &b->d_elem_pre, elem_pre)) ||
-      (rc = bupload(b, &b->d_cta_pre, cta_pre)))
+      (rc = bupload(b, &b->d_col_pre, col_pre)))
     return rc;
   b->total_tiles = tile_pre[R];
   b->total_elems = elem_pre[R];
-  b->total_ctas = cta_pre[R];
+  b->total_cols = col_pre[R];
   BCK(cudaStreamSynchronize(b->st));
   // capture one step for all runs
   cudaGraph_t g;
@@ -2527,16 +2579,16 @@ int batch_prepare(mattohf_batch* b, int nt) {
     cudaError_t es = cudaStreamWaitEvent(b->st_side, b->ev_fork, 0);
     if (es == cudaSuccess) es = launch_density_batch(NG, b->d_dens[s], R, b->st_side);
     if (es == cudaSuccess)
-      es = launch_combine_batch(NG, b->d_comb_pre[s], b->d_cta_pre, R, b->total_ctas, b->st_side);
+      es = launch_combine_batch(NG, b->d_comb_pre[s], b->d_col_pre, R, b->total_cols, b->st_side);
     const cudaError_t ej = cudaEventRecord(b->ev_join, b->st_side);
     e = batch_exchange(b, s);
     const cudaError_t ew = cudaStreamWaitEvent(b->st, b->ev_join, 0);
     if (e == cudaSuccess) e = es != cudaSuccess ? es : (ej != cudaSuccess ? ej : ew);
-    if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[s], b->d_cta_pre, R, b->total_ctas, b->st);
+    if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[s], b->d_col_pre, R, b->total_cols, b->st);
     if (e == cudaSuccess && s == 0) e = launch_ex_finalize_batch(b->d_ex, R, b->st);
   }
   if (e == cudaSuccess) e = launch_density_batch(NG, b->d_dens[4], R, b->st);
-  if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[4], b->d_cta_pre, R, b->total_ctas, b->st);
+  if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[4], b->d_col_pre, R, b->total_cols, b->st);
   if (e == cudaSuccess) e = launch_obs_reduce_batch(b->d_obs, R, b->st);
   if (e == cudaSuccess) e = launch_step_advance(b->d_int, b->st);
   cudaError_t ec = cudaStreamEndCapture(b->st, &g);
@@ -2597,9 +2649,10 @@ int mattohf_batch_destroy(mattohf_batch* b) {
     cudaFree(b->d_dens[v]);
     cudaFree(b->d_fsym[v]);
     cudaFree(b->d_fsym_df[v]);
+    cudaFree(b->d_fsym_fx[v]);
     cudaFree(b->d_comb[v]);
   }
-  void* ptrs[] = {b->d_obs, b->d_ex, b->d_exf, b->d_tile_pre, b->d_elem_pre, b->d_cta_pre, b->d_int};
+  void* ptrs[] = {b->d_obs, b->d_ex, b->d_exf, b->d_tile_pre, b->d_elem_pre, b->d_col_pre, b->d_int};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto* c : b->runs) mattohf_destroy(c);
@@ -2671,7 +2724,7 @@ int mattohf_batch_rk4_run(mattohf_batch* b, int nt, const double* dt, const doub
   const int NG = b->NG;
   BCK(launch_density_batch(NG, b->d_dens[5], b->R, b->st));
   BCK(batch_exchange(b, 5));
-  BCK(launch_combine_batch(NG, b->d_comb[5], b->d_cta_pre, b->R, b->total_ctas, b->st));
+  BCK(launch_combine_batch(NG, b->d_comb[5], b->d_col_pre, b->R, b->total_cols, b->st));
   BCK(launch_ex_finalize_batch(b->d_exf, b->R, b->st));
   BCK(cudaEventRecord(e1, b->st));
   BCK(cudaEventSynchronize(e1));
@@ -2746,7 +2799,7 @@ int mattohf_batch_autotune(mattohf_batch* b, int steps, int* tile, double* us) {
   std::vector<double> A((size_t)b->R * steps, 0.0), dt(b->R, 1e-4);
   double best = 1e300;
   int bestS = 0, rc = MATTOHF_OK;
-  for (int S = fock_sym_teams(b->NG); S >= 1 && rc == MATTOHF_OK; S >>= 1) {
+  for (int S = b->opt_df ? fock_sym_teams(b->NG) : std::min(kFxMaxTile, fock_sym_teams(b->NG)); S >= 1 && rc == MATTOHF_OK; S >>= 1) {
     b->opt_tile = S;
     b->built_nt = -1;
     double t = 0.0;

@@ -5,9 +5,13 @@
 
 namespace mattohf {
 
+namespace fx {  // fft_fx.cuh
+struct cx;
+struct lc;
+}  // namespace fx
+
 constexpr int kThreads = 128;  // threads per CTA for the column/pair kernels (4 warps)
 constexpr int kDensChunks = 32; // column chunks of the two-stage density reduction
-constexpr int kCombineWarps = 1; // warps per CTA of the per-column combine kernels (spread over SMs)
 
 // How a kernel obtains the vector potential of the current launch.
 //   AVAL : use `A_val` directly
@@ -51,7 +55,7 @@ struct DensArgs {
   double occ;         // 2/NK for occupied bands, 0 otherwise (src/Initialization.f90:179-186)
   const double* vCG;  // NG
   const double* vion; // NG
-  const double2* tw;  // NG forward twiddles
+  const fx::lc* twfx; // fixed-point twiddles
   double dvcell;
   double* rho;        // NG out
   double* vloc;       // NG out: vH + vion
@@ -108,6 +112,48 @@ cudaError_t launch_fock_sym_df_batch(int NG, const FockSymArgs* d_src, const Foc
 cudaError_t launch_to_df_tables(const double* kern, int nkern, float2* kern_df, const double2* tw, int ntw,
                                 float4* tw_df, cudaStream_t s);
 
+// Fixed-point exchange (k_fock_fx.cu).
+constexpr int kFxTerms = 16;   // terms that a fixed-point accumulator takes
+constexpr int kFxMaxTile = 8;  // largest tile (a row and a column accumulator take one term per round)
+constexpr int kRowsThreads = 128;   // CTA of the exchange on other functions
+constexpr int kRowsCtasPerSm = 12;  // its CTAs per SM to aim at
+struct FockFxArgs {
+  Block u;              // occupied orbitals (bands 0..nbocc-1 used)
+  int nk, nbocc;
+  int S, T;             // tile size (<= kFxMaxTile), tiles
+  int2* sizes;          // [NK*nbocc]: largest |component| and squared norm (k_fx_sizes)
+  fx::lc* ufx;          // [NK*nbocc][NG] fixed-point orbitals in limbs
+  int* shift;           // [NK*nbocc] extra scale 2^d of an orbital with a small norm
+  double2* fscale;      // [NK*nbocc] F = F^ * (x + y)
+  int2* uscale;         // the orbitals' common scale (c, k)
+  const int2* kern;     // kernel table in limbs
+  const int2* kscale;   // its scale (c, k)
+  const fx::lc* tw;
+  unsigned long long* acc;  // [NK*nbocc][4][NG] sums F^ (fx_accumulate), zeroed by the conversion
+};
+// Functions w that the exchange operator of the orbitals acts on.
+struct FockFxRows {
+  Block w;
+  int ncols;            // k-points of w times w.nb
+  fx::lc* wfx;          // [ncols][NG] w in limbs
+  double2* wscale;      // [ncols] F = F^ * (x + y)
+  unsigned long long* acc;  // [ncols][4][NG] sums F^, zeroed by the conversion
+  int nchunks, chunk;   // chunks of the sources, sources per chunk
+};
+// orbitals to fixed point: before either exchange
+cudaError_t launch_fx_orbitals(int NG, const FockFxArgs& a, cudaStream_t s);
+cudaError_t launch_fock_sym_fx(int NG, const FockFxArgs& a, cudaStream_t s);
+// kern of the arguments starts at the row of w's first k-point
+cudaError_t launch_fock_fx(int NG, const FockFxArgs& a, const FockFxRows& r, cudaStream_t s);
+int fx_rows_teams(int NG);
+void fx_rows_split(int NG, int ncols, int npairs, int nsm, int fixed, int* nchunks, int* chunk);
+cudaError_t launch_fock_sym_fx_batch(int NG, const FockFxArgs* d_args, const int* d_tile_pre, int nruns, int S,
+                                     int total_tiles, const int* d_elem_pre, int total_elems, cudaStream_t s);
+// kernel table in limbs and its scale (device)
+cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int2* out, cudaStream_t s);
+int fx_twiddle_table(int NG, int4* out);  // host table in limbs; returns its length (out may be null)
+cudaError_t configure_fx_kernels();
+
 __host__ __device__ __forceinline__ int sym_tp(int i, int j, int T) {
   return i * T - (i * (i - 1)) / 2 + (j - i);
 }
@@ -157,21 +203,39 @@ enum CombineMode : int {
   CM_T = 7,     // out = T_A w only (kinetic term alone)
 };
 
+// run owning work item `i` given exclusive prefix sums pre[0..nruns] (pre[0] = 0)
+__device__ __forceinline__ int find_run(const int* __restrict__ pre, int nruns, int i) {
+  int lo = 0, hi = nruns - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pre[mid] <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Exchange term of a set of columns, [columns][NG]: fixed-point sums with a scale
+// per column, or double2 values; none when both are null.
+struct ExSource {
+  const unsigned long long* acc;
+  const double2* scale;
+  const double2* f;
+};
+
 struct CombineArgs {
   Block w;                  // columns being processed (the h-apply's wbk)
-  const double2* sym;       // reduced symmetric exchange [NK*nbocc][NG] for occupied columns (or null)
-  int sym_S, sym_T;
-  int chunk_b0;             // first band whose exchange comes from the chunked partials
+  // exchange of the columns (ExSource, indexed k * (bands) + band): bands below
+  // nbocc from occ_ex, or all bands from b0 on from row_ex
+  ExSource occ_ex, row_ex;
+  int row_b0;
   int ex_cols;              // CM_RK0: also store <w|F> per occupied column (deferred Ex)
   BlockOut out;             // h output (CM_H / CM_F / CM_T) or stage input (CM_RK0..2)
   double2* u0;              // RK4 base state [NK][NB][NG] (CM_RK*)
   double2* kbuf[4];         // RK4 stage derivatives [NK][NB][NG]
-  const double2* scratch;   // Fock partials (may be null when the Fock term is off)
-  int nchunks;
   const double* vloc;       // NG
   const double* Gx;         // NG
   const double* kx;         // NK
-  const double2* tw;
+  const fx::lc* twfx;       // fixed-point twiddles
   AField af;
   double dt;
   int mode;
@@ -294,11 +358,9 @@ struct ObsReduceArgs {
 // Launchers (defined in k_hpsi.cu); all return cudaGetLastError() of the launch.
 cudaError_t launch_density(int NG, const DensArgs& a, cudaStream_t s);
 cudaError_t launch_fock(int NG, const FockArgs& a, int ncols, cudaStream_t s);
-cudaError_t launch_fock_sym(int NG, const FockSymArgs& a, cudaStream_t s);
 int fock_sym_teams(int NG);  // teams of a full symmetric-exchange CTA (largest tile size)
 int choose_sym_tile(int NG, int M, int nsm);  // tile size for a single run of M occupied orbitals on nsm SMs
 cudaError_t sym_launch_params(int NG, int S, int* threads, size_t* smem);
-cudaError_t configure_kernels();
 struct ExArgs {
   const double* colbuf;
   int nk, nb, nbocc;
@@ -315,12 +377,8 @@ cudaError_t launch_obs_reduce(const ObsReduceArgs& a, cudaStream_t s);
 // Batched launchers: per-run argument structs live in device memory; work
 // items map to runs through exclusive prefix arrays (pre[0] = 0, pre[nruns] = total).
 cudaError_t launch_density_batch(int NG, const DensArgs* d_args, int nruns, cudaStream_t s);
-cudaError_t launch_fock_sym_batch(int NG, const FockSymArgs* d_args, const int* d_tile_pre, int nruns,
-                                  int total_tiles, const int* d_elem_pre, int total_elems,
-                                  cudaStream_t s);
-int combine_cols_per_cta(int NG);
-cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d_cta_pre, int nruns,
-                                 int total_ctas, cudaStream_t s);
+cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d_col_pre, int nruns,
+                                 int total_cols, cudaStream_t s);
 cudaError_t launch_obs_reduce_batch(const ObsReduceArgs* d_args, int nruns, cudaStream_t s);
 cudaError_t launch_ex_finalize_batch(const ExArgs* d_args, int nruns, cudaStream_t s);
 cudaError_t launch_step_advance(int* it, cudaStream_t s);

@@ -1,0 +1,602 @@
+// Fock exchange (src/Functions.f90:237-261) with 64-bit fixed-point pair
+// transforms (fft_fx.cuh).
+//
+// Scales.  Orbitals are converted once per apply to u^ = u s 2^d with one
+// scale s for all of them (k_fx_stats, k_fx_convert): a short factor times a
+// power of two, so that u^ keeps every bit of u, with
+//     |u^|_2 <= 2^60.2      (a pair density's absolute sum stays below 2^60.4)
+//     max |u^| <= 2^58.4    (16 terms phi^ u^ / 2^60 stay below 2^63).
+// d = 0 except for an orbital whose norm is under half the largest one: d
+// then brings it up to that, and a term that it enters twice is shifted back.
+// The kernel table is K^ = kern s_k with sum_G |K^(G)| <= 2^60 for every k - k'.
+// A pair's chain is then
+//     p^ = u_a^ conj(u_b^) / 2^60,  phi^ = IFFT(K^ FFT(p^) / 2^60),
+//     F_a^ += phi^ u_b^ / 2^60,     F = F^ 2^180 / (s^3 s_k 2^d_a),
+// every sum exact in integers, so the order of summation does not matter.
+// Orbitals that are not finite, or whose squared norm overflows, give NaN.
+//
+// What bounds it and what it measured.  k_fock_sym_fx at NG = 256, NK = 64,
+// Nocc = 4 (32896 pairs): 165 us, against 918 us of the same pairs in FP64 (89 % FP64
+// pipe).  It issues about 390 instructions per point and pair, 87 of them
+// 32 x 32 + 64-bit multiply-adds at half the rate of the others; the multiplier
+// pipe is 69 % busy, the adder pipe 53 %, shared memory 39 %.  Two CTAs of 128
+// threads a SM at least (a register limit for four of them spills: 183 us).
+// Error of one apply against long double, same table, smooth orthonormal
+// orbitals, here / FP64: NG = 64 0.7e-16 / 1.2e-16, NG = 256 1.0e-16 / 1.8e-16,
+// NG = 512 1.3e-16 / 1.9e-16.
+//
+// Sums over tiles and chunks go to 64-bit atomics in global memory (29 us by
+// themselves at that size, mostly beside the pair loop) instead of 68 MB of
+// partials and a reduction launch (13 + 24 us).
+#include <algorithm>
+
+#include "fx_convert.cuh"
+#include "internal.h"
+
+namespace mattohf {
+
+__device__ __forceinline__ const double2* fx_column(const Block& u, int nb, int col, int N) {
+  return u.p + (size_t)(col / nb) * u.kstride + (size_t)(col % nb) * N;
+}
+
+// One column to fixed point, by a CTA.  scan: the CTA takes the sizes of all
+// columns itself (few orbitals); else k_fx_sizes has left them in a.sizes.
+__device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, int N, int col, bool scan) {
+  __shared__ int2 own[4];
+  __shared__ Scale out;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int M = a.nk * a.nbocc;
+  // largest size over the columns, each warp over its share, then over warps
+  int m = 0;
+  float g2 = 0.0f, n2 = 0.0f;
+  int mc = 0;
+  for (int i = scan ? warp : tid; i < M; i += scan ? 4 : 128) {
+    const int2 z = scan ? fx_column_size<32>(fx_column(a.u, a.nbocc, i, N), N, lane) : a.sizes[i];
+    const float s = __int_as_float(z.y);
+    if (i == col) {
+      mc = z.x;
+      n2 = s;
+    }
+    // s and g2 in units of their own exponents, compared as s 2^(2 (e - e'))
+    const int d = (z.x >> 20) - (m >> 20);
+    g2 = d > 0 ? fmaxf(s, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(s, 2 * d));
+    m = max(m, z.x);
+  }
+  if (!scan) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const int mo = __shfl_xor_sync(0xffffffffu, m, o);
+      const float go = __shfl_xor_sync(0xffffffffu, g2, o);
+      const int d = (mo >> 20) - (m >> 20);
+      g2 = d > 0 ? fmaxf(go, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(go, 2 * d));
+      m = max(m, mo);
+      const int co = __shfl_xor_sync(0xffffffffu, mc, o);
+      const float no = __shfl_xor_sync(0xffffffffu, n2, o);
+      mc = max(mc, co);  // one lane has the column
+      n2 = fmaxf(n2, no);
+    }
+  }
+  __shared__ int2 ownc[4];
+  if (lane == 0) {
+    own[warp] = make_int2(m, __float_as_int(g2));
+    ownc[warp] = make_int2(mc, __float_as_int(n2));
+  }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < 4; ++w) {
+      const float go = __int_as_float(own[w].y);
+      const int d = (own[w].x >> 20) - (m >> 20);
+      g2 = d > 0 ? fmaxf(go, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(go, 2 * d));
+      m = max(m, own[w].x);
+      mc = max(mc, ownc[w].x);
+      n2 = fmaxf(n2, __int_as_float(ownc[w].y));
+    }
+    const int e = m >> 20;
+    const Scale s = fx_scale(m, g2, fx_mantissa(m, e), kSquareMax);
+    // a column with less than half the largest norm is lifted by 2^d
+    const int dc = (mc >> 20) - e;
+    int d = 0;
+    if (n2 > 0.0f) {
+      const int lg = ilogbf(g2) - ilogbf(n2) - 2 * dc;  // log2 of the squared norms' ratio, to 1
+      if (lg > 2) d = min(60, (lg - 1) >> 1);
+    }
+    const Scale sd{s.c, s.k + d};
+    out = sd;
+    a.shift[col] = d;
+    if (col == 0) *a.uscale = make_int2(s.c, s.k);
+    // a column of zeros has a sum of zero; the roundings of its terms do not count
+    a.fscale[col] = n2 > 0.0f || s.c == 0 ? fx_output_scale(s, sd, Scale{a.kscale->x, a.kscale->y}) : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const Scale sd = out;
+  const bool ok = sd.c != 0;
+  const double2* p = fx_column(a.u, a.nbocc, col, N);
+  lc* o = a.ufx + (size_t)col * N;
+  for (int i = tid; i < N; i += 128) {
+    const double2 z = p[i];
+    o[i] = ok ? fx::limbs(cx{fx_convert(z.x, sd), fx_convert(z.y, sd)}) : lc{0, 0, 0, 0};
+  }
+  unsigned long long* acc = a.acc + (size_t)col * 4 * N;
+  for (int i = tid; i < 4 * N; i += 128) acc[i] = 0;
+}
+
+__global__ void __launch_bounds__(128) k_fx_sizes(FockFxArgs a, int N) {
+  const int col = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (col >= a.nk * a.nbocc) return;
+  const int2 z = fx_column_size<32>(fx_column(a.u, a.nbocc, col, N), N, threadIdx.x & 31);
+  if ((threadIdx.x & 31) == 0) a.sizes[col] = z;
+}
+__global__ void __launch_bounds__(128) k_fx_convert(FockFxArgs a, int N, int scan) {
+  fx_convert_body(a, N, blockIdx.x, scan);
+}
+// element prefix: pre[r] = sum over earlier runs of M_r * N
+__global__ void __launch_bounds__(128) k_fx_sizes_batch(const FockFxArgs* __restrict__ args,
+                                                        const int* __restrict__ pre, int nruns, int N) {
+  const int c = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (c * N >= pre[nruns]) return;
+  const int r = find_run(pre, nruns, c * N), col = c - pre[r] / N;
+  const int2 z = fx_column_size<32>(fx_column(args[r].u, args[r].nbocc, col, N), N, threadIdx.x & 31);
+  if ((threadIdx.x & 31) == 0) args[r].sizes[col] = z;
+}
+__global__ void __launch_bounds__(128) k_fx_convert_batch(const FockFxArgs* __restrict__ args,
+                                                          const int* __restrict__ pre, int nruns, int N) {
+  const int r = find_run(pre, nruns, blockIdx.x * N);
+  fx_convert_body(args[r], N, blockIdx.x - pre[r] / N, false);
+}
+
+// t / 2^s for s > 0, rounded (a floor would be biased by half a place per term)
+__device__ __forceinline__ cx fx_shift(cx t, int s) {
+  s = min(s, 62);
+  const i64 r = 1ll << (s - 1);
+  return cx{(t.x + r) >> s, (t.y + r) >> s};
+}
+
+// Adds a 64-bit partial sum to a column's accumulators, as its high and low words:
+// planes [4][N] of x high, x low, y high, y low.  Exact, so in any order.
+__device__ __forceinline__ void fx_accumulate(unsigned long long* acc, int N, int q, cx v) {
+  atomicAdd(acc + q, (unsigned long long)(v.x >> 32));
+  atomicAdd(acc + N + q, (unsigned long long)(unsigned)v.x);
+  atomicAdd(acc + 2 * N + q, (unsigned long long)(v.y >> 32));
+  atomicAdd(acc + 3 * N + q, (unsigned long long)(unsigned)v.y);
+}
+
+// x = conj(phi_ab) of the pair (a, b); returns R_ab[N/2], the transform of the
+// pair density at the self-aliased frequency.
+template <int N>
+__device__ __forceinline__ cx pair_potential(cx (&x)[fx::Team<N>::E], const lc* __restrict__ ua,
+                                             const lc* __restrict__ ub, const int2* __restrict__ kab, cx* buf,
+                                             const lc* tw_s, const int2* twn_s, int tl, int team) {
+  using TM = fx::Team<N>;
+  constexpr int E = TM::E, T = TM::T;
+  cx rn{0, 0};
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int q = TM::pos(tl, e);
+    x[e] = fx::cmulc(ua[q], ub[q]);
+  }
+  // forward transform, kernel product, backward transform of the conjugate
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    fx::forward<N>(x, buf, tw_s, twn_s, tl, team);
+    if (h == 0) {
+      rn = x[TM::kNyquistSlot];  // in the team's lane 0
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int2 k = __ldg(kab + TM::pos(tl, e));
+        x[e] = cx{fx::rmul(x[e].x, k), -fx::rmul(x[e].y, k)};
+      }
+    }
+  }
+  if constexpr (T > 32) {  // the team's two warps share lane 0's value through the buffer
+    fx::team_sync<T>(team);
+    if (tl == 0) buf[0] = rn;
+    fx::team_sync<T>(team);
+    return buf[0];
+  } else {
+    const int lane0 = (threadIdx.x & 31) / T * T;
+    return cx{__shfl_sync(0xffffffffu, rn.x, lane0), __shfl_sync(0xffffffffu, rn.y, lane0)};
+  }
+}
+
+// Twiddles to shared memory: tw_s, and the negated imaginary parts to twn_s.
+template <int N>
+__device__ __forceinline__ void load_twiddles(const lc* __restrict__ tw, lc* tw_s, int2* twn_s) {
+  for (int i = threadIdx.x; i < fx::Team<N>::kTwCount; i += blockDim.x) {
+    const lc w = tw[i];
+    tw_s[i] = w;
+    twn_s[i] = make_int2(fx::neg_hi(w.yh), fx::neg_lo(w.yl));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Symmetric exchange (w == u, occupied pairs), tile pairs as k_fock_sym of
+// k_hpsi.cu: team w owns row a = i S + w in registers and in round r visits
+// column b = j S + (w + r) % S, whose accumulator in shared memory has one
+// writer per round.
+// ---------------------------------------------------------------------------
+template <int N>
+__device__ __forceinline__ void fock_sym_fx_body(const FockFxArgs& a, const int tile) {
+  using TM = fx::Team<N>;
+  constexpr int E = TM::E, T = TM::T;
+  const int S = a.S;
+  const int nteam = blockDim.x / T;
+  extern __shared__ int4 sm_fx[];
+  lc* tw_s = reinterpret_cast<lc*>(sm_fx);                 // kTwCount
+  cx* bufs = reinterpret_cast<cx*>(sm_fx + TM::kTwCount);  // nteam * N
+  cx* cacc = bufs + nteam * N;                             // S * N
+  const int tid = threadIdx.x, tl = tid % T, tw_ = tid / T;
+  cx* buf = bufs + tw_ * N;
+  int2* twn_s = reinterpret_cast<int2*>(cacc + S * N);  // kTwCount
+  load_twiddles<N>(a.tw, tw_s, twn_s);
+  for (int i = tid; i < S * N; i += blockDim.x) cacc[i] = cx{0, 0};
+  int ti = 0, rem = tile;
+  while (rem >= a.T - ti) { rem -= a.T - ti; ++ti; }
+  const int tj = ti + rem;
+  const int M = a.nk * a.nbocc;
+  const int ia = ti * S + tw_;
+  const bool va = tw_ < S && ia < M;
+  const int oa = va ? ia : 0;
+  const int ka = oa / a.nbocc;
+  const lc* ua = a.ufx + (size_t)oa * N;
+  const int sa = 2 * a.shift[oa];
+  cx racc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) racc[e] = cx{0, 0};
+  __syncthreads();
+  const bool diag = (ti == tj);
+  const int nrounds = diag ? (S / 2 + 1) : S;
+  for (int r = 0; r < nrounds; ++r) {
+    const int lb = (tw_ + r) % S;
+    const int ib = tj * S + lb;
+    bool valid = va && ib < M;
+    if (diag && (S % 2 == 0) && r == S / 2 && tw_ >= S / 2) valid = false;  // counted by the partner
+    const bool self = diag && r == 0;
+    const int ob = ib < M ? ib : 0;
+    const int kb = ob / a.nbocc;
+    const lc* ub = a.ufx + (size_t)ob * N;
+    const int2* kab = a.kern + (size_t)(ka - kb + a.nk - 1) * N;
+    cx x[E];
+    const cx rn = pair_potential<N>(x, ua, ub, kab, buf, tw_s, twn_s, tl, tw_);
+    if (valid) {
+      const int sb = 2 * a.shift[ob];
+      // phi u_b = conj(x) u_b
+      if (sb == 0) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) racc[e] = fx::add(racc[e], fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])));
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          racc[e] = fx::add(racc[e], fx_shift(fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])), sb));
+      }
+      if (!self) {
+        // phi_ba = conj(phi_ab + c (-1)^x), c = (K_ba - K_ab)(N/2) R_ab(N/2)
+        const int2 kba = __ldg(a.kern + (size_t)(kb - ka + a.nk - 1) * N + N / 2), kn = __ldg(kab + N / 2);
+        cx c{fx::rmul(rn.x, kba) - fx::rmul(rn.x, kn), fx::rmul(rn.y, kn) - fx::rmul(rn.y, kba)};
+        if (tl & 1) c = cx{-c.x, -c.y};  // T and N/R0 are even: the sign is the lane's
+        cx* col = cacc + lb * N;
+        if (sa == 0) {
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int q = TM::pos(tl, e);
+            col[q] = fx::add(col[q], fx::cmul(fx::limbs(fx::add(x[e], c)), ua[q]));
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int q = TM::pos(tl, e);
+            col[q] = fx::add(col[q], fx_shift(fx::cmul(fx::limbs(fx::add(x[e], c)), ua[q]), sa));
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (va) {
+    unsigned long long* dst = a.acc + (size_t)ia * 4 * N;
+#pragma unroll
+    for (int e = 0; e < E; ++e) fx_accumulate(dst, N, TM::pos(tl, e), racc[e]);
+  }
+  for (int i = tid; i < S * N; i += blockDim.x) {
+    const int ib = tj * S + i / N;
+    if (ib < M) fx_accumulate(a.acc + (size_t)ib * 4 * N, N, i % N, cacc[i]);
+  }
+}
+
+// threads of a CTA with the largest tile
+template <int N>
+constexpr int sym_fx_threads() {
+  return kFxMaxTile * fx::Team<N>::T < 32 ? 32 : kFxMaxTile * fx::Team<N>::T > 256 ? 256 : kFxMaxTile * fx::Team<N>::T;
+}
+
+template <int N>
+__global__ void __launch_bounds__(sym_fx_threads<N>(), 2) k_fock_sym_fx(FockFxArgs a) { fock_sym_fx_body<N>(a, blockIdx.x); }
+
+template <int N>
+__global__ void __launch_bounds__(sym_fx_threads<N>(), 2) k_fock_sym_fx_batch(const FockFxArgs* __restrict__ args,
+                                                                           const int* __restrict__ pre, int nruns) {
+  const int r = find_run(pre, nruns, blockIdx.x);
+  fock_sym_fx_body<N>(args[r], blockIdx.x - pre[r]);
+}
+
+// ---------------------------------------------------------------------------
+// Exchange on other functions w (Krylov blocks, empty bands, a rank's rows):
+// F_w = sum over all occupied b of phi_wb u_b, no symmetry.  Each column of w
+// has a scale of its own (|w^|_2 <= 2^60.2), since it enters every term once.
+// A CTA takes kRowsThreads / T columns, one per team, against one chunk of the
+// sources, which all its teams read together.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_fx_rows(FockFxArgs a, FockFxRows r, int N) {
+  const int lane = threadIdx.x & 31, col = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (col >= r.ncols) return;
+  const double2* p = fx_column(r.w, r.w.nb, col, N);
+  const int2 z = fx_column_size<32>(p, N, lane);
+  const Scale s = fx_scale(z.x, __int_as_float(z.y), 1e-30f, kSquareMax), su{a.uscale->x, a.uscale->y};
+  const bool ok = s.c != 0;
+  lc* o = r.wfx + (size_t)col * N;
+  for (int i = lane; i < N; i += 32) {
+    const double2 v = p[i];
+    o[i] = ok ? fx::limbs(cx{fx_convert(v.x, s), fx_convert(v.y, s)}) : lc{0, 0, 0, 0};
+  }
+  for (int i = lane; i < 4 * N; i += 32) r.acc[(size_t)col * 4 * N + i] = 0;
+  if (lane == 0) r.wscale[col] = fx_output_scale(su, s, Scale{a.kscale->x, a.kscale->y});
+}
+
+template <int N>
+constexpr int rows_fx_teams() { return kRowsThreads / fx::Team<N>::T; }
+
+template <int N>
+__global__ void __launch_bounds__(kRowsThreads, 2) k_fock_fx(FockFxArgs a, FockFxRows r) {
+  using TM = fx::Team<N>;
+  constexpr int E = TM::E, T = TM::T, R = kRowsThreads / TM::T;
+  extern __shared__ int4 sm_fx[];
+  lc* tw_s = reinterpret_cast<lc*>(sm_fx);                      // kTwCount
+  cx* bufs = reinterpret_cast<cx*>(sm_fx + TM::kTwCount);       // R * N
+  int2* twn_s = reinterpret_cast<int2*>(bufs + R * N);          // kTwCount
+  const int tl = threadIdx.x % T, team = threadIdx.x / T;
+  cx* buf = bufs + team * N;
+  load_twiddles<N>(a.tw, tw_s, twn_s);
+  __syncthreads();
+  const int col = (blockIdx.x / r.nchunks) * R + team, chunk = blockIdx.x % r.nchunks;
+  const bool valid = col < r.ncols;
+  const int c = valid ? col : 0;
+  const int kr = c / r.w.nb;
+  const lc* wa = r.wfx + (size_t)c * N;
+  unsigned long long* dst = r.acc + (size_t)c * 4 * N;
+  const int p0 = chunk * r.chunk, p1 = min(a.nk * a.nbocc, p0 + r.chunk);
+  cx acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = cx{0, 0};
+  for (int p = p0; p < p1; ++p) {
+    if (p != p0 && (p - p0) % kFxTerms == 0) {  // before the accumulators could overflow
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        if (valid) fx_accumulate(dst, N, TM::pos(tl, e), acc[e]);
+        acc[e] = cx{0, 0};
+      }
+    }
+    const lc* ub = a.ufx + (size_t)p * N;
+    const int2* kab = a.kern + (size_t)(kr - p / a.nbocc + a.nk - 1) * N;
+    cx x[E];
+    pair_potential<N>(x, wa, ub, kab, buf, tw_s, twn_s, tl, team);
+    const int sb = 2 * a.shift[p];
+    if (sb == 0) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[e] = fx::add(acc[e], fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])));
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        acc[e] = fx::add(acc[e], fx_shift(fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])), sb));
+    }
+  }
+  if (!valid) return;
+#pragma unroll
+  for (int e = 0; e < E; ++e) fx_accumulate(dst, N, TM::pos(tl, e), acc[e]);
+}
+
+// Kernel table: K^ = kern s_k, with s_k the largest short factor that keeps
+// sum_G |K^(G)| below 2^60 for every k - k'.
+__global__ void __launch_bounds__(1024) k_fx_kern_scale(const double* __restrict__ kern, int nd, int N, int2* kscale) {
+  __shared__ double red[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double m = 0.0;
+  for (int d = warp; d < nd; d += 32) {
+    double s = 0.0;
+    for (int i = lane; i < N; i += 32) s += fabs(kern[(size_t)d * N + i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    m = fmax(m, s);
+  }
+  if (lane == 0) red[warp] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 32; ++w) m = fmax(m, red[w]);
+    // 2^60 (1 - 2e-5) / m
+    int e = 0;
+    const float f = m > 1e-280 ? (float)(2.0 * frexp(1.1529e18 / m, &e)) : 1.0f;
+    const Scale s = m > 1e-280 ? fx_short_scale(f * (1.0f - 1.0f / 65536.0f), e - 1) : Scale{8, -3};
+    *kscale = make_int2(s.c, s.k);
+  }
+}
+__global__ void k_fx_kern(const double* __restrict__ kern, int n, const int2* __restrict__ kscale, int2* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const i64 v = fx_convert(kern[i], Scale{kscale->x, kscale->y});
+  out[i] = fx::real_limbs(v);
+}
+
+// ---------------------------------------------------------------------------
+// Launchers
+// ---------------------------------------------------------------------------
+template <int N>
+static void sym_fx_shape(int S, int* threads, size_t* smem) {
+  using TM = fx::Team<N>;
+  *threads = (S * TM::T + 31) / 32 * 32;
+  *smem = 24 * (size_t)TM::kTwCount + 16 * (size_t)N * (*threads / TM::T + S);
+}
+
+template <int N>
+static cudaError_t fock_sym_fx_impl(const FockFxArgs& a, cudaStream_t s) {
+  const int tiles = a.T * (a.T + 1) / 2;
+  if (tiles == 0) return cudaSuccess;
+  int threads;
+  size_t smem;
+  sym_fx_shape<N>(a.S, &threads, &smem);
+  k_fock_sym_fx<N><<<tiles, threads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+#define MATTOHF_DISPATCH(NG, CALL)                 \
+  switch (NG) {                                    \
+    case 16: return CALL(16);                      \
+    case 32: return CALL(32);                      \
+    case 64: return CALL(64);                      \
+    case 128: return CALL(128);                    \
+    case 256: return CALL(256);                    \
+    case 512: return CALL(512);                    \
+    default: return cudaErrorInvalidValue;         \
+  }
+
+// after launch_fx_orbitals
+cudaError_t launch_fock_sym_fx(int NG, const FockFxArgs& a, cudaStream_t s) {
+#define CALL(n) fock_sym_fx_impl<n>(a, s)
+  MATTOHF_DISPATCH(NG, CALL)
+#undef CALL
+}
+
+template <int N>
+static cudaError_t fock_sym_fx_batch_impl(const FockFxArgs* d_args, const int* d_tile_pre, int nruns, int S,
+                                          int total_tiles, const int* d_elem_pre, int total_elems, cudaStream_t s) {
+  int threads;
+  size_t smem;
+  sym_fx_shape<N>(S, &threads, &smem);
+  k_fx_sizes_batch<<<(total_elems / N + 3) / 4, 128, 0, s>>>(d_args, d_elem_pre, nruns, N);
+  k_fx_convert_batch<<<total_elems / N, 128, 0, s>>>(d_args, d_elem_pre, nruns, N);
+  k_fock_sym_fx_batch<N><<<total_tiles, threads, smem, s>>>(d_args, d_tile_pre, nruns);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fock_sym_fx_batch(int NG, const FockFxArgs* d_args, const int* d_tile_pre, int nruns, int S,
+                                     int total_tiles, const int* d_elem_pre, int total_elems, cudaStream_t s) {
+  if (total_tiles <= 0) return cudaSuccess;
+#define CALL(n) fock_sym_fx_batch_impl<n>(d_args, d_tile_pre, nruns, S, total_tiles, d_elem_pre, total_elems, s)
+  MATTOHF_DISPATCH(NG, CALL)
+#undef CALL
+}
+
+cudaError_t launch_fx_orbitals(int NG, const FockFxArgs& a, cudaStream_t s) {
+  const int M = a.nk * a.nbocc;
+  // up to 2^13 values every CTA takes all the sizes itself: a launch less
+  const int scan = M * NG <= 8192;
+  if (!scan) k_fx_sizes<<<(M + 3) / 4, 128, 0, s>>>(a, NG);
+  k_fx_convert<<<M, 128, 0, s>>>(a, NG, scan);
+  return cudaGetLastError();
+}
+
+template <int N>
+static constexpr size_t rows_fx_smem() {
+  return 24 * (size_t)fx::Team<N>::kTwCount + 16 * (size_t)N * rows_fx_teams<N>();
+}
+
+template <int N>
+static cudaError_t fock_fx_impl(const FockFxArgs& a, const FockFxRows& r, cudaStream_t s) {
+  constexpr int R = rows_fx_teams<N>();
+  k_fx_rows<<<(r.ncols + 3) / 4, 128, 0, s>>>(a, r, N);
+  k_fock_fx<N><<<(r.ncols + R - 1) / R * r.nchunks, kRowsThreads, rows_fx_smem<N>(), s>>>(a, r);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fock_fx(int NG, const FockFxArgs& a, const FockFxRows& r, cudaStream_t s) {
+  if (r.ncols <= 0) return cudaSuccess;
+#define CALL(n) fock_fx_impl<n>(a, r, s)
+  MATTOHF_DISPATCH(NG, CALL)
+#undef CALL
+}
+
+// Chunks of the sources for ncols columns: enough CTAs to fill the device's
+// SMs several times over.
+void fx_rows_split(int NG, int ncols, int npairs, int nsm, int fixed, int* nchunks, int* chunk) {
+  int nch = fixed;
+  if (nch <= 0) {
+    const int groups = (ncols + fx_rows_teams(NG) - 1) / fx_rows_teams(NG);
+    nch = (std::max(1, nsm) * kRowsCtasPerSm + groups - 1) / groups;
+  }
+  nch = std::max(1, std::min(nch, npairs));
+  const int ch = (npairs + nch - 1) / nch;
+  *chunk = ch;
+  *nchunks = (npairs + ch - 1) / ch;
+}
+
+int fx_rows_teams(int NG) {
+  switch (NG) {
+    case 16: return rows_fx_teams<16>();
+    case 32: return rows_fx_teams<32>();
+    case 64: return rows_fx_teams<64>();
+    case 128: return rows_fx_teams<128>();
+    case 256: return rows_fx_teams<256>();
+    default: return rows_fx_teams<512>();
+  }
+}
+
+cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int2* out, cudaStream_t s) {
+  k_fx_kern_scale<<<1, 1024, 0, s>>>(kern, nd, NG, kscale);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  k_fx_kern<<<(nd * NG + 255) / 256, 256, 0, s>>>(kern, nd * NG, kscale, out);
+  return cudaGetLastError();
+}
+
+template <int N>
+static int fx_twiddles(int4* out) {
+  using TM = fx::Team<N>;
+  int n = 0;
+  auto put = [&](int num, int den) {
+    const long double th = -2.0L * acosl(-1.0L) * (long double)(num % den) / (long double)den;
+    const long long x = llrintl(ldexpl(cosl(th), fx::kOne)), y = llrintl(ldexpl(sinl(th), fx::kOne));
+    const long long m = (1ll << fx::kLimb) - 1;
+    if (out) out[n] = make_int4((int)(x >> fx::kLimb), (int)(x & m), (int)(y >> fx::kLimb), (int)(y & m));
+    ++n;
+  };
+  if (TM::R1 > 1)
+    for (int r = 0; r < TM::R1; ++r)
+      for (int k = 0; k < TM::R0; ++k) put(r * k, TM::R0 * TM::R1);
+  for (int r = 0; r < TM::R0; ++r)
+    for (int j = 0; j < TM::STRIDE; ++j) put(r * j, N);
+  return n;
+}
+
+int fx_twiddle_table(int NG, int4* out) {
+  switch (NG) {
+    case 16: return fx_twiddles<16>(out);
+    case 32: return fx_twiddles<32>(out);
+    case 64: return fx_twiddles<64>(out);
+    case 128: return fx_twiddles<128>(out);
+    case 256: return fx_twiddles<256>(out);
+    case 512: return fx_twiddles<512>(out);
+    default: return 0;
+  }
+}
+
+template <int N>
+static cudaError_t configure_fx_impl() {
+  int threads;
+  size_t smem;
+  sym_fx_shape<N>(sym_fx_threads<N>() / fx::Team<N>::T, &threads, &smem);
+  const cudaError_t e = cudaFuncSetAttribute(k_fock_sym_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const cudaError_t e2 =
+      cudaFuncSetAttribute(k_fock_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_fx_smem<N>());
+  if (e2 != cudaSuccess) return e2;
+  return cudaFuncSetAttribute(k_fock_sym_fx_batch<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+cudaError_t configure_fx_kernels() {
+  cudaError_t e;
+  if ((e = configure_fx_impl<16>()) != cudaSuccess) return e;
+  if ((e = configure_fx_impl<32>()) != cudaSuccess) return e;
+  if ((e = configure_fx_impl<64>()) != cudaSuccess) return e;
+  if ((e = configure_fx_impl<128>()) != cudaSuccess) return e;
+  if ((e = configure_fx_impl<256>()) != cudaSuccess) return e;
+  return configure_fx_impl<512>();
+}
+
+}  // namespace mattohf

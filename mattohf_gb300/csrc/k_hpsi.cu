@@ -6,6 +6,7 @@
 // (F:94-119), ubk_Ex (F:165-183), ubk_Je (F:289-318); RK4 stages from
 // src/RT_calculation.f90:154-173.
 #include "fft.cuh"
+#include "fx_convert.cuh"
 #include "internal.h"
 
 namespace mattohf {
@@ -53,41 +54,84 @@ __global__ void __launch_bounds__(256) k_dens_partial_batch(const DensArgs* __re
   dens_partial_body(args[blockIdx.y], N, blockIdx.x);
 }
 
-// Stage 2 (one CTA): rho = ordered sum of the chunk partials, then the
-// Hartree potential (F:147-162), vloc = vH + vion and the density scalars.
+// Twiddles in shared memory (fixed point), loaded by the whole CTA.
 template <int N>
-__device__ __forceinline__ void density_body(const DensArgs& a) {
-  using TM = Team<N>;
-  __shared__ double rho_s[N];
-  __shared__ double vh_s[N];
-  __shared__ double2 tw_s[N];
-  __shared__ double2 buf_s[TM::PER_WARP][N];
-  const int tid = threadIdx.x;
-  for (int i = tid; i < N; i += blockDim.x) tw_s[i] = a.tw[i];
-  for (int ig = tid; ig < N; ig += blockDim.x) {
-    double s = a.part[ig];
-    for (int ch = 1; ch < kDensChunks; ++ch) s += a.part[(size_t)ch * N + ig];
-    rho_s[ig] = s;
-    a.rho[ig] = s;
+struct FxTwiddles {
+  lc w[fx::Team<N>::kTwCount];
+  int2 n[fx::Team<N>::kTwCount];
+  __device__ __forceinline__ void load(const lc* __restrict__ tw) {
+    for (int i = threadIdx.x; i < fx::Team<N>::kTwCount; i += blockDim.x) {
+      const lc v = tw[i];
+      w[i] = v;
+      n[i] = make_int2(fx::neg_hi(v.yh), fx::neg_lo(v.yl));
+    }
+  }
+};
+
+// Transform of buf (N fixed-point values) in place by the CTA's first team; every
+// thread calls it, with buf complete, and finds it complete.
+template <int N>
+__device__ __forceinline__ void fx_block_forward(cx* buf, const FxTwiddles<N>& tw) {
+  using TM = fx::Team<N>;
+  __syncthreads();
+  const int tl = threadIdx.x;
+  if (tl < TM::T) {
+    cx x[TM::E];
+#pragma unroll
+    for (int e = 0; e < TM::E; ++e) x[e] = buf[TM::pos(tl, e)];
+    fx::forward<N, true>(x, buf, tw.w, tw.n, tl, 0);
+    fx::team_sync<TM::T, true>(0);
+#pragma unroll
+    for (int e = 0; e < TM::E; ++e) buf[TM::pos(tl, e)] = x[e];
   }
   __syncthreads();
-  if (tid < 32) {
-    const int lane = tid, tl = lane % TM::T, team = lane / TM::T;
-    double2 x[TM::E];
-#pragma unroll
-    for (int e = 0; e < TM::E; ++e) x[e] = make_double2(rho_s[TM::pos(tl, e)], 0.0);
-    fft_team<N, -1>(x, buf_s[team], tw_s, tl);
-#pragma unroll
-    for (int e = 0; e < TM::E; ++e) {
-      const double v = a.vCG[TM::pos(tl, e)];
-      x[e] = make_double2(v * x[e].x, v * x[e].y);
-    }
-    fft_team<N, +1>(x, buf_s[team], tw_s, tl);
-    if (team == 0) {
-#pragma unroll
-      for (int e = 0; e < TM::E; ++e) vh_s[TM::pos(tl, e)] = x[e].x / (double)N;
-    }
+}
+
+// Threads of a CTA that holds one column of N values, and values per thread.
+template <int N>
+struct ColumnCta {
+  static constexpr int TH = N < 32 ? 32 : N > 128 ? 128 : N;
+  static constexpr int PER = N > TH ? N / TH : 1;
+  static constexpr int NW = TH / 32;
+};
+
+// Stage 2 (one CTA): rho = ordered sum of the chunk partials, then the
+// Hartree potential (F:147-162), vloc = vH + vion and the density scalars.
+// The transforms are fixed-point (fft_fx.cuh); the product with vCG is FP64, one
+// value per thread, with a new scale for the second transform.
+template <int N>
+__device__ __forceinline__ void density_body(const DensArgs& a) {
+  constexpr int TH = N < 64 ? 64 : N, NW = TH / 32;
+  __shared__ double rho_s[N];
+  __shared__ double vh_s[N];
+  __shared__ FxTwiddles<N> tw_s;
+  __shared__ cx buf[N];
+  __shared__ int red[2 * NW];
+  const int tid = threadIdx.x;
+  const bool in = tid < N;
+  tw_s.load(a.twfx);
+  double2 v[1] = {make_double2(0.0, 0.0)};
+  if (in) {
+    double s = a.part[tid];
+#pragma unroll 8
+    for (int ch = 1; ch < kDensChunks; ++ch) s += a.part[(size_t)ch * N + tid];
+    rho_s[tid] = s;
+    a.rho[tid] = s;
+    v[0].x = s;
   }
+  int2 z = fx_block_size<1, NW>(v, red);
+  const Scale s1 = fx_fft_scale(z, N);
+  if (in) buf[tid] = cx{fx_convert(v[0].x, s1), 0};
+  fx_block_forward<N>(buf, tw_s);
+  if (in) {
+    const double f = a.vCG[tid] * fx_unscale(s1) * (1.0 / N);
+    v[0] = make_double2(f * (double)buf[tid].x, -f * (double)buf[tid].y);  // conjugate: backward next
+  }
+  z = fx_block_size<1, NW>(v, red);
+  const Scale s2 = fx_fft_scale(z, N);
+  if (in) buf[tid] = cx{fx_convert(v[0].x, s2), fx_convert(v[0].y, s2)};
+  fx_block_forward<N>(buf, tw_s);
+  if (in) vh_s[tid] = (double)buf[tid].x * fx_unscale(s2);
   __syncthreads();
   if (a.mu != nullptr) {
     for (int ig = tid; ig < N; ig += blockDim.x) {
@@ -124,17 +168,6 @@ __global__ void __launch_bounds__(512) k_density(DensArgs a) { density_body<N>(a
 template <int N>
 __global__ void __launch_bounds__(512) k_density_batch(const DensArgs* __restrict__ args) {
   density_body<N>(args[blockIdx.x]);
-}
-
-// run owning work item `i` given exclusive prefix sums pre[0..nruns] (pre[0] = 0)
-__device__ __forceinline__ int find_run(const int* __restrict__ pre, int nruns, int i) {
-  int lo = 0, hi = nruns - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (pre[mid] <= i) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
 }
 
 // ---------------------------------------------------------------------------
@@ -204,108 +237,6 @@ __global__ void __launch_bounds__(kThreads) k_fock(FockArgs a) {
 }
 
 
-// ---------------------------------------------------------------------------
-// Symmetric exchange for w == u over occupied pairs (same F:237-261 sum).
-//
-// For occupied orbitals a=(ka,ba), b=(kb,bb) the pair potentials obey
-//   phi_ba(x_m) = conj(phi_ab(x_m)) + (kern_ba[N/2] - kern_ab[N/2]) conj(R_ab[N/2]) (-1)^m
-// (the soft-Coulomb kernel is even; only the self-aliased Nyquist frequency
-// breaks the conjugate symmetry, R_ab being FFT(u_a conj(u_b))).  One pair of
-// transforms therefore yields both out(a) += phi_ab u_b and
-// out(b) += phi_ba u_a.  A CTA handles a tile pair (i <= j) of S orbitals:
-// team w owns row a = i*S + w (accumulated in registers) and in round r
-// visits b = j*S + (w + r) % S, so within a round every column accumulator
-// (shared memory) has exactly one writer.  Diagonal tiles visit each
-// unordered pair once (rounds 0..S/2).
-// ---------------------------------------------------------------------------
-template <int N>
-__device__ __forceinline__ void fock_sym_body(const FockSymArgs& a, const int tile) {
-  using TM = Team<N>;
-  constexpr int E = TM::E, T = TM::T, PW = TM::PER_WARP;
-  const int S = a.S;                          // tile size (runtime, <= teams per CTA)
-  const int nteam = (blockDim.x >> 5) * PW;    // teams in this CTA (>= S)
-  extern __shared__ double2 sm[];
-  double2* tw_s = sm;                  // N
-  double2* bufs = sm + N;              // nteam * N  (team FFT buffers)
-  double2* cacc = bufs + nteam * N;    // S * N  (column accumulators)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tl = lane % T, tw_ = warp * PW + lane / T;
-  const int team_lane0 = (lane / T) * T;
-  double2* buf = bufs + tw_ * N;
-  for (int i = tid; i < N; i += blockDim.x) tw_s[i] = a.tw[i];
-  for (int i = tid; i < S * N; i += blockDim.x) cacc[i] = make_double2(0.0, 0.0);
-  // tile pair (ti, tj), ti <= tj, from the linear block index
-  int ti = 0, rem = tile;
-  while (rem >= a.T - ti) { rem -= a.T - ti; ++ti; }
-  const int tj = ti + rem;
-  const int M = a.nk * a.nbocc;
-  const int ia = ti * S + tw_;
-  const bool va = tw_ < S && ia < M;
-  const int ka = (va ? ia : 0) / a.nbocc, ba = (va ? ia : 0) % a.nbocc;
-  // orbitals are re-read from global memory (L1/L2-resident) where needed
-  // rather than held in registers: the kernel is FP64-pipe bound, and this
-  // keeps the largest grids free of register spills
-  const double2* ucol_a = a.u.p + (size_t)ka * a.u.kstride + (size_t)ba * N;
-  double2 racc[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) racc[e] = make_double2(0.0, 0.0);
-  __syncthreads();
-  const bool diag = (ti == tj);
-  const int nrounds = diag ? (S / 2 + 1) : S;
-  for (int r = 0; r < nrounds; ++r) {
-    const int lb = (tw_ + r) % S;
-    const int ib = tj * S + lb;
-    bool valid = va && ib < M;
-    if (diag && (S % 2 == 0) && r == S / 2 && tw_ >= S / 2) valid = false;  // counted by the partner
-    const bool self = diag && r == 0;
-    const int kb = (ib < M ? ib : 0) / a.nbocc, bb = (ib < M ? ib : 0) % a.nbocc;
-    const double2* ucol_b = a.u.p + (size_t)kb * a.u.kstride + (size_t)bb * N;
-    double2 x[E];
-    fft_team_in<N, -1>(InConjProduct<N>{ucol_a, ucol_b, tl}, x, buf, tw_s, tl);
-    // Nyquist coefficient R_ab[N/2] lives in slot (p=0, r=R0/2) of the team's lane 0
-    const double2 rn_own = x[TM::R0 / 2];
-    const double rnx = __shfl_sync(0xffffffffu, rn_own.x, team_lane0);
-    const double rny = __shfl_sync(0xffffffffu, rn_own.y, team_lane0);
-    const int dab = ka - kb + a.nk - 1, dba = kb - ka + a.nk - 1;
-    const double* kab = a.kern + (size_t)dab * N;
-    fft_team_in<N, +1>(InScaled<N>{x, kab, tl}, x, buf, tw_s, tl);
-    if (valid) {
-#pragma unroll
-      for (int e = 0; e < E; ++e) racc[e] = cfma(x[e], ucol_b[TM::pos(tl, e)], racc[e]);
-      if (!self) {
-        const double dk = __ldg(a.kern + (size_t)dba * N + N / 2) - __ldg(kab + N / 2);
-        const double cx = dk * rnx, cy = -dk * rny;  // dk * conj(R)
-        double2* col = cacc + lb * N;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int q = TM::pos(tl, e);
-          const double sg = (q & 1) ? -1.0 : 1.0;
-          const double2 pba = make_double2(fma(sg, cx, x[e].x), fma(sg, cy, -x[e].y));
-          col[q] = cfma(pba, ucol_a[q], col[q]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // write partials: rows from registers, columns from shared memory
-  double2* dst = a.scratch + (size_t)tile * 2 * S * N;
-  if (tw_ < S) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) dst[(size_t)tw_ * N + TM::pos(tl, e)] = racc[e];
-  }
-  for (int i = tid; i < S * N; i += blockDim.x) dst[(size_t)S * N + i] = cacc[i];
-}
-
-template <int N>
-__global__ void __launch_bounds__(kThreads) k_fock_sym(FockSymArgs a) { fock_sym_body<N>(a, blockIdx.x); }
-
-template <int N>
-__global__ void __launch_bounds__(kThreads) k_fock_sym_batch(const FockSymArgs* __restrict__ args,
-                                                           const int* __restrict__ pre, int nruns) {
-  const int r = find_run(pre, nruns, blockIdx.x);
-  fock_sym_body<N>(args[r], blockIdx.x - pre[r]);
-}
-
 // Sum the tile-pair partials of every occupied output into F[o][q] (fixed
 // order over tiles: column partials of earlier tiles, the diagonal tile's row
 // and column partials, row partials of later tiles).
@@ -345,123 +276,147 @@ __global__ void __launch_bounds__(kRedQ* kRedE) k_sym_reduce(const double2* __re
   sym_reduce_finish(f, valid, F + (valid ? idx : 0));
 }
 
-// element prefix: pre[r] = sum over earlier runs of M_r * N
-__global__ void __launch_bounds__(kRedQ* kRedE) k_sym_reduce_batch(const FockSymArgs* __restrict__ args,
-                                                                   const int* __restrict__ pre, int nruns,
-                                                                   int N) {
-  const int e = threadIdx.x % kRedE, c = threadIdx.x / kRedE;
-  const int idx = blockIdx.x * kRedE + e;
-  const bool valid = idx < pre[nruns];
-  double2 f = make_double2(0.0, 0.0);
-  double2* out = nullptr;
-  if (valid) {
-    const int r = find_run(pre, nruns, idx);
-    const FockSymArgs& a = args[r];
-    f = sym_run_sum(a.scratch, a.S, a.T, N, idx - pre[r], c);
-    out = a.F + (idx - pre[r]);
+__device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, int q, int N) {
+  if (s.f != nullptr) return s.f[(size_t)col * N + q];
+  const unsigned long long* p = s.acc + (size_t)col * 4 * N + q;
+  const i64 hx = (i64)p[0], lx = (i64)p[N], hy = (i64)p[2 * N], ly = (i64)p[3 * N];
+  const double2 f = s.scale[col];
+  const double x = fma((double)hx, 4294967296.0, (double)lx), y = fma((double)hy, 4294967296.0, (double)ly);
+  return make_double2(fma(x, f.x, x * f.y), fma(y, f.x, y * f.y));
+}
+// Exchange term of output column (ik, ib) at grid point q; false: none.
+__device__ __forceinline__ bool exchange_at(const CombineArgs& a, int ik, int ib, int q, int N, double2* f) {
+  if (ib < a.nbocc && (a.occ_ex.acc != nullptr || a.occ_ex.f != nullptr)) {
+    *f = exchange_value(a.occ_ex, ik * a.nbocc + ib, q, N);
+    return true;
   }
-  sym_reduce_finish(f, valid, out);
+  if (a.row_ex.acc == nullptr) return false;
+  *f = exchange_value(a.row_ex, ik * (a.w.nb - a.row_b0) + (ib - a.row_b0), q, N);
+  return true;
 }
 
-// Exchange term of output column (ik, ib) at grid point q, summed over the
-// partials in a fixed order.
-__device__ __forceinline__ double2 exchange_at(const CombineArgs& a, int ik, int ib, int q, int N) {
-  if (a.sym != nullptr && ib < a.nbocc) return a.sym[(size_t)(ik * a.nbocc + ib) * N + q];
-  const int nbc = a.w.nb - a.chunk_b0;
-  const int c = ik * nbc + (ib - a.chunk_b0);
-  const double2* src = a.scratch + (size_t)c * a.nchunks * N + q;
-  double2 f = src[0];
-  for (int ch = 1; ch < a.nchunks; ++ch) f = cadd(f, src[(size_t)ch * N]);
-  return f;
+// Sum over a CTA, result in every thread of warp 0 (fixed order).
+template <int NW>
+__device__ __forceinline__ double block_sum(double v, double* red) {
+  v = warp_sum(v);
+  if constexpr (NW == 1) return v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+#pragma unroll
+  for (int w = 1; w < NW; ++w) v += red[w];
+  __syncthreads();
+  return v;
 }
 
 // ---------------------------------------------------------------------------
-// Combine: kinetic (F:212-234) + local potential (F:199-203) + Fock partials,
-// then the mode's epilogue (RK4 stages RT:166-170, observables F:94-119,
-// F:165-183, F:289-318).  One team per output column.
+// Combine: kinetic (F:212-234) + local potential (F:199-203) + exchange, then
+// the mode's epilogue (RK4 stages RT:166-170, observables F:94-119, F:165-183,
+// F:289-318).  One CTA per output column.
+//
+// FP64 is slow here in both throughput and latency (one instruction per 64
+// cycles and warp), so the transforms run in fixed point on the CTA's first
+// team and the FP64 work is spread over all threads, a value or a few each.
+// With FP64 transforms on one warp per column a launch took 26 us at NG = 64 and
+// 43 us at NG = 128.
 // ---------------------------------------------------------------------------
 template <int N>
-__device__ __forceinline__ void combine_body(const CombineArgs& a, const int ncols, const int cta) {
-  using TM = Team<N>;
-  constexpr int E = TM::E, T = TM::T, PW = TM::PER_WARP;
-  constexpr int NTEAM = kCombineWarps * PW;
-  __shared__ double2 tw_s[N];
-  __shared__ double2 bufs[NTEAM][N];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tl = lane % T, team = warp * PW + lane / T;
-  for (int i = tid; i < N; i += kCombineWarps * 32) tw_s[i] = a.tw[i];
-  __syncthreads();
-  const double A = afield_value(a.af);
-  // warp-uniform: whole warps go idle together
-  const int col0 = (cta * kCombineWarps + warp) * PW;
-  if (col0 >= ncols) return;
-  const int col = col0 + lane / T;
-  const bool valid = col < ncols;
-  const int c = valid ? col : col0;
+__device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) {
+  using CC = ColumnCta<N>;
+  constexpr int TH = CC::TH, PER = CC::PER, NW = CC::NW;
+  __shared__ FxTwiddles<N> tw_s;
+  __shared__ cx buf[N];
+  __shared__ int red[2 * NW];
+  __shared__ double redd[NW];
+  const int tid = threadIdx.x;
   const int ik = c / a.w.nb, ib = c % a.w.nb;
   const double2* wcol = a.w.p + (size_t)ik * a.w.kstride + (size_t)ib * N;
-  double2 wv[E], x[E];
+  const bool in = tid < N;
+  double2 wv[PER];
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    wv[e] = wcol[TM::pos(tl, e)];
-    x[e] = wv[e];
-  }
+  for (int p = 0; p < PER; ++p) wv[p] = in ? wcol[tid + TH * p] : make_double2(0.0, 0.0);
   // split == 2: the kinetic and local-potential part was made by the split == 1
   // pass (beside the exchange); only the exchange and the epilogue remain
   const bool post = a.split == 2;
-  if (!post) fft_team<N, -1>(x, bufs[team], tw_s, tl);
-  const double kAx = a.kx[ik] + A;
-  const double kA2 = kAx * kAx;
-  if (a.mode == CM_OBS) {
-    // Ekin and Je of this column by Parseval on FFT(u):
-    //   sum_x conj(u) IFFT(f * FFT(u)) = sum_G f(G) |FFT(u)(G)|^2
-    double ek = 0.0, je = 0.0;
+  double2 kin[PER];
+  if (!post && a.mode != CM_F) {
+    const double A = afield_value(a.af);
+    const double kAx = a.kx[ik] + A;
+    const double kA2 = kAx * kAx;
+    tw_s.load(a.twfx);
+    int2 z = fx_block_size<PER, NW>(wv, red);
+    const Scale s1 = fx_fft_scale(z, N);
+    if (in) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const double G = a.Gx[TM::pos(tl, e)];
-      const double m2 = x[e].x * x[e].x + x[e].y * x[e].y;
-      ek += 0.5 * (G * G + 2.0 * G * kAx + kA2) * m2;
-      je += (G + a.kx[ik] + A) * m2;
+      for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(wv[p].x, s1), fx_convert(wv[p].y, s1)};
     }
-    ek = team_sum<T>(ek) / (double)N;
-    je = team_sum<T>(je) / (double)N;
-    double fr = 0.0, fi = 0.0;
-    if ((a.scratch != nullptr || a.sym != nullptr) && ib < a.nbocc) {
+    fx_block_forward<N>(buf, tw_s);
+    const double u1 = fx_unscale(s1);
+    if (a.mode == CM_OBS) {
+      // Ekin and Je of this column by Parseval on FFT(u):
+      //   sum_x conj(u) IFFT(f * FFT(u)) = sum_G f(G) |FFT(u)(G)|^2
+      double ek = 0.0, je = 0.0, fr = 0.0, fi = 0.0;
+      if (in) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const double2 f = exchange_at(a, ik, ib, TM::pos(tl, e), N);
-        fr += wv[e].x * f.x + wv[e].y * f.y;
-        fi += wv[e].x * f.y - wv[e].y * f.x;
+        for (int p = 0; p < PER; ++p) {
+          const int q = tid + TH * p;
+          const double G = a.Gx[q];
+          const double xr = (double)buf[q].x * u1, xi = (double)buf[q].y * u1;
+          const double m2 = xr * xr + xi * xi;
+          ek += 0.5 * (G * G + 2.0 * G * kAx + kA2) * m2;
+          je += (G + a.kx[ik] + A) * m2;
+          double2 f;
+          if (ib < a.nbocc && exchange_at(a, ik, ib, q, N, &f)) {
+            fr += wv[p].x * f.x + wv[p].y * f.y;
+            fi += wv[p].x * f.y - wv[p].y * f.x;
+          }
+        }
+      }
+      ek = block_sum<NW>(ek, redd) / (double)N;
+      je = block_sum<NW>(je, redd) / (double)N;
+      fr = block_sum<NW>(fr, redd);
+      fi = block_sum<NW>(fi, redd);
+      if (tid == 0) {
+        double* cb = a.colbuf + (size_t)c * 4;
+        cb[0] = ek;
+        cb[1] = je;
+        cb[2] = fr;
+        cb[3] = fi;
+      }
+      return;
+    }
+    // kinetic energy in FP64, then back with a new scale
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int q = tid + TH * p;
+      kin[p] = make_double2(0.0, 0.0);
+      if (in) {
+        const double G = a.Gx[q];
+        const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2) * (u1 * (1.0 / N));
+        kin[p] = make_double2(m * (double)buf[q].x, -m * (double)buf[q].y);  // conjugate: backward next
       }
     }
-    fr = team_sum<T>(fr);
-    fi = team_sum<T>(fi);
-    if (valid && tl == 0) {
-      double* cb = a.colbuf + (size_t)c * 4;
-      cb[0] = ek;
-      cb[1] = je;
-      cb[2] = fr;
-      cb[3] = fi;
-    }
-    return;
-  }
-  if (!post) {
+    z = fx_block_size<PER, NW>(kin, red);
+    const Scale s2 = fx_fft_scale(z, N);
+    if (in) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const double G = a.Gx[TM::pos(tl, e)];
-      const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2);
-      x[e] = make_double2(m * x[e].x / (double)N, m * x[e].y / (double)N);
+      for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(kin[p].x, s2), fx_convert(kin[p].y, s2)};
     }
-    fft_team<N, +1>(x, bufs[team], tw_s, tl);
+    fx_block_forward<N>(buf, tw_s);
+    const double u2 = fx_unscale(s2);
+    if (in) {
+#pragma unroll
+      for (int p = 0; p < PER; ++p) kin[p] = make_double2((double)buf[tid + TH * p].x * u2, (double)buf[tid + TH * p].y * -u2);
+    }
   }
   const size_t ocol = (size_t)ik * a.w.nb * N + (size_t)ib * N;  // [NK][NB][NG]
   if (a.split == 1) {
-    if (valid) {
+    if (in) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int q = TM::pos(tl, e);
+      for (int p = 0; p < PER; ++p) {
+        const int q = tid + TH * p;
         const double v = a.vloc[q];
-        a.hpre[ocol + q] = make_double2(x[e].x + v * wv[e].x, x[e].y + v * wv[e].y);
+        a.hpre[ocol + q] = make_double2(kin[p].x + v * wv[p].x, kin[p].y + v * wv[p].y);
       }
     }
     return;
@@ -470,28 +425,28 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int nco
   double exr = 0.0, exi = 0.0;
   bool bad = false;
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int q = TM::pos(tl, e);
+  for (int p = 0; p < PER; ++p) {
+    if (!in) continue;
+    const int q = tid + TH * p;
     double2 h;
     if (a.mode == CM_T) {
-      h = x[e];
+      h = kin[p];
     } else {
       if (a.mode == CM_F) h = make_double2(0.0, 0.0);
       else if (post) h = a.hpre[ocol + q];
       else {
         const double v = a.vloc[q];
-        h = make_double2(x[e].x + v * wv[e].x, x[e].y + v * wv[e].y);
+        h = make_double2(kin[p].x + v * wv[p].x, kin[p].y + v * wv[p].y);
       }
-      if (a.scratch != nullptr || a.sym != nullptr) {
-        const double2 f = exchange_at(a, ik, ib, q, N);
+      double2 f;
+      if (exchange_at(a, ik, ib, q, N, &f)) {
         if (a.ex_cols) {
-          exr += wv[e].x * f.x + wv[e].y * f.y;
-          exi += wv[e].x * f.y - wv[e].y * f.x;
+          exr += wv[p].x * f.x + wv[p].y * f.y;
+          exi += wv[p].x * f.y - wv[p].y * f.x;
         }
         h = cadd(h, f);
       }
     }
-    if (!valid) continue;
     if (a.mode == CM_H || a.mode == CM_F || a.mode == CM_T) {
       a.out.p[(size_t)ik * a.out.kstride + (size_t)ib * N + q] = h;
       bad |= !(isfinite(h.x) && isfinite(h.y));
@@ -499,7 +454,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int nco
     }
     // RK4: k = -i h
     const double2 k = make_double2(h.y, -h.x);
-    const size_t o = (size_t)ik * a.w.nb * N + (size_t)ib * N + q;  // [NK][NB][NG]
+    const size_t o = ocol + q;
     const double2 u0 = a.u0[o];
     double2 nx;
     if (a.mode == CM_RK0 || a.mode == CM_RK1 || a.mode == CM_RK2) {
@@ -522,9 +477,9 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int nco
     bad |= !(isfinite(nx.x) && isfinite(nx.y));
   }
   if (a.ex_cols) {
-    exr = team_sum<T>(exr);
-    exi = team_sum<T>(exi);
-    if (valid && tl == 0) {
+    exr = block_sum<NW>(exr, redd);
+    exi = block_sum<NW>(exi, redd);
+    if (tid == 0) {
       a.colbuf[(size_t)c * 4 + 2] = exr;
       a.colbuf[(size_t)c * 4 + 3] = exi;
     }
@@ -533,17 +488,16 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int nco
 }
 
 template <int N>
-__global__ void __launch_bounds__(kCombineWarps * 32) k_combine(CombineArgs a, int ncols) {
-  combine_body<N>(a, ncols, blockIdx.x);
+__global__ void __launch_bounds__(ColumnCta<N>::TH) k_combine(CombineArgs a) {
+  combine_body<N>(a, blockIdx.x);
 }
 
-// CTA prefix: pre[r] = sum over earlier runs of ceil(ncols_r / columns per CTA)
+// column prefix: pre[r] = sum over earlier runs of their columns
 template <int N>
-__global__ void __launch_bounds__(kCombineWarps * 32) k_combine_batch(const CombineArgs* __restrict__ args,
-                                                          const int* __restrict__ pre, int nruns) {
+__global__ void __launch_bounds__(ColumnCta<N>::TH) k_combine_batch(const CombineArgs* __restrict__ args,
+                                                                    const int* __restrict__ pre, int nruns) {
   const int r = find_run(pre, nruns, blockIdx.x);
-  const CombineArgs& a = args[r];
-  combine_body<N>(a, a.nk * a.w.nb, blockIdx.x - pre[r]);
+  combine_body<N>(args[r], blockIdx.x - pre[r]);
 }
 
 // Deferred exchange energy Ex = 0.5 sum_occ occ <u|F u> dvcell (F:165-183),
@@ -659,35 +613,9 @@ static void sym_launch_shape(int S, int* threads, size_t* smem) {
 }
 
 template <int N>
-static cudaError_t fock_sym_impl(const FockSymArgs& a, cudaStream_t s) {
-  const int tiles = a.T * (a.T + 1) / 2;
-  if (tiles == 0) return cudaSuccess;
-  int threads;
-  size_t smem;
-  sym_launch_shape<N>(a.S, &threads, &smem);
-  k_fock_sym<N><<<tiles, threads, smem, s>>>(a);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const int M = a.nk * a.nbocc;
-  k_sym_reduce<<<(M * N + kRedE - 1) / kRedE, kRedQ * kRedE, 0, s>>>(a.scratch, a.S, a.T, M, N, a.F);
-  return cudaGetLastError();
-}
-
-template <int N>
-static cudaError_t configure_impl() {
-  // the single-run and the batched symmetric exchange (above 48 KB at NG = 512)
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_fock_sym<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym_smem<N>());
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_fock_sym_batch<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym_smem<N>());
-}
-
-template <int N>
 static cudaError_t combine_impl(const CombineArgs& a, int ncols, cudaStream_t s) {
-  constexpr int PER_CTA = kCombineWarps * Team<N>::PER_WARP;
-  const int blocks = (ncols + PER_CTA - 1) / PER_CTA;
-  if (blocks == 0) return cudaSuccess;
-  k_combine<N><<<blocks, kCombineWarps * 32, 0, s>>>(a, ncols);
+  if (ncols == 0) return cudaSuccess;
+  k_combine<N><<<ncols, ColumnCta<N>::TH, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -713,12 +641,6 @@ cudaError_t launch_density(int NG, const DensArgs& a, cudaStream_t s) {
 
 cudaError_t launch_fock(int NG, const FockArgs& a, int ncols, cudaStream_t s) {
 #define CALL(n) fock_impl<n>(a, ncols, s)
-  MATTOHF_DISPATCH(NG, CALL)
-#undef CALL
-}
-
-cudaError_t launch_fock_sym(int NG, const FockSymArgs& a, cudaStream_t s) {
-#define CALL(n) fock_sym_impl<n>(a, s)
   MATTOHF_DISPATCH(NG, CALL)
 #undef CALL
 }
@@ -763,18 +685,6 @@ int fock_sym_teams(int NG) {
   }
 }
 
-// Per-device kernel attributes (larger dynamic shared memory); call with the
-// device current.
-cudaError_t configure_kernels() {
-  cudaError_t e;
-  if ((e = configure_impl<16>()) != cudaSuccess) return e;
-  if ((e = configure_impl<32>()) != cudaSuccess) return e;
-  if ((e = configure_impl<64>()) != cudaSuccess) return e;
-  if ((e = configure_impl<128>()) != cudaSuccess) return e;
-  if ((e = configure_impl<256>()) != cudaSuccess) return e;
-  return configure_impl<512>();
-}
-
 cudaError_t launch_ex_finalize(const ExArgs& a, cudaStream_t s) {
   k_ex_finalize<<<1, 32, 0, s>>>(a);
   return cudaGetLastError();
@@ -796,42 +706,10 @@ cudaError_t launch_density_batch(int NG, const DensArgs* d_args, int nruns, cuda
 #undef CALL
 }
 
-template <int N>
-static cudaError_t fock_sym_batch_impl(const FockSymArgs* d_args, const int* d_tile_pre, int nruns,
-                                       int total_tiles, const int* d_elem_pre, int total_elems,
-                                       cudaStream_t s) {
-  if (total_tiles <= 0) return cudaSuccess;
-  k_fock_sym_batch<N><<<total_tiles, kThreads, sym_smem<N>(), s>>>(d_args, d_tile_pre, nruns);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_sym_reduce_batch<<<(total_elems + kRedE - 1) / kRedE, kRedQ * kRedE, 0, s>>>(d_args, d_elem_pre, nruns, N);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_fock_sym_batch(int NG, const FockSymArgs* d_args, const int* d_tile_pre, int nruns,
-                                  int total_tiles, const int* d_elem_pre, int total_elems,
-                                  cudaStream_t s) {
-#define CALL(n) fock_sym_batch_impl<n>(d_args, d_tile_pre, nruns, total_tiles, d_elem_pre, total_elems, s)
-  MATTOHF_DISPATCH(NG, CALL)
-#undef CALL
-}
-
-int combine_cols_per_cta(int NG) {
-  switch (NG) {
-    case 16: return kCombineWarps * Team<16>::PER_WARP;
-    case 32: return kCombineWarps * Team<32>::PER_WARP;
-    case 64: return kCombineWarps * Team<64>::PER_WARP;
-    case 128: return kCombineWarps * Team<128>::PER_WARP;
-    case 256: return kCombineWarps * Team<256>::PER_WARP;
-    case 512: return kCombineWarps * Team<512>::PER_WARP;
-    default: return 0;
-  }
-}
-
-cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d_cta_pre, int nruns,
-                                 int total_ctas, cudaStream_t s) {
-  if (total_ctas <= 0) return cudaSuccess;
-#define CALL(n) (k_combine_batch<n><<<total_ctas, kCombineWarps * 32, 0, s>>>(d_args, d_cta_pre, nruns), cudaGetLastError())
+cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d_col_pre, int nruns,
+                                 int total_cols, cudaStream_t s) {
+  if (total_cols <= 0) return cudaSuccess;
+#define CALL(n) (k_combine_batch<n><<<total_cols, ColumnCta<n>::TH, 0, s>>>(d_args, d_col_pre, nruns), cudaGetLastError())
   MATTOHF_DISPATCH(NG, CALL)
 #undef CALL
 }
