@@ -145,8 +145,9 @@ struct mattohf_ctx {
   std::vector<cudaEvent_t> step_events;
   // adjoint work
   double2 *d_ckpt = nullptr, *d_store = nullptr, *d_lam = nullptr, *d_lamu = nullptr, *d_vbuf = nullptr,
-          *d_Fa = nullptr, *d_uN = nullptr, *d_u0 = nullptr;
+          *d_uN = nullptr, *d_u0 = nullptr;
   double2* d_lamk[4] = {nullptr, nullptr, nullptr, nullptr};
+  int4* d_mufx = nullptr;  // adjoint orbitals in limbs
   double *d_psi = nullptr, *d_sig = nullptr, *d_gcol = nullptr, *d_gstage = nullptr, *d_gvion = nullptr,
          *d_vloc_adj = nullptr, *d_dpart2 = nullptr;
   int* d_adj_int = nullptr;  // [0] step n, [1] segment start
@@ -333,7 +334,7 @@ int ensure_fx(mattohf_ctx* ctx) {
   if (!ctx->d_fx_sizes) CKR(dalloc(ctx, &ctx->d_fx_sizes, M));
   if (!ctx->d_fx_shift) CKR(dalloc(ctx, &ctx->d_fx_shift, M));
   if (!ctx->d_fx_fscale) CKR(dalloc(ctx, &ctx->d_fx_fscale, M));
-  if (!ctx->d_uscale) CKR(dalloc(ctx, &ctx->d_uscale, 1));
+  if (!ctx->d_uscale) CKR(dalloc(ctx, &ctx->d_uscale, 2));
   if (!ctx->d_fx_acc) CKR(dalloc(ctx, &ctx->d_fx_acc, M * 4 * ctx->NG));
   return MATTOHF_OK;
 }
@@ -355,6 +356,9 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   a.kscale = ctx->d_kscale;
   a.tw = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
   a.acc = ctx->d_fx_acc;
+  a.lift = 1;
+  a.halve = 0;
+  a.vscale = nullptr;
   return a;
 }
 
@@ -1027,7 +1031,6 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
     e = configure_fx_kernels();
-    if (e == cudaSuccess) e = configure_adjoint_kernels();
     if (e == cudaSuccess) e = configure_df_kernels();
     if (e == cudaSuccess) e = configure_small_kernels();
     if (e == cudaSuccess) e = configure_small_adj_kernels();
@@ -1082,7 +1085,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   destroy_graph(ctx);
   {
-    void* adj[] = {ctx->d_ckpt, ctx->d_store, ctx->d_lam, ctx->d_lamu, ctx->d_vbuf, ctx->d_Fa, ctx->d_uN,
+    void* adj[] = {ctx->d_ckpt, ctx->d_store, ctx->d_lam, ctx->d_lamu, ctx->d_vbuf, ctx->d_mufx, ctx->d_uN,
                    ctx->d_u0, ctx->d_lamk[0], ctx->d_lamk[1], ctx->d_lamk[2], ctx->d_lamk[3], ctx->d_psi,
                    ctx->d_sig, ctx->d_gcol, ctx->d_gstage, ctx->d_gvion, ctx->d_vloc_adj, ctx->d_dpart2,
                    ctx->d_adj_int};
@@ -1974,9 +1977,7 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
     }
     return MATTOHF_OK;
   }
-  const int M = NK * ctx->NBocc;
-  const int S = sym_tile(ctx);
-  const int T = (M + S - 1) / S;
+  const int S = fx_tile(ctx);
   const bool side = ctx->hf != 0;
   cudaStream_t ss = side ? ctx->st_side : ctx->st;
   for (int s = 3; s >= 0; --s) {
@@ -2009,12 +2010,12 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
     AdjCombineArgs c;
     c.mu = ctx->d_lamk[s];
     c.v = ctx->d_vbuf;
-    c.Fa = ctx->d_Fa;
+    c.fa = ctx->hf ? occ_source(ctx, false) : ExSource{nullptr, nullptr, nullptr};
     c.psi = ctx->d_psi;
     c.vloc = ctx->d_vloc;
     c.Gx = ctx->d_Gx;
     c.kx = ctx->d_kx;
-    c.tw = ctx->tw;
+    c.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
     c.af.mode = amodes[s];
     c.af.val = 0.0;
     c.af.A = ctx->d_A;
@@ -2039,20 +2040,29 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
       c.split = 2;
     }
     if (ctx->hf) {
-      AdjFockArgs f;
-      f.v = ctx->d_vbuf;
-      f.mu = ctx->d_lamk[s];
-      f.kstride = NB * NG;
+      FockFxArgs fv = fx_args(ctx, vb, S), fm = fx_args(ctx, blk(ctx->d_lamk[s], NB, NG, NB), S);
+      fv.lift = fm.lift = 0;
+      fv.shift = fm.shift = nullptr;
+      fv.fscale = nullptr;
+      fv.acc = nullptr;
+      fm.halve = 1;  // the second pass subtracts two pair densities
+      fm.ufx = reinterpret_cast<fx::lc*>(ctx->d_mufx);
+      fm.vscale = ctx->d_uscale;
+      fm.uscale = ctx->d_uscale + 1;
+      FockAdjFxArgs f;
+      f.v = fv.ufx;
+      f.mu = fm.ufx;
       f.nk = NK;
       f.nbocc = ctx->NBocc;
       f.S = S;
-      f.T = T;
-      f.kern = ctx->d_kern;
-      f.tw = ctx->tw;
-      f.scratch = ctx->d_sym;
+      f.T = fv.T;
+      f.kern = fv.kern;
+      f.tw = fv.tw;
+      f.acc = fm.acc;
       CKR(timed_begin(ctx));
-      CK(launch_fock_adj(NG, f, ctx->st));
-      CK(launch_sym_reduce(ctx->d_sym, S, T, M, NG, ctx->d_Fa, ctx->st));
+      CK(launch_fx_orbitals(NG, fv, ctx->st));
+      CK(launch_fx_orbitals(NG, fm, ctx->st));
+      CK(launch_fock_adj_fx(NG, f, ctx->st));
       CKR(timed_end(ctx));
     }
     if (side) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
@@ -2103,6 +2113,7 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   // (4 per step), checkpoints and work buffers fit in three quarters of the
   // free device memory.
   release_adjoint_storage(ctx);   // a previous call's segments do not count against this one
+  CKR(ensure_fock_buffers(ctx));
   size_t freeb = 0, totalb = 0;
   CK(cudaMemGetInfo(&freeb, &totalb));
   int C = ckpt_every;
@@ -2120,15 +2131,11 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   if (need > freeb) return fail(ctx, MATTOHF_ERR_ALLOC, "checkpoint storage exceeds free device memory; lower ckpt_every");
   CKR(ensure_series(ctx, nt));
   CKR(ensure_scratch(ctx, NK * NB));
-  const int M = NK * ctx->NBocc;
-  const int S = sym_tile(ctx);
-  const int T = (M + S - 1) / S;
-  CKR(ensure_sym(ctx, (size_t)T * (T + 1) / 2 * 2 * S * NG));
-  if (!ctx->d_symF) CKR(dalloc(ctx, &ctx->d_symF, (size_t)M * NG));
   destroy_graph(ctx);
+  CKR(dalloc(ctx, &ctx->d_mufx, elems));
   CKR(dalloc(ctx, &ctx->d_ckpt, elems * nseg));
   CKR(dalloc(ctx, &ctx->d_store, elems * 4 * C));
-  double2** bufs[] = {&ctx->d_lam, &ctx->d_lamu, &ctx->d_vbuf, &ctx->d_Fa, &ctx->d_uN, &ctx->d_u0,
+  double2** bufs[] = {&ctx->d_lam, &ctx->d_lamu, &ctx->d_vbuf, &ctx->d_uN, &ctx->d_u0,
                       &ctx->d_lamk[0], &ctx->d_lamk[1], &ctx->d_lamk[2], &ctx->d_lamk[3]};
   for (double2** b : bufs) CKR(dalloc(ctx, b, elems));
   CKR(dalloc(ctx, &ctx->d_psi, NG));

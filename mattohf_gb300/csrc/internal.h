@@ -130,7 +130,19 @@ struct FockFxArgs {
   const int2* kscale;   // its scale (c, k)
   const fx::lc* tw;
   unsigned long long* acc;  // [NK*nbocc][4][NG] sums F^ (fx_accumulate), zeroed by the conversion
+  // conversions for the adjoint (shift, fscale, acc may be null there): no lifting,
+  // a further 2^-halve in the scale, and the scale of v for mu's output scale
+  int lift, halve;
+  const int2* vscale;
 };
+struct FockAdjFxArgs {
+  const fx::lc *v, *mu;     // [NK*nbocc][NG] in limbs (FockFxArgs::ufx of two conversions)
+  int nk, nbocc, S, T;
+  const int2* kern;
+  const fx::lc* tw;
+  unsigned long long* acc;  // sums, as FockFxArgs::acc
+};
+cudaError_t launch_fock_adj_fx(int NG, const FockAdjFxArgs& a, cudaStream_t s);
 // Functions w that the exchange operator of the orbitals acts on.
 struct FockFxRows {
   Block w;
@@ -384,24 +396,15 @@ cudaError_t launch_ex_finalize_batch(const ExArgs* d_args, int nruns, cudaStream
 cudaError_t launch_step_advance(int* it, cudaStream_t s);
 
 // ---- adjoint (k_adjoint.cu) ----
-struct AdjFockArgs {
-  const double2* v;     // stage input [NK][NB][NG]
-  const double2* mu;    // adjoint of the stage derivative, same layout
-  int kstride;          // NB * NG
-  int nk, nbocc, S, T;
-  const double* kern;
-  const double2* tw;
-  double2* scratch;     // tile partials, as FockSymArgs
-};
 struct AdjCombineArgs {
   const double2* mu;
   const double2* v;
-  const double2* Fa;    // reduced exchange part of J^T mu (includes the factor i)
+  ExSource fa;          // exchange part of J^T mu without its factor i
   const double* psi;    // vH[sigma]
   const double* vloc;   // vH[rho(v)] + vion
   const double* Gx;
   const double* kx;
-  const double2* tw;
+  const fx::lc* twfx;
   AField af;
   int nb;
   double occ;
@@ -418,9 +421,6 @@ struct AdjCombineArgs {
   int split;
   double2* lpre;        // [NK][NB][NG]
 };
-cudaError_t launch_fock_adj(int NG, const AdjFockArgs& a, cudaStream_t s);
-cudaError_t configure_adjoint_kernels();
-cudaError_t launch_sym_reduce(const double2* part, int S, int T, int M, int N, double2* F, cudaStream_t s);
 cudaError_t launch_adj_combine(int NG, const AdjCombineArgs& a, int ncols, cudaStream_t s);
 cudaError_t launch_adj_init(const double2* lam, double2* lam_u, double2* const* lamk, double dt, size_t n,
                             cudaStream_t s);

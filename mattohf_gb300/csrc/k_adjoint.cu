@@ -15,10 +15,11 @@
 // Nyquist index N/2, where it stays kern_ji.  So
 //   Phi~_ji[f] = Phi_ij[f] + dk_ij Nyq(f) (-1)^m,  dk_ij = kern_ji[N/2] - kern_ij[N/2],
 // Nyq(f) = sum_m (-1)^m f(m) the Nyquist coefficient of the forward transform.
-// k_fock_adj evaluates the two exchange sums over unordered occupied pairs
+// k_fock_adj_fx (k_fock_fx.cu) evaluates the two exchange sums over unordered occupied pairs
 // with two transform pairs per pair (pair densities v_i conj(v_j) and
 // mu_i conj(v_j) - v_i conj(mu_j)), using the same conjugate-plus-Nyquist
 // relation as the forward symmetric kernel.
+#include "column_fx.cuh"
 #include "fft.cuh"
 #include "internal.h"
 
@@ -26,214 +27,106 @@ namespace mattohf {
 
 __device__ __forceinline__ double2 mul_i(double2 a) { return make_double2(-a.y, a.x); }
 
-template <int N>
-__global__ void __launch_bounds__(kThreads) k_fock_adj(AdjFockArgs a) {
-  using TM = Team<N>;
-  constexpr int E = TM::E, T = TM::T, PW = TM::PER_WARP;
-  const int S = a.S;
-  const int nteam = (blockDim.x >> 5) * PW;
-  extern __shared__ double2 sm[];
-  double2* tw_s = sm;
-  double2* bufs = sm + N;
-  double2* cacc = bufs + nteam * N;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tl = lane % T, tw_ = warp * PW + lane / T;
-  const int team_lane0 = (lane / T) * T;
-  double2* buf = bufs + tw_ * N;
-  for (int i = tid; i < N; i += blockDim.x) tw_s[i] = a.tw[i];
-  for (int i = tid; i < S * N; i += blockDim.x) cacc[i] = make_double2(0.0, 0.0);
-  int ti = 0, rem = blockIdx.x;
-  while (rem >= a.T - ti) { rem -= a.T - ti; ++ti; }
-  const int tj = ti + rem;
-  const int M = a.nk * a.nbocc;
-  const int ia = ti * S + tw_;
-  const bool va = tw_ < S && ia < M;
-  const int ka = (va ? ia : 0) / a.nbocc, ba = (va ? ia : 0) % a.nbocc;
-  const size_t oa = (size_t)ka * a.kstride + (size_t)ba * N;
-  // orbitals and adjoints are re-read (L1/L2) where needed instead of held in
-  // registers (the kernel is FP64-pipe bound; this avoids spills at NG=512)
-  const double2* vA = a.v + oa;
-  const double2* mA = a.mu + oa;
-  double2 racc[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) racc[e] = make_double2(0.0, 0.0);
-  __syncthreads();
-  const bool diag = (ti == tj);
-  const int nrounds = diag ? (S / 2 + 1) : S;
-  for (int r = 0; r < nrounds; ++r) {
-    const int lb = (tw_ + r) % S;
-    const int ib = tj * S + lb;
-    bool valid = va && ib < M;
-    if (diag && (S % 2 == 0) && r == S / 2 && tw_ >= S / 2) valid = false;
-    const bool self = diag && r == 0;
-    const int kb = (ib < M ? ib : 0) / a.nbocc, bb = (ib < M ? ib : 0) % a.nbocc;
-    const size_t ob = (size_t)kb * a.kstride + (size_t)bb * N;
-    const int dab = ka - kb + a.nk - 1, dba = kb - ka + a.nk - 1;
-    const double* kab = a.kern + (size_t)dab * N;
-    const double dk = __ldg(a.kern + (size_t)dba * N + N / 2) - __ldg(kab + N / 2);
-    const double2* vB = a.v + ob;
-    const double2* mB = a.mu + ob;
-    double2 x[E];
-    // ---- pass A: phi_ab = Phi_ab[v_a conj(v_b)]
-    fft_team_in<N, -1>(InConjProduct<N>{vA, vB, tl}, x, buf, tw_s, tl);
-    const double rnx = __shfl_sync(0xffffffffu, x[TM::R0 / 2].x, team_lane0);
-    const double rny = __shfl_sync(0xffffffffu, x[TM::R0 / 2].y, team_lane0);
-    fft_team_in<N, +1>(InScaled<N>{x, kab, tl}, x, buf, tw_s, tl);
-    if (valid) {
-      if (self) {
-        // out_a += i conj(phi_aa) mu_a
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-          racc[e] = cadd(racc[e], mul_i(cmul(make_double2(x[e].x, -x[e].y), mA[TM::pos(tl, e)])));
-      } else {
-        // c = dk * conj(R); out_a += i (phi_ab + conj(c)(-1)^m) mu_b ; out_b += i conj(phi_ab) mu_a
-        const double cx = dk * rnx, cy = -dk * rny;
-        double2* col = cacc + lb * N;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int q = TM::pos(tl, e);
-          const double sg = (q & 1) ? -1.0 : 1.0;
-          const double2 pr = make_double2(fma(sg, cx, x[e].x), fma(-sg, cy, x[e].y));
-          racc[e] = cadd(racc[e], mul_i(cmul(pr, mB[q])));
-          col[q] = cadd(col[q], mul_i(cmul(make_double2(x[e].x, -x[e].y), mA[q])));
-        }
-      }
-    }
-    // ---- pass B: phi'_ab = Phi_ab[mu_a conj(v_b) - v_a conj(mu_b)], and
-    //      n2 = Nyq(v_a conj(mu_b)) for the transposed operator's Nyquist term
-    double n2x = 0.0, n2y = 0.0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int q = TM::pos(tl, e);
-      const double sg = (q & 1) ? -1.0 : 1.0;
-      const double2 t2 = cmulc(vA[q], mB[q]);
-      x[e] = csub(cmulc(mA[q], vB[q]), t2);
-      n2x = fma(sg, t2.x, n2x);
-      n2y = fma(sg, t2.y, n2y);
-    }
-    n2x = team_sum<T>(n2x);
-    n2y = team_sum<T>(n2y);
-    fft_team<N, -1>(x, buf, tw_s, tl);
-    fft_team_in<N, +1>(InScaled<N>{x, kab, tl}, x, buf, tw_s, tl);
-    if (valid) {
-      // y = Phi_ab[mu_a conj(v_b)] - Phi~_ba[v_a conj(mu_b)] = phi'_ab - dk n2 (-1)^m;
-      // out_a += i v_b y.  The pair's reversed term is its mirror image:
-      // Phi_ba[mu_b conj(v_a)] - Phi~_ab[v_b conj(mu_a)] = -conj(y), so
-      // out_b += i v_a (-conj(y)).  (dk = 0 on the diagonal.)
-      const double cx = dk * n2x, cy = dk * n2y;
-      double2* col = cacc + lb * N;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int q = TM::pos(tl, e);
-        const double sg = (q & 1) ? -1.0 : 1.0;
-        const double2 y = make_double2(fma(-sg, cx, x[e].x), fma(-sg, cy, x[e].y));
-        racc[e] = cadd(racc[e], mul_i(cmul(vB[q], y)));
-        if (!self) col[q] = cadd(col[q], mul_i(cmul(vA[q], make_double2(-y.x, y.y))));
-      }
-    }
-    __syncthreads();
-  }
-  double2* dst = a.scratch + (size_t)blockIdx.x * 2 * S * N;
-  if (tw_ < S) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) dst[(size_t)tw_ * N + TM::pos(tl, e)] = racc[e];
-  }
-  for (int i = tid; i < S * N; i += blockDim.x) dst[(size_t)S * N + i] = cacc[i];
-}
-
-// Adjoint combine of one RK4 stage, one team per column:
-//   lu   = i (T_a + vloc) mu + Fa + 2 occ psi v
+// Adjoint combine of one RK4 stage, one CTA per column (fixed-point transforms on
+// the first team, FP64 spread over the threads, as combine_body of k_hpsi.cu):
+//   lu   = i (T_a + vloc) mu + i fa + 2 occ psi v
 //   g_a += sum_G (G+k+a) Im(conj(FFT mu) FFT v) / N     (field gradient partial)
 //   lam_u += lu ; lam_prev += c_prev * lu               (RK4 stage bookkeeping)
 template <int N>
-__global__ void __launch_bounds__(kThreads) k_adj_combine(AdjCombineArgs a, int ncols) {
-  using TM = Team<N>;
-  constexpr int E = TM::E, T = TM::T, PW = TM::PER_WARP;
-  constexpr int NTEAM = (kThreads / 32) * PW;
-  __shared__ double2 tw_s[N];
-  __shared__ double2 bufs[NTEAM][N];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tl = lane % T, team = warp * PW + lane / T;
-  for (int i = tid; i < N; i += kThreads) tw_s[i] = a.tw[i];
-  __syncthreads();
-  const double A = afield_value(a.af);
-  const int col0 = (blockIdx.x * (kThreads / 32) + warp) * PW;
-  if (col0 >= ncols) return;
-  const int col = col0 + lane / T;
-  const bool valid = col < ncols;
-  const int c = valid ? col : col0;
+__global__ void __launch_bounds__(ColumnCta<N>::TH) k_adj_combine(AdjCombineArgs a) {
+  using CC = ColumnCta<N>;
+  constexpr int TH = CC::TH, PER = CC::PER, NW = CC::NW;
+  __shared__ FxTwiddles<N> tw_s;
+  __shared__ cx buf[N];
+  __shared__ int red[2 * NW];
+  __shared__ double redd[NW];
+  const int tid = threadIdx.x, c = blockIdx.x;
   const int ik = c / a.nb;
   const size_t o = (size_t)c * N;
-  if (a.split == 2) {
-    if (!valid) return;
+  const bool in = tid < N;
+  double2 mu[PER], v[PER], lu[PER];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int q = TM::pos(tl, e);
-      double2 lu = cadd(a.lpre[o + q], a.Fa[o + q]);
-      const double ps = 2.0 * a.occ * a.psi[q];
-      const double2 vv = a.v[o + q];
-      lu = make_double2(fma(ps, vv.x, lu.x), fma(ps, vv.y, lu.y));
-      a.lam_u[o + q] = cadd(a.lam_u[o + q], lu);
-      if (a.lam_prev) {
-        const double2 p = a.lam_prev[o + q];
-        a.lam_prev[o + q] = make_double2(fma(a.cprev, lu.x, p.x), fma(a.cprev, lu.y, p.y));
-      }
+  for (int p = 0; p < PER; ++p) {
+    const int q = tid + TH * p;
+    mu[p] = in && a.split != 2 ? a.mu[o + q] : make_double2(0.0, 0.0);
+    v[p] = in ? a.v[o + q] : make_double2(0.0, 0.0);
+    lu[p] = in && a.split == 2 ? a.lpre[o + q] : make_double2(0.0, 0.0);
+  }
+  if (a.split != 2) {
+    const double A = afield_value(a.af);
+    const double kAx = a.kx[ik] + A, kA2 = kAx * kAx;
+    tw_s.load(a.twfx);
+    int2 z = fx_block_size<PER, NW>(v, red);
+    const Scale sv = fx_fft_scale(z, N);
+    if (in) {
+#pragma unroll
+      for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(v[p].x, sv), fx_convert(v[p].y, sv)};
     }
-    return;
-  }
-  double2 mu[E], v[E], x[E];
+    fx_block_forward<N>(buf, tw_s);
+    cx vf[PER];
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int q = TM::pos(tl, e);
-    mu[e] = a.mu[o + q];
-    v[e] = a.v[o + q];
-    x[e] = mu[e];
-  }
-  fft_team<N, -1>(x, bufs[team], tw_s, tl);
-  // field-gradient partial needs FFT(v) too
-  double2 vf[E];
+    for (int p = 0; p < PER; ++p) vf[p] = in ? buf[tid + TH * p] : cx{0, 0};
+    z = fx_block_size<PER, NW>(mu, red);  // its barriers also separate the reads above from the writes below
+    const Scale s1 = fx_fft_scale(z, N);
+    if (in) {
 #pragma unroll
-  for (int e = 0; e < E; ++e) vf[e] = v[e];
-  fft_team<N, -1>(vf, bufs[team], tw_s, tl);
-  const double kAx = a.kx[ik] + A, kA2 = kAx * kAx;
-  double gp = 0.0;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const double G = a.Gx[TM::pos(tl, e)];
-    gp += (G + a.kx[ik] + A) * (x[e].x * vf[e].y - x[e].y * vf[e].x);
-    const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2);
-    x[e] = make_double2(m * x[e].x / (double)N, m * x[e].y / (double)N);
-  }
-  gp = team_sum<T>(gp) / (double)N;
-  fft_team<N, +1>(x, bufs[team], tw_s, tl);
-  if (valid && tl == 0) a.gcol[c] = gp;
-  if (!valid) return;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int q = TM::pos(tl, e);
-    const double vl = a.vloc[q];
-    double2 lu = mul_i(make_double2(x[e].x + vl * mu[e].x, x[e].y + vl * mu[e].y));
-    if (a.split == 1) {
-      a.lpre[o + q] = lu;
-      continue;
+      for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(mu[p].x, s1), fx_convert(mu[p].y, s1)};
     }
-    lu = cadd(lu, a.Fa[o + q]);
+    fx_block_forward<N>(buf, tw_s);
+    const double u1 = fx_unscale(s1), uv = fx_unscale(sv);
+    double gp = 0.0;
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      if (!in) continue;
+      const int q = tid + TH * p;
+      const double G = a.Gx[q];
+      const double mx = (double)buf[q].x * u1, my = (double)buf[q].y * u1;
+      gp += (G + a.kx[ik] + A) * (mx * ((double)vf[p].y * uv) - my * ((double)vf[p].x * uv));
+      const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2) * (1.0 / N);
+      lu[p] = make_double2(m * mx, -m * my);  // conjugate: backward next
+    }
+    gp = block_sum<NW>(gp, redd) / (double)N;
+    if (tid == 0) a.gcol[c] = gp;
+    z = fx_block_size<PER, NW>(lu, red);
+    const Scale s2 = fx_fft_scale(z, N);
+    if (in) {
+#pragma unroll
+      for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(lu[p].x, s2), fx_convert(lu[p].y, s2)};
+    }
+    fx_block_forward<N>(buf, tw_s);
+    const double u2 = fx_unscale(s2);
+    if (!in) return;
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int q = tid + TH * p;
+      const double vl = a.vloc[q];
+      lu[p] = mul_i(make_double2((double)buf[q].x * u2 + vl * mu[p].x, (double)buf[q].y * -u2 + vl * mu[p].y));
+      if (a.split == 1) a.lpre[o + q] = lu[p];
+    }
+    if (a.split == 1) return;
+  }
+  if (!in) return;
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int q = tid + TH * p;
+    double2 l = lu[p];
+    if (a.fa.acc != nullptr) l = cadd(l, mul_i(exchange_value(a.fa, c, q, N)));
     const double ps = 2.0 * a.occ * a.psi[q];
-    lu = make_double2(fma(ps, v[e].x, lu.x), fma(ps, v[e].y, lu.y));
-    a.lam_u[o + q] = cadd(a.lam_u[o + q], lu);
+    l = make_double2(fma(ps, v[p].x, l.x), fma(ps, v[p].y, l.y));
+    a.lam_u[o + q] = cadd(a.lam_u[o + q], l);
     if (a.lam_prev) {
-      const double2 p = a.lam_prev[o + q];
-      a.lam_prev[o + q] = make_double2(fma(a.cprev, lu.x, p.x), fma(a.cprev, lu.y, p.y));
+      const double2 lp = a.lam_prev[o + q];
+      a.lam_prev[o + q] = make_double2(fma(a.cprev, l.x, lp.x), fma(a.cprev, l.y, lp.y));
     }
   }
 }
 
-// Ordered sum of the per-column field-gradient partials into g[slot].
+// Sum of the per-column field-gradient partials into g[slot] (one warp, fixed order).
 __global__ void k_adj_gsum(const double* __restrict__ gcol, int ncols, double* g, const int* n, int s) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double acc = 0.0;
-  for (int i = 0; i < ncols; ++i) acc += gcol[i];
-  g[(size_t)(*n) * 4 + s] = acc;
+  for (int i = threadIdx.x; i < ncols; i += 32) acc += gcol[i];
+  acc = warp_sum(acc);
+  if (threadIdx.x == 0) g[(size_t)(*n) * 4 + s] = acc;
 }
 
 // lam_k[s] = w_s lam (w = dt/6, dt/3, dt/3, dt/6); lam_u = lam.
@@ -330,45 +223,8 @@ __global__ void k_scale2(double2* x, double s, size_t n) {
   }
 
 template <int N>
-static size_t adj_smem() { return sizeof(double2) * (size_t)N * (1 + 2 * (kThreads / 32) * Team<N>::PER_WARP); }
-
-template <int N>
-static cudaError_t fock_adj_impl(const AdjFockArgs& a, cudaStream_t s) {
-  const int tiles = a.T * (a.T + 1) / 2;
-  if (tiles == 0) return cudaSuccess;
-  int threads;
-  size_t smem;
-  cudaError_t e = sym_launch_params(N, a.S, &threads, &smem);
-  if (e != cudaSuccess) return e;
-  k_fock_adj<N><<<tiles, threads, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-template <int N>
-static cudaError_t configure_adj_impl() {
-  return cudaFuncSetAttribute(k_fock_adj<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem<N>());
-}
-
-cudaError_t configure_adjoint_kernels() {
-  cudaError_t e;
-  if ((e = configure_adj_impl<16>()) != cudaSuccess) return e;
-  if ((e = configure_adj_impl<32>()) != cudaSuccess) return e;
-  if ((e = configure_adj_impl<64>()) != cudaSuccess) return e;
-  if ((e = configure_adj_impl<128>()) != cudaSuccess) return e;
-  if ((e = configure_adj_impl<256>()) != cudaSuccess) return e;
-  return configure_adj_impl<512>();
-}
-
-cudaError_t launch_fock_adj(int NG, const AdjFockArgs& a, cudaStream_t s) {
-#define CALL(n) fock_adj_impl<n>(a, s)
-  MATTOHF_DISPATCH(NG, CALL)
-#undef CALL
-}
-
-template <int N>
 static cudaError_t adj_combine_impl(const AdjCombineArgs& a, int ncols, cudaStream_t s) {
-  constexpr int PER_CTA = (kThreads / 32) * Team<N>::PER_WARP;
-  k_adj_combine<N><<<(ncols + PER_CTA - 1) / PER_CTA, kThreads, 0, s>>>(a, ncols);
+  k_adj_combine<N><<<ncols, ColumnCta<N>::TH, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || a.split == 2) return e;  // the field-gradient partials come from the other passes
   k_adj_gsum<<<1, 32, 0, s>>>(a.gcol, ncols, a.gstage, a.n, a.slot);

@@ -92,20 +92,24 @@ __device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, int N, int 
       n2 = fmaxf(n2, __int_as_float(ownc[w].y));
     }
     const int e = m >> 20;
-    const Scale s = fx_scale(m, g2, fx_mantissa(m, e), kSquareMax);
+    Scale s = fx_scale(m, g2, fx_mantissa(m, e), kSquareMax);
+    s.k -= a.halve;
     // a column with less than half the largest norm is lifted by 2^d
     const int dc = (mc >> 20) - e;
     int d = 0;
-    if (n2 > 0.0f) {
+    if (n2 > 0.0f && a.lift) {
       const int lg = ilogbf(g2) - ilogbf(n2) - 2 * dc;  // log2 of the squared norms' ratio, to 1
       if (lg > 2) d = min(60, (lg - 1) >> 1);
     }
     const Scale sd{s.c, s.k + d};
     out = sd;
-    a.shift[col] = d;
+    if (a.shift) a.shift[col] = d;
     if (col == 0) *a.uscale = make_int2(s.c, s.k);
-    // a column of zeros has a sum of zero; the roundings of its terms do not count
-    a.fscale[col] = n2 > 0.0f || s.c == 0 ? fx_output_scale(s, sd, Scale{a.kscale->x, a.kscale->y}) : make_double2(0.0, 0.0);
+    if (a.fscale) {
+      const Scale so = a.vscale ? Scale{a.vscale->x, a.vscale->y} : s;
+      // a column of zeros has a sum of zero; the roundings of its terms do not count
+      a.fscale[col] = n2 > 0.0f || s.c == 0 || a.vscale ? fx_output_scale(so, sd, Scale{a.kscale->x, a.kscale->y}) : make_double2(0.0, 0.0);
+    }
   }
   __syncthreads();
   const Scale sd = out;
@@ -116,6 +120,7 @@ __device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, int N, int 
     const double2 z = p[i];
     o[i] = ok ? fx::limbs(cx{fx_convert(z.x, sd), fx_convert(z.y, sd)}) : lc{0, 0, 0, 0};
   }
+  if (a.acc == nullptr) return;
   unsigned long long* acc = a.acc + (size_t)col * 4 * N;
   for (int i = tid; i < 4 * N; i += 128) acc[i] = 0;
 }
@@ -160,20 +165,14 @@ __device__ __forceinline__ void fx_accumulate(unsigned long long* acc, int N, in
   atomicAdd(acc + 3 * N + q, (unsigned long long)(unsigned)v.y);
 }
 
-// x = conj(phi_ab) of the pair (a, b); returns R_ab[N/2], the transform of the
-// pair density at the self-aliased frequency.
+// x: pair density in, conj(its potential) out; returns the density's transform at
+// the self-aliased frequency N/2.
 template <int N>
-__device__ __forceinline__ cx pair_potential(cx (&x)[fx::Team<N>::E], const lc* __restrict__ ua,
-                                             const lc* __restrict__ ub, const int2* __restrict__ kab, cx* buf,
-                                             const lc* tw_s, const int2* twn_s, int tl, int team) {
+__device__ __forceinline__ cx potential(cx (&x)[fx::Team<N>::E], const int2* __restrict__ kab, cx* buf,
+                                        const lc* tw_s, const int2* twn_s, int tl, int team) {
   using TM = fx::Team<N>;
   constexpr int E = TM::E, T = TM::T;
   cx rn{0, 0};
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int q = TM::pos(tl, e);
-    x[e] = fx::cmulc(ua[q], ub[q]);
-  }
   // forward transform, kernel product, backward transform of the conjugate
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
@@ -196,6 +195,19 @@ __device__ __forceinline__ cx pair_potential(cx (&x)[fx::Team<N>::E], const lc* 
     const int lane0 = (threadIdx.x & 31) / T * T;
     return cx{__shfl_sync(0xffffffffu, rn.x, lane0), __shfl_sync(0xffffffffu, rn.y, lane0)};
   }
+}
+// the same for the density of the pair (a, b): x = conj(phi_ab)
+template <int N>
+__device__ __forceinline__ cx pair_potential(cx (&x)[fx::Team<N>::E], const lc* __restrict__ ua,
+                                             const lc* __restrict__ ub, const int2* __restrict__ kab, cx* buf,
+                                             const lc* tw_s, const int2* twn_s, int tl, int team) {
+  using TM = fx::Team<N>;
+#pragma unroll
+  for (int e = 0; e < TM::E; ++e) {
+    const int q = TM::pos(tl, e);
+    x[e] = fx::cmulc(ua[q], ub[q]);
+  }
+  return potential<N>(x, kab, buf, tw_s, twn_s, tl, team);
 }
 
 // Twiddles to shared memory: tw_s, and the negated imaginary parts to twn_s.
@@ -393,6 +405,128 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_fock_fx(FockFxArgs a, FockF
   for (int e = 0; e < E; ++e) fx_accumulate(dst, N, TM::pos(tl, e), acc[e]);
 }
 
+// ---------------------------------------------------------------------------
+// Adjoint of the exchange (k_adjoint.cu has the formulas): tile pairs as
+// k_fock_sym_fx, two transform pairs per pair of orbitals.  v and mu have one
+// scale each, without lifting small columns: the two pair densities of the second
+// pass are subtracted, and a gradient takes absolute errors.  The factor i is left
+// to the combine.  Bounded like the forward kernel; a gradient over 3 steps at
+// NG = 256, NK = 32, Nocc = 4 went from 10.3 to 5.1 ms with it and the column-wise
+// combine (13.1 ms with the forward exchange in FP64 as well).
+// ---------------------------------------------------------------------------
+template <int N>
+__global__ void __launch_bounds__(sym_fx_threads<N>(), 2) k_fock_adj_fx(FockAdjFxArgs a) {
+  using TM = fx::Team<N>;
+  constexpr int E = TM::E, T = TM::T;
+  const int S = a.S;
+  const int nteam = blockDim.x / T;
+  extern __shared__ int4 sm_fx[];
+  lc* tw_s = reinterpret_cast<lc*>(sm_fx);                 // kTwCount
+  cx* bufs = reinterpret_cast<cx*>(sm_fx + TM::kTwCount);  // nteam * N
+  cx* cacc = bufs + nteam * N;                             // S * N
+  const int tid = threadIdx.x, tl = tid % T, tw_ = tid / T;
+  cx* buf = bufs + tw_ * N;
+  int2* twn_s = reinterpret_cast<int2*>(cacc + S * N);  // kTwCount
+  load_twiddles<N>(a.tw, tw_s, twn_s);
+  for (int i = tid; i < S * N; i += blockDim.x) cacc[i] = cx{0, 0};
+  int ti = 0, rem = blockIdx.x;
+  while (rem >= a.T - ti) { rem -= a.T - ti; ++ti; }
+  const int tj = ti + rem;
+  const int M = a.nk * a.nbocc;
+  const int ia = ti * S + tw_;
+  const bool va = tw_ < S && ia < M;
+  const int oa = va ? ia : 0;
+  const int ka = oa / a.nbocc;
+  const lc* vA = a.v + (size_t)oa * N;
+  const lc* mA = a.mu + (size_t)oa * N;
+  cx racc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) racc[e] = cx{0, 0};
+  __syncthreads();
+  const bool diag = (ti == tj);
+  const int nrounds = diag ? (S / 2 + 1) : S;
+  for (int r = 0; r < nrounds; ++r) {
+    const int lb = (tw_ + r) % S;
+    const int ib = tj * S + lb;
+    bool valid = va && ib < M;
+    if (diag && (S % 2 == 0) && r == S / 2 && tw_ >= S / 2) valid = false;
+    const bool self = diag && r == 0;
+    const int ob = ib < M ? ib : 0;
+    const int kb = ob / a.nbocc;
+    const lc* vB = a.v + (size_t)ob * N;
+    const lc* mB = a.mu + (size_t)ob * N;
+    const int2* kab = a.kern + (size_t)(ka - kb + a.nk - 1) * N;
+    const int2 kba = __ldg(a.kern + (size_t)(kb - ka + a.nk - 1) * N + N / 2), kn = __ldg(kab + N / 2);
+    cx* col = cacc + lb * N;
+    cx x[E];
+    // ---- pass A: x = conj(phi_ab), c = dk conj(R_ab) (-1)^m;
+    //      out_a += conj(x + c) mu_b, out_b += x mu_a (on the diagonal out_a += x mu_a)
+    {
+      const cx rn = pair_potential<N>(x, vA, vB, kab, buf, tw_s, twn_s, tl, tw_);
+      if (valid) {
+        if (self) {
+#pragma unroll
+          for (int e = 0; e < E; ++e) racc[e] = fx::add(racc[e], fx::cmul(fx::limbs(x[e]), mA[TM::pos(tl, e)]));
+        } else {
+          cx c{fx::rmul(rn.x, kba) - fx::rmul(rn.x, kn), fx::rmul(rn.y, kn) - fx::rmul(rn.y, kba)};
+          if (tl & 1) c = cx{-c.x, -c.y};
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int q = TM::pos(tl, e);
+            racc[e] = fx::add(racc[e], fx::cmulc(mB[q], fx::limbs(fx::add(x[e], c))));
+            col[q] = fx::add(col[q], fx::cmul(fx::limbs(x[e]), mA[q]));
+          }
+        }
+      }
+    }
+    // ---- pass B: x = conj(Phi_ab[mu_a conj(v_b) - v_a conj(mu_b)]),
+    //      n2 = sum_m (-1)^m v_a conj(mu_b); conj(y) = x - dk conj(n2) (-1)^m;
+    //      out_a += v_b y, out_b -= v_a conj(y)
+    cx n2{0, 0};
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int q = TM::pos(tl, e);
+      const cx t = fx::cmulc(vA[q], mB[q]);
+      x[e] = fx::sub(fx::cmulc(mA[q], vB[q]), t);
+      n2 = fx::add(n2, t);
+    }
+    if (tl & 1) n2 = cx{-n2.x, -n2.y};
+#pragma unroll
+    for (int o = (T < 32 ? T : 32) / 2; o > 0; o >>= 1) {
+      n2.x += __shfl_xor_sync(0xffffffffu, n2.x, o);
+      n2.y += __shfl_xor_sync(0xffffffffu, n2.y, o);
+    }
+    if constexpr (T > 32) {
+      fx::team_sync<T>(tw_);
+      if ((tl & 31) == 0) buf[tl >> 5] = n2;
+      fx::team_sync<T>(tw_);
+      n2 = fx::add(buf[0], buf[1]);
+    }
+    potential<N>(x, kab, buf, tw_s, twn_s, tl, tw_);
+    if (valid) {
+      cx c{fx::rmul(n2.x, kn) - fx::rmul(n2.x, kba), fx::rmul(n2.y, kba) - fx::rmul(n2.y, kn)};  // -dk conj(n2)
+      if (tl & 1) c = cx{-c.x, -c.y};
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int q = TM::pos(tl, e);
+        const lc y = fx::limbs(fx::add(x[e], c));
+        racc[e] = fx::add(racc[e], fx::cmulc(vB[q], y));
+        if (!self) col[q] = fx::sub(col[q], fx::cmul(y, vA[q]));
+      }
+    }
+    __syncthreads();
+  }
+  if (va) {
+    unsigned long long* dst = a.acc + (size_t)ia * 4 * N;
+#pragma unroll
+    for (int e = 0; e < E; ++e) fx_accumulate(dst, N, TM::pos(tl, e), racc[e]);
+  }
+  for (int i = tid; i < S * N; i += blockDim.x) {
+    const int ib = tj * S + i / N;
+    if (ib < M) fx_accumulate(a.acc + (size_t)ib * 4 * N, N, i % N, cacc[i]);
+  }
+}
+
 // Kernel table: K^ = kern s_k, with s_k the largest short factor that keeps
 // sum_G |K^(G)| below 2^60 for every k - k'.
 __global__ void __launch_bounds__(1024) k_fx_kern_scale(const double* __restrict__ kern, int nd, int N, int2* kscale) {
@@ -537,6 +671,22 @@ int fx_rows_teams(int NG) {
   }
 }
 
+template <int N>
+static cudaError_t fock_adj_fx_impl(const FockAdjFxArgs& a, cudaStream_t s) {
+  int threads;
+  size_t smem;
+  sym_fx_shape<N>(a.S, &threads, &smem);
+  k_fock_adj_fx<N><<<a.T * (a.T + 1) / 2, threads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fock_adj_fx(int NG, const FockAdjFxArgs& a, cudaStream_t s) {
+  if (a.T <= 0) return cudaSuccess;
+#define CALL(n) fock_adj_fx_impl<n>(a, s)
+  MATTOHF_DISPATCH(NG, CALL)
+#undef CALL
+}
+
 cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int2* out, cudaStream_t s) {
   k_fx_kern_scale<<<1, 1024, 0, s>>>(kern, nd, NG, kscale);
   cudaError_t e = cudaGetLastError();
@@ -583,6 +733,8 @@ static cudaError_t configure_fx_impl() {
   sym_fx_shape<N>(sym_fx_threads<N>() / fx::Team<N>::T, &threads, &smem);
   const cudaError_t e = cudaFuncSetAttribute(k_fock_sym_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
+  const cudaError_t e1 = cudaFuncSetAttribute(k_fock_adj_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e1 != cudaSuccess) return e1;
   const cudaError_t e2 =
       cudaFuncSetAttribute(k_fock_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_fx_smem<N>());
   if (e2 != cudaSuccess) return e2;

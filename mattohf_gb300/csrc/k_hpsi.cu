@@ -6,17 +6,10 @@
 // (F:94-119), ubk_Ex (F:165-183), ubk_Je (F:289-318); RK4 stages from
 // src/RT_calculation.f90:154-173.
 #include "fft.cuh"
-#include "fx_convert.cuh"
+#include "column_fx.cuh"
 #include "internal.h"
 
 namespace mattohf {
-
-// Fixed xor-shuffle tree over the 32 lanes of a warp (deterministic order).
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // ---------------------------------------------------------------------------
 // Density (F:55-71) and Hartree potential (F:147-162), one CTA.
@@ -53,47 +46,6 @@ __global__ void __launch_bounds__(256) k_dens_partial(DensArgs a, int N) { dens_
 __global__ void __launch_bounds__(256) k_dens_partial_batch(const DensArgs* __restrict__ args, int N) {
   dens_partial_body(args[blockIdx.y], N, blockIdx.x);
 }
-
-// Twiddles in shared memory (fixed point), loaded by the whole CTA.
-template <int N>
-struct FxTwiddles {
-  lc w[fx::Team<N>::kTwCount];
-  int2 n[fx::Team<N>::kTwCount];
-  __device__ __forceinline__ void load(const lc* __restrict__ tw) {
-    for (int i = threadIdx.x; i < fx::Team<N>::kTwCount; i += blockDim.x) {
-      const lc v = tw[i];
-      w[i] = v;
-      n[i] = make_int2(fx::neg_hi(v.yh), fx::neg_lo(v.yl));
-    }
-  }
-};
-
-// Transform of buf (N fixed-point values) in place by the CTA's first team; every
-// thread calls it, with buf complete, and finds it complete.
-template <int N>
-__device__ __forceinline__ void fx_block_forward(cx* buf, const FxTwiddles<N>& tw) {
-  using TM = fx::Team<N>;
-  __syncthreads();
-  const int tl = threadIdx.x;
-  if (tl < TM::T) {
-    cx x[TM::E];
-#pragma unroll
-    for (int e = 0; e < TM::E; ++e) x[e] = buf[TM::pos(tl, e)];
-    fx::forward<N, true>(x, buf, tw.w, tw.n, tl, 0);
-    fx::team_sync<TM::T, true>(0);
-#pragma unroll
-    for (int e = 0; e < TM::E; ++e) buf[TM::pos(tl, e)] = x[e];
-  }
-  __syncthreads();
-}
-
-// Threads of a CTA that holds one column of N values, and values per thread.
-template <int N>
-struct ColumnCta {
-  static constexpr int TH = N < 32 ? 32 : N > 128 ? 128 : N;
-  static constexpr int PER = N > TH ? N / TH : 1;
-  static constexpr int NW = TH / 32;
-};
 
 // Stage 2 (one CTA): rho = ordered sum of the chunk partials, then the
 // Hartree potential (F:147-162), vloc = vH + vion and the density scalars.
@@ -237,53 +189,6 @@ __global__ void __launch_bounds__(kThreads) k_fock(FockArgs a) {
 }
 
 
-// Sum the tile-pair partials of every occupied output into F[o][q] (fixed
-// order over tiles: column partials of earlier tiles, the diagonal tile's row
-// and column partials, row partials of later tiles).
-// Run c of the ordered partial sum of output element idx (see sym_term).
-__device__ __forceinline__ double2 sym_run_sum(const double2* __restrict__ part, int S, int T, int N, int idx,
-                                               int c) {
-  const int o = idx / N, q = idx % N;
-  const int i = o / S, l = o % S;
-  int t0, t1;
-  sym_run_bounds(T, c, &t0, &t1);
-  double2 f = make_double2(0.0, 0.0);
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t) f = cadd(f, part[sym_term(t, i, l, q, S, T, N)]);
-  return f;
-}
-
-// kRedQ runs per element through shared memory, added in run order.
-__device__ __forceinline__ void sym_reduce_finish(double2 f, bool valid, double2* __restrict__ out) {
-  __shared__ double2 red[kRedQ][kRedE];
-  const int e = threadIdx.x % kRedE, c = threadIdx.x / kRedE;
-  red[c][e] = f;
-  __syncthreads();
-  if (c == 0 && valid) {
-    double2 s = red[0][e];
-#pragma unroll
-    for (int k = 1; k < kRedQ; ++k) s = cadd(s, red[k][e]);
-    *out = s;
-  }
-}
-
-__global__ void __launch_bounds__(kRedQ* kRedE) k_sym_reduce(const double2* __restrict__ part, int S, int T,
-                                                             int M, int N, double2* __restrict__ F) {
-  const int e = threadIdx.x % kRedE, c = threadIdx.x / kRedE;
-  const int idx = blockIdx.x * kRedE + e;
-  const bool valid = idx < M * N;
-  const double2 f = valid ? sym_run_sum(part, S, T, N, idx, c) : make_double2(0.0, 0.0);
-  sym_reduce_finish(f, valid, F + (valid ? idx : 0));
-}
-
-__device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, int q, int N) {
-  if (s.f != nullptr) return s.f[(size_t)col * N + q];
-  const unsigned long long* p = s.acc + (size_t)col * 4 * N + q;
-  const i64 hx = (i64)p[0], lx = (i64)p[N], hy = (i64)p[2 * N], ly = (i64)p[3 * N];
-  const double2 f = s.scale[col];
-  const double x = fma((double)hx, 4294967296.0, (double)lx), y = fma((double)hy, 4294967296.0, (double)ly);
-  return make_double2(fma(x, f.x, x * f.y), fma(y, f.x, y * f.y));
-}
 // Exchange term of output column (ik, ib) at grid point q; false: none.
 __device__ __forceinline__ bool exchange_at(const CombineArgs& a, int ik, int ib, int q, int N, double2* f) {
   if (ib < a.nbocc && (a.occ_ex.acc != nullptr || a.occ_ex.f != nullptr)) {
@@ -293,20 +198,6 @@ __device__ __forceinline__ bool exchange_at(const CombineArgs& a, int ik, int ib
   if (a.row_ex.acc == nullptr) return false;
   *f = exchange_value(a.row_ex, ik * (a.w.nb - a.row_b0) + (ib - a.row_b0), q, N);
   return true;
-}
-
-// Sum over a CTA, result in every thread of warp 0 (fixed order).
-template <int NW>
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  v = warp_sum(v);
-  if constexpr (NW == 1) return v;
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  v = red[0];
-#pragma unroll
-  for (int w = 1; w < NW; ++w) v += red[w];
-  __syncthreads();
-  return v;
 }
 
 // ---------------------------------------------------------------------------
@@ -726,11 +617,6 @@ cudaError_t launch_ex_finalize_batch(const ExArgs* d_args, int nruns, cudaStream
 
 cudaError_t launch_step_advance(int* it, cudaStream_t s) {
   k_step_advance<<<1, 32, 0, s>>>(it);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_sym_reduce(const double2* part, int S, int T, int M, int N, double2* F, cudaStream_t s) {
-  k_sym_reduce<<<(M * N + kRedE - 1) / kRedE, kRedQ * kRedE, 0, s>>>(part, S, T, M, N, F);
   return cudaGetLastError();
 }
 
