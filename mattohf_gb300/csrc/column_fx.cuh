@@ -60,7 +60,16 @@ __device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, in
   const unsigned long long* p = s.acc + (size_t)col * 4 * N + q;
   const i64 hx = (i64)p[0], lx = (i64)p[N], hy = (i64)p[2 * N], ly = (i64)p[3 * N];
   const double2 f = s.scale[col];
-  const double x = fma((double)hx, 4294967296.0, (double)lx), y = fma((double)hy, 4294967296.0, (double)ly);
+  double x, y;
+  // one conversion where the sums fit 64 bits (they can only outgrow them when
+  // very many equal localised orbitals add up)
+  if (((hx + (1ll << 29)) >> 30) == 0 && ((hy + (1ll << 29)) >> 30) == 0) {
+    x = (double)((hx << 32) + lx);
+    y = (double)((hy << 32) + ly);
+  } else {
+    x = fma((double)hx, 4294967296.0, (double)lx);
+    y = fma((double)hy, 4294967296.0, (double)ly);
+  }
   return make_double2(fma(x, f.x, x * f.y), fma(y, f.x, y * f.y));
 }
 // Sum over a CTA, result in every thread of warp 0 (fixed order).

@@ -246,7 +246,7 @@ AField aval(double A) {
   return f;
 }
 
-int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr) {
+int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scalars = true) {
   DensArgs a;
   a.u = u;
   a.nbocc = ctx->NBocc;
@@ -257,7 +257,7 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr) {
   a.dvcell = ctx->dvcell;
   a.rho = ctx->d_rho;
   a.vloc = ctx->d_vloc;
-  a.scal = ctx->d_scal;
+  a.scal = scalars ? ctx->d_scal : nullptr;
   a.nk = ctx->NK;
   a.part = ctx->d_dpart;
   a.mu = nullptr;
@@ -367,21 +367,15 @@ size_t sym_partials(int M, int S, int NG) {
   return T * (T + 1) / 2 * 2 * S * NG;
 }
 
-// The exchange on columns w (k-points from k0 on) of the occupied orbitals of u,
-// which are already in fixed point.
-int enq_fock_rows(mattohf_ctx* ctx, Block u, Block w, int nk_w, int k0) {
-  const int ncols = nk_w * w.nb;
-  CKR(ensure_scratch(ctx, ncols));
-  FockFxArgs a = fx_args(ctx, u, 1);
-  a.kern += (size_t)k0 * ctx->NG;
-  FockFxRows r;
-  r.w = w;
-  r.ncols = ncols;
-  r.wfx = reinterpret_cast<fx::lc*>(ctx->d_wfx);
-  r.wscale = ctx->d_wscale;
-  r.acc = ctx->d_wacc;
-  fock_split(ctx, ncols, &r.nchunks, &r.chunk);
-  CK(launch_fock_fx(ctx->NG, a, r, ctx->st));
+// The rows' arguments for columns w (nk_w k-points).
+int fx_rows_args(mattohf_ctx* ctx, Block w, int nk_w, FockFxRows* r) {
+  r->w = w;
+  r->ncols = nk_w * w.nb;
+  CKR(ensure_scratch(ctx, r->ncols));
+  r->wfx = reinterpret_cast<fx::lc*>(ctx->d_wfx);
+  r->wscale = ctx->d_wscale;
+  r->acc = ctx->d_wacc;
+  fock_split(ctx, r->ncols, &r->nchunks, &r->chunk);
   return MATTOHF_OK;
 }
 
@@ -394,51 +388,54 @@ int ensure_fock_buffers(mattohf_ctx* ctx) {
   return MATTOHF_OK;
 }
 
-// Exchange partials of h[u] w.  When w is u itself (all RK4 stages, Ex,
-// Subspace_diag, eps) the occupied rows use the symmetric pair kernel and only
-// the unoccupied rows (if any) take the chunked kernel.
-int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = false) {
+// Exchange of h[u] w.  When w is u itself (all RK4 stages, Ex, Subspace_diag,
+// eps) the occupied rows use the symmetric pair kernel and only the unoccupied
+// rows (if any) the kernel for other functions.  have_sizes: the orbitals' sizes
+// are there (left by the kernel that made them).
+int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = false, bool have_sizes = false) {
   *plan = FockPlan();
   plan->any = true;
   const bool same = (w.p == u.p) && (w.kstride == u.kstride) && (w.nb == u.nb);
   const int NG = ctx->NG;
-  if (same && ctx->opt_sym) {
-    const int M = ctx->NK * ctx->NBocc;
-    const int S = ctx->opt_df ? sym_tile(ctx) : fx_tile(ctx);
-    const int T = (M + S - 1) / S;
-    if (ctx->opt_df) CKR(ensure_sym(ctx, sym_partials(M, S, NG)));
-    CKR(ensure_fx(ctx));
-    CKR(timed_begin(ctx));
-    if (ctx->opt_df) {
-      if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * NG));
-      FockSymDfArgs d;
-      d.u = ctx->d_udf;
-      d.nk = ctx->NK;
-      d.nbocc = ctx->NBocc;
-      d.S = S;
-      d.T = T;
-      d.kern = ctx->d_kern_df;
-      d.tw = ctx->d_tw_df;
-      d.scratch = reinterpret_cast<float4*>(ctx->d_sym);  // same 16-byte elements
-      d.F = ctx->d_symF;
-      CK(launch_fock_sym_df(NG, d, u.p, u.kstride, ctx->d_udf, ctx->st));
-    } else {
-      CK(launch_fx_orbitals(NG, fx_args(ctx, u, S), ctx->st));
-      CK(launch_fock_sym_fx(NG, fx_args(ctx, u, S), ctx->st));
-    }
-    CKR(timed_end(ctx));
-    plan->occ = true;
-    plan->b0 = ctx->NBocc;
-    if (w.nb == ctx->NBocc) return MATTOHF_OK;
-  }
-  Block wr = w;
-  wr.p = w.p + (size_t)plan->b0 * NG;
-  wr.nb = w.nb - plan->b0;
+  const int M = ctx->NK * ctx->NBocc;
+  plan->occ = same && ctx->opt_sym;
+  plan->b0 = plan->occ ? ctx->NBocc : 0;
+  plan->rows = w.nb > plan->b0;
   CKR(ensure_fx(ctx));
+  const int S = fx_tile(ctx);
+  const FockFxArgs a = fx_args(ctx, u, S);
+  FockFxRows r;
+  if (plan->rows) {
+    Block wr = w;
+    wr.p = w.p + (size_t)plan->b0 * NG;
+    wr.nb = w.nb - plan->b0;
+    CKR(fx_rows_args(ctx, wr, ctx->NK, &r));
+  }
+  const bool df = plan->occ && ctx->opt_df;
+  if (df) {
+    const int Sd = sym_tile(ctx);
+    CKR(ensure_sym(ctx, sym_partials(M, Sd, NG)));
+    if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * NG));
+  }
   CKR(timed_begin(ctx));
-  if (!same_u && (!plan->occ || ctx->opt_df)) CK(launch_fx_orbitals(NG, fx_args(ctx, u, 1), ctx->st));
-  CKR(enq_fock_rows(ctx, u, wr, ctx->NK, 0));
-  plan->rows = true;
+  if (plan->rows || !df)
+    CK(launch_fx_convert(NG, a, plan->rows ? &r : nullptr, have_sizes, same_u && !plan->occ, ctx->st));
+  if (df) {
+    FockSymDfArgs d;
+    d.u = ctx->d_udf;
+    d.nk = ctx->NK;
+    d.nbocc = ctx->NBocc;
+    d.S = sym_tile(ctx);
+    d.T = (M + d.S - 1) / d.S;
+    d.kern = ctx->d_kern_df;
+    d.tw = ctx->d_tw_df;
+    d.scratch = reinterpret_cast<float4*>(ctx->d_sym);  // same 16-byte elements
+    d.F = ctx->d_symF;
+    CK(launch_fock_sym_df(NG, d, u.p, u.kstride, ctx->d_udf, ctx->st));
+  } else if (plan->occ) {
+    CK(launch_fock_sym_fx(NG, a, ctx->st));
+  }
+  if (plan->rows) CK(launch_fock_fx(NG, a, r, ctx->st));
   CKR(timed_end(ctx));
   return MATTOHF_OK;
 }
@@ -505,73 +502,60 @@ BlockOut blko(double2* p, int ld, int NG, int nb) {
   return b;
 }
 
-// Observables of `u` at field af (RT:43-47): density scalars, Fock partials,
-// per-column Ekin/Je/<u|F u>, then the ordered reduction.
-// With `defer_ex` the exchange energy is left out of Etot (and no Fock apply
-// is made); the next RK4 step's first stage, which applies the exchange
-// operator of the same orbitals, adds it (k_ex_finalize).
-int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, bool advance, bool defer_ex,
-                    FockPlan* plan_out = nullptr) {
-  const int NG = ctx->NG, NB = ctx->NB;
-  Block ub = blk(u, NB, NG, NB);
-  CKR(enq_density(ctx, ub));
-  FockPlan fp;
-  fp.any = false;
-  if (ctx->hf && !defer_ex) CKR(enq_fock(ctx, ub, ub, &fp));
-  CKR(ensure_scratch(ctx, ctx->NK * NB));
-  if (plan_out) *plan_out = fp;
-  CombineArgs a = combine_base(ctx, ub, af, CM_OBS, fp);
-  CK(launch_combine(NG, a, ctx->NK * NB, ctx->st));
+ObsReduceArgs obs_args(mattohf_ctx* ctx, int advance) {
   ObsReduceArgs r;
   r.colbuf = ctx->d_colbuf;
   r.scal = ctx->d_scal;
   r.nk = ctx->NK;
-  r.nb = NB;
+  r.nb = ctx->NB;
   r.nbocc = ctx->NBocc;
   r.occ = ctx->occ;
   r.dvcell = ctx->dvcell;
   r.vcell = ctx->vcell;
-  r.NGd = (double)NG;
+  r.NGd = (double)ctx->NG;
   r.hf = ctx->hf;
-  r.defer_ex = defer_ex ? 1 : 0;
   r.out = ctx->d_out;
   r.series_E = advance ? ctx->d_sE : nullptr;
   r.series_J = advance ? ctx->d_sJ : nullptr;
   r.series_N = advance ? ctx->d_sN : nullptr;
   r.it = ctx->d_int;
-  r.advance = advance ? 1 : 0;
+  r.advance = advance;
   r.nonfinite = ctx->d_int + 1;
-  CK(launch_obs_reduce(r, ctx->st));
+  return r;
+}
+
+// Observables of `u` at field af (RT:43-47): density scalars, Fock partials,
+// per-column Ekin/Je/<u|F u>, then the ordered reduction.
+// advance: the series are written at the step counter, which is then incremented
+// (1), or at the counter less one (3).
+int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, int advance, FockPlan* plan_out = nullptr) {
+  const int NG = ctx->NG, NB = ctx->NB;
+  Block ub = blk(u, NB, NG, NB);
+  CKR(enq_density(ctx, ub));
+  FockPlan fp;
+  fp.any = false;
+  if (ctx->hf) CKR(enq_fock(ctx, ub, ub, &fp));
+  CKR(ensure_scratch(ctx, ctx->NK * NB));
+  if (plan_out) *plan_out = fp;
+  CombineArgs a = combine_base(ctx, ub, af, CM_OBS, fp);
+  CK(launch_combine(NG, a, ctx->NK * NB, ctx->st));
+  CK(launch_obs_reduce(obs_args(ctx, advance), ctx->st));
   return MATTOHF_OK;
 }
 
-// One RK4 step (RT:165-170); fields either from host values or from the
-// device series indexed by the device step counter.
-ExArgs ex_args(mattohf_ctx* ctx, double* series, int idx, double* out) {
-  ExArgs e;
-  e.colbuf = ctx->d_colbuf;
-  e.nk = ctx->NK;
-  e.nb = ctx->NB;
-  e.nbocc = ctx->NBocc;
-  e.occ = ctx->occ;
-  e.dvcell = ctx->dvcell;
-  e.series_E = series;
-  e.it = ctx->d_int;
-  e.idx = idx;
-  e.out = out;
-  return e;
-}
-
-// One RK4 step (RT:165-170); fields either from host values or from the
-// device series indexed by the device step counter.  With `ex_series` the
-// first stage also completes Etot(it-1) with the exchange energy of the
-// step's input orbitals (the same exchange operator the stage applies).
 int launch_store_stage(mattohf_ctx* ctx, const double2* src, int slot);
 
-// One RK4 step.  With `store`, the four stage inputs also go to the adjoint's
-// stage store at slot (it - seg0) * 4 + s.
-int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
-            double* ex_series = nullptr, bool store = false) {
+// One RK4 step (RT:165-170); fields either from host values or from the device
+// series indexed by the device step counter.  With `store`, the four stage inputs
+// also go to the adjoint's stage store at slot (it - seg0) * 4 + s.
+// With `run` (mattohf_rk4_run) the step is one of a loop: the sizes of its input
+// are there (left by the step before, or taken before the loop), and the first
+// stage, which needs the density, the kinetic transform and the exchange of the
+// step's input anyway, leaves the observables of that input (the previous step's
+// state, at the previous step's field) for a reduction on the side stream, beside
+// the second stage; the last stage's combine increments the counter.
+int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt, bool run = false,
+            bool store = false) {
   const int NG = ctx->NG, NB = ctx->NB;
   const int modes[4] = {CM_RK0, CM_RK1, CM_RK2, CM_RK3};
   const AField fs[4] = {f_m, f_ave, f_ave, f_cur};
@@ -582,18 +566,25 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
     Block ub = blk(in, NB, NG, NB);
     FockPlan fp;
     const bool side = ctx->hf != 0;
+    const bool obs = run && side && s == 0;
     if (side) {
       // The density and the kinetic + local-potential part of h w need only
       // the stage input: they run on the side stream beside the exchange.
       CK(cudaEventRecord(ctx->ev_fork, ctx->st));
       CK(cudaStreamWaitEvent(ctx->st_side, ctx->ev_fork, 0));
-      CKR(enq_density(ctx, ub, ctx->st_side));
+      CKR(enq_density(ctx, ub, ctx->st_side, !run || obs));
       CombineArgs pre = combine_base(ctx, ub, fs[s], modes[s], FockPlan());
       pre.split = 1;
       pre.hpre = ctx->d_hpre;
+      if (obs) {
+        pre.obs = 1;
+        pre.af_obs = fs[s];
+        pre.af_obs.mode = APREV;
+      }
       CK(launch_combine(NG, pre, ctx->NK * NB, ctx->st_side));
       CK(cudaEventRecord(ctx->ev_join, ctx->st_side));
-      CKR(enq_fock(ctx, ub, ub, &fp));
+      if (run && s == 1) CK(launch_obs_reduce(obs_args(ctx, 3), ctx->st_side));  // joined by stage 2
+      CKR(enq_fock(ctx, ub, ub, &fp, false, run || s > 0));
       CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
     } else {
       CKR(enq_density(ctx, ub));
@@ -601,15 +592,19 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
     CombineArgs a = combine_base(ctx, ub, fs[s], modes[s], fp);
     a.out = blko(ctx->d_us, NB, NG, NB);
     a.dt = dt;
-    a.ex_cols = (s == 0 && ex_series != nullptr && ctx->hf) ? 1 : 0;
+    a.ex_cols = obs ? 1 : 0;
     if (side) {
       a.split = 2;
       a.hpre = ctx->d_hpre;
+      a.sizes = ctx->d_fx_sizes;
+      a.advance = run && s == 3 ? ctx->d_int : nullptr;
     }
     CK(launch_combine(NG, a, ctx->NK * NB, ctx->st));
-    if (a.ex_cols) CK(launch_ex_finalize(ex_args(ctx, ex_series, -1, nullptr), ctx->st));
     if (store && s < 3) CKR(launch_store_stage(ctx, ctx->d_us, s + 1));
   }
+  // without exchange there is no first-stage apply to share: the observables of
+  // the step's result follow it, and advance the counter
+  if (run && !ctx->hf) CKR(enq_observables(ctx, ctx->d_u, f_cur, 1));
   return MATTOHF_OK;
 }
 
@@ -1325,8 +1320,12 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   FockPlan fp;
   if (ctx->hf && mode != CM_T) {
     CKR(ensure_fx(ctx));
-    CK(launch_fx_orbitals(NG, fx_args(ctx, u, 1), ctx->st));
-    CKR(enq_fock_rows(ctx, u, w, nkl, k0));
+    FockFxArgs a = fx_args(ctx, u, 1);
+    a.kern += (size_t)k0 * NG;
+    FockFxRows r;
+    CKR(fx_rows_args(ctx, w, nkl, &r));
+    CK(launch_fx_convert(NG, a, &r, false, false, ctx->st));
+    CK(launch_fock_fx(NG, a, r, ctx->st));
     fp.any = true;
     fp.rows = true;
   } else if (mode == CM_F) {
@@ -1404,7 +1403,7 @@ int mattohf_density(mattohf_ctx* ctx, const double* ubk, double* dns, double* vH
 
 int mattohf_observables(mattohf_ctx* ctx, double A, double* Ecomps, double* Etot, double* Je, double* Nele) {
   CKR(check_ctx(ctx));
-  CKR(enq_observables(ctx, ctx->d_u, aval(A), false, false));
+  CKR(enq_observables(ctx, ctx->d_u, aval(A), 0));
   double o[8];
   CK(cudaMemcpyAsync(o, ctx->d_out, sizeof(double) * 7, cudaMemcpyDeviceToHost, ctx->st));
   CKR(sync_and_flag(ctx));
@@ -1467,8 +1466,7 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
         if (small) {
           rc = enq_small_step(ctx, fm, fave, fcur, dt);
         } else {
-          rc = enq_rk4(ctx, fm, fave, fcur, dt, ctx->d_sE);
-          if (rc == MATTOHF_OK) rc = enq_observables(ctx, ctx->d_u, fcur, true, true);
+          rc = enq_rk4(ctx, fm, fave, fcur, dt, true);
         }
       }
       cudaError_t ec = cudaStreamEndCapture(ctx->st, &g);
@@ -1504,6 +1502,7 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
   CK(e0.create());
   CK(e1.create());
   CK(cudaEventRecord(e0, ctx->st));
+  if (!small && ctx->hf) CK(launch_fx_sizes(ctx->NG, fx_args(ctx, blk(ctx->d_u, ctx->NB, ctx->NG, ctx->NB), 1), ctx->st));
   int flag = 0;
   int bad_at = -1;
   for (int it = 0; it < nt; ++it) {
@@ -1519,8 +1518,7 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
     } else if (small) {
       CKR(enq_small_step(ctx, fm, fave, fcur, dt));
     } else {
-      CKR(enq_rk4(ctx, fm, fave, fcur, dt, ctx->d_sE));
-      CKR(enq_observables(ctx, ctx->d_u, fcur, true, true));
+      CKR(enq_rk4(ctx, fm, fave, fcur, dt, true));
     }
     if (stepwise) CK(cudaEventRecord(ctx->step_events[2 * it + 1], ctx->st));
     // bounded detection of a blow-up: poll the flag every 256 steps
@@ -1535,9 +1533,8 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
     }
   }
   {
-    // exchange energy of the last step's orbitals (the next stage-1 apply that
-    // would supply it does not happen)
-    const int last = bad_at >= 0 ? bad_at : nt - 1;
+    // observables of the last step's orbitals (the next step's first stage, which
+    // would supply them, does not happen)
     if (stepwise) {
       CK(cudaMemsetAsync(ctx->d_flush, 0x5a, (size_t)ctx->opt_flush, ctx->st));
       CK(cudaEventRecord(ctx->step_events[2 * nt], ctx->st));
@@ -1545,10 +1542,9 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
     if (small) {
       CKR(enq_small_close(ctx));
     } else if (ctx->hf) {
-      FockPlan fp;
-      CKR(enq_observables(ctx, ctx->d_u, aval(0.0), false, false, &fp));
-      (void)fp;
-      CK(launch_ex_finalize(ex_args(ctx, ctx->d_sE, last, nullptr), ctx->st));
+      AField fp = fcur;
+      fp.mode = APREV;
+      CKR(enq_observables(ctx, ctx->d_u, fp, 3));
     }
   }
   CK(cudaEventRecord(e1, ctx->st));
@@ -1792,7 +1788,7 @@ int mattohf_gs_run(mattohf_ctx* ctx, int nscf, int ncg, double* Etot_iter, doubl
   std::vector<double> dprev(NG), dnew(NG);
   double o[8];
   // Etotscf(0) and dnsscf(:,1) (GS:26-27)
-  CKR(enq_observables(ctx, ctx->d_u, aval(0.0), false, false));
+  CKR(enq_observables(ctx, ctx->d_u, aval(0.0), 0));
   CK(cudaMemcpyAsync(o, ctx->d_out, sizeof(double) * 7, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(dprev.data(), ctx->d_rho, sizeof(double) * NG, cudaMemcpyDeviceToHost, ctx->st));
   CKR(sync_and_flag(ctx));
@@ -1825,7 +1821,7 @@ int mattohf_gs_run(mattohf_ctx* ctx, int nscf, int ncg, double* Etot_iter, doubl
     // Etot, Je (GS:36-38); the Fock partials of h[u]u are then reused for the
     // Ritz values and residuals (GS:42-43), which apply the same operator.
     FockPlan fp;
-    CKR(enq_observables(ctx, ctx->d_u, aval(0.0), false, false, &fp));
+    CKR(enq_observables(ctx, ctx->d_u, aval(0.0), 0, &fp));
     {
       CombineArgs a = combine_base(ctx, ub, aval(0.0), CM_H, fp);
       a.out = blko(ctx->d_hwork, NB, NG, NB);
@@ -1926,7 +1922,7 @@ namespace {
 // segment store at slot (it - seg0)*4 + s.
 int enq_recompute_step(mattohf_ctx* ctx, AField fm, AField fave, AField fcur, double dt) {
   if (use_small(ctx)) return enq_small_step(ctx, fm, fave, fcur, dt, true);  // advances the counter itself
-  CKR(enq_rk4(ctx, fm, fave, fcur, dt, nullptr, true));
+  CKR(enq_rk4(ctx, fm, fave, fcur, dt, false, true));
   CK(launch_counter_add(ctx->d_int, 1, ctx->st));
   return MATTOHF_OK;
 }
@@ -2060,8 +2056,8 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
       f.tw = fv.tw;
       f.acc = fm.acc;
       CKR(timed_begin(ctx));
-      CK(launch_fx_orbitals(NG, fv, ctx->st));
-      CK(launch_fx_orbitals(NG, fm, ctx->st));
+      CK(launch_fx_convert(NG, fv, nullptr, false, false, ctx->st));
+      CK(launch_fx_convert(NG, fm, nullptr, false, false, ctx->st));
       CK(launch_fock_adj_fx(NG, f, ctx->st));
       CKR(timed_end(ctx));
     }
@@ -2169,7 +2165,7 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   // ---- objective at t = 0 and the forward pass with checkpoints
   double o0[8];
   std::vector<double> rho0(NG), rhoN(NG);
-  CKR(enq_observables(ctx, ctx->d_u, aval(0.0), false, false));
+  CKR(enq_observables(ctx, ctx->d_u, aval(0.0), 0));
   CK(cudaMemcpyAsync(o0, ctx->d_out, sizeof(double) * 7, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(rho0.data(), ctx->d_rho, sizeof(double) * NG, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(ctx->d_u0, ctx->d_u, sizeof(double2) * elems, cudaMemcpyDeviceToDevice, ctx->st));
@@ -2215,7 +2211,7 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
       // the fused stage 0 writes the checkpoint itself
       if (use_small(ctx)) return enq_small_step(ctx, fm, fave, fcur, dt, false, C, phase);
       CK(launch_checkpoint(ctx->d_ckpt, ctx->d_u, ctx->d_int, C, phase, elems, ctx->st));
-      CKR(enq_rk4(ctx, fm, fave, fcur, dt, nullptr));
+      CKR(enq_rk4(ctx, fm, fave, fcur, dt));
       CK(launch_counter_add(ctx->d_int, 1, ctx->st));
       return MATTOHF_OK;
     });
@@ -2231,7 +2227,7 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   // ---- objective at t = T and its gradient
   const double Afin = Ah[nt - 1];
   double oN[8];
-  CKR(enq_observables(ctx, ctx->d_u, aval(Afin), false, false));
+  CKR(enq_observables(ctx, ctx->d_u, aval(Afin), 0));
   CK(cudaMemcpyAsync(oN, ctx->d_out, sizeof(double) * 7, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(rhoN.data(), ctx->d_rho, sizeof(double) * NG, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(ctx->d_uN, ctx->d_u, sizeof(double2) * elems, cudaMemcpyDeviceToDevice, ctx->st));
@@ -2364,7 +2360,7 @@ struct mattohf_batch {
   std::vector<mattohf_ctx*> runs;
   cudaStream_t st = nullptr;
   int* d_int = nullptr;  // [0] step counter, [1] non-finite flag
-  static constexpr int kVariants = 6;  // stages 0..3, observables, observables with exchange
+  static constexpr int kVariants = 5;  // stages 0..3, observables
   DensArgs* d_dens[kVariants] = {};
   FockSymArgs* d_fsym[kVariants] = {};
   FockSymDfArgs* d_fsym_df[kVariants] = {};
@@ -2376,8 +2372,6 @@ struct mattohf_batch {
   int opt_df = 0;  // exchange transforms in double-float arithmetic
   int opt_tile = 0;  // symmetric-exchange tile of every run (0 = the CTA's teams)
   ObsReduceArgs* d_obs = nullptr;
-  ExArgs* d_ex = nullptr;
-  ExArgs* d_exf = nullptr;
   int *d_tile_pre = nullptr, *d_elem_pre = nullptr, *d_col_pre = nullptr;
   int total_tiles = 0, total_elems = 0, total_cols = 0;
   cudaGraphExec_t exec = nullptr;
@@ -2441,7 +2435,6 @@ int batch_prepare(mattohf_batch* b, int nt) {
   std::vector<CombineArgs> comb[mattohf_batch::kVariants];
   std::vector<CombineArgs> comb_pre[4];
   std::vector<ObsReduceArgs> obs(R);
-  std::vector<ExArgs> ex(R), exf(R);
   std::vector<int> tile_pre(R + 1, 0), elem_pre(R + 1, 0), col_pre(R + 1, 0);
   // one launch shape (a CTA's teams) for every run; a smaller tile leaves
   // teams idle but gives small runs more CTAs
@@ -2484,7 +2477,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
       d.dvcell = ctx->dvcell;
       d.rho = ctx->d_rho;
       d.vloc = ctx->d_vloc;
-      d.scal = ctx->d_scal;
+      d.scal = v >= 1 && v <= 3 ? nullptr : ctx->d_scal;
       d.nk = ctx->NK;
       d.part = ctx->d_dpart;
       d.mu = nullptr;
@@ -2514,13 +2507,13 @@ int batch_prepare(mattohf_batch* b, int nt) {
       fsdf[v].push_back(fd);
       fsfx[v].push_back(fx_args(ctx, ub, S));
       FockPlan fp;
-      fp.any = (v != 4);
+      fp.any = true;
       fp.occ = true;
       fp.b0 = ctx->NBocc;
       const AField af = v < 4 ? fld[v] : fld[3];
       CombineArgs c = combine_base(ctx, ub, af, v < 4 ? modes[v] : CM_OBS, fp);
-      if (v != 4 && ctx->hf) c.occ_ex = occ_source(ctx, b->opt_df);
-      if (v == 5) c.af = aval(0.0);
+      if (ctx->hf) c.occ_ex = occ_source(ctx, b->opt_df);
+      if (v == 4) c.af.mode = APREV;
       c.out = blko(ctx->d_us, ctx->NB, NG, ctx->NB);
       c.dt = b->dts[r];
       c.ex_cols = (v == 0 && ctx->hf) ? 1 : 0;
@@ -2529,36 +2522,22 @@ int batch_prepare(mattohf_batch* b, int nt) {
         CombineArgs cp = c;
         cp.split = 1;
         cp.hpre = ctx->d_hpre;
+        if (v == 0) {
+          cp.obs = 1;
+          cp.af_obs = af;
+          cp.af_obs.mode = APREV;
+        }
+        c.sizes = ctx->d_fx_sizes;
         comb_pre[v].push_back(cp);
         c.split = 2;
         c.hpre = ctx->d_hpre;
       }
       comb[v].push_back(c);
     }
-    ObsReduceArgs o;
-    o.colbuf = ctx->d_colbuf;
-    o.scal = ctx->d_scal;
-    o.nk = ctx->NK;
-    o.nb = ctx->NB;
-    o.nbocc = ctx->NBocc;
-    o.occ = ctx->occ;
-    o.dvcell = ctx->dvcell;
-    o.vcell = ctx->vcell;
-    o.NGd = (double)NG;
-    o.hf = ctx->hf;
-    o.defer_ex = 1;
-    o.out = ctx->d_out;
-    o.series_E = ctx->d_sE;
-    o.series_J = ctx->d_sJ;
-    o.series_N = ctx->d_sN;
+    ObsReduceArgs o = obs_args(ctx, 3);
     o.it = b->d_int;
-    o.advance = 2;
     o.nonfinite = b->d_int + 1;
     obs[r] = o;
-    ex[r] = ex_args(ctx, ctx->d_sE, -1, nullptr);
-    ex[r].it = b->d_int;
-    exf[r] = ex_args(ctx, ctx->d_sE, nt - 1, nullptr);
-    exf[r].it = b->d_int;
   }
   int rc;
   for (int v = 0; v < mattohf_batch::kVariants; ++v) {
@@ -2567,7 +2546,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
       return rc;
     if (v < 4 && (rc = bupload(b, &b->d_comb_pre[v], comb_pre[v]))) return rc;
   }
-  if ((rc = bupload(b, &b->d_obs, obs)) || (rc = bupload(b, &b->d_ex, ex)) || (rc = bupload(b, &b->d_exf, exf)) ||
+  if ((rc = bupload(b, &b->d_obs, obs)) ||
       (rc = bupload(b, &b->d_tile_pre, tile_pre)) || (rc = bupload(b, &b->d_elem_pre, elem_pre)) ||
       (rc = bupload(b, &b->d_col_pre, col_pre)))
     return rc;
@@ -2588,15 +2567,13 @@ int batch_prepare(mattohf_batch* b, int nt) {
     if (es == cudaSuccess)
       es = launch_combine_batch(NG, b->d_comb_pre[s], b->d_col_pre, R, b->total_cols, b->st_side);
     const cudaError_t ej = cudaEventRecord(b->ev_join, b->st_side);
+    // the observables of the step's input, beside the second stage (joined by the third)
+    if (es == cudaSuccess && s == 1) es = launch_obs_reduce_batch(b->d_obs, R, b->st_side);
     e = batch_exchange(b, s);
     const cudaError_t ew = cudaStreamWaitEvent(b->st, b->ev_join, 0);
     if (e == cudaSuccess) e = es != cudaSuccess ? es : (ej != cudaSuccess ? ej : ew);
     if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[s], b->d_col_pre, R, b->total_cols, b->st);
-    if (e == cudaSuccess && s == 0) e = launch_ex_finalize_batch(b->d_ex, R, b->st);
   }
-  if (e == cudaSuccess) e = launch_density_batch(NG, b->d_dens[4], R, b->st);
-  if (e == cudaSuccess) e = launch_combine_batch(NG, b->d_comb[4], b->d_col_pre, R, b->total_cols, b->st);
-  if (e == cudaSuccess) e = launch_obs_reduce_batch(b->d_obs, R, b->st);
   if (e == cudaSuccess) e = launch_step_advance(b->d_int, b->st);
   cudaError_t ec = cudaStreamEndCapture(b->st, &g);
   BCK(e);
@@ -2659,7 +2636,7 @@ int mattohf_batch_destroy(mattohf_batch* b) {
     cudaFree(b->d_fsym_fx[v]);
     cudaFree(b->d_comb[v]);
   }
-  void* ptrs[] = {b->d_obs, b->d_ex, b->d_exf, b->d_tile_pre, b->d_elem_pre, b->d_col_pre, b->d_int};
+  void* ptrs[] = {b->d_obs, b->d_tile_pre, b->d_elem_pre, b->d_col_pre, b->d_int};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto* c : b->runs) mattohf_destroy(c);
@@ -2694,14 +2671,6 @@ int mattohf_batch_rk4_run(mattohf_batch* b, int nt, const double* dt, const doub
     b->built_nt = -1;
     int rc = batch_prepare(b, nt);
     if (rc != MATTOHF_OK) return rc;
-  } else {
-    // the final-exchange arguments depend on nt
-    std::vector<ExArgs> exf(b->R);
-    for (int r = 0; r < b->R; ++r) {
-      exf[r] = ex_args(b->runs[r], b->runs[r]->d_sE, nt - 1, nullptr);
-      exf[r].it = b->d_int;
-    }
-    BCK(cudaMemcpyAsync(b->d_exf, exf.data(), sizeof(ExArgs) * b->R, cudaMemcpyHostToDevice, b->st));
   }
   // every run's orbitals were set on its own stream
   for (auto* c : b->runs) BCK(cudaStreamSynchronize(c->st));
@@ -2715,6 +2684,8 @@ int mattohf_batch_rk4_run(mattohf_batch* b, int nt, const double* dt, const doub
   BCK(e0.create());
   BCK(e1.create());
   BCK(cudaEventRecord(e0, b->st));
+  const int NG = b->NG;
+  if (!b->opt_df) BCK(launch_fx_sizes_batch(NG, b->d_fsym_fx[0], b->d_elem_pre, b->R, b->total_elems, b->st));
   int flag = 0, bad_at = -1;
   for (int it = 0; it < nt; ++it) {
     BCK(cudaGraphLaunch(b->exec, b->st));
@@ -2727,12 +2698,11 @@ int mattohf_batch_rk4_run(mattohf_batch* b, int nt, const double* dt, const doub
       }
     }
   }
-  // exchange energy of the last step's orbitals
-  const int NG = b->NG;
-  BCK(launch_density_batch(NG, b->d_dens[5], b->R, b->st));
-  BCK(batch_exchange(b, 5));
-  BCK(launch_combine_batch(NG, b->d_comb[5], b->d_col_pre, b->R, b->total_cols, b->st));
-  BCK(launch_ex_finalize_batch(b->d_exf, b->R, b->st));
+  // observables of the last step's orbitals
+  BCK(launch_density_batch(NG, b->d_dens[4], b->R, b->st));
+  BCK(batch_exchange(b, 4));
+  BCK(launch_combine_batch(NG, b->d_comb[4], b->d_col_pre, b->R, b->total_cols, b->st));
+  BCK(launch_obs_reduce_batch(b->d_obs, b->R, b->st));
   BCK(cudaEventRecord(e1, b->st));
   BCK(cudaEventSynchronize(e1));
   float ms = 0;

@@ -15,26 +15,34 @@ __device__ __forceinline__ float fx_mantissa(int h, int e) {  // |component| wit
   const int x = (h >> 20) - e + 127;
   return x > 0 && h >= 0x100000 ? __int_as_float((x << 23) | ((h & 0xfffff) << 3)) : 0.0f;
 }
-template <int LANES>
+// A size: x = high word of the largest |component|, y = the squared norm as a key
+// that orders like it: 13 bits of binary exponent (biased by 2 * 1023), 18 of mantissa.
+__device__ __forceinline__ int2 fx_size(int m, float s) {
+  const int b = __float_as_int(s);
+  return make_int2(m, m < 0x100000 ? 0 : (2 * (m >> 20) + (b >> 23) - 127) << 18 | ((b >> 5) & 0x3ffff));
+}
+__device__ __forceinline__ int2 fx_larger(int2 a, int2 b) { return make_int2(max(a.x, b.x), max(a.y, b.y)); }
+
+// Size of one column, by a warp.
 __device__ __forceinline__ int2 fx_column_size(const double2* __restrict__ p, int N, int lane) {
   int m = 0;
-  for (int i = lane; i < N; i += LANES) {
+  for (int i = lane; i < N; i += 32) {
     const double2 z = p[i];
     m = max(m, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  m = __reduce_max_sync(0xffffffffu, m);
   const int e = m >> 20;
   float s = 0.0f;
-  for (int i = lane; i < N; i += LANES) {
+  for (int i = lane; i < N; i += 32) {
     const double2 z = p[i];
     const float x = fx_mantissa(__double2hiint(z.x) & 0x7fffffff, e), y = fx_mantissa(__double2hiint(z.y) & 0x7fffffff, e);
     s = fmaf(x, x, fmaf(y, y, s));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return make_int2(m, __float_as_int(s));
+  return fx_size(m, s);
 }
+
 // A short scale c 2^k, c in {8 .. 15}.  Conversions and scales below are integer
 // and FP32 work: one FP64 instruction after another takes 64 cycles a warp, and
 // with FP64 square roots and divisions a conversion launch took 14 us for 1536
@@ -61,16 +69,18 @@ __device__ __forceinline__ i64 fx_convert(double v, Scale s) {
 // 2^60.2 for the norm, 2^58.4 for a component
 constexpr float kNorm = 1.3241e18f, kPeak = 3.803e17f;
 
-// s of a set whose largest component has the high word m (largest squared norm g2
-// and largest component gm in units of its exponent): both are short of the true
-// ones by less than 2^-18.  Not a number when the set holds a value that is not
-// finite or has an exponent field from emax on; for a set of zeros (or
-// denormal numbers), so large that every result scales back to zero.
-__device__ __forceinline__ Scale fx_scale(int m, float g2, float gm, int emax) {
-  const int e = m >> 20;
+// s of a set of size z (largest component, largest squared norm; both short of the
+// true ones by less than 2^-17).  Not a number when the set holds a value that is
+// not finite or has an exponent field from emax on; for a set of zeros (or
+// denormal numbers), so large that every result scales back to zero.  peak: the
+// bound of a component, n: further factor under the norm's.
+__device__ __forceinline__ Scale fx_scale(int2 z, float peak, float n, int emax) {
+  const int e = z.x >> 20;
   if (e >= emax) return Scale{0, 0};
-  if (m < 0x100000) return Scale{8, 2000};
-  return fx_short_scale(fminf(kNorm * rsqrtf(g2), kPeak / gm) * (1.0f - 1.0f / 16384.0f), 1023 - e);
+  if (z.x < 0x100000) return Scale{8, 2000};
+  // norm^2 = g 2^(2 (e - 1023)); the key's exponent is within a few units of 2 e
+  const float g = __int_as_float(((z.y >> 18) - 2 * e + 127) << 23 | (z.y & 0x3ffff) << 5);
+  return fx_short_scale(fminf(kNorm * rsqrtf(g * n), peak / fx_mantissa(z.x, e)) * (1.0f - 1.0f / 16384.0f), 1023 - e);
 }
 constexpr int kSquareMax = 1023 + 510;  // the squared norm overflows
 
@@ -96,14 +106,13 @@ __device__ __forceinline__ double2 fx_output_scale(Scale s, Scale sd, Scale sk) 
 // Scale of N values of size z (fx_block_size) that a transform takes: every partial sum is below sqrt(N) |v|_2 <= 2^60.2.  A power
 // of two, so that scaling back is exact.
 __device__ __forceinline__ Scale fx_fft_scale(int2 z, int N) {
-  Scale s = fx_scale(z.x, __int_as_float(z.y) * (float)N, 1e-30f, 2047);
+  Scale s = fx_scale(z, 1e30f, (float)N, 2047);
   if (s.c) s.c = 8;
   return s;
 }
 __device__ __forceinline__ double fx_unscale(Scale s) { return s.c ? pow2(-(s.k + 3)) : __longlong_as_double(0x7ff8000000000000ll); }
 
-// Size of the values that a CTA's threads hold (z.x = high word of the largest
-// component, z.y = squared norm); red: two words per warp.  Two barriers.
+// Size of the values that a CTA's threads hold; red: two words per warp.  Two barriers.
 template <int PER, int NWARP>
 __device__ __forceinline__ int2 fx_block_size(const double2 (&v)[PER], int* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -130,7 +139,7 @@ __device__ __forceinline__ int2 fx_block_size(const double2 (&v)[PER], int* red)
   s = 0.0f;
 #pragma unroll
   for (int w = 0; w < NWARP; ++w) s += __int_as_float(red[NWARP + w]);
-  return make_int2(m, __float_as_int(s));
+  return fx_size(m, s);
 }
 
 }  // namespace mattohf

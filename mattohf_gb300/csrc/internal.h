@@ -11,14 +11,16 @@ struct lc;
 }  // namespace fx
 
 constexpr int kThreads = 128;  // threads per CTA for the column/pair kernels (4 warps)
-constexpr int kDensChunks = 32; // column chunks of the two-stage density reduction
+constexpr int kDensChunks = 16; // most column chunks of the two-stage density reduction
+constexpr int kDensSub = 4;     // sub-chunks that a CTA of it adds up
 
 // How a kernel obtains the vector potential of the current launch.
 //   AVAL : use `A_val` directly
 //   AM   : A(it-1) recovered as 2*Aave(it) - A(it)        (src/RT_calculation.f90:165)
 //   AAVE : Aave(it)
 //   ACUR : A(it)
-enum AMode : int { AVAL = 0, AM = 1, AAVE = 2, ACUR = 3 };
+//   APREV: A(it-1), 0 for it = 0
+enum AMode : int { AVAL = 0, AM = 1, AAVE = 2, ACUR = 3, APREV = 4 };
 
 struct AField {
   int mode;
@@ -33,6 +35,7 @@ __device__ __forceinline__ double afield_value(const AField& f) {
   const int it = *f.it;
   if (f.mode == AM) return 2.0 * f.Aave[it] - f.A[it];
   if (f.mode == AAVE) return f.Aave[it];
+  if (f.mode == APREV) return it > 0 ? f.A[it - 1] : 0.0;
   return f.A[it];
 }
 
@@ -59,7 +62,7 @@ struct DensArgs {
   double dvcell;
   double* rho;        // NG out
   double* vloc;       // NG out: vH + vion
-  double* scal;       // out: [0]=Nele, [1]=Eion, [2]=EH
+  double* scal;       // out: [0]=Nele, [1]=Eion, [2]=EH (or null)
   int nk;
   double* part;       // scratch [kDensChunks][NG] partial densities
   // adjoint mode (mu != null): accumulate sigma = sum_cols Im(conj(mu) u)
@@ -121,7 +124,7 @@ struct FockFxArgs {
   Block u;              // occupied orbitals (bands 0..nbocc-1 used)
   int nk, nbocc;
   int S, T;             // tile size (<= kFxMaxTile), tiles
-  int2* sizes;          // [NK*nbocc]: largest |component| and squared norm (k_fx_sizes)
+  int2* sizes;          // [NK*nbocc]: largest |component| and squared norm (fx_size)
   fx::lc* ufx;          // [NK*nbocc][NG] fixed-point orbitals in limbs
   int* shift;           // [NK*nbocc] extra scale 2^d of an orbital with a small norm
   double2* fscale;      // [NK*nbocc] F = F^ * (x + y)
@@ -152,8 +155,13 @@ struct FockFxRows {
   unsigned long long* acc;  // [ncols][4][NG] sums F^, zeroed by the conversion
   int nchunks, chunk;   // chunks of the sources, sources per chunk
 };
-// orbitals to fixed point: before either exchange
-cudaError_t launch_fx_orbitals(int NG, const FockFxArgs& a, cudaStream_t s);
+// Orbitals (unless have_orbitals: still there from the last call) and rows (if any)
+// to fixed point, before either exchange; have_sizes: a.sizes holds.
+cudaError_t launch_fx_convert(int NG, const FockFxArgs& a, const FockFxRows* r, bool have_sizes, bool have_orbitals,
+                              cudaStream_t s);
+cudaError_t launch_fx_sizes(int NG, const FockFxArgs& a, cudaStream_t s);
+cudaError_t launch_fx_sizes_batch(int NG, const FockFxArgs* d_args, const int* d_elem_pre, int nruns, int total_elems,
+                                  cudaStream_t s);
 cudaError_t launch_fock_sym_fx(int NG, const FockFxArgs& a, cudaStream_t s);
 // kern of the arguments starts at the row of w's first k-point
 cudaError_t launch_fock_fx(int NG, const FockFxArgs& a, const FockFxRows& r, cudaStream_t s);
@@ -240,7 +248,7 @@ struct CombineArgs {
   // nbocc from occ_ex, or all bands from b0 on from row_ex
   ExSource occ_ex, row_ex;
   int row_b0;
-  int ex_cols;              // CM_RK0: also store <w|F> per occupied column (deferred Ex)
+  int ex_cols;              // CM_RK0: also store <w|F> per occupied column
   BlockOut out;             // h output (CM_H / CM_F / CM_T) or stage input (CM_RK0..2)
   double2* u0;              // RK4 base state [NK][NB][NG] (CM_RK*)
   double2* kbuf[4];         // RK4 stage derivatives [NK][NB][NG]
@@ -260,6 +268,11 @@ struct CombineArgs {
   // exchange).  2: hpre + exchange, then the mode's epilogue (no transforms).
   int split;
   double2* hpre;            // [NK][NB][NG]
+  // split == 1: also the columns' Ekin and Je parts at field af_obs
+  int obs;
+  AField af_obs;
+  int2* sizes;              // RK modes: sizes of the output's occupied columns (fx_size), or null
+  int* advance;             // split == 2: step counter to increment, or null (nothing here reads it)
 };
 
 // Fused RK4 stage for small problems (k_small.cu).  Each output column (k, b)
@@ -357,13 +370,13 @@ struct ObsReduceArgs {
   int nk, nb, nbocc;
   double occ, dvcell, vcell, NGd;
   int hf;
-  int defer_ex;             // 1: Etot excludes Ex (added later by k_ex_finalize)
   double* out;              // [0]=Etot [1]=Ekin [2]=Eion [3]=EH [4]=Ex [5]=Je [6]=Nele
   double* series_E;         // per step (may be null)
   double* series_J;
   double* series_N;
   int* it;                  // step counter
-  int advance;              // 0: no series; 1: write series[it] and increment it; 2: write only
+  int advance;              // 0: no series; 1: write series[it] and increment it; 3: write
+                            // series[it - 1] (of the state that step it starts from)
   int* nonfinite;
 };
 
@@ -373,16 +386,6 @@ cudaError_t launch_fock(int NG, const FockArgs& a, int ncols, cudaStream_t s);
 int fock_sym_teams(int NG);  // teams of a full symmetric-exchange CTA (largest tile size)
 int choose_sym_tile(int NG, int M, int nsm);  // tile size for a single run of M occupied orbitals on nsm SMs
 cudaError_t sym_launch_params(int NG, int S, int* threads, size_t* smem);
-struct ExArgs {
-  const double* colbuf;
-  int nk, nb, nbocc;
-  double occ, dvcell;
-  double* series_E;   // Etot series; Ex added to entry it-1 (or `idx` when >= 0)
-  const int* it;
-  int idx;
-  double* out;        // optional: [0] += Ex, [4] = Ex
-};
-cudaError_t launch_ex_finalize(const ExArgs& a, cudaStream_t s);
 cudaError_t launch_combine(int NG, const CombineArgs& a, int ncols, cudaStream_t s);
 cudaError_t launch_obs_reduce(const ObsReduceArgs& a, cudaStream_t s);
 
@@ -392,7 +395,6 @@ cudaError_t launch_density_batch(int NG, const DensArgs* d_args, int nruns, cuda
 cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d_col_pre, int nruns,
                                  int total_cols, cudaStream_t s);
 cudaError_t launch_obs_reduce_batch(const ObsReduceArgs* d_args, int nruns, cudaStream_t s);
-cudaError_t launch_ex_finalize_batch(const ExArgs* d_args, int nruns, cudaStream_t s);
 cudaError_t launch_step_advance(int* it, cudaStream_t s);
 
 // ---- adjoint (k_adjoint.cu) ----

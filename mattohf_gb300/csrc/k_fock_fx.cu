@@ -39,100 +39,83 @@ __device__ __forceinline__ const double2* fx_column(const Block& u, int nb, int 
   return u.p + (size_t)(col / nb) * u.kstride + (size_t)(col % nb) * N;
 }
 
-// One column to fixed point, by a CTA.  scan: the CTA takes the sizes of all
-// columns itself (few orbitals); else k_fx_sizes has left them in a.sizes.
-__device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, int N, int col, bool scan) {
-  __shared__ int2 own[4];
-  __shared__ Scale out;
+// One column to fixed point, by a CTA of 128 threads: column i < M of the orbitals
+// (one scale for all), or column i - M of the rows (a scale of its own).  The
+// orbitals' sizes are in a.sizes, or (scan: few orbitals) taken here.
+__device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, const FockFxRows& r, int N, int i, bool scan) {
+  constexpr int PER = 4;  // N <= 512
+  __shared__ int2 red[4], own_s;
+  __shared__ int redr[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int M = a.nk * a.nbocc;
-  // largest size over the columns, each warp over its share, then over warps
-  int m = 0;
-  float g2 = 0.0f, n2 = 0.0f;
-  int mc = 0;
-  for (int i = scan ? warp : tid; i < M; i += scan ? 4 : 128) {
-    const int2 z = scan ? fx_column_size<32>(fx_column(a.u, a.nbocc, i, N), N, lane) : a.sizes[i];
-    const float s = __int_as_float(z.y);
-    if (i == col) {
-      mc = z.x;
-      n2 = s;
-    }
-    // s and g2 in units of their own exponents, compared as s 2^(2 (e - e'))
-    const int d = (z.x >> 20) - (m >> 20);
-    g2 = d > 0 ? fmaxf(s, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(s, 2 * d));
-    m = max(m, z.x);
-  }
-  if (!scan) {
+  const bool row = i >= M;
+  const int col = row ? i - M : i;
+  const double2* p = row ? fx_column(r.w, r.w.nb, col, N) : fx_column(a.u, a.nbocc, col, N);
+  double2 v[PER];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int mo = __shfl_xor_sync(0xffffffffu, m, o);
-      const float go = __shfl_xor_sync(0xffffffffu, g2, o);
-      const int d = (mo >> 20) - (m >> 20);
-      g2 = d > 0 ? fmaxf(go, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(go, 2 * d));
-      m = max(m, mo);
-      const int co = __shfl_xor_sync(0xffffffffu, mc, o);
-      const float no = __shfl_xor_sync(0xffffffffu, n2, o);
-      mc = max(mc, co);  // one lane has the column
-      n2 = fmaxf(n2, no);
+  for (int j = 0; j < PER; ++j) v[j] = tid + 128 * j < N ? p[tid + 128 * j] : make_double2(0.0, 0.0);
+  int2 g = make_int2(0, 0), own = make_int2(0, 0);
+  if (scan) {
+    for (int c = warp; c < M; c += 4) {
+      const int2 z = fx_column_size(fx_column(a.u, a.nbocc, c, N), N, lane);
+      g = fx_larger(g, z);
+      if (c == i && lane == 0) {
+        own_s = z;
+        a.sizes[c] = z;
+      }
     }
+  } else {
+    for (int c = tid; c < M; c += 128) g = fx_larger(g, a.sizes[c]);
+    g = make_int2(__reduce_max_sync(0xffffffffu, g.x), __reduce_max_sync(0xffffffffu, g.y));
+    if (!row && tid == 0) own_s = a.sizes[col];
   }
-  __shared__ int2 ownc[4];
-  if (lane == 0) {
-    own[warp] = make_int2(m, __float_as_int(g2));
-    ownc[warp] = make_int2(mc, __float_as_int(n2));
+  if (lane == 0) red[warp] = g;
+  if (row) own = fx_block_size<PER, 4>(v, redr);  // has barriers
+  else __syncthreads();
+  g = fx_larger(fx_larger(red[0], red[1]), fx_larger(red[2], red[3]));
+  if (!row) own = own_s;
+  Scale s = fx_scale(g, kPeak, 1.0f, kSquareMax);
+  s.k -= a.halve;
+  Scale sd = s;
+  int d = 0;
+  if (row) {
+    sd = fx_scale(own, 1e30f, 1.0f, kSquareMax);
+  } else if (a.lift && own.y > 0) {  // a column with less than half the largest norm is lifted by 2^d
+    const int lg = (g.y >> 18) - (own.y >> 18);  // log2 of the squared norms' ratio, to 1
+    if (lg > 2) d = min(60, (lg - 1) >> 1);
+    sd.k += d;
   }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < 4; ++w) {
-      const float go = __int_as_float(own[w].y);
-      const int d = (own[w].x >> 20) - (m >> 20);
-      g2 = d > 0 ? fmaxf(go, d > 60 ? 0.0f : scalbnf(g2, -2 * d)) : fmaxf(g2, d < -60 ? 0.0f : scalbnf(go, 2 * d));
-      m = max(m, own[w].x);
-      mc = max(mc, ownc[w].x);
-      n2 = fmaxf(n2, __int_as_float(ownc[w].y));
-    }
-    const int e = m >> 20;
-    Scale s = fx_scale(m, g2, fx_mantissa(m, e), kSquareMax);
-    s.k -= a.halve;
-    // a column with less than half the largest norm is lifted by 2^d
-    const int dc = (mc >> 20) - e;
-    int d = 0;
-    if (n2 > 0.0f && a.lift) {
-      const int lg = ilogbf(g2) - ilogbf(n2) - 2 * dc;  // log2 of the squared norms' ratio, to 1
-      if (lg > 2) d = min(60, (lg - 1) >> 1);
-    }
-    const Scale sd{s.c, s.k + d};
-    out = sd;
-    if (a.shift) a.shift[col] = d;
-    if (col == 0) *a.uscale = make_int2(s.c, s.k);
-    if (a.fscale) {
-      const Scale so = a.vscale ? Scale{a.vscale->x, a.vscale->y} : s;
-      // a column of zeros has a sum of zero; the roundings of its terms do not count
-      a.fscale[col] = n2 > 0.0f || s.c == 0 || a.vscale ? fx_output_scale(so, sd, Scale{a.kscale->x, a.kscale->y}) : make_double2(0.0, 0.0);
-    }
-  }
-  __syncthreads();
-  const Scale sd = out;
   const bool ok = sd.c != 0;
-  const double2* p = fx_column(a.u, a.nbocc, col, N);
-  lc* o = a.ufx + (size_t)col * N;
-  for (int i = tid; i < N; i += 128) {
-    const double2 z = p[i];
-    o[i] = ok ? fx::limbs(cx{fx_convert(z.x, sd), fx_convert(z.y, sd)}) : lc{0, 0, 0, 0};
+  lc* o = (row ? r.wfx : a.ufx) + (size_t)col * N;
+#pragma unroll
+  for (int j = 0; j < PER; ++j)
+    if (tid + 128 * j < N) o[tid + 128 * j] = ok ? fx::limbs(cx{fx_convert(v[j].x, sd), fx_convert(v[j].y, sd)}) : lc{0, 0, 0, 0};
+  unsigned long long* acc = row ? r.acc : a.acc;
+  if (acc != nullptr)
+    for (int j = tid; j < 4 * N; j += 128) acc[(size_t)col * 4 * N + j] = 0;
+  if (tid != 0) return;
+  const Scale sk{a.kscale->x, a.kscale->y};
+  if (row) {
+    r.wscale[col] = fx_output_scale(s, sd, sk);
+    return;
   }
-  if (a.acc == nullptr) return;
-  unsigned long long* acc = a.acc + (size_t)col * 4 * N;
-  for (int i = tid; i < 4 * N; i += 128) acc[i] = 0;
+  if (a.shift) a.shift[col] = d;
+  if (col == 0) *a.uscale = make_int2(s.c, s.k);
+  if (a.fscale) {
+    const Scale so = a.vscale ? Scale{a.vscale->x, a.vscale->y} : s;
+    // a column of zeros has a sum of zero; the roundings of its terms do not count
+    a.fscale[col] = own.y > 0 || s.c == 0 || a.vscale ? fx_output_scale(so, sd, sk) : make_double2(0.0, 0.0);
+  }
 }
 
 __global__ void __launch_bounds__(128) k_fx_sizes(FockFxArgs a, int N) {
   const int col = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (col >= a.nk * a.nbocc) return;
-  const int2 z = fx_column_size<32>(fx_column(a.u, a.nbocc, col, N), N, threadIdx.x & 31);
+  const int2 z = fx_column_size(fx_column(a.u, a.nbocc, col, N), N, threadIdx.x & 31);
   if ((threadIdx.x & 31) == 0) a.sizes[col] = z;
 }
-__global__ void __launch_bounds__(128) k_fx_convert(FockFxArgs a, int N, int scan) {
-  fx_convert_body(a, N, blockIdx.x, scan);
+__global__ void __launch_bounds__(128) k_fx_convert(FockFxArgs a, FockFxRows r, int N, int first, int scan) {
+  fx_convert_body(a, r, N, first + blockIdx.x, scan);
 }
 // element prefix: pre[r] = sum over earlier runs of M_r * N
 __global__ void __launch_bounds__(128) k_fx_sizes_batch(const FockFxArgs* __restrict__ args,
@@ -140,13 +123,13 @@ __global__ void __launch_bounds__(128) k_fx_sizes_batch(const FockFxArgs* __rest
   const int c = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (c * N >= pre[nruns]) return;
   const int r = find_run(pre, nruns, c * N), col = c - pre[r] / N;
-  const int2 z = fx_column_size<32>(fx_column(args[r].u, args[r].nbocc, col, N), N, threadIdx.x & 31);
+  const int2 z = fx_column_size(fx_column(args[r].u, args[r].nbocc, col, N), N, threadIdx.x & 31);
   if ((threadIdx.x & 31) == 0) args[r].sizes[col] = z;
 }
 __global__ void __launch_bounds__(128) k_fx_convert_batch(const FockFxArgs* __restrict__ args,
                                                           const int* __restrict__ pre, int nruns, int N) {
   const int r = find_run(pre, nruns, blockIdx.x * N);
-  fx_convert_body(args[r], N, blockIdx.x - pre[r] / N, false);
+  fx_convert_body(args[r], FockFxRows{}, N, blockIdx.x - pre[r] / N, false);
 }
 
 // t / 2^s for s > 0, rounded (a floor would be biased by half a place per term)
@@ -337,22 +320,6 @@ __global__ void __launch_bounds__(sym_fx_threads<N>(), 2) k_fock_sym_fx_batch(co
 // A CTA takes kRowsThreads / T columns, one per team, against one chunk of the
 // sources, which all its teams read together.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_fx_rows(FockFxArgs a, FockFxRows r, int N) {
-  const int lane = threadIdx.x & 31, col = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (col >= r.ncols) return;
-  const double2* p = fx_column(r.w, r.w.nb, col, N);
-  const int2 z = fx_column_size<32>(p, N, lane);
-  const Scale s = fx_scale(z.x, __int_as_float(z.y), 1e-30f, kSquareMax), su{a.uscale->x, a.uscale->y};
-  const bool ok = s.c != 0;
-  lc* o = r.wfx + (size_t)col * N;
-  for (int i = lane; i < N; i += 32) {
-    const double2 v = p[i];
-    o[i] = ok ? fx::limbs(cx{fx_convert(v.x, s), fx_convert(v.y, s)}) : lc{0, 0, 0, 0};
-  }
-  for (int i = lane; i < 4 * N; i += 32) r.acc[(size_t)col * 4 * N + i] = 0;
-  if (lane == 0) r.wscale[col] = fx_output_scale(su, s, Scale{a.kscale->x, a.kscale->y});
-}
-
 template <int N>
 constexpr int rows_fx_teams() { return kRowsThreads / fx::Team<N>::T; }
 
@@ -590,7 +557,7 @@ static cudaError_t fock_sym_fx_impl(const FockFxArgs& a, cudaStream_t s) {
     default: return cudaErrorInvalidValue;         \
   }
 
-// after launch_fx_orbitals
+// after launch_fx_convert
 cudaError_t launch_fock_sym_fx(int NG, const FockFxArgs& a, cudaStream_t s) {
 #define CALL(n) fock_sym_fx_impl<n>(a, s)
   MATTOHF_DISPATCH(NG, CALL)
@@ -603,7 +570,6 @@ static cudaError_t fock_sym_fx_batch_impl(const FockFxArgs* d_args, const int* d
   int threads;
   size_t smem;
   sym_fx_shape<N>(S, &threads, &smem);
-  k_fx_sizes_batch<<<(total_elems / N + 3) / 4, 128, 0, s>>>(d_args, d_elem_pre, nruns, N);
   k_fx_convert_batch<<<total_elems / N, 128, 0, s>>>(d_args, d_elem_pre, nruns, N);
   k_fock_sym_fx_batch<N><<<total_tiles, threads, smem, s>>>(d_args, d_tile_pre, nruns);
   return cudaGetLastError();
@@ -617,12 +583,29 @@ cudaError_t launch_fock_sym_fx_batch(int NG, const FockFxArgs* d_args, const int
 #undef CALL
 }
 
-cudaError_t launch_fx_orbitals(int NG, const FockFxArgs& a, cudaStream_t s) {
+cudaError_t launch_fx_sizes(int NG, const FockFxArgs& a, cudaStream_t s) {
+  k_fx_sizes<<<(a.nk * a.nbocc + 3) / 4, 128, 0, s>>>(a, NG);
+  return cudaGetLastError();
+}
+cudaError_t launch_fx_sizes_batch(int NG, const FockFxArgs* d_args, const int* d_elem_pre, int nruns, int total_elems,
+                                  cudaStream_t s) {
+  if (total_elems <= 0) return cudaSuccess;
+  k_fx_sizes_batch<<<(total_elems / NG + 3) / 4, 128, 0, s>>>(d_args, d_elem_pre, nruns, NG);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_convert(int NG, const FockFxArgs& a, const FockFxRows* r, bool have_sizes, bool have_orbitals,
+                              cudaStream_t s) {
   const int M = a.nk * a.nbocc;
-  // up to 2^13 values every CTA takes all the sizes itself: a launch less
-  const int scan = M * NG <= 8192;
-  if (!scan) k_fx_sizes<<<(M + 3) / 4, 128, 0, s>>>(a, NG);
-  k_fx_convert<<<M, 128, 0, s>>>(a, NG, scan);
+  // up to 16 orbitals every CTA takes all the sizes itself: a launch less
+  const bool scan = !have_sizes && !have_orbitals && M <= 16;
+  if (!have_sizes && !have_orbitals && !scan) {
+    const cudaError_t e = launch_fx_sizes(NG, a, s);
+    if (e != cudaSuccess) return e;
+  }
+  const int n = (have_orbitals ? 0 : M) + (r ? r->ncols : 0);
+  if (n == 0) return cudaSuccess;
+  k_fx_convert<<<n, 128, 0, s>>>(a, r ? *r : FockFxRows{}, NG, have_orbitals ? M : 0, scan);
   return cudaGetLastError();
 }
 
@@ -634,7 +617,6 @@ static constexpr size_t rows_fx_smem() {
 template <int N>
 static cudaError_t fock_fx_impl(const FockFxArgs& a, const FockFxRows& r, cudaStream_t s) {
   constexpr int R = rows_fx_teams<N>();
-  k_fx_rows<<<(r.ncols + 3) / 4, 128, 0, s>>>(a, r, N);
   k_fock_fx<N><<<(r.ncols + R - 1) / R * r.nchunks, kRowsThreads, rows_fx_smem<N>(), s>>>(a, r);
   return cudaGetLastError();
 }

@@ -14,22 +14,34 @@ namespace mattohf {
 // ---------------------------------------------------------------------------
 // Density (F:55-71) and Hartree potential (F:147-162), one CTA.
 // ---------------------------------------------------------------------------
-// Stage 1: partial densities over a contiguous range of columns (one CTA per
-// chunk, thread per grid point); the FP64 work is spread over many SMs.
-__device__ __forceinline__ void dens_partial_body(const DensArgs& a, int N, int chunk) {
-  const int ncol = a.nk * a.u.nb;
-  const int per = (ncol + kDensChunks - 1) / kDensChunks;
-  const int c0 = chunk * per, c1 = min(ncol, c0 + per);
-  for (int ig = threadIdx.x; ig < N; ig += blockDim.x) {
-    double s = 0.0;
+// Stage 1: partial densities of kDensChunks chunks of columns (fewer for few
+// columns).  A CTA takes one chunk at 64 grid points, a quarter of the chunk per
+// group of 64 threads: FP64 instructions of a warp come 64 cycles apart, so the
+// columns of a thread are what the launch's time goes by.
+__host__ __device__ __forceinline__ int dens_chunks(int ncol) {
+  const int n = (ncol + 4 * kDensSub - 1) / (4 * kDensSub);
+  return n < 1 ? 1 : n > kDensChunks ? kDensChunks : n;
+}
+__device__ __forceinline__ void dens_partial_body(const DensArgs& a, int N, int chunk, int group) {
+  __shared__ double part_s[kDensSub][64];
+  const int ncol = a.nk * a.u.nb, nch = dens_chunks(ncol);
+  if (chunk >= nch) return;
+  const int per = (ncol + nch * kDensSub - 1) / (nch * kDensSub);
+  const int pt = threadIdx.x & 63, sub = threadIdx.x >> 6;
+  const int ig = group * 64 + pt;
+  const int c0 = (chunk * kDensSub + sub) * per, c1 = min(ncol, c0 + per);
+  double s = 0.0;
+  if (ig < N) {
     if (a.mu == nullptr) {
-      for (int c = c0; c < c1; ++c) {   // ik outer, ib inner within the chunk (reference order)
+#pragma unroll 4
+      for (int c = c0; c < c1; ++c) {
         const int ik = c / a.u.nb, ib = c % a.u.nb;
         const double occ = ib < a.nbocc ? a.occ : 0.0;
         const double2 z = a.u.p[(size_t)ik * a.u.kstride + (size_t)ib * N + ig];
         s += fma(occ * z.x, z.x, (occ * z.y) * z.y);
       }
     } else {
+#pragma unroll 4
       for (int c = c0; c < c1; ++c) {   // adjoint source: Im(conj(mu) u)
         const int ik = c / a.u.nb, ib = c % a.u.nb;
         const size_t o = (size_t)ik * a.u.kstride + (size_t)ib * N + ig;
@@ -37,14 +49,21 @@ __device__ __forceinline__ void dens_partial_body(const DensArgs& a, int N, int 
         s += fma(m.x, z.y, -(m.y * z.x));
       }
     }
+  }
+  part_s[sub][pt] = s;
+  __syncthreads();
+  if (sub == 0 && ig < N) {
+    for (int j = 1; j < kDensSub; ++j) s += part_s[j][pt];
     a.part[(size_t)chunk * N + ig] = s;
   }
 }
 
-__global__ void __launch_bounds__(256) k_dens_partial(DensArgs a, int N) { dens_partial_body(a, N, blockIdx.x); }
+__global__ void __launch_bounds__(64 * kDensSub) k_dens_partial(DensArgs a, int N) {
+  dens_partial_body(a, N, blockIdx.x, blockIdx.y);
+}
 
-__global__ void __launch_bounds__(256) k_dens_partial_batch(const DensArgs* __restrict__ args, int N) {
-  dens_partial_body(args[blockIdx.y], N, blockIdx.x);
+__global__ void __launch_bounds__(64 * kDensSub) k_dens_partial_batch(const DensArgs* __restrict__ args, int N) {
+  dens_partial_body(args[blockIdx.z], N, blockIdx.x, blockIdx.y);
 }
 
 // Stage 2 (one CTA): rho = ordered sum of the chunk partials, then the
@@ -64,9 +83,10 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
   tw_s.load(a.twfx);
   double2 v[1] = {make_double2(0.0, 0.0)};
   if (in) {
+    const int nch = dens_chunks(a.nk * a.u.nb);
     double s = a.part[tid];
-#pragma unroll 8
-    for (int ch = 1; ch < kDensChunks; ++ch) s += a.part[(size_t)ch * N + tid];
+#pragma unroll 4
+    for (int ch = 1; ch < nch; ++ch) s += a.part[(size_t)ch * N + tid];
     rho_s[tid] = s;
     a.rho[tid] = s;
     v[0].x = s;
@@ -93,21 +113,26 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
     return;
   }
   for (int ig = tid; ig < N; ig += blockDim.x) a.vloc[ig] = vh_s[ig] + a.vion[ig];
-  if (tid < 32) {
-    // Nele, Eion, EH: lane-strided partial sums, then a fixed shuffle tree
-    double sn = 0.0, si = 0.0, sh = 0.0;
-    for (int ig = tid; ig < N; ig += 32) {
-      sn += rho_s[ig];
-      si += a.vion[ig] * rho_s[ig];
-      sh += vh_s[ig] * rho_s[ig];
+  if (a.scal != nullptr && tid < 64) {
+    // Nele, Eion, EH: lane-strided partial sums, then a fixed shuffle tree; two
+    // warps (one for the first two sums)
+    const int lane = tid & 31;
+    double x = 0.0, y = 0.0;
+    if (tid < 32) {
+      for (int ig = lane; ig < N; ig += 32) {
+        x += rho_s[ig];
+        y += a.vion[ig] * rho_s[ig];
+      }
+    } else {
+      for (int ig = lane; ig < N; ig += 32) x += vh_s[ig] * rho_s[ig];
     }
-    sn = warp_sum(sn);
-    si = warp_sum(si);
-    sh = warp_sum(sh);
+    x = warp_sum(x);
+    y = warp_sum(y);
     if (tid == 0) {
-      a.scal[0] = sn * a.dvcell;
-      a.scal[1] = si * a.dvcell;
-      a.scal[2] = 0.5 * sh * a.dvcell;
+      a.scal[0] = x * a.dvcell;
+      a.scal[1] = y * a.dvcell;
+    } else if (tid == 32) {
+      a.scal[2] = 0.5 * x * a.dvcell;
     }
   }
 }
@@ -243,9 +268,11 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
     }
     fx_block_forward<N>(buf, tw_s);
     const double u1 = fx_unscale(s1);
-    if (a.mode == CM_OBS) {
+    if (a.mode == CM_OBS || a.obs) {
       // Ekin and Je of this column by Parseval on FFT(u):
       //   sum_x conj(u) IFFT(f * FFT(u)) = sum_G f(G) |FFT(u)(G)|^2
+      const double Ao = a.obs ? afield_value(a.af_obs) : A;
+      const double kAo = a.kx[ik] + Ao, kAo2 = kAo * kAo;
       double ek = 0.0, je = 0.0, fr = 0.0, fi = 0.0;
       if (in) {
 #pragma unroll
@@ -254,10 +281,10 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
           const double G = a.Gx[q];
           const double xr = (double)buf[q].x * u1, xi = (double)buf[q].y * u1;
           const double m2 = xr * xr + xi * xi;
-          ek += 0.5 * (G * G + 2.0 * G * kAx + kA2) * m2;
-          je += (G + a.kx[ik] + A) * m2;
+          ek += 0.5 * (G * G + 2.0 * G * kAo + kAo2) * m2;
+          je += (G + a.kx[ik] + Ao) * m2;
           double2 f;
-          if (ib < a.nbocc && exchange_at(a, ik, ib, q, N, &f)) {
+          if (a.mode == CM_OBS && ib < a.nbocc && exchange_at(a, ik, ib, q, N, &f)) {
             fr += wv[p].x * f.x + wv[p].y * f.y;
             fi += wv[p].x * f.y - wv[p].y * f.x;
           }
@@ -265,16 +292,20 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       }
       ek = block_sum<NW>(ek, redd) / (double)N;
       je = block_sum<NW>(je, redd) / (double)N;
-      fr = block_sum<NW>(fr, redd);
-      fi = block_sum<NW>(fi, redd);
+      double* cb = a.colbuf + (size_t)c * 4;
       if (tid == 0) {
-        double* cb = a.colbuf + (size_t)c * 4;
         cb[0] = ek;
         cb[1] = je;
-        cb[2] = fr;
-        cb[3] = fi;
       }
-      return;
+      if (a.mode == CM_OBS) {
+        fr = block_sum<NW>(fr, redd);
+        fi = block_sum<NW>(fi, redd);
+        if (tid == 0) {
+          cb[2] = fr;
+          cb[3] = fi;
+        }
+        return;
+      }
     }
     // kinetic energy in FP64, then back with a new scale
 #pragma unroll
@@ -315,8 +346,11 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
   // deferred exchange energy: <w|F> of occupied columns (stage 1 of an RK4 step)
   double exr = 0.0, exi = 0.0;
   bool bad = false;
+  double2 next[PER];
+  const double dt6 = a.dt / 6.0;
 #pragma unroll
   for (int p = 0; p < PER; ++p) {
+    next[p] = make_double2(0.0, 0.0);
     if (!in) continue;
     const int q = tid + TH * p;
     double2 h;
@@ -360,12 +394,16 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       sy = sy + 2.0 * k2.y;
       sx = sx + k.x;
       sy = sy + k.y;
-      sx = sx * a.dt / 6.0;
-      sy = sy * a.dt / 6.0;
-      nx = make_double2(u0.x + sx, u0.y + sy);
+      nx = make_double2(fma(sx, dt6, u0.x), fma(sy, dt6, u0.y));
       a.u0[o] = nx;
     }
+    next[p] = nx;
     bad |= !(isfinite(nx.x) && isfinite(nx.y));
+  }
+  if (a.advance != nullptr && c == 0 && tid == 0) *a.advance = *a.advance + 1;
+  if (a.sizes != nullptr && ib < a.nbocc) {
+    const int2 z = fx_block_size<PER, NW>(next, red);
+    if (tid == 0) a.sizes[ik * a.nbocc + ib] = z;
   }
   if (a.ex_cols) {
     exr = block_sum<NW>(exr, redd);
@@ -391,40 +429,11 @@ __global__ void __launch_bounds__(ColumnCta<N>::TH) k_combine_batch(const Combin
   combine_body<N>(args[r], blockIdx.x - pre[r]);
 }
 
-// Deferred exchange energy Ex = 0.5 sum_occ occ <u|F u> dvcell (F:165-183),
-// added to the Etot of the step whose orbitals produced F.
-__device__ __forceinline__ void ex_finalize_body(const ExArgs& a, int lane) {
-  int idx = a.idx;
-  if (idx < 0) idx = *a.it - 1;
-  if (idx < 0) return;
-  double ex = 0.0;
-  const int ncol = a.nk * a.nbocc;
-  for (int o = lane; o < ncol; o += 32) {
-    const int ik = o / a.nbocc, ib = o % a.nbocc;
-    ex += a.occ * a.colbuf[(size_t)(ik * a.nb + ib) * 4 + 2] * a.dvcell;
-  }
-  ex = 0.5 * warp_sum(ex);
-  if (lane != 0) return;
-  if (a.series_E) a.series_E[idx] = a.series_E[idx] + ex;
-  if (a.out) {
-    a.out[0] = a.out[0] + ex;
-    a.out[4] = ex;
-  }
-}
-
-__global__ void k_ex_finalize(ExArgs a) {
-  if (blockIdx.x == 0 && threadIdx.x < 32) ex_finalize_body(a, threadIdx.x);
-}
-
-__global__ void k_ex_finalize_batch(const ExArgs* __restrict__ args, int nruns) {
-  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (r < nruns) ex_finalize_body(args[r], threadIdx.x & 31);
-}
-
 // ---------------------------------------------------------------------------
 // Observable reduction (F:74-91, F:165-183, F:289-318) in reference order.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void obs_reduce_body(const ObsReduceArgs& a, int lane) {
+  if (a.advance == 3 && *a.it == 0) return;
   double ekin = 0.0, jre = 0.0, exr = 0.0;
   const int ncol = a.nk * a.nb;
   for (int c = lane; c < ncol; c += 32) {
@@ -433,15 +442,15 @@ __device__ __forceinline__ void obs_reduce_body(const ObsReduceArgs& a, int lane
     const double* cb = a.colbuf + (size_t)c * 4;
     ekin += occ * cb[0] * a.dvcell;
     jre += occ * cb[1];
-    if (ib < a.nbocc && !a.defer_ex) exr += occ * cb[2] * a.dvcell;
+    if (ib < a.nbocc && a.hf) exr += occ * cb[2] * a.dvcell;
   }
   ekin = warp_sum(ekin);
   jre = warp_sum(jre);
   exr = warp_sum(exr);
   if (lane != 0) return;
-  const double Ex = (a.hf && !a.defer_ex) ? 0.5 * exr : 0.0;
+  const double Ex = a.hf ? 0.5 * exr : 0.0;
   const double Eion = a.scal[1], EH = a.scal[2], Nele = a.scal[0];
-  const double Etot = a.defer_ex ? (ekin + Eion + EH) : (ekin + Eion + EH + Ex);
+  const double Etot = ekin + Eion + EH + Ex;
   const double Je = -(jre * a.dvcell / a.vcell);
   a.out[0] = Etot;
   a.out[1] = ekin;
@@ -451,7 +460,7 @@ __device__ __forceinline__ void obs_reduce_body(const ObsReduceArgs& a, int lane
   a.out[5] = Je;
   a.out[6] = Nele;
   if (a.advance) {
-    const int it = *a.it;
+    const int it = a.advance == 3 ? *a.it - 1 : *a.it;
     if (a.series_E) a.series_E[it] = Etot;
     if (a.series_J) a.series_J[it] = Je;
     if (a.series_N) a.series_N[it] = Nele;
@@ -522,7 +531,7 @@ static cudaError_t combine_impl(const CombineArgs& a, int ncols, cudaStream_t s)
   }
 
 cudaError_t launch_density(int NG, const DensArgs& a, cudaStream_t s) {
-  k_dens_partial<<<kDensChunks, 256, 0, s>>>(a, NG);
+  k_dens_partial<<<dim3(dens_chunks(a.nk * a.u.nb), (NG + 63) / 64), 64 * kDensSub, 0, s>>>(a, NG);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
 #define CALL(n) (k_density<n><<<1, (n) < 64 ? 64 : (n), 0, s>>>(a), cudaGetLastError())
@@ -576,11 +585,6 @@ int fock_sym_teams(int NG) {
   }
 }
 
-cudaError_t launch_ex_finalize(const ExArgs& a, cudaStream_t s) {
-  k_ex_finalize<<<1, 32, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_combine(int NG, const CombineArgs& a, int ncols, cudaStream_t s) {
 #define CALL(n) combine_impl<n>(a, ncols, s)
   MATTOHF_DISPATCH(NG, CALL)
@@ -589,7 +593,7 @@ cudaError_t launch_combine(int NG, const CombineArgs& a, int ncols, cudaStream_t
 
 // ---- batched launchers (many independent runs per launch) ----
 cudaError_t launch_density_batch(int NG, const DensArgs* d_args, int nruns, cudaStream_t s) {
-  k_dens_partial_batch<<<dim3(kDensChunks, nruns), 256, 0, s>>>(d_args, NG);
+  k_dens_partial_batch<<<dim3(kDensChunks, (NG + 63) / 64, nruns), 64 * kDensSub, 0, s>>>(d_args, NG);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
 #define CALL(n) (k_density_batch<n><<<nruns, (n) < 64 ? 64 : (n), 0, s>>>(d_args), cudaGetLastError())
@@ -607,11 +611,6 @@ cudaError_t launch_combine_batch(int NG, const CombineArgs* d_args, const int* d
 
 cudaError_t launch_obs_reduce_batch(const ObsReduceArgs* d_args, int nruns, cudaStream_t s) {
   k_obs_reduce_batch<<<(nruns + 3) / 4, 128, 0, s>>>(d_args, nruns);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ex_finalize_batch(const ExArgs* d_args, int nruns, cudaStream_t s) {
-  k_ex_finalize_batch<<<(nruns + 3) / 4, 128, 0, s>>>(d_args, nruns);
   return cudaGetLastError();
 }
 
