@@ -147,7 +147,8 @@ struct mattohf_ctx {
   double2 *d_ckpt = nullptr, *d_store = nullptr, *d_lam = nullptr, *d_lamu = nullptr, *d_vbuf = nullptr,
           *d_uN = nullptr, *d_u0 = nullptr;
   double2* d_lamk[4] = {nullptr, nullptr, nullptr, nullptr};
-  int4* d_mufx = nullptr;  // adjoint orbitals in limbs
+  int4* d_mufx = nullptr;  // adjoint orbitals in limbs and their sizes
+  int2* d_mu_sizes = nullptr;
   double *d_psi = nullptr, *d_sig = nullptr, *d_gcol = nullptr, *d_gstage = nullptr, *d_gvion = nullptr,
          *d_vloc_adj = nullptr, *d_dpart2 = nullptr;
   int* d_adj_int = nullptr;  // [0] step n, [1] segment start
@@ -358,7 +359,6 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   a.acc = ctx->d_fx_acc;
   a.lift = 1;
   a.halve = 0;
-  a.vscale = nullptr;
   return a;
 }
 
@@ -1080,7 +1080,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   destroy_graph(ctx);
   {
-    void* adj[] = {ctx->d_ckpt, ctx->d_store, ctx->d_lam, ctx->d_lamu, ctx->d_vbuf, ctx->d_mufx, ctx->d_uN,
+    void* adj[] = {ctx->d_ckpt, ctx->d_store, ctx->d_lam, ctx->d_lamu, ctx->d_vbuf, ctx->d_mufx, ctx->d_mu_sizes, ctx->d_uN,
                    ctx->d_u0, ctx->d_lamk[0], ctx->d_lamk[1], ctx->d_lamk[2], ctx->d_lamk[3], ctx->d_psi,
                    ctx->d_sig, ctx->d_gcol, ctx->d_gstage, ctx->d_gvion, ctx->d_vloc_adj, ctx->d_dpart2,
                    ctx->d_adj_int};
@@ -2039,12 +2039,12 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
       FockFxArgs fv = fx_args(ctx, vb, S), fm = fx_args(ctx, blk(ctx->d_lamk[s], NB, NG, NB), S);
       fv.lift = fm.lift = 0;
       fv.shift = fm.shift = nullptr;
-      fv.fscale = nullptr;
+      fv.fscale = fm.fscale = nullptr;
       fv.acc = nullptr;
       fm.halve = 1;  // the second pass subtracts two pair densities
       fm.ufx = reinterpret_cast<fx::lc*>(ctx->d_mufx);
-      fm.vscale = ctx->d_uscale;
       fm.uscale = ctx->d_uscale + 1;
+      fm.sizes = ctx->d_mu_sizes;
       FockAdjFxArgs f;
       f.v = fv.ufx;
       f.mu = fm.ufx;
@@ -2055,9 +2055,12 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
       f.kern = fv.kern;
       f.tw = fv.tw;
       f.acc = fm.acc;
+      f.vscale = fv.uscale;
+      f.muscale = fm.uscale;
+      f.kscale = fv.kscale;
+      f.fscale = ctx->d_fx_fscale;
       CKR(timed_begin(ctx));
-      CK(launch_fx_convert(NG, fv, nullptr, false, false, ctx->st));
-      CK(launch_fx_convert(NG, fm, nullptr, false, false, ctx->st));
+      CK(launch_fx_convert2(NG, fv, fm, ctx->st));
       CK(launch_fock_adj_fx(NG, f, ctx->st));
       CKR(timed_end(ctx));
     }
@@ -2129,6 +2132,7 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   CKR(ensure_scratch(ctx, NK * NB));
   destroy_graph(ctx);
   CKR(dalloc(ctx, &ctx->d_mufx, elems));
+  CKR(dalloc(ctx, &ctx->d_mu_sizes, (size_t)NK * NB));
   CKR(dalloc(ctx, &ctx->d_ckpt, elems * nseg));
   CKR(dalloc(ctx, &ctx->d_store, elems * 4 * C));
   double2** bufs[] = {&ctx->d_lam, &ctx->d_lamu, &ctx->d_vbuf, &ctx->d_uN, &ctx->d_u0,

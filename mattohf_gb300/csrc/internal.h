@@ -134,17 +134,20 @@ struct FockFxArgs {
   const fx::lc* tw;
   unsigned long long* acc;  // [NK*nbocc][4][NG] sums F^ (fx_accumulate), zeroed by the conversion
   // conversions for the adjoint (shift, fscale, acc may be null there): no lifting,
-  // a further 2^-halve in the scale, and the scale of v for mu's output scale
+  // a further 2^-halve in the scale
   int lift, halve;
-  const int2* vscale;
 };
 struct FockAdjFxArgs {
   const fx::lc *v, *mu;     // [NK*nbocc][NG] in limbs (FockFxArgs::ufx of two conversions)
   int nk, nbocc, S, T;
   const int2* kern;
   const fx::lc* tw;
+  const int2 *vscale, *muscale, *kscale;
   unsigned long long* acc;  // sums, as FockFxArgs::acc
+  double2* fscale;          // [NK*nbocc] their scale, written here
 };
+// v (a) and mu (b) to fixed point
+cudaError_t launch_fx_convert2(int NG, const FockFxArgs& a, const FockFxArgs& b, cudaStream_t s);
 cudaError_t launch_fock_adj_fx(int NG, const FockAdjFxArgs& a, cudaStream_t s);
 // Functions w that the exchange operator of the orbitals acts on.
 struct FockFxRows {

@@ -102,9 +102,8 @@ __device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, const FockF
   if (a.shift) a.shift[col] = d;
   if (col == 0) *a.uscale = make_int2(s.c, s.k);
   if (a.fscale) {
-    const Scale so = a.vscale ? Scale{a.vscale->x, a.vscale->y} : s;
     // a column of zeros has a sum of zero; the roundings of its terms do not count
-    a.fscale[col] = own.y > 0 || s.c == 0 || a.vscale ? fx_output_scale(so, sd, sk) : make_double2(0.0, 0.0);
+    a.fscale[col] = own.y > 0 || s.c == 0 ? fx_output_scale(s, sd, sk) : make_double2(0.0, 0.0);
   }
 }
 
@@ -116,6 +115,17 @@ __global__ void __launch_bounds__(128) k_fx_sizes(FockFxArgs a, int N) {
 }
 __global__ void __launch_bounds__(128) k_fx_convert(FockFxArgs a, FockFxRows r, int N, int first, int scan) {
   fx_convert_body(a, r, N, first + blockIdx.x, scan);
+}
+// two sets at once (blockIdx.y): the adjoint's v and mu
+__global__ void __launch_bounds__(128) k_fx_sizes2(FockFxArgs a, FockFxArgs b, int N) {
+  const FockFxArgs& c = blockIdx.y ? b : a;
+  const int col = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (col >= c.nk * c.nbocc) return;
+  const int2 z = fx_column_size(fx_column(c.u, c.nbocc, col, N), N, threadIdx.x & 31);
+  if ((threadIdx.x & 31) == 0) c.sizes[col] = z;
+}
+__global__ void __launch_bounds__(128) k_fx_convert2(FockFxArgs a, FockFxArgs b, int N) {
+  fx_convert_body(blockIdx.y ? b : a, FockFxRows{}, N, blockIdx.x, false);
 }
 // element prefix: pre[r] = sum over earlier runs of M_r * N
 __global__ void __launch_bounds__(128) k_fx_sizes_batch(const FockFxArgs* __restrict__ args,
@@ -395,6 +405,11 @@ __global__ void __launch_bounds__(sym_fx_threads<N>(), 2) k_fock_adj_fx(FockAdjF
   cx* buf = bufs + tw_ * N;
   int2* twn_s = reinterpret_cast<int2*>(cacc + S * N);  // kTwCount
   load_twiddles<N>(a.tw, tw_s, twn_s);
+  if (blockIdx.x == 0) {
+    const double2 f = fx_output_scale(Scale{a.vscale->x, a.vscale->y}, Scale{a.muscale->x, a.muscale->y},
+                                      Scale{a.kscale->x, a.kscale->y});
+    for (int i = tid; i < a.nk * a.nbocc; i += blockDim.x) a.fscale[i] = f;
+  }
   for (int i = tid; i < S * N; i += blockDim.x) cacc[i] = cx{0, 0};
   int ti = 0, rem = blockIdx.x;
   while (rem >= a.T - ti) { rem -= a.T - ti; ++ti; }
@@ -659,6 +674,13 @@ static cudaError_t fock_adj_fx_impl(const FockAdjFxArgs& a, cudaStream_t s) {
   size_t smem;
   sym_fx_shape<N>(a.S, &threads, &smem);
   k_fock_adj_fx<N><<<a.T * (a.T + 1) / 2, threads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_convert2(int NG, const FockFxArgs& a, const FockFxArgs& b, cudaStream_t s) {
+  const int M = a.nk * a.nbocc;
+  k_fx_sizes2<<<dim3((M + 3) / 4, 2), 128, 0, s>>>(a, b, NG);
+  k_fx_convert2<<<dim3(M, 2), 128, 0, s>>>(a, b, NG);
   return cudaGetLastError();
 }
 
