@@ -153,6 +153,13 @@ struct mattohf_ctx {
          *d_vloc_adj = nullptr, *d_dpart2 = nullptr;
   int* d_adj_int = nullptr;  // [0] step n, [1] segment start
   double last_adj_ms = 0, last_adj_fwd_ms = 0;
+  size_t ckpt_cap = 0, store_cap = 0;  // elements of d_ckpt and d_store
+  int gstage_cap = 0;                  // steps of d_gstage
+  // the adjoint's step graphs (forward, recompute, reverse; one step, then
+  // kGraphSteps) and what they were captured for
+  cudaGraphExec_t adj_exec[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  double adj_dt = 0;
+  int adj_C = 0, adj_phase = 0;
   // graph of one RK4 step
   cudaGraphExec_t step_exec = nullptr;
   cudaGraphExec_t multi_exec = nullptr;  // kGraphSteps steps in one graph
@@ -780,6 +787,10 @@ int sync_and_flag(mattohf_ctx* ctx) {
 }
 
 void destroy_graph(mattohf_ctx* c) {
+  for (auto& g : c->adj_exec) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
   if (c->step_exec) {
     cudaGraphExecDestroy(c->step_exec);
     c->step_exec = nullptr;
@@ -930,8 +941,10 @@ void ion_param_grad(const mattohf_ctx* c, const double* g, double* dZ, double* d
 // The adjoint's segment storage (checkpoints and stage inputs), the only
 // buffers of the adjoint that scale with the window.
 void release_adjoint_storage(mattohf_ctx* ctx) {
+  destroy_graph(ctx);
   dalloc(ctx, &ctx->d_ckpt, 0);
   dalloc(ctx, &ctx->d_store, 0);
+  ctx->ckpt_cap = ctx->store_cap = 0;
 }
 
 int ensure_series(mattohf_ctx* ctx, int nt) {
@@ -2111,10 +2124,11 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   // C >= nt).  Automatic (ckpt_every <= 0): the largest C whose stage inputs
   // (4 per step), checkpoints and work buffers fit in three quarters of the
   // free device memory.
-  release_adjoint_storage(ctx);   // a previous call's segments do not count against this one
   CKR(ensure_fock_buffers(ctx));
   size_t freeb = 0, totalb = 0;
   CK(cudaMemGetInfo(&freeb, &totalb));
+  // a previous call's segments do not count against this one
+  freeb += sizeof(double2) * (ctx->ckpt_cap + ctx->store_cap);
   int C = ckpt_every;
   if (C <= 0) {
     const long long slots = (long long)(freeb / 4 * 3 / (sizeof(double2) * elems));   // stage-input sized
@@ -2130,22 +2144,35 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   if (need > freeb) return fail(ctx, MATTOHF_ERR_ALLOC, "checkpoint storage exceeds free device memory; lower ckpt_every");
   CKR(ensure_series(ctx, nt));
   CKR(ensure_scratch(ctx, NK * NB));
-  destroy_graph(ctx);
-  CKR(dalloc(ctx, &ctx->d_mufx, elems));
-  CKR(dalloc(ctx, &ctx->d_mu_sizes, (size_t)NK * NB));
-  CKR(dalloc(ctx, &ctx->d_ckpt, elems * nseg));
-  CKR(dalloc(ctx, &ctx->d_store, elems * 4 * C));
-  double2** bufs[] = {&ctx->d_lam, &ctx->d_lamu, &ctx->d_vbuf, &ctx->d_uN, &ctx->d_u0,
-                      &ctx->d_lamk[0], &ctx->d_lamk[1], &ctx->d_lamk[2], &ctx->d_lamk[3]};
-  for (double2** b : bufs) CKR(dalloc(ctx, b, elems));
-  CKR(dalloc(ctx, &ctx->d_psi, NG));
-  CKR(dalloc(ctx, &ctx->d_sig, NG));
-  CKR(dalloc(ctx, &ctx->d_vloc_adj, NG));
-  CKR(dalloc(ctx, &ctx->d_gvion, NG));
-  CKR(dalloc(ctx, &ctx->d_dpart2, (size_t)kDensChunks * NG));
-  CKR(dalloc(ctx, &ctx->d_gcol, (size_t)NK * NB));
-  CKR(dalloc(ctx, &ctx->d_gstage, (size_t)nt * 4));
-  CKR(dalloc(ctx, &ctx->d_adj_int, 4));
+  // buffers and step graphs are kept for the next call: an optimisation loop
+  // calls this once per iterate, and 17 allocations and six captures took 2 ms
+  if (!ctx->d_mufx) {
+    double2** bufs[] = {&ctx->d_lam, &ctx->d_lamu, &ctx->d_vbuf, &ctx->d_uN, &ctx->d_u0,
+                        &ctx->d_lamk[0], &ctx->d_lamk[1], &ctx->d_lamk[2], &ctx->d_lamk[3]};
+    for (double2** b : bufs) CKR(dalloc(ctx, b, elems));
+    CKR(dalloc(ctx, &ctx->d_mu_sizes, (size_t)NK * NB));
+    CKR(dalloc(ctx, &ctx->d_psi, NG));
+    CKR(dalloc(ctx, &ctx->d_sig, NG));
+    CKR(dalloc(ctx, &ctx->d_vloc_adj, NG));
+    CKR(dalloc(ctx, &ctx->d_gvion, NG));
+    CKR(dalloc(ctx, &ctx->d_dpart2, (size_t)kDensChunks * NG));
+    CKR(dalloc(ctx, &ctx->d_gcol, (size_t)NK * NB));
+    CKR(dalloc(ctx, &ctx->d_adj_int, 4));
+    CKR(dalloc(ctx, &ctx->d_mufx, elems));
+  }
+  if (elems * nseg > ctx->ckpt_cap || elems * 4 * C > ctx->store_cap) {
+    release_adjoint_storage(ctx);
+    CKR(dalloc(ctx, &ctx->d_ckpt, elems * nseg));
+    ctx->ckpt_cap = elems * nseg;
+    CKR(dalloc(ctx, &ctx->d_store, elems * 4 * C));
+    ctx->store_cap = elems * 4 * C;
+  }
+  if (nt > ctx->gstage_cap) {
+    destroy_graph(ctx);
+    ctx->gstage_cap = 0;
+    CKR(dalloc(ctx, &ctx->d_gstage, (size_t)nt * 4));
+    ctx->gstage_cap = nt;
+  }
   // fields (RT:227-230)
   std::vector<double> Ah(A, A + nt), Aave(nt);
   Aave[0] = 0.5 * (Ah[0] + 0.0);
@@ -2174,27 +2201,28 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   CK(cudaMemcpyAsync(rho0.data(), ctx->d_rho, sizeof(double) * NG, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaMemcpyAsync(ctx->d_u0, ctx->d_u, sizeof(double2) * elems, cudaMemcpyDeviceToDevice, ctx->st));
   CK(cudaMemsetAsync(ctx->d_int, 0, 2 * sizeof(int), ctx->st));
-  // the three step graphs, destroyed on every exit path
-  // each loop also as kGraphSteps steps in one graph (a graph launch is a
-  // full dependency; inside a graph the stages overlap)
-  struct Execs {
-    cudaGraphExec_t g[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    ~Execs() {
-      for (auto x : g)
-        if (x) cudaGraphExecDestroy(x);
-    }
-  } ex;
-  cudaGraphExec_t &gfwd = ex.g[0], &grec = ex.g[1], &gadj = ex.g[2];
-  cudaGraphExec_t &gfwd8 = ex.g[3], &grec8 = ex.g[4], &gadj8 = ex.g[5];
-  auto capture_steps = [&](cudaGraphExec_t* one, cudaGraphExec_t* many, const std::function<int()>& body) {
-    int rc = capture(ctx, one, body);
-    if (rc == MATTOHF_OK)
-      rc = capture(ctx, many, [&]() {
+  // the three step graphs, each also as kGraphSteps steps in one graph (a graph
+  // launch is a full dependency; inside a graph the stages overlap), captured when
+  // a call first replays that many steps
+  if (ctx->adj_dt != dt || ctx->adj_C != C || ctx->adj_phase != phase) {
+    destroy_graph(ctx);
+    ctx->adj_dt = dt;
+    ctx->adj_C = C;
+    ctx->adj_phase = phase;
+  }
+  cudaGraphExec_t* const gx = ctx->adj_exec;
+  auto capture_steps = [&](int which, bool one, bool many, const std::function<int()>& body) -> int {
+    if (one && !gx[which]) CKR(capture(ctx, &gx[which], body));
+    if (many && !gx[which + 3])
+      CKR(capture(ctx, &gx[which + 3], [&]() -> int {
         for (int k = 0; k < kGraphSteps; ++k) CKR(body());
         return MATTOHF_OK;
-      });
-    return rc;
+      }));
+    return MATTOHF_OK;
   };
+  // does a replay of n steps launch the single step, the multiple one?
+  auto ones = [](int n) { return n % kGraphSteps != 0; };
+  auto manys = [](int n) { return n >= kGraphSteps; };
   auto replay = [&](cudaGraphExec_t one, cudaGraphExec_t many, int n) -> int {
     int j = 0;
     for (; j + kGraphSteps <= n; j += kGraphSteps) CK(cudaGraphLaunch(many, ctx->st));
@@ -2209,20 +2237,20 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   // gfwd: a step that keeps the segment checkpoint; grec: a step that stores
   // its stage inputs (the last segment in the forward pass, and every
   // recomputed segment)
-  int rc = MATTOHF_OK;
+  const int len0 = nseg > 1 ? C - phase : nt;  // steps of the first segment; the others have C
   if (nseg > 1)
-    rc = capture_steps(&gfwd, &gfwd8, [&]() {
+    CKR(capture_steps(0, ones(s_last), manys(s_last), [&]() -> int {
       // the fused stage 0 writes the checkpoint itself
       if (use_small(ctx)) return enq_small_step(ctx, fm, fave, fcur, dt, false, C, phase);
       CK(launch_checkpoint(ctx->d_ckpt, ctx->d_u, ctx->d_int, C, phase, elems, ctx->st));
       CKR(enq_rk4(ctx, fm, fave, fcur, dt));
       CK(launch_counter_add(ctx->d_int, 1, ctx->st));
       return MATTOHF_OK;
-    });
-  if (rc == MATTOHF_OK)
-    rc = capture_steps(&grec, &grec8, [&]() { return enq_recompute_step(ctx, fm, fave, fcur, dt); });
-  if (rc == MATTOHF_OK) rc = capture_steps(&gadj, &gadj8, [&]() { return enq_adjoint_step(ctx, dt, elems); });
-  if (rc != MATTOHF_OK) return rc;
+    }));
+  const bool one = ones(len0) || (nseg > 1 && ones(C)), many = manys(len0) || (nseg > 1 && manys(C));
+  CKR(capture_steps(1, one, many, [&]() { return enq_recompute_step(ctx, fm, fave, fcur, dt); }));
+  CKR(capture_steps(2, one, many, [&]() { return enq_adjoint_step(ctx, dt, elems); }));
+  const cudaGraphExec_t gfwd = gx[0], grec = gx[1], gadj = gx[2], gfwd8 = gx[3], grec8 = gx[4], gadj8 = gx[5];
   if (nseg > 1) CKR(replay(gfwd, gfwd8, s_last));
   // the last segment's stage inputs go to store slots it - s_last
   CK(cudaMemcpyAsync(ctx->d_adj_int + 1, &s_last, sizeof(int), cudaMemcpyHostToDevice, ctx->st));
