@@ -57,9 +57,17 @@ struct ColumnCta {
 // Value of an exchange source.
 __device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, int q, int N) {
   if (s.f != nullptr) return s.f[(size_t)col * N + q];
-  const unsigned long long* p = s.acc + (size_t)col * 4 * N + q;
-  const i64 hx = (i64)p[0], lx = (i64)p[N], hy = (i64)p[2 * N], ly = (i64)p[3 * N];
   const double2 f = s.scale[col];
+  const unsigned long long* p;
+  size_t stride;
+  if (s.dm != nullptr) {
+    stride = s.dm_nk;
+    p = s.dm + 4 * ((size_t)q * s.dm_nb + col % s.dm_nb) * stride + col / s.dm_nb;
+  } else {
+    stride = N;
+    p = s.acc + (size_t)col * 4 * N + q;
+  }
+  const i64 hx = (i64)p[0], lx = (i64)p[stride], hy = (i64)p[2 * stride], ly = (i64)p[3 * stride];
   double x, y;
   // one conversion where the sums fit 64 bits (they can only outgrow them when
   // very many equal localised orbitals add up)

@@ -109,6 +109,14 @@ struct mattohf_ctx {
   double2* d_wscale = nullptr;
   unsigned long long *d_fx_acc = nullptr, *d_wacc = nullptr;  // exchange sums
   size_t wfx_cap = 0;
+  // exchange through the density matrix (k_fock_dm.cu), made when first used
+  int4 *d_dm_ut = nullptr, *d_dm_wt = nullptr, *d_dm_table = nullptr, *d_dm_tw = nullptr, *d_dm_W = nullptr;
+  int2* d_dm_tscale = nullptr;
+  unsigned long long* d_dm_acc = nullptr;
+  double2* d_dm_wscale = nullptr;
+  size_t dm_cols = 0;         // columns of d_dm_wt and d_dm_acc
+  bool dm_last = false;       // the last exchange went through it
+  int opt_dm = -1;            // 1 / 0: the autotuner's choice; -1: by rule
   int2* d_kern_fx = nullptr;  // kernel table in limbs, its scale, the twiddles
   int2* d_kscale = nullptr;
   int4* d_tw_fx = nullptr;
@@ -279,6 +287,7 @@ struct FockPlan {
   bool occ = false;           // occupied bands by the symmetric exchange
   int b0 = 0;                 // first band of the others
   bool rows = false;          // bands >= b0 by the exchange on rows
+  bool dm = false;            // all bands through the density matrix
   bool any = false;           // exchange present at all
 };
 
@@ -369,6 +378,10 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   return a;
 }
 
+std::vector<int4> fx_twiddles_host(int NG);
+bool use_dm(const mattohf_ctx* c, int nbw, bool same);
+int ensure_dm(mattohf_ctx* ctx, int ncols);
+
 size_t sym_partials(int M, int S, int NG) {
   const size_t T = (M + S - 1) / S;
   return T * (T + 1) / 2 * 2 * S * NG;
@@ -391,7 +404,118 @@ int ensure_fock_buffers(mattohf_ctx* ctx) {
   const int M = ctx->NK * ctx->NBocc;
   if (ctx->opt_df) CKR(ensure_sym(ctx, sym_partials(M, sym_tile(ctx), ctx->NG)));
   CKR(ensure_fx(ctx));
+  if (use_dm(ctx, ctx->NB, true)) CKR(ensure_dm(ctx, ctx->NK * ctx->NB));  // or to the pairs
   if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * ctx->NG));
+  return MATTOHF_OK;
+}
+
+// Is the exchange of h[u] on nbw bands per k-point (w = u: same) cheaper through
+// the density matrix (k_fock_dm.cu) than by pairs (k_fock_fx.cu)?  In 32 x 32 +
+// 64-bit multiply-adds; those of the density matrix run a third faster (0.186
+// against 0.248 us a million, 512 / 32 / 8) and its five launches cost about 16 us
+// more, the time of 65 million.  Measured, us per RK4 step, NG / NK / bands, pairs
+// against density matrix: 64/32/4 132 176, 128/16/8 162 172, 128/32/4 163 195,
+// 256/16/8 253 275, 256/32/4 250 330, 512/64/4 1510 1901; 256/64/4 746 588,
+// 512/32/8 1510 1332.  Grids below 64 points stay with pairs: few terms average
+// less of W's rounding, 2.1e-16 at 16 / 33 / 2 and 1.4e-16 at 32 / 40 / 2 against
+// 7e-17 and 5e-17 (from 64 points on at most 1.2e-16).
+bool fock_dm_wins(const mattohf_ctx* c, int nbw, bool same) {
+  const double N = c->NG, NK = c->NK, no = c->NBocc, M = NK * no;
+  const int lh = dm_length(c->NK) / 2;
+  if (2 * lh > 512 || c->NG < 64) return false;
+  if (N * (N + 1) / 2 * NK * 16 > 2147483648.0) return false;  // bytes of W
+  const double pairs = same ? 87.0 * M * M / 2 * N + 75.0 * M * NK * (nbw - no) * N : 75.0 * M * NK * nbw * N;
+  const double dm = N * N / 2 * lh * (12 * no + 114) + N * N * NK * 12 * nbw;
+  return 0.75 * dm + 6.5e7 < pairs;
+}
+bool use_dm(const mattohf_ctx* c, int nbw, bool same) {
+  if (!c->opt_sym || c->opt_df || c->opt_chunks > 0 || c->opt_dm == 0) return false;
+  if (c->opt_dm < 0 && c->opt_tile > 0) return false;  // a tile asked for: pairs
+  return fock_dm_wins(c, nbw, same);
+}
+
+// No memory for W or the sums: the pair kernels take over, which need none of it.
+int dm_no_room(mattohf_ctx* ctx) {
+  cudaGetLastError();
+  ctx->opt_dm = 0;
+  ctx->err.clear();
+  return MATTOHF_OK;
+}
+
+// Its buffers for ncols columns of w, and (once) its tables.  Where there is no
+// memory for them, opt_dm = 0 afterwards.
+int ensure_dm(mattohf_ctx* ctx, int ncols) {
+  const int NG = ctx->NG, NK = ctx->NK, L = dm_length(NK);
+  if (!ctx->d_dm_table) {
+    if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "density-matrix tables during capture");
+    const std::vector<int4> tw = fx_twiddles_host(L);
+    struct Tmp {
+      int4* p = nullptr;
+      ~Tmp() {
+        if (p) cudaFree(p);
+      }
+    } v, raw, mx, roots;
+    std::vector<longlong2> rt(L);  // exp(-2 pi i t / L) 2^60
+    for (int t = 0; t < L; ++t) {
+      const long double th = -2.0L * acosl(-1.0L) * (long double)t / (long double)L;
+      rt[t] = make_longlong2(llrintl(ldexpl(cosl(th), 60)), llrintl(ldexpl(sinl(th), 60)));
+    }
+    const size_t nu = (size_t)NG * ctx->NBocc * (L / 2);
+    int4* table = nullptr;
+    if (dalloc(ctx, &ctx->d_dm_W, (size_t)NG * (NG + 1) / 2 * NK) || dalloc(ctx, &ctx->d_dm_ut, nu)) return dm_no_room(ctx);
+    CKR(dalloc(ctx, &v.p, (size_t)(2 * NK - 1) * NG));
+    CKR(dalloc(ctx, &raw.p, (size_t)NG * L));
+    CKR(dalloc(ctx, &mx.p, 1));
+    CKR(dalloc(ctx, &roots.p, (size_t)L));
+    CK(cudaMemcpyAsync(roots.p, rt.data(), L * sizeof(longlong2), cudaMemcpyHostToDevice, ctx->st));
+    CKR(dalloc(ctx, &ctx->d_dm_tw, tw.size()));
+    CKR(dalloc(ctx, &ctx->d_dm_tscale, 2));  // and the largest density
+    CK(cudaMemsetAsync(ctx->d_dm_tscale, 0, 2 * sizeof(int2), ctx->st));
+    CKR(dalloc(ctx, &table, (size_t)NG * L));
+    CK(cudaMemcpyAsync(ctx->d_dm_tw, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemsetAsync(ctx->d_dm_ut, 0, nu * sizeof(int4), ctx->st));
+    CK(launch_dm_table(NG, NK, ctx->d_kern_fx, reinterpret_cast<const fx::lc*>(ctx->d_tw_fx),
+                       reinterpret_cast<const fx::cx*>(roots.p), reinterpret_cast<fx::cx*>(v.p),
+                       reinterpret_cast<fx::cx*>(raw.p), reinterpret_cast<int*>(mx.p), reinterpret_cast<fx::lc*>(table),
+                       ctx->d_dm_tscale, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    ctx->d_dm_table = table;
+  }
+  if ((size_t)ncols > ctx->dm_cols) {
+    if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
+    destroy_graph(ctx);
+    ctx->dm_cols = 0;
+    if (dalloc(ctx, &ctx->d_dm_wt, (size_t)ncols * NG) || dalloc(ctx, &ctx->d_dm_acc, (size_t)ncols * NG * 4) ||
+        dalloc(ctx, &ctx->d_dm_wscale, (size_t)ncols))
+      return dm_no_room(ctx);
+    ctx->dm_cols = ncols;
+  }
+  return MATTOHF_OK;
+}
+
+int enq_fock_dm(mattohf_ctx* ctx, Block u, Block w, bool same_u, bool have_sizes) {
+  FockDmArgs a;
+  a.u = u;
+  a.w = w;
+  a.nk = ctx->NK;
+  a.nbocc = ctx->NBocc;
+  a.lh = dm_length(ctx->NK) / 2;
+  a.sizes = ctx->d_fx_sizes;
+  a.uscale = ctx->d_uscale;
+  a.kscale = ctx->d_kscale;
+  a.tscale = ctx->d_dm_tscale;
+  a.nmax = reinterpret_cast<int*>(ctx->d_dm_tscale + 1);
+  a.ut = reinterpret_cast<fx::lc*>(ctx->d_dm_ut);
+  a.wt = reinterpret_cast<fx::lc*>(ctx->d_dm_wt);
+  a.table = reinterpret_cast<const fx::lc*>(ctx->d_dm_table);
+  a.twL = reinterpret_cast<const fx::lc*>(ctx->d_dm_tw);
+  a.W = reinterpret_cast<fx::lc*>(ctx->d_dm_W);
+  a.acc = ctx->d_dm_acc;
+  a.wscale = ctx->d_dm_wscale;
+  if (!have_sizes && !same_u) CK(launch_fx_sizes(ctx->NG, fx_args(ctx, u, 1), ctx->st));
+  CK(launch_dm_convert(ctx->NG, a, same_u, ctx->st));
+  if (!same_u) CK(launch_dm_build(ctx->NG, a, ctx->nsm, ctx->st));
+  CK(launch_dm_apply(ctx->NG, a, ctx->nsm, ctx->st));
   return MATTOHF_OK;
 }
 
@@ -405,6 +529,24 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = f
   const bool same = (w.p == u.p) && (w.kstride == u.kstride) && (w.nb == u.nb);
   const int NG = ctx->NG;
   const int M = ctx->NK * ctx->NBocc;
+  bool dm = use_dm(ctx, w.nb, same);
+  if (dm) {
+    CKR(ensure_fx(ctx));
+    CKR(ensure_dm(ctx, ctx->NK * w.nb));
+    dm = ctx->opt_dm != 0;
+  }
+  if (dm) {
+    plan->dm = true;
+    // W of the same u: only if it was made by this path
+    const bool have_W = same_u && ctx->dm_last;
+    CKR(timed_begin(ctx));
+    CKR(enq_fock_dm(ctx, u, w, have_W, have_sizes || same_u));
+    CKR(timed_end(ctx));
+    ctx->dm_last = true;
+    return MATTOHF_OK;
+  }
+  if (same_u && ctx->dm_last) same_u = false;  // its orbitals are not in this path's fixed point
+  ctx->dm_last = false;
   plan->occ = same && ctx->opt_sym;
   plan->b0 = plan->occ ? ctx->NBocc : 0;
   plan->rows = w.nb > plan->b0;
@@ -449,7 +591,8 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = f
 
 // The symmetric exchange's result, of the fixed-point or the double-float kernels.
 ExSource occ_source(const mattohf_ctx* ctx, bool df) {
-  return df ? ExSource{nullptr, nullptr, ctx->d_symF} : ExSource{ctx->d_fx_acc, ctx->d_fx_fscale, nullptr};
+  return df ? ExSource{nullptr, nullptr, ctx->d_symF, nullptr, 0, 0}
+            : ExSource{ctx->d_fx_acc, ctx->d_fx_fscale, nullptr, nullptr, 0, 0};
 }
 
 CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const FockPlan& fp) {
@@ -458,7 +601,9 @@ CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const F
   a.w = w;
   const bool ex = ctx->hf && mode != CM_T && fp.any;
   if (ex && fp.occ) a.occ_ex = occ_source(ctx, ctx->opt_df);
-  if (ex && fp.rows) a.row_ex = ExSource{ctx->d_wacc, ctx->d_wscale, nullptr};
+  if (ex && fp.rows) a.row_ex = ExSource{ctx->d_wacc, ctx->d_wscale, nullptr, nullptr, 0, 0};
+  if (ex && fp.dm)
+    a.row_ex = ExSource{nullptr, ctx->d_dm_wscale, nullptr, ctx->d_dm_acc, w.nb, ctx->NK};
   a.row_b0 = fp.b0;
   a.vloc = ctx->d_vloc;
   a.Gx = ctx->d_Gx;
@@ -620,14 +765,14 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
 bool use_small(const mattohf_ctx* ctx) {
   if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
   if (ctx->opt_small == 1) return true;
-  // measured on GB300 with mattohf_autotune (us per step, fused vs tiled):
-  // NG=64 NK=8 Nocc=2 29 vs 129; NG=128 NK=16 Nocc=2 and NK=8 Nocc=4 96 vs 235
-  // (M^2 NG = 2^17); NG=64 NK=16 Nocc=4 171 vs 156, NG=64 NK=32 Nocc=2 173 vs
-  // 158 (2^18); NG=256 NK=8 Nocc=4 178 vs 253 (2^18, M = 32); NG=128 NK=32
-  // Nocc=2 320 vs 285 (2^19)
+  // us per RK4 step, fused against tiled, NG / NK / occupied bands: 16/4/2 24 57;
+  // 32/16/2 29 70; 64/8/2 29 78; 128/8/2 71 89; 128/8/3 72 90; 64/8/4 86 80 and
+  // 128/8/4 95 92, both even with the adjoint's reverse steps (208 221, 259 263);
+  // 64/16/4 (M^2 NG = 2^18) 172 97.  At 256 points an FP64 pair takes a warp twice as
+  // long: 256/8/2 83 104, 256/6/4 177 105, 256/8/4 257 107.
   const size_t M = (size_t)ctx->NK * ctx->NBocc;
   if (ctx->NK * ctx->NB > 64) return false;
-  return M * M * ctx->NG <= ((size_t)1 << 17) || (ctx->NG == 256 && M <= 32);
+  return M * M * ctx->NG <= ((size_t)1 << 17) && (ctx->NG < 256 || M <= 16);
 }
 
 // CTAs per column.  A warp issues at most one FP64 instruction per ~64
@@ -1039,6 +1184,7 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
     e = configure_fx_kernels();
+    if (e == cudaSuccess) e = configure_dm_kernels();
     if (e == cudaSuccess) e = configure_df_kernels();
     if (e == cudaSuccess) e = configure_small_kernels();
     if (e == cudaSuccess) e = configure_small_adj_kernels();
@@ -1114,7 +1260,8 @@ int mattohf_destroy(mattohf_ctx* ctx) {
                   ctx->d_eps, ctx->d_err, ctx->d_sym, ctx->d_symF, ctx->d_dpart,
                   ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale,
                   ctx->d_wfx, ctx->d_wscale, ctx->d_fx_acc, ctx->d_wacc, ctx->d_kern_fx, ctx->d_kscale,
-                  ctx->d_tw_fx, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
+                  ctx->d_tw_fx, ctx->d_dm_ut, ctx->d_dm_wt, ctx->d_dm_table, ctx->d_dm_tw, ctx->d_dm_W,
+                  ctx->d_dm_tscale, ctx->d_dm_acc, ctx->d_dm_wscale, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
                   ctx->d_small_part, ctx->d_small_obs};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1141,6 +1288,7 @@ int mattohf_set_option(mattohf_ctx* ctx, int option, long long value) {
       if (value < 0 || value > fock_sym_teams(ctx->NG) || (value & (value - 1)))
         return fail(ctx, MATTOHF_ERR_ARG, "tile size must be 0 or a power of two up to the CTA's teams");
       ctx->opt_tile = (int)value;
+      ctx->opt_dm = -1;
       break;
     case MATTOHF_OPT_SMALL_STAGES:
       if (value < 0 || value > 2) return fail(ctx, MATTOHF_ERR_ARG, "small-stage option must be 0, 1 or 2");
@@ -1651,12 +1799,7 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
   if (ctx->hf && ctx->opt_sym && ctx->NBocc > 0) {
     const int reps = std::max(2, std::min(steps, 20));
     double best = 1e300;
-    const int M = NK * ctx->NBocc, Smax = ctx->opt_df ? fock_sym_teams(NG) : std::min(kFxMaxTile, fock_sym_teams(NG));
-    for (int S = 1; S <= Smax; S <<= 1) {
-      // tiles far beyond a few waves only add partial-sum traffic (and scratch)
-      const long long T = (M + S - 1) / S;
-      if (S < Smax && T * (T + 1) / 2 > 32LL * ctx->nsm) continue;
-      ctx->opt_tile = S;
+    auto time_exchange = [&](double* t) -> int {
       CKR(ensure_fock_buffers(ctx));
       const Block ub = blk(ctx->d_u, NB, NG, NB);
       FockPlan fp;
@@ -1667,13 +1810,33 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
       CK(cudaEventSynchronize(e1));
       float ms = 0;
       CK(cudaEventElapsedTime(&ms, e0, e1));
-      const double t = 1e3 * ms / reps;
+      *t = 1e3 * ms / reps;
+      return MATTOHF_OK;
+    };
+    const int M = NK * ctx->NBocc, Smax = ctx->opt_df ? fock_sym_teams(NG) : std::min(kFxMaxTile, fock_sym_teams(NG));
+    ctx->opt_dm = 0;
+    for (int S = 1; S <= Smax; S <<= 1) {
+      // tiles far beyond a few waves only add partial-sum traffic (and scratch)
+      const long long T = (M + S - 1) / S;
+      if (S < Smax && T * (T + 1) / 2 > 32LL * ctx->nsm) continue;
+      ctx->opt_tile = S;
+      double t = 0.0;
+      CKR(time_exchange(&t));
       if (t < best) {
         best = t;
         bestS = S;
       }
     }
     ctx->opt_tile = bestS;
+    // the density-matrix form, where it is in question, against the best tile
+    ctx->opt_dm = -1;
+    if (!ctx->opt_df && ctx->opt_chunks == 0 && fock_dm_wins(ctx, NB, true)) {
+      ctx->opt_dm = 1;
+      double t = 0.0;
+      CKR(time_exchange(&t));
+      ctx->opt_dm = t < best ? 1 : 0;
+      best = std::min(best, t);
+    }
     tS = best;
   }
   // ---- stepping: tiled, then the fused stages for each P
@@ -2019,7 +2182,7 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
     AdjCombineArgs c;
     c.mu = ctx->d_lamk[s];
     c.v = ctx->d_vbuf;
-    c.fa = ctx->hf ? occ_source(ctx, false) : ExSource{nullptr, nullptr, nullptr};
+    c.fa = ctx->hf ? occ_source(ctx, false) : ExSource{nullptr, nullptr, nullptr, nullptr, 0, 0};
     c.psi = ctx->d_psi;
     c.vloc = ctx->d_vloc;
     c.Gx = ctx->d_Gx;

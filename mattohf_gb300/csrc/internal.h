@@ -149,6 +149,30 @@ struct FockAdjFxArgs {
 // v (a) and mu (b) to fixed point
 cudaError_t launch_fx_convert2(int NG, const FockFxArgs& a, const FockFxArgs& b, cudaStream_t s);
 cudaError_t launch_fock_adj_fx(int NG, const FockAdjFxArgs& a, cudaStream_t s);
+// Exchange through the density matrix (k_fock_dm.cu).
+constexpr int kDmThreads = 128;  // CTA of its first kernel
+constexpr int kDmTerms = 32;     // terms that its accumulators take
+struct FockDmArgs {
+  Block u, w;               // occupied orbitals; functions w, [nk][w.nb]
+  int nk, nbocc, lh;        // lh = half the transform length over k
+  const int2* sizes;        // of the orbitals (fx_size)
+  int* nmax;                // largest density (k_dm_density); zero between applies
+  int2* uscale;
+  const int2 *kscale, *tscale;
+  fx::lc *ut, *wt;          // [NG][nbocc][lh], [NG][w.nb][nk] in limbs
+  const fx::lc* table;      // [NG][2 lh]
+  const fx::lc* twL;
+  fx::lc* W;                // [NG (NG + 1) / 2][nk]
+  unsigned long long* acc;  // [NG][w.nb][4][nk]: words as FockFxArgs::acc
+  double2* wscale;          // [nk][w.nb]
+};
+int dm_length(int NK);
+cudaError_t launch_dm_table(int N, int NK, const int2* kern, const fx::lc* twN, const fx::cx* roots, fx::cx* v, fx::cx* raw,
+                            int* maxsum, fx::lc* table, int2* scale, cudaStream_t s);
+cudaError_t launch_dm_convert(int NG, const FockDmArgs& a, bool have_orbitals, cudaStream_t s);
+cudaError_t launch_dm_build(int NG, const FockDmArgs& a, int nsm, cudaStream_t s);
+cudaError_t launch_dm_apply(int NG, const FockDmArgs& a, int nsm, cudaStream_t s);
+cudaError_t configure_dm_kernels();
 // Functions w that the exchange operator of the orbitals acts on.
 struct FockFxRows {
   Block w;
@@ -243,6 +267,9 @@ struct ExSource {
   const unsigned long long* acc;
   const double2* scale;
   const double2* f;
+  // or sums with k fastest, [NG][dm_nb][4][dm_nk] (k_fock_dm.cu), and scale
+  const unsigned long long* dm;
+  int dm_nb, dm_nk;
 };
 
 struct CombineArgs {

@@ -220,7 +220,7 @@ __device__ __forceinline__ bool exchange_at(const CombineArgs& a, int ik, int ib
     *f = exchange_value(a.occ_ex, ik * a.nbocc + ib, q, N);
     return true;
   }
-  if (a.row_ex.acc == nullptr) return false;
+  if (a.row_ex.acc == nullptr && a.row_ex.dm == nullptr) return false;
   *f = exchange_value(a.row_ex, ik * (a.w.nb - a.row_b0) + (ib - a.row_b0), q, N);
   return true;
 }
