@@ -437,6 +437,13 @@ bool use_dm(const mattohf_ctx* c, int nbw, bool same) {
 // No memory for W or the sums: the pair kernels take over, which need none of it.
 int dm_no_room(mattohf_ctx* ctx) {
   cudaGetLastError();
+  destroy_graph(ctx);
+  CKR(dalloc(ctx, &ctx->d_dm_W, 0));
+  CKR(dalloc(ctx, &ctx->d_dm_ut, 0));
+  CKR(dalloc(ctx, &ctx->d_dm_table, 0));
+  CKR(dalloc(ctx, &ctx->d_dm_wt, 0));
+  CKR(dalloc(ctx, &ctx->d_dm_acc, 0));
+  ctx->dm_cols = 0;
   ctx->opt_dm = 0;
   ctx->err.clear();
   return MATTOHF_OK;
@@ -455,11 +462,7 @@ int ensure_dm(mattohf_ctx* ctx, int ncols) {
         if (p) cudaFree(p);
       }
     } v, raw, mx, roots;
-    std::vector<longlong2> rt(L);  // exp(-2 pi i t / L) 2^60
-    for (int t = 0; t < L; ++t) {
-      const long double th = -2.0L * acosl(-1.0L) * (long double)t / (long double)L;
-      rt[t] = make_longlong2(llrintl(ldexpl(cosl(th), 60)), llrintl(ldexpl(sinl(th), 60)));
-    }
+    const std::vector<longlong2> rt = fx_roots(L);
     const size_t nu = (size_t)NG * ctx->NBocc * (L / 2);
     int4* table = nullptr;
     if (dalloc(ctx, &ctx->d_dm_W, (size_t)NG * (NG + 1) / 2 * NK) || dalloc(ctx, &ctx->d_dm_ut, nu)) return dm_no_room(ctx);

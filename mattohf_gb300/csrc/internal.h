@@ -1,5 +1,6 @@
 // Internal declarations shared by the host runtime and the kernel translation units.
 #pragma once
+#include <vector>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -198,6 +199,7 @@ cudaError_t launch_fock_sym_fx_batch(int NG, const FockFxArgs* d_args, const int
                                      int total_tiles, const int* d_elem_pre, int total_elems, cudaStream_t s);
 // kernel table in limbs and its scale (device)
 cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int2* out, cudaStream_t s);
+std::vector<longlong2> fx_roots(int N);   // exp(-2 pi i t / N) 2^60, N a power of two from 8 on
 int fx_twiddle_table(int NG, int4* out);  // host table in limbs; returns its length (out may be null)
 cudaError_t configure_fx_kernels();
 

@@ -699,16 +699,31 @@ cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int
   return cudaGetLastError();
 }
 
+// The first eighth of the circle gives the others: where long double has 113 bits
+// in software, a context of 256 points spent 0.3 ms on 544 sines.
+std::vector<longlong2> fx_roots(int N) {
+  std::vector<longlong2> c(N / 8 + 1), r(N);  // (cos, sin) of 2 pi j / N
+  const long double step = 2.0L * acosl(-1.0L) / (long double)N;
+  for (int j = 0; j <= N / 8; ++j)
+    c[j] = make_longlong2(llrintl(ldexpl(cosl(step * j), fx::kOne)), llrintl(ldexpl(sinl(step * j), fx::kOne)));
+  for (int t = 0; t < N; ++t) {
+    const int q = t / (N / 4), j = t % (N / 4);
+    const longlong2 z = j <= N / 8 ? c[j] : make_longlong2(c[N / 4 - j].y, c[N / 4 - j].x);
+    r[t] = q == 0 ? make_longlong2(z.x, -z.y) : q == 1 ? make_longlong2(-z.y, -z.x) : q == 2 ? make_longlong2(-z.x, z.y) : make_longlong2(z.y, z.x);
+  }
+  return r;
+}
+
 template <int N>
 static int fx_twiddles(int4* out) {
   using TM = fx::Team<N>;
+  if (!out) return TM::kTwCount;
+  const std::vector<longlong2> roots = fx_roots(N);
   int n = 0;
   auto put = [&](int num, int den) {
-    const long double th = -2.0L * acosl(-1.0L) * (long double)(num % den) / (long double)den;
-    const long long x = llrintl(ldexpl(cosl(th), fx::kOne)), y = llrintl(ldexpl(sinl(th), fx::kOne));
+    const longlong2 z = roots[num % den * (N / den)];
     const long long m = (1ll << fx::kLimb) - 1;
-    if (out) out[n] = make_int4((int)(x >> fx::kLimb), (int)(x & m), (int)(y >> fx::kLimb), (int)(y & m));
-    ++n;
+    out[n++] = make_int4((int)(z.x >> fx::kLimb), (int)(z.x & m), (int)(z.y >> fx::kLimb), (int)(z.y & m));
   };
   if (TM::R1 > 1)
     for (int r = 0; r < TM::R1; ++r)
