@@ -120,6 +120,7 @@ struct mattohf_ctx {
   int2* d_kern_fx = nullptr;  // kernel table in limbs, its scale, the twiddles
   int2* d_kscale = nullptr;
   int4* d_tw_fx = nullptr;
+  int4* d_tw_small = nullptr;  // of the fused fixed-point stages' plan
   float4* d_udf = nullptr;    // double-float copy of the occupied orbitals
   float2* d_kern_df = nullptr;
   float4* d_tw_df = nullptr;
@@ -378,7 +379,7 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   return a;
 }
 
-std::vector<int4> fx_twiddles_host(int NG);
+std::vector<int4> fx_twiddles_host(int NG, bool latency = false);
 bool use_dm(const mattohf_ctx* c, int nbw, bool same);
 int ensure_dm(mattohf_ctx* ctx, int ncols);
 
@@ -768,14 +769,20 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
 bool use_small(const mattohf_ctx* ctx) {
   if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
   if (ctx->opt_small == 1) return true;
-  // us per RK4 step, fused against tiled, NG / NK / occupied bands: 16/4/2 24 57;
-  // 32/16/2 29 70; 64/8/2 29 78; 128/8/2 71 89; 128/8/3 72 90; 64/8/4 86 80 and
-  // 128/8/4 95 92, both even with the adjoint's reverse steps (208 221, 259 263);
-  // 64/16/4 (M^2 NG = 2^18) 172 97.  At 256 points an FP64 pair takes a warp twice as
-  // long: 256/8/2 83 104, 256/6/4 177 105, 256/8/4 257 107.
-  const size_t M = (size_t)ctx->NK * ctx->NBocc;
+  // us per RK4 step, fused against tiled, NG / NK / occupied bands, in fixed point
+  // (k_small_fx.cu): 64/8/4 44 77, 64/16/3 83 85, 128/8/2 65 86, 128/16/2 81 90, 256/8/2
+  // 77 101, but 64/16/4 (M^2 NG = 2^18) 93 93, 128/12/4 148 98, 256/8/4 149 107.  In FP64
+  // (k_small.cu): 16/4/2 24 54, 64/8/2 29 75, 64/12/2 44 80, 32/16/2 30 64, but 32/16/4
+  // (2^17) 100 79.
+  const size_t M = (size_t)ctx->NK * ctx->NBocc, work = M * M * ctx->NG;
   if (ctx->NK * ctx->NB > 64) return false;
-  return M * M * ctx->NG <= ((size_t)1 << 17) && (ctx->NG < 256 || M <= 16);
+  return work <= (small_stage_fx(ctx->NG, (int)M) ? (size_t)1 << 17 : (size_t)3 << 15);
+}
+// The adjoint's reverse stages, which are in FP64 (k_small_adj.cu): us per reverse
+// step, fused against separate launches, 64/8/4 120 134, 128/8/2 101 146, 128/16/2 161
+// 160, 256/4/2 132 155; 256/8/2 228 165.
+bool use_small_reverse(const mattohf_ctx* ctx) {
+  return use_small(ctx) && (ctx->opt_small == 1 || ctx->NG < 256 || ctx->NK * ctx->NBocc <= 8);
 }
 
 // CTAs per column.  A warp issues at most one FP64 instruction per ~64
@@ -819,6 +826,8 @@ int small_adj_ctas_per_column(const mattohf_ctx* ctx) {
 }
 
 // Buffers of the fused stages, sized before any capture.
+bool small_fx(const mattohf_ctx* ctx) { return small_stage_fx(ctx->NG, ctx->NK * ctx->NBocc); }
+
 int ensure_small_buffers(mattohf_ctx* ctx) {
   ctx->small_P = small_ctas_per_column(ctx);
   ctx->small_P_adj = small_adj_ctas_per_column(ctx);
@@ -829,6 +838,15 @@ int ensure_small_buffers(mattohf_ctx* ctx) {
     destroy_graph(ctx);  // a captured step holds the old pointer
     CKR(dalloc(ctx, &ctx->d_small_part, need));
     ctx->small_part_cap = need;
+  }
+  if (!ctx->d_tw_small && small_fx(ctx)) {
+    if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "fused-stage scratch growth during capture");
+    const std::vector<int4> tw = fx_twiddles_host(ctx->NG, true);
+    int4* p = nullptr;
+    CKR(dalloc(ctx, &p, tw.size()));
+    ctx->d_tw_small = p;
+    CK(cudaMemcpyAsync(p, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
   }
   if (!ctx->d_small_obs) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "fused-stage scratch growth during capture");
@@ -856,6 +874,9 @@ SmallStageArgs small_base(mattohf_ctx* ctx, double dt) {
   a.Gx = ctx->d_Gx;
   a.kx = ctx->d_kx;
   a.tw = ctx->tw;
+  a.kern_fx = ctx->d_kern_fx;
+  a.kscale = ctx->d_kscale;
+  a.tw_fx = reinterpret_cast<const fx::lc*>(ctx->d_tw_small);
   a.P = ctx->small_P;
   a.part = ctx->d_small_part;
   a.Aobs = ctx->d_A;
@@ -905,7 +926,7 @@ int enq_small_step(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, dou
     a.it = s == 3 ? shadow : ctx->d_int;
     a.it_out = s == 0 ? shadow : s == 3 ? ctx->d_int : nullptr;
     a.it_inc = s == 3 ? 1 : 0;
-    CK(launch_small_stage(ctx->NG, a, ctx->st));
+    CK((small_fx(ctx) ? launch_small_stage_fx : launch_small_stage)(ctx->NG, a, ctx->st));
   }
   return MATTOHF_OK;
 }
@@ -918,7 +939,7 @@ int enq_small_close(mattohf_ctx* ctx) {
   a.mode = 4;
   a.af = aval(0.0);
   a.out_obs = ctx->d_out;
-  CK(launch_small_stage(ctx->NG, a, ctx->st));
+  CK((small_fx(ctx) ? launch_small_stage_fx : launch_small_stage)(ctx->NG, a, ctx->st));
   return MATTOHF_OK;
 }
 
@@ -1010,9 +1031,9 @@ int compute_tables(mattohf_ctx* ctx) {
   return MATTOHF_OK;
 }
 
-std::vector<int4> fx_twiddles_host(int NG) {
-  std::vector<int4> t(fx_twiddle_table(NG, nullptr));
-  fx_twiddle_table(NG, t.data());
+std::vector<int4> fx_twiddles_host(int NG, bool latency) {
+  std::vector<int4> t(fx_twiddle_table(NG, nullptr, latency));
+  fx_twiddle_table(NG, t.data(), latency);
   return t;
 }
 
@@ -1190,6 +1211,7 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
     if (e == cudaSuccess) e = configure_dm_kernels();
     if (e == cudaSuccess) e = configure_df_kernels();
     if (e == cudaSuccess) e = configure_small_kernels();
+    if (e == cudaSuccess) e = configure_small_fx_kernels();
     if (e == cudaSuccess) e = configure_small_adj_kernels();
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
   }
@@ -1263,7 +1285,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
                   ctx->d_eps, ctx->d_err, ctx->d_sym, ctx->d_symF, ctx->d_dpart,
                   ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale,
                   ctx->d_wfx, ctx->d_wscale, ctx->d_fx_acc, ctx->d_wacc, ctx->d_kern_fx, ctx->d_kscale,
-                  ctx->d_tw_fx, ctx->d_dm_ut, ctx->d_dm_wt, ctx->d_dm_table, ctx->d_dm_tw, ctx->d_dm_W,
+                  ctx->d_tw_fx, ctx->d_tw_small, ctx->d_dm_ut, ctx->d_dm_wt, ctx->d_dm_table, ctx->d_dm_tw, ctx->d_dm_W,
                   ctx->d_dm_tscale, ctx->d_dm_acc, ctx->d_dm_wscale, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
                   ctx->d_small_part, ctx->d_small_obs};
   for (void* p : ptrs)
@@ -2114,7 +2136,7 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
   CK(launch_adj_init(ctx->d_lam, ctx->d_lamu, ctx->d_lamk, dt, elems, ctx->st));
   const double cst[3] = {0.5 * dt, 0.5 * dt, dt};
   const int amodes[4] = {AM, AAVE, AAVE, ACUR};
-  if (use_small(ctx)) {
+  if (use_small_reverse(ctx)) {
     // one fused launch per reverse stage; stage 0 also copies lam = lam_u and
     // steps the counter back
     SmallAdjArgs a;

@@ -144,17 +144,19 @@ template <> struct Dft<8> {
   }
 };
 
-// Radices (first = last; R1 = 1: two passes) and lanes.
-template <int N> struct Plan;
-template <> struct Plan<16> { static constexpr int R0 = 4, R1 = 1, T = 4; };
-template <> struct Plan<32> { static constexpr int R0 = 4, R1 = 2, T = 8; };
-template <> struct Plan<64> { static constexpr int R0 = 8, R1 = 1, T = 8; };
-template <> struct Plan<128> { static constexpr int R0 = 4, R1 = 8, T = 16; };
-template <> struct Plan<256> { static constexpr int R0 = 8, R1 = 4, T = 32; };
-template <> struct Plan<512> { static constexpr int R0 = 8, R1 = 8, T = 64; };
+// Radices (first = last; R1 = 1: two passes) and lanes.  V = 1: where few
+// transforms run at a time, 64 points on 16 lanes (half the chain of a lane).
+template <int N, int V = 0> struct Plan : Plan<N, 0> {};
+template <> struct Plan<16, 0> { static constexpr int R0 = 4, R1 = 1, T = 4; };
+template <> struct Plan<32, 0> { static constexpr int R0 = 4, R1 = 2, T = 8; };
+template <> struct Plan<64, 0> { static constexpr int R0 = 8, R1 = 1, T = 8; };
+template <> struct Plan<128, 0> { static constexpr int R0 = 4, R1 = 8, T = 16; };
+template <> struct Plan<256, 0> { static constexpr int R0 = 8, R1 = 4, T = 32; };
+template <> struct Plan<512, 0> { static constexpr int R0 = 8, R1 = 8, T = 64; };
+template <> struct Plan<64, 1> { static constexpr int R0 = 4, R1 = 4, T = 16; };
 
-template <int N> struct Team {
-  static constexpr int R0 = Plan<N>::R0, R1 = Plan<N>::R1, T = Plan<N>::T;
+template <int N, int V = 0> struct Team {
+  static constexpr int R0 = Plan<N, V>::R0, R1 = Plan<N, V>::R1, T = Plan<N, V>::T;
   static constexpr int E = N / T, STRIDE = N / R0;
   __device__ __forceinline__ static int pos(int tl, int e) { return tl + T * (e / R0) + STRIDE * (e % R0); }
   // register slot of lane 0 that holds the self-aliased frequency N/2
@@ -179,10 +181,10 @@ __device__ __forceinline__ void team_sync(int team) {
 
 // Forward transform of x in place (slots pos); twn: the negated imaginary parts
 // of the twiddles, as neg_hi and neg_lo.
-template <int N, bool ALONE = false>
-__device__ __forceinline__ void forward(cx (&x)[Team<N>::E], cx* buf, const lc* __restrict__ tw,
+template <int N, bool ALONE = false, int V = 0>
+__device__ __forceinline__ void forward(cx (&x)[Team<N, V>::E], cx* buf, const lc* __restrict__ tw,
                                         const int2* __restrict__ twn, int tl, int team) {
-  using TM = Team<N>;
+  using TM = Team<N, V>;
   constexpr int R0 = TM::R0, R1 = TM::R1, T = TM::T, E = TM::E;
 #pragma unroll
   for (int p = 0; p < E / R0; ++p) Dft<R0>::run(&x[p * R0]);

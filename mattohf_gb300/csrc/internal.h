@@ -200,7 +200,8 @@ cudaError_t launch_fock_sym_fx_batch(int NG, const FockFxArgs* d_args, const int
 // kernel table in limbs and its scale (device)
 cudaError_t launch_fx_kern(const double* kern, int nd, int NG, int2* kscale, int2* out, cudaStream_t s);
 std::vector<longlong2> fx_roots(int N);   // exp(-2 pi i t / N) 2^60, N a power of two from 8 on
-int fx_twiddle_table(int NG, int4* out);  // host table in limbs; returns its length (out may be null)
+// host table in limbs; returns its length (out may be null); latency: of Plan<NG, 1>
+int fx_twiddle_table(int NG, int4* out, bool latency = false);
 cudaError_t configure_fx_kernels();
 
 __host__ __device__ __forceinline__ int sym_tp(int i, int j, int T) {
@@ -331,6 +332,10 @@ struct SmallStageArgs {
   const double* Gx;
   const double* kx;
   const double2* tw;
+  // for the fixed-point form: kernel table and its scale, twiddles of Plan<NG, 1>
+  const int2* kern_fx;
+  const int2* kscale;
+  const fx::lc* tw_fx;
   double2* part;            // [ncols][P][NG] exchange partials, then [ncols][NG] (rho, vH),
                             // then [ncols][NG] kinetic term T_A w
   double* colbuf;           // [ncols][4]: Ekin part, J part, Re<u|F>, Im<u|F>
@@ -356,6 +361,10 @@ struct SmallStageArgs {
 // (the portable cluster size)
 constexpr int kSmallMaxCtas = 8;
 cudaError_t launch_small_stage(int NG, const SmallStageArgs& a, cudaStream_t s);
+// in fixed point (k_small_fx.cu), for M occupied orbitals where small_stage_fx
+bool small_stage_fx(int NG, int M);
+cudaError_t launch_small_stage_fx(int NG, const SmallStageArgs& a, cudaStream_t s);
+cudaError_t configure_small_fx_kernels();
 bool small_stage_supported(int NG);
 int small_pair_teams(int NG);
 cudaError_t configure_small_kernels();

@@ -714,9 +714,9 @@ std::vector<longlong2> fx_roots(int N) {
   return r;
 }
 
-template <int N>
+template <int N, int V = 0>
 static int fx_twiddles(int4* out) {
-  using TM = fx::Team<N>;
+  using TM = fx::Team<N, V>;
   if (!out) return TM::kTwCount;
   const std::vector<longlong2> roots = fx_roots(N);
   int n = 0;
@@ -733,7 +733,8 @@ static int fx_twiddles(int4* out) {
   return n;
 }
 
-int fx_twiddle_table(int NG, int4* out) {
+int fx_twiddle_table(int NG, int4* out, bool latency) {
+  if (latency && NG == 64) return fx_twiddles<64, 1>(out);
   switch (NG) {
     case 16: return fx_twiddles<16>(out);
     case 32: return fx_twiddles<32>(out);
