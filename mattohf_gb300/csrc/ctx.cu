@@ -158,7 +158,7 @@ struct mattohf_ctx {
   double2* d_lamk[4] = {nullptr, nullptr, nullptr, nullptr};
   int4* d_mufx = nullptr;  // adjoint orbitals in limbs and their sizes
   int2* d_mu_sizes = nullptr;
-  double *d_psi = nullptr, *d_sig = nullptr, *d_gcol = nullptr, *d_gstage = nullptr, *d_gvion = nullptr,
+  double *d_psi = nullptr, *d_gcol = nullptr, *d_gstage = nullptr, *d_gvion = nullptr,
          *d_vloc_adj = nullptr, *d_dpart2 = nullptr;
   int* d_adj_int = nullptr;  // [0] step n, [1] segment start
   double last_adj_ms = 0, last_adj_fwd_ms = 0;
@@ -263,8 +263,9 @@ AField aval(double A) {
   return f;
 }
 
-int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scalars = true) {
+DensArgs density_args(const mattohf_ctx* ctx, Block u, bool scalars = true) {
   DensArgs a;
+  std::memset(&a, 0, sizeof(a));
   a.u = u;
   a.nbocc = ctx->NBocc;
   a.occ = ctx->occ;
@@ -277,9 +278,10 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scala
   a.scal = scalars ? ctx->d_scal : nullptr;
   a.nk = ctx->NK;
   a.part = ctx->d_dpart;
-  a.mu = nullptr;
-  a.gvion = nullptr;
-  CK(launch_density(ctx->NG, a, st ? st : ctx->st));
+  return a;
+}
+int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scalars = true) {
+  CK(launch_density(ctx->NG, density_args(ctx, u, scalars), st ? st : ctx->st));
   return MATTOHF_OK;
 }
 
@@ -779,10 +781,12 @@ bool use_small(const mattohf_ctx* ctx) {
   return work <= (small_stage_fx(ctx->NG, (int)M) ? (size_t)1 << 17 : (size_t)3 << 15);
 }
 // The adjoint's reverse stages, which are in FP64 (k_small_adj.cu): us per reverse
-// step, fused against separate launches, 64/8/4 120 134, 128/8/2 101 146, 128/16/2 161
-// 160, 256/4/2 132 155; 256/8/2 228 165.
+// step, fused against separate launches, 16/4/2 52 74, 32/16/2 76 91, 64/12/2 96 115,
+// 128/8/2 102 112; 64/8/4 120 108, 128/8/3 138 130, 128/16/2 161 131, 256/4/2 132 126,
+// 256/8/2 228 132.
 bool use_small_reverse(const mattohf_ctx* ctx) {
-  return use_small(ctx) && (ctx->opt_small == 1 || ctx->NG < 256 || ctx->NK * ctx->NBocc <= 8);
+  const size_t M = (size_t)ctx->NK * ctx->NBocc;
+  return use_small(ctx) && (ctx->opt_small == 1 || M * M * ctx->NG <= (ctx->NG < 256 ? (size_t)3 << 14 : (size_t)1 << 13));
 }
 
 // CTAs per column.  A warp issues at most one FP64 instruction per ~64
@@ -1266,7 +1270,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
   {
     void* adj[] = {ctx->d_ckpt, ctx->d_store, ctx->d_lam, ctx->d_lamu, ctx->d_vbuf, ctx->d_mufx, ctx->d_mu_sizes, ctx->d_uN,
                    ctx->d_u0, ctx->d_lamk[0], ctx->d_lamk[1], ctx->d_lamk[2], ctx->d_lamk[3], ctx->d_psi,
-                   ctx->d_sig, ctx->d_gcol, ctx->d_gstage, ctx->d_gvion, ctx->d_vloc_adj, ctx->d_dpart2,
+                   ctx->d_gcol, ctx->d_gstage, ctx->d_gvion, ctx->d_vloc_adj, ctx->d_dpart2,
                    ctx->d_adj_int};
     for (void* p : adj)
       if (p) cudaFree(p);
@@ -1786,9 +1790,9 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
 
 // Autotuner: times the context's tunable launch shapes on its own orbitals
 // and keeps the fastest.  The orbitals (and the step counter) are restored.
-//   * symmetric-exchange tile S: one exchange apply h[u]u (k_fock_sym +
-//     k_sym_reduce, or the double-float kernels) for S = 1, 2, 4, ... up to the
-//     teams of a CTA;
+//   * symmetric-exchange tile S: one exchange apply h[u]u by pairs (or in
+//     double-float) for S = 1, 2, 4, ... up to the teams of a CTA, and, where it is
+//     in question, the exchange through the density matrix;
 //   * fused-stage CTAs per column P, for the grids the fused stages support:
 //     graph-replayed mattohf_rk4_run steps for every P from one round of all
 //     pair teams up to twice the multiprocessors over the columns (at most 8);
@@ -2186,22 +2190,12 @@ int enq_adjoint_step(mattohf_ctx* ctx, double dt, size_t elems) {
       CK(cudaEventRecord(ctx->ev_fork, ctx->st));
       CK(cudaStreamWaitEvent(ctx->st_side, ctx->ev_fork, 0));
     }
-    CKR(enq_density(ctx, vb, ss));  // vloc = vH[rho(v)] + vion
-    // sigma = sum Im(conj(mu) v) -> psi = vH[sigma]; accumulate the vion gradient
-    DensArgs d;
-    d.u = vb;
-    d.nbocc = ctx->NBocc;
-    d.occ = ctx->occ;
-    d.vCG = ctx->d_vCG;
-    d.vion = ctx->d_vion;
-    d.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
-    d.dvcell = ctx->dvcell;
-    d.rho = ctx->d_sig;
-    d.vloc = ctx->d_psi;
-    d.scal = ctx->d_scal + 4;
-    d.nk = NK;
-    d.part = ctx->d_dpart2;
+    // vloc = vH[rho(v)] + vion; sigma = sum Im(conj(mu) v) -> psi = vH[sigma] and the
+    // vion gradient
+    DensArgs d = density_args(ctx, vb, false);
     d.mu = ctx->d_lamk[s];
+    d.part_sig = ctx->d_dpart2;
+    d.psi = ctx->d_psi;
     d.gvion = ctx->d_gvion;
     CK(launch_density(NG, d, ss));
     AdjCombineArgs c;
@@ -2340,7 +2334,6 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
     for (double2** b : bufs) CKR(dalloc(ctx, b, elems));
     CKR(dalloc(ctx, &ctx->d_mu_sizes, (size_t)NK * NB));
     CKR(dalloc(ctx, &ctx->d_psi, NG));
-    CKR(dalloc(ctx, &ctx->d_sig, NG));
     CKR(dalloc(ctx, &ctx->d_vloc_adj, NG));
     CKR(dalloc(ctx, &ctx->d_gvion, NG));
     CKR(dalloc(ctx, &ctx->d_dpart2, (size_t)kDensChunks * NG));
@@ -2687,21 +2680,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
     for (int v = 0; v < mattohf_batch::kVariants; ++v) {
       const double2* uin = (v >= 1 && v <= 3) ? ctx->d_us : ctx->d_u;
       Block ub = blk(uin, ctx->NB, NG, ctx->NB);
-      DensArgs d;
-      d.u = ub;
-      d.nbocc = ctx->NBocc;
-      d.occ = ctx->occ;
-      d.vCG = ctx->d_vCG;
-      d.vion = ctx->d_vion;
-      d.twfx = reinterpret_cast<const fx::lc*>(ctx->d_tw_fx);
-      d.dvcell = ctx->dvcell;
-      d.rho = ctx->d_rho;
-      d.vloc = ctx->d_vloc;
-      d.scal = v >= 1 && v <= 3 ? nullptr : ctx->d_scal;
-      d.nk = ctx->NK;
-      d.part = ctx->d_dpart;
-      d.mu = nullptr;
-      d.gvion = nullptr;
+      const DensArgs d = density_args(ctx, ub, v < 1 || v > 3);
       dens[v].push_back(d);
       FockSymArgs f;
       f.u = ub;

@@ -66,10 +66,11 @@ struct DensArgs {
   double* scal;       // out: [0]=Nele, [1]=Eion, [2]=EH (or null)
   int nk;
   double* part;       // scratch [kDensChunks][NG] partial densities
-  // adjoint mode (mu != null): accumulate sigma = sum_cols Im(conj(mu) u)
-  // instead of the density, write vH[sigma] to vloc (no vion), and add
-  // sigma to gvion (if non-null)
+  // adjoint (mu != null): also sigma = sum_cols Im(conj(mu) u), vH[sigma] to psi,
+  // sigma added to gvion
   const double2* mu;
+  double* part_sig;   // scratch [kDensChunks][NG]
+  double* psi;
   double* gvion;
 };
 

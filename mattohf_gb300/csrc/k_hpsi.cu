@@ -23,14 +23,14 @@ __host__ __device__ __forceinline__ int dens_chunks(int ncol) {
   return n < 1 ? 1 : n > kDensChunks ? kDensChunks : n;
 }
 __device__ __forceinline__ void dens_partial_body(const DensArgs& a, int N, int chunk, int group) {
-  __shared__ double part_s[kDensSub][64];
+  __shared__ double part_s[kDensSub][64], sig_s[kDensSub][64];
   const int ncol = a.nk * a.u.nb, nch = dens_chunks(ncol);
   if (chunk >= nch) return;
   const int per = (ncol + nch * kDensSub - 1) / (nch * kDensSub);
   const int pt = threadIdx.x & 63, sub = threadIdx.x >> 6;
   const int ig = group * 64 + pt;
   const int c0 = (chunk * kDensSub + sub) * per, c1 = min(ncol, c0 + per);
-  double s = 0.0;
+  double s = 0.0, t = 0.0;
   if (ig < N) {
     if (a.mu == nullptr) {
 #pragma unroll 4
@@ -42,19 +42,24 @@ __device__ __forceinline__ void dens_partial_body(const DensArgs& a, int N, int 
       }
     } else {
 #pragma unroll 4
-      for (int c = c0; c < c1; ++c) {   // adjoint source: Im(conj(mu) u)
+      for (int c = c0; c < c1; ++c) {   // the adjoint's: all bands are occupied
         const int ik = c / a.u.nb, ib = c % a.u.nb;
         const size_t o = (size_t)ik * a.u.kstride + (size_t)ib * N + ig;
         const double2 z = a.u.p[o], m = a.mu[o];
-        s += fma(m.x, z.y, -(m.y * z.x));
+        s += fma(a.occ * z.x, z.x, (a.occ * z.y) * z.y);
+        t += fma(m.x, z.y, -(m.y * z.x));
       }
     }
   }
   part_s[sub][pt] = s;
+  if (a.mu != nullptr) sig_s[sub][pt] = t;
   __syncthreads();
   if (sub == 0 && ig < N) {
     for (int j = 1; j < kDensSub; ++j) s += part_s[j][pt];
     a.part[(size_t)chunk * N + ig] = s;
+    if (a.mu == nullptr) return;
+    for (int j = 1; j < kDensSub; ++j) t += sig_s[j][pt];
+    a.part_sig[(size_t)chunk * N + ig] = t;
   }
 }
 
@@ -81,7 +86,7 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
   const int tid = threadIdx.x;
   const bool in = tid < N;
   tw_s.load(a.twfx);
-  double2 v[1] = {make_double2(0.0, 0.0)};
+  double2 v[1] = {make_double2(0.0, 0.0)}, sg[1] = {make_double2(0.0, 0.0)};
   if (in) {
     const int nch = dens_chunks(a.nk * a.u.nb);
     double s = a.part[tid];
@@ -90,8 +95,39 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
     rho_s[tid] = s;
     a.rho[tid] = s;
     v[0].x = s;
+    if (a.mu != nullptr) {
+      s = a.part_sig[tid];
+#pragma unroll 4
+      for (int ch = 1; ch < nch; ++ch) s += a.part_sig[(size_t)ch * N + tid];
+      sg[0].x = s;
+    }
   }
   int2 z = fx_block_size<1, NW>(v, red);
+  if (a.mu != nullptr) {
+    // Both potentials by one transform pair: vCG is real and even, so rho + i sigma
+    // goes to vH[rho] + i vH[sigma].  Each has its own scale, whatever the size of mu.
+    const Scale sr = fx_fft_scale(z, 2 * N);
+    __syncthreads();
+    const Scale ss = fx_fft_scale(fx_block_size<1, NW>(sg, red), 2 * N);
+    if (in) buf[tid] = cx{fx_convert(v[0].x, sr), fx_convert(sg[0].x, ss)};
+    fx_block_forward<N>(buf, tw_s);
+    const double sig = sg[0].x;
+    if (in) {
+      const double f = a.vCG[tid] * (1.0 / N);
+      v[0] = make_double2(f * (double)buf[tid].x, -f * (double)buf[tid].y);  // conjugate: backward next
+    }
+    z = fx_block_size<1, NW>(v, red);
+    const Scale sb = fx_fft_scale(z, N);
+    if (in) buf[tid] = cx{fx_convert(v[0].x, sb), fx_convert(v[0].y, sb)};
+    fx_block_forward<N>(buf, tw_s);
+    if (in) {
+      const double u = fx_unscale(sb);
+      a.vloc[tid] = (double)buf[tid].x * u * fx_unscale(sr) + a.vion[tid];
+      a.psi[tid] = (double)buf[tid].y * -u * fx_unscale(ss);
+      a.gvion[tid] += sig;
+    }
+    return;
+  }
   const Scale s1 = fx_fft_scale(z, N);
   if (in) buf[tid] = cx{fx_convert(v[0].x, s1), 0};
   fx_block_forward<N>(buf, tw_s);
@@ -105,13 +141,6 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
   fx_block_forward<N>(buf, tw_s);
   if (in) vh_s[tid] = (double)buf[tid].x * fx_unscale(s2);
   __syncthreads();
-  if (a.mu != nullptr) {
-    for (int ig = tid; ig < N; ig += blockDim.x) {
-      a.vloc[ig] = vh_s[ig];
-      if (a.gvion) a.gvion[ig] += rho_s[ig];
-    }
-    return;
-  }
   for (int ig = tid; ig < N; ig += blockDim.x) a.vloc[ig] = vh_s[ig] + a.vion[ig];
   if (a.scal != nullptr && tid < 64) {
     // Nele, Eion, EH: lane-strided partial sums, then a fixed shuffle tree; two
