@@ -80,8 +80,8 @@ struct mattohf_ctx {
   std::vector<int> Kion;
   cudaStream_t st = nullptr;
   // side stream: the density of an RK4 stage runs beside that stage's exchange
-  cudaStream_t st_side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t st_side = nullptr, st_dens = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_dens = nullptr;
   // tables
   double2* tw = nullptr;
   double *d_Gx = nullptr, *d_kx = nullptr, *d_vCG = nullptr, *d_vcq = nullptr, *d_kern = nullptr;
@@ -726,11 +726,14 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
     const bool side = ctx->hf != 0;
     const bool obs = run && side && s == 0;
     if (side) {
-      // The density and the kinetic + local-potential part of h w need only
-      // the stage input: they run on the side stream beside the exchange.
+      // The density and the kinetic part of h w need only the stage input: each
+      // has a stream beside the exchange (one after the other on one stream, their
+      // 22 us were a small problem's longest chain).
       CK(cudaEventRecord(ctx->ev_fork, ctx->st));
       CK(cudaStreamWaitEvent(ctx->st_side, ctx->ev_fork, 0));
-      CKR(enq_density(ctx, ub, ctx->st_side, !run || obs));
+      CK(cudaStreamWaitEvent(ctx->st_dens, ctx->ev_fork, 0));
+      CKR(enq_density(ctx, ub, ctx->st_dens, !run || obs));
+      CK(cudaEventRecord(ctx->ev_dens, ctx->st_dens));
       CombineArgs pre = combine_base(ctx, ub, fs[s], modes[s], FockPlan());
       pre.split = 1;
       pre.hpre = ctx->d_hpre;
@@ -743,6 +746,7 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
       CK(cudaEventRecord(ctx->ev_join, ctx->st_side));
       if (run && s == 1) CK(launch_obs_reduce(obs_args(ctx, 3), ctx->st_side));  // joined by stage 2
       CKR(enq_fock(ctx, ub, ub, &fp, false, run || s > 0));
+      CK(cudaStreamWaitEvent(ctx->st, ctx->ev_dens, 0));
       CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
     } else {
       CKR(enq_density(ctx, ub));
@@ -772,13 +776,12 @@ bool use_small(const mattohf_ctx* ctx) {
   if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
   if (ctx->opt_small == 1) return true;
   // us per RK4 step, fused against tiled, NG / NK / occupied bands, in fixed point
-  // (k_small_fx.cu): 64/8/4 44 77, 64/16/3 83 85, 128/8/2 65 86, 128/16/2 81 90, 256/8/2
-  // 77 101, but 64/16/4 (M^2 NG = 2^18) 93 93, 128/12/4 148 98, 256/8/4 149 107.  In FP64
-  // (k_small.cu): 16/4/2 24 54, 64/8/2 29 75, 64/12/2 44 80, 32/16/2 30 64, but 32/16/4
-  // (2^17) 100 79.
-  const size_t M = (size_t)ctx->NK * ctx->NBocc, work = M * M * ctx->NG;
-  if (ctx->NK * ctx->NB > 64) return false;
-  return work <= (small_stage_fx(ctx->NG, (int)M) ? (size_t)1 << 17 : (size_t)3 << 15);
+  // (k_small_fx.cu): 64/8/4 44 61, 128/8/2 65 68, 256/4/2 70 83, 256/8/2 77 85, but
+  // 64/16/3 (M^2 NG = 2^17.2) 83 73, 128/8/3 (2^16.2) 76 68, 128/16/2 81 69, 256/8/4 150
+  // 94.  In FP64 (k_small.cu): 32/16/2 30 52, 64/8/2 29 61, 64/12/2 44 61, but 32/16/4
+  // (2^17) 79 65.
+  const size_t M = (size_t)ctx->NK * ctx->NBocc;
+  return ctx->NK * ctx->NB <= 64 && M * M * ctx->NG <= (size_t)1 << 16;
 }
 // The adjoint's reverse stages, which are in FP64 (k_small_adj.cu): us per reverse
 // step, fused against separate launches, 16/4/2 52 74, 32/16/2 76 91, 64/12/2 96 115,
@@ -1208,6 +1211,8 @@ int mattohf_create(const mattohf_config* cfg, mattohf_ctx** out) {
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
     e = cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->st_side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->st_dens, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_dens, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(MATTOHF_ERR_CUDA);
@@ -1297,6 +1302,8 @@ int mattohf_destroy(mattohf_ctx* ctx) {
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   if (ctx->st_side) cudaStreamDestroy(ctx->st_side);
+  if (ctx->ev_dens) cudaEventDestroy(ctx->ev_dens);
+  if (ctx->st_dens) cudaStreamDestroy(ctx->st_dens);
   if (ctx->st) cudaStreamDestroy(ctx->st);
   delete ctx;
   return MATTOHF_OK;

@@ -298,8 +298,8 @@ struct CombineArgs {
   double occ;
   double* colbuf;           // CM_OBS: [ncols][4] = Ekin part, J part, Re<w|F>, Im<w|F>
   int* nonfinite;           // set to 1 if any output is not finite
-  // 0: whole combine.  1: only T_A w + vloc w -> hpre (runs beside the
-  // exchange).  2: hpre + exchange, then the mode's epilogue (no transforms).
+  // 0: whole combine.  1: only T_A w -> hpre (runs beside the exchange).  2: hpre +
+  // vloc w + exchange, then the mode's epilogue (no transforms).
   int split;
   double2* hpre;            // [NK][NB][NG]
   // split == 1: also the columns' Ekin and Je parts at field af_obs

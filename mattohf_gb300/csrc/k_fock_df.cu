@@ -1,8 +1,8 @@
 // Symmetric exchange (src/Functions.f90:237-261, w == u) with the pair
 // transforms in double-float arithmetic (fft_df.cuh).
 //
-// Same tile-pair decomposition, Nyquist correction and partial-sum layout as
-// k_fock_sym in k_hpsi.cu; only the arithmetic of the pair chain (pair
+// Same tile pairs and Nyquist correction as k_fock_sym_fx in k_fock_fx.cu, with tile
+// partials in global memory; the arithmetic of the pair chain (pair
 // density, forward transform, kernel, inverse transform, the two
 // accumulations) runs on the FP32 pipe as unevaluated hi+lo pairs.  Inputs are
 // converted from FP64 once per apply, the partial sums back to FP64 on the way
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kThreads) k_fock_sym_df_batch(const FockSymDfA
 }
 
 // Ordered double-float sum of the tile partials of every occupied output,
-// converted to FP64 once (same term order and runs as k_sym_reduce).
+// converted to FP64 once (in kRedQ runs of the tiles).
 __device__ __forceinline__ df::cdf sym_run_sum_df(const float4* __restrict__ part, int S, int T, int N, int idx,
                                                   int c) {
   const int o = idx / N, q = idx % N;

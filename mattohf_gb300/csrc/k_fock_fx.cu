@@ -214,8 +214,8 @@ __device__ __forceinline__ void load_twiddles(const lc* __restrict__ tw, lc* tw_
 }
 
 // ---------------------------------------------------------------------------
-// Symmetric exchange (w == u, occupied pairs), tile pairs as k_fock_sym of
-// k_hpsi.cu: team w owns row a = i S + w in registers and in round r visits
+// Symmetric exchange (w == u, occupied pairs).  A CTA has a tile pair (ti <= tj) of
+// S orbitals each: team w owns row a = i S + w in registers and in round r visits
 // column b = j S + (w + r) % S, whose accumulator in shared memory has one
 // writer per round.
 // ---------------------------------------------------------------------------

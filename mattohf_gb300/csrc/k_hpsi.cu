@@ -280,8 +280,8 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
   double2 wv[PER];
 #pragma unroll
   for (int p = 0; p < PER; ++p) wv[p] = in ? wcol[tid + TH * p] : make_double2(0.0, 0.0);
-  // split == 2: the kinetic and local-potential part was made by the split == 1
-  // pass (beside the exchange); only the exchange and the epilogue remain
+  // split == 2: the kinetic part was made by the split == 1 pass (beside the
+  // exchange and the density); the potential, the exchange and the epilogue remain
   const bool post = a.split == 2;
   double2 kin[PER];
   if (!post && a.mode != CM_F) {
@@ -365,9 +365,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
     if (in) {
 #pragma unroll
       for (int p = 0; p < PER; ++p) {
-        const int q = tid + TH * p;
-        const double v = a.vloc[q];
-        a.hpre[ocol + q] = make_double2(kin[p].x + v * wv[p].x, kin[p].y + v * wv[p].y);
+        a.hpre[ocol + tid + TH * p] = kin[p];
       }
     }
     return;
@@ -387,10 +385,10 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       h = kin[p];
     } else {
       if (a.mode == CM_F) h = make_double2(0.0, 0.0);
-      else if (post) h = a.hpre[ocol + q];
       else {
         const double v = a.vloc[q];
-        h = make_double2(kin[p].x + v * wv[p].x, kin[p].y + v * wv[p].y);
+        const double2 t = post ? a.hpre[ocol + q] : kin[p];
+        h = make_double2(t.x + v * wv[p].x, t.y + v * wv[p].y);
       }
       double2 f;
       if (exchange_at(a, ik, ib, q, N, &f)) {

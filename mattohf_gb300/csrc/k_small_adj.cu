@@ -26,7 +26,7 @@
 //                              - dk_ab Nyq(v_a conj(mu_b)) (-1)^m),
 //         the second part being the Nyquist term of the transposed pair
 //         operator (see k_adjoint.cu), Nyq(f) = sum_m (-1)^m f(m);
-//     these are the row-a terms of the symmetric adjoint exchange (k_fock_adj)
+//     these are the row-a terms of the symmetric adjoint exchange (k_fock_adj_fx)
 //     with the column terms written as the rows of the reversed pairs.  The
 //     transforms use the 32-lane latency plans, so a unit is one team;
 //   * the column's last CTA (per-column ticket) adds the P partials in chunk

@@ -9,8 +9,8 @@
 // One FP64 instruction becomes 12 to 20 integer ones, which a warp runs once a launch
 // and so fetches cold: with few orbitals k_small.cu stays faster.  us per RK4 step
 // at NG / NK / bands, FP64 against this: 16/4/2 24 34, 32/16/2 29 37, 64/8/2 29 37;
-// 64/8/4 86 44, 128/8/2 71 64, 128/16/2 95 79, 256/8/2 83 76 (the other path: 76, 84, 88,
-// 99 from 64/8/4 on).  Hence from 64 points and M NG = 2048 on (small_stage_fx).
+// 64/8/4 86 44, 128/8/2 71 65, 256/4/2 79 70, 256/8/2 83 77 (separate launches: 61, 68, 83,
+// 85 from 64/8/4 on).  Hence from 64 points and M NG = 2048 on (small_stage_fx).
 #include "fx_convert.cuh"
 #include "small_stage.cuh"
 
