@@ -33,8 +33,9 @@ WORKLOAD = dict(acell=10.0, NG=256, NK=64, NB=4, NBocc=4, Zeff=[1.5, 0.5], alpha
                 Rion=[0.25, 0.75], Kion=[1, 2])
 PULSE = dict(A0=0.1, w=0.057, T=600.0)
 DT = 7e-4
-# DRAM bytes (read + write) of one symmetric-exchange launch on WORKLOAD, ncu
-FOCK_SYM_DRAM_BYTES_NG256_NK64_NB4 = 1_242_624 + 7_576_064
+# DRAM bytes (read + write) of one exchange apply on WORKLOAD (density, conversion,
+# k_dm_build, k_dm_apply), ncu
+EXCHANGE_DRAM_BYTES = 1_060_608 + 1_084_928 + 1_639_936 + 36_843_776
 NSCF_INIT, NCG_INIT = 3, 4
 METRIC = "TDHF RK4 steps/s"
 WORKLOAD_NAME = ("plain HF RK4, exchange-dominated: a=10, NG=256, NK=64, Nocc=NB=4, "
@@ -46,6 +47,16 @@ def fock_flops_per_apply(NG, NK, NB, NBocc):
     L = int(np.log2(NG))
     P = NK * NK * NB * NBocc
     return P * (10 * NG * L + 16 * NG)
+
+
+def exchange_multiply_adds(NG, NK, NB, NBocc):
+    """32 x 32 + 64-bit multiply-adds of one exchange apply through the density matrix (w == u):
+    half of the grid-point pairs each take two transforms over L >= 2 NK k-points
+    (114 a point and the density matrix's 12 a band), the product 12 a term."""
+    L = 16
+    while L < 2 * NK:
+        L *= 2
+    return NG * NG // 2 * (L // 2) * (12 * NBocc + 114) + NG * NG * NK * 12 * NB
 
 
 def fock_sym_flops_per_apply(NG, NK, NBocc):
@@ -283,23 +294,20 @@ def run_gpu(args, dist):
     value = dist.ws * K / (total_ms * 1e-3)
     clocks = clk.summary()
 
-    # --- dominant kernel (Fock pair kernel): per-launch CUDA-event time
+    # --- the exchange (conversion, k_dm_build, k_dm_apply): CUDA-event time per apply
     ctx.set_option(_capi.OPT_KERNEL_TIMING, 1)
     ctx.set_orbitals(u0)
     ctx.rk4_run(A[:2], Aave[:2], cfg.dt)
     _, fock_ms, nf = ctx.last_run_timing()
     ctx.set_option(_capi.OPT_KERNEL_TIMING, 0)
-    flops = fock_sym_flops_per_apply(cfg.NG, cfg.NK, cfg.NBocc)
-    achieved = flops / (fock_ms / nf * 1e-3) / 1e12
+    mads = exchange_multiply_adds(cfg.NG, cfg.NK, cfg.NB, cfg.NBocc)
+    achieved = mads / (fock_ms / nf * 1e-3) / 1e12
+    # 32 a clock and multiprocessor with three different registers each
+    peak_mads = 32 * 152 * (clocks.get("sm_mhz") or 1920.0) * 1e6 / 1e12
     peak = C.c_double()
     lib.mattohf_diag_fp64_peak(dev, C.byref(peak))
     dmma = C.c_double()
     lib.mattohf_diag_dmma_peak(dev, C.byref(dmma))
-    # dram__bytes_read.sum + dram__bytes_write.sum of one k_fock_sym<256> launch on
-    # this workload, from the ncu capture in profiles/k_fock_sym_ng256_nk64_nb4.md
-    prof_traffic = None
-    if (cfg.NG, cfg.NK, cfg.NBocc) == (256, 64, 4):
-        prof_traffic = FOCK_SYM_DRAM_BYTES_NG256_NK64_NB4
 
     # --- the same timed region with the exchange transforms in double-float
     #     arithmetic (MATTOHF_OPT_FOCK_DF64; parity-tested at the FP64 tolerances)
@@ -353,28 +361,30 @@ def run_gpu(args, dist):
                "sample": f"{steps_cpu} RK4+observable steps of the same workload (C restatement, "
                          f"OpenMP over output columns)",
                "one_core": {"value": 1.0 / t1, "unit": "steps/s", "cores": 1, "sample": "1 step"}}
-    # per step: 4 stages x (k_dens_partial, k_density, kinetic k_combine pass, k_fock_sym,
-    # k_sym_reduce, exchange k_combine pass) + k_ex_finalize + observables (k_dens_partial,
-    # k_density, k_combine, k_obs_reduce); per run: the closing exchange apply (7 launches)
-    launches_per_step = 4 * 6 + 1 + 4
+    # per step: 4 stages x (k_dens_partial, k_density, kinetic k_combine pass, k_dm_density,
+    # k_dm_convert, k_dm_build, k_dm_apply, exchange k_combine pass) + k_obs_reduce; per run:
+    # the first sizes and the closing exchange apply with its observables
+    launches_per_step = 4 * 8 + 1
     line = {"metric": METRIC, "value": value, "unit": "steps/s", "n_gpus": dist.ws, "steps": K,
             "warmup": W, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": bench_config(cfg), "graph": True,
-            "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-                         "frac": achieved / peak.value if peak.value else None,
-                         "traffic": prof_traffic, "kernel": "k_fock_sym",
-                         "flops_per_launch": flops, "launch_ms": fock_ms / nf,
-                         "peak_source": "measured DFMA throughput on this GPU (mattohf_diag_fp64_peak)",
-                         "fp64_tensor_peak": dmma.value,
+            "roofline": {"bound": "int-mad", "achieved": achieved, "peak": peak_mads, "unit": "T multiply-adds/s",
+                         "frac": achieved / peak_mads, "traffic": EXCHANGE_DRAM_BYTES,
+                         "kernel": "k_dm_build + k_dm_apply",
+                         "mads_per_apply": mads, "apply_ms": fock_ms / nf,
+                         "peak_source": "32 multiply-adds (32 x 32 + 64 bits) a clock and multiprocessor, measured, "
+                                        "x 152 x the sampled SM clock",
+                         "fp64_peak_tflops": peak.value, "fp64_tensor_peak": dmma.value,
                          "fp64_tensor_peak_source": "measured DMMA (mma.sync m8n8k4 f64) throughput, "
                                                     "mattohf_diag_dmma_peak",
                          "hbm_peak_gbs": hbm_peak(),
-                         "flops_model": "symmetric exchange: M(M+1)/2 pairs x (10 N log2 N + 16 N) + M(M-1)/2 x 8 N, M = NK*NBocc"},
+                         "work_model": "64-bit fixed point through the density matrix: NG^2/2 L/2 (12 Nocc + 114) "
+                                       "+ NG^2 NK 12 NB, L >= 2 NK"},
             "ground_state": {"value": gs_timing.get("gs_scf_iterations_per_s"), "unit": "SCF iterations/s",
                              "note": f"GS_calculation, Krylov dim NB*NCG = {cfg.NB * NCG_INIT}, "
                                      f"{2 * NCG_INIT + 2} h-applies per iteration, host wall clock"},
-            "cpu_baseline": cpu, "e2e": e2e, "double_float_exchange": double_float, "gpu_launches": launches_per_step * K + 7, "clocks": clocks}
+            "cpu_baseline": cpu, "e2e": e2e, "double_float_exchange": double_float, "gpu_launches": launches_per_step * K + 9, "clocks": clocks}
     ctx.close()
     if dist.rank == 0 and dist.ws == 1 and not args.no_extras:
         # the metric's other clauses, each on its own workload (outside the
@@ -412,7 +422,6 @@ def measure_ensemble(R: int, K: int, W: int, with_df: bool = True) -> dict:
     """
     import math
     from mattohf_gb300 import Batch, RunConfig, define_afield, _capi
-    import ctypes as C
     import dataclasses
     rng = np.random.default_rng(1)
     nks = rng.choice([8, 16, 32, 64], size=R)
@@ -463,20 +472,15 @@ def measure_ensemble(R: int, K: int, W: int, with_df: bool = True) -> dict:
         t_plain += m.last_run_timing()[0]
     b.close()
     kb = float(sum(c.NK * c.NB for c in cfgs))
-    # executed algorithmic FP64 work of one ensemble step: 4 symmetric exchange
-    # applies per run (the first stage's doubles as the previous step's Ex)
+    # algorithmic work of one ensemble step: 4 symmetric exchange applies per run (the
+    # first stage's doubles as the previous step's Ex)
     flops_step = float(sum(4 * fock_sym_flops_per_apply(c.NG, c.NK, c.NBocc) for c in cfgs))
-    peak = C.c_double()
-    _capi.load().mattohf_diag_fp64_peak(0, C.byref(peak))
-    achieved = flops_step * K / (t_batch * 1e-3) / 1e12
     out = {"metric": "TDHF RK4 steps/s (ensemble aggregate)", "value": R * K / (t_batch * 1e-3),
            "unit": "run-steps/s", "steps": K, "warmup": W, "higher_is_better": True,
            "plain_value": R * K / (t_plain * 1e-3), "batched_over_plain": t_plain / t_batch,
            "kpoint_orbital_steps_per_s": kb * K / (t_batch * 1e-3),
-           "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-                        "frac": achieved / peak.value if peak.value else None,
-                        "flops_per_step": flops_step,
-                        "flops_model": "exchange only: 4 symmetric applies per run per step"},
+           "exchange_tflops": flops_step * K / (t_batch * 1e-3) / 1e12,
+           "flops_model": "exchange only: 4 symmetric applies per run per step, 5 N log2 N a transform",
            "double_float_exchange": None if t_batch_df is None else R * K / (t_batch_df * 1e-3),
            "dtype": "f64", "data": "synthetic",
            "config": {"workload": f"{R} runs, NK in {{8,16,32,64}}, Nocc in {{1..4}}, NG=128, a in [8,14], "
