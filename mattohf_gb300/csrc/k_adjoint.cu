@@ -286,59 +286,68 @@ cudaError_t launch_scale2(double2* x, double sc, size_t n, cudaStream_t s) {
 // Phi_ji[p_ji] except at the self-aliased Nyquist index; so the gradient is
 // 2 occ dvcell h[u] u plus, for column i,
 //   g_i += sc sum_j (kern_ji - kern_ij)[N/2] Nyq(p_ij) (-1)^m u_j,
-// Nyq(p) = sum_m (-1)^m p(m), sc = occ dvcell.  One CTA per column i; the
-// orbitals j are visited in order, each dot product reduced in a fixed order.
+// Nyq(p) = sum_m (-1)^m p(m), sc = occ dvcell.  One CTA per column i, one orbital j
+// per warp at a time, so that eight chains of FP64 run side by side (with all warps on
+// one j, a reduction over the CTA each, 112 us at NG = 128, NK = 16, 2 bands, now 46,
+// bound by the SM's FP64 rate; an energy gradient at 256 / 32 / 4 3.12 -> 2.81 ms);
+// the warps' sums are added in order.
 constexpr int kNyqThreads = 256;
 __global__ void __launch_bounds__(kNyqThreads) k_energy_grad_nyquist(const double2* __restrict__ u, double2* g,
                                                                       const double* __restrict__ kern, int N,
                                                                       int nk, int nb, double sc) {
-  __shared__ double2 red[kNyqThreads / 32];
+  constexpr int kMaxPer = 512 / 32;    // N <= 512
+  __shared__ double2 s_s[512], sum_s[512];
   const int i = blockIdx.x, ki = i / nb;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const double2* ui = u + (size_t)i * N;
   const int M = nk * nb;
-  constexpr int kMaxPer = 512 / kNyqThreads;    // N <= 512
+  for (int m = tid; m < N; m += kNyqThreads) {
+    const double sg = (m & 1) ? -1.0 : 1.0;
+    s_s[m] = make_double2(sg * ui[m].x, sg * ui[m].y);
+    sum_s[m] = make_double2(0.0, 0.0);
+  }
+  __syncthreads();
   double2 acc[kMaxPer];
 #pragma unroll
   for (int r = 0; r < kMaxPer; ++r) acc[r] = make_double2(0.0, 0.0);
-  for (int j = 0; j < M; ++j) {
+  for (int j = warp; j < M; j += kNyqThreads / 32) {
     const int kj = j / nb;
     if (kj == ki) continue;   // the two multipliers coincide
     const double d = kern[(size_t)(kj - ki + nk - 1) * N + N / 2] - kern[(size_t)(ki - kj + nk - 1) * N + N / 2];
     const double2* uj = u + (size_t)j * N;
     double px = 0.0, py = 0.0;
-    for (int m = tid; m < N; m += kNyqThreads) {
-      const double sg = (m & 1) ? -1.0 : 1.0;
-      const double2 t = cmulc(ui[m], uj[m]);
-      px = fma(sg, t.x, px);
-      py = fma(sg, t.y, py);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      px += __shfl_xor_sync(0xffffffffu, px, o);
-      py += __shfl_xor_sync(0xffffffffu, py, o);
-    }
-    if (lane == 0) red[warp] = make_double2(px, py);
-    __syncthreads();
-    double2 c = red[0];
-    for (int w = 1; w < kNyqThreads / 32; ++w) c = cadd(c, red[w]);
-    __syncthreads();
-    const double2 f = make_double2(sc * d * c.x, sc * d * c.y);
 #pragma unroll
     for (int r = 0; r < kMaxPer; ++r) {
-      const int m = tid + r * kNyqThreads;
+      const int m = lane + 32 * r;
       if (m < N) {
-        const double sg = (m & 1) ? -1.0 : 1.0;
-        const double2 t = cmul(f, uj[m]);
-        acc[r] = make_double2(fma(sg, t.x, acc[r].x), fma(sg, t.y, acc[r].y));
+        const double2 z = uj[m], w = s_s[m];
+        px = fma(w.x, z.x, fma(w.y, z.y, px));
+        py = fma(w.y, z.x, fma(-w.x, z.y, py));
       }
     }
+    px = warp_sum(px);
+    py = warp_sum(py);
+    const double2 f = make_double2(sc * d * px, sc * d * py);
+#pragma unroll
+    for (int r = 0; r < kMaxPer; ++r) {
+      const int m = lane + 32 * r;
+      if (m < N) acc[r] = cfma(f, uj[m], acc[r]);
+    }
+  }
+  for (int w = 0; w < kNyqThreads / 32; ++w) {
+    if (warp == w) {
+#pragma unroll
+      for (int r = 0; r < kMaxPer; ++r) {
+        const int m = lane + 32 * r;
+        if (m < N) sum_s[m] = cadd(sum_s[m], acc[r]);
+      }
+    }
+    __syncthreads();
   }
   double2* gi = g + (size_t)i * N;
-#pragma unroll
-  for (int r = 0; r < kMaxPer; ++r) {
-    const int m = tid + r * kNyqThreads;
-    if (m < N) gi[m] = cadd(gi[m], acc[r]);
+  for (int m = tid; m < N; m += kNyqThreads) {
+    const double sg = (m & 1) ? -1.0 : 1.0;
+    gi[m] = make_double2(fma(sg, sum_s[m].x, gi[m].x), fma(sg, sum_s[m].y, gi[m].y));
   }
 }
 
