@@ -285,6 +285,22 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scala
   return MATTOHF_OK;
 }
 
+// The density and local potential of u on a stream of its own, beside the exchange
+// that follows on the main one (without exchange: on the main one); the main stream
+// has them after join_density.
+int fork_density(mattohf_ctx* ctx, Block u) {
+  if (!ctx->hf) return enq_density(ctx, u);
+  CK(cudaEventRecord(ctx->ev_fork, ctx->st));
+  CK(cudaStreamWaitEvent(ctx->st_dens, ctx->ev_fork, 0));
+  CKR(enq_density(ctx, u, ctx->st_dens));
+  CK(cudaEventRecord(ctx->ev_dens, ctx->st_dens));
+  return MATTOHF_OK;
+}
+int join_density(mattohf_ctx* ctx) {
+  if (ctx->hf) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_dens, 0));
+  return MATTOHF_OK;
+}
+
 // Which exchange partials a combine launch reads.
 struct FockPlan {
   bool occ = false;           // occupied bands by the symmetric exchange
@@ -631,16 +647,18 @@ CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const F
 // same_u: the previous enq_hpsi applied the operator of the same, unchanged u,
 // whose local potential and fixed-point orbitals still hold.
 int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mode, bool same_u = false) {
+  CKR(ensure_scratch(ctx, ctx->NK * w.nb));
   FockPlan fp;
-  if (mode == CM_H && !same_u) CKR(enq_density(ctx, u));
+  const bool dens = mode == CM_H && !same_u;
+  if (dens) CKR(fork_density(ctx, u));
   if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp, same_u));
   else if (mode == CM_F) {
     CK(cudaMemsetAsync(out.p, 0, sizeof(double2) * (size_t)ctx->NK * out.kstride, ctx->st));
     return MATTOHF_OK;
   }
-  CKR(ensure_scratch(ctx, ctx->NK * w.nb));
   CombineArgs a = combine_base(ctx, w, af, mode, fp);
   a.out = out;
+  if (dens) CKR(join_density(ctx));
   CK(launch_combine(ctx->NG, a, ctx->NK * w.nb, ctx->st));
   return MATTOHF_OK;
 }
@@ -689,7 +707,7 @@ ObsReduceArgs obs_args(mattohf_ctx* ctx, int advance) {
 int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, int advance, FockPlan* plan_out = nullptr) {
   const int NG = ctx->NG, NB = ctx->NB;
   Block ub = blk(u, NB, NG, NB);
-  CKR(enq_density(ctx, ub));
+  CKR(fork_density(ctx, ub));
   FockPlan fp;
   fp.any = false;
   if (ctx->hf) CKR(enq_fock(ctx, ub, ub, &fp));
@@ -697,6 +715,7 @@ int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, int advance, 
   if (plan_out) *plan_out = fp;
   CombineArgs a = combine_base(ctx, ub, af, CM_OBS, fp);
   CK(launch_combine(NG, a, ctx->NK * NB, ctx->st));
+  CKR(join_density(ctx));
   CK(launch_obs_reduce(obs_args(ctx, advance), ctx->st));
   return MATTOHF_OK;
 }
@@ -1512,8 +1531,9 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   Block u = blk((const double2*)d_uocc, ctx->NBocc, NG, ctx->NBocc);
   Block w = blk((const double2*)d_w, nbw, NG, nbw);
   const int ncols = nkl * nbw;
-  if (mode == CM_H || mode == CM_OBS) CKR(enq_density(ctx, u));
   CKR(ensure_scratch(ctx, ncols));
+  const bool dens = mode == CM_H || mode == CM_OBS;
+  if (dens) CKR(fork_density(ctx, u));
   FockPlan fp;
   if (ctx->hf && mode != CM_T) {
     CKR(ensure_fx(ctx));
@@ -1533,6 +1553,7 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   c.kx = ctx->d_kx + k0;
   c.nk = nkl;
   c.out = out;
+  if (dens) CKR(join_density(ctx));
   CK(launch_combine(NG, c, ncols, ctx->st));
   return MATTOHF_OK;
 }
