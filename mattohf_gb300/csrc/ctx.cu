@@ -438,14 +438,14 @@ int ensure_fock_buffers(mattohf_ctx* ctx) {
 // 512/32/8 1510 1332.  Grids below 64 points stay with pairs: few terms average
 // less of W's rounding, 2.1e-16 at 16 / 33 / 2 and 1.4e-16 at 32 / 40 / 2 against
 // 7e-17 and 5e-17 (from 64 points on at most 1.2e-16).
-bool fock_dm_wins(const mattohf_ctx* c, int nbw, bool same) {
+bool fock_dm_wins(const mattohf_ctx* c, int nbw, bool same, double launches = 6.5e7) {
   const double N = c->NG, NK = c->NK, no = c->NBocc, M = NK * no;
   const int lh = dm_length(c->NK) / 2;
   if (2 * lh > 512 || c->NG < 64) return false;
   if (N * (N + 1) / 2 * NK * 16 > 2147483648.0) return false;  // bytes of W
   const double pairs = same ? 87.0 * M * M / 2 * N + 75.0 * M * NK * (nbw - no) * N : 75.0 * M * NK * nbw * N;
   const double dm = N * N / 2 * lh * (12 * no + 114) + N * N * NK * 12 * nbw;
-  return 0.75 * dm + 6.5e7 < pairs;
+  return 0.75 * dm + launches < pairs;
 }
 bool use_dm(const mattohf_ctx* c, int nbw, bool same) {
   if (!c->opt_sym || c->opt_df || c->opt_chunks > 0 || c->opt_dm == 0) return false;
@@ -458,8 +458,6 @@ int dm_no_room(mattohf_ctx* ctx) {
   cudaGetLastError();
   destroy_graph(ctx);
   CKR(dalloc(ctx, &ctx->d_dm_W, 0));
-  CKR(dalloc(ctx, &ctx->d_dm_ut, 0));
-  CKR(dalloc(ctx, &ctx->d_dm_table, 0));
   CKR(dalloc(ctx, &ctx->d_dm_wt, 0));
   CKR(dalloc(ctx, &ctx->d_dm_acc, 0));
   ctx->dm_cols = 0;
@@ -468,40 +466,50 @@ int dm_no_room(mattohf_ctx* ctx) {
   return MATTOHF_OK;
 }
 
-// Its buffers for ncols columns of w, and (once) its tables.  Where there is no
-// memory for them, opt_dm = 0 afterwards.
-int ensure_dm(mattohf_ctx* ctx, int ncols) {
+// Its tables and the orbitals' place, once per context.
+int ensure_dm_tables(mattohf_ctx* ctx) {
+  if (ctx->d_dm_table) return MATTOHF_OK;
   const int NG = ctx->NG, NK = ctx->NK, L = dm_length(NK);
-  if (!ctx->d_dm_table) {
-    if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "density-matrix tables during capture");
-    const std::vector<int4> tw = fx_twiddles_host(L);
-    struct Tmp {
-      int4* p = nullptr;
-      ~Tmp() {
-        if (p) cudaFree(p);
-      }
-    } v, raw, mx, roots;
-    const std::vector<longlong2> rt = fx_roots(L);
-    const size_t nu = (size_t)NG * ctx->NBocc * (L / 2);
-    int4* table = nullptr;
-    if (dalloc(ctx, &ctx->d_dm_W, (size_t)NG * (NG + 1) / 2 * NK) || dalloc(ctx, &ctx->d_dm_ut, nu)) return dm_no_room(ctx);
-    CKR(dalloc(ctx, &v.p, (size_t)(2 * NK - 1) * NG));
-    CKR(dalloc(ctx, &raw.p, (size_t)NG * L));
-    CKR(dalloc(ctx, &mx.p, 1));
-    CKR(dalloc(ctx, &roots.p, (size_t)L));
-    CK(cudaMemcpyAsync(roots.p, rt.data(), L * sizeof(longlong2), cudaMemcpyHostToDevice, ctx->st));
-    CKR(dalloc(ctx, &ctx->d_dm_tw, tw.size()));
-    CKR(dalloc(ctx, &ctx->d_dm_tscale, 2));  // and the largest density
-    CK(cudaMemsetAsync(ctx->d_dm_tscale, 0, 2 * sizeof(int2), ctx->st));
-    CKR(dalloc(ctx, &table, (size_t)NG * L));
-    CK(cudaMemcpyAsync(ctx->d_dm_tw, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemsetAsync(ctx->d_dm_ut, 0, nu * sizeof(int4), ctx->st));
-    CK(launch_dm_table(NG, NK, ctx->d_kern_fx, reinterpret_cast<const fx::lc*>(ctx->d_tw_fx),
-                       reinterpret_cast<const fx::cx*>(roots.p), reinterpret_cast<fx::cx*>(v.p),
-                       reinterpret_cast<fx::cx*>(raw.p), reinterpret_cast<int*>(mx.p), reinterpret_cast<fx::lc*>(table),
-                       ctx->d_dm_tscale, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    ctx->d_dm_table = table;
+  if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "density-matrix tables during capture");
+  const std::vector<int4> tw = fx_twiddles_host(L);
+  struct Tmp {
+    int4* p = nullptr;
+    ~Tmp() {
+      if (p) cudaFree(p);
+    }
+  } v, raw, mx, roots;
+  const std::vector<longlong2> rt = fx_roots(L);
+  const size_t nu = (size_t)NG * ctx->NBocc * (L / 2);
+  int4* table = nullptr;
+  CKR(dalloc(ctx, &ctx->d_dm_ut, nu));
+  CKR(dalloc(ctx, &v.p, (size_t)(2 * NK - 1) * NG));
+  CKR(dalloc(ctx, &raw.p, (size_t)NG * L));
+  CKR(dalloc(ctx, &mx.p, 1));
+  CKR(dalloc(ctx, &roots.p, (size_t)L));
+  CK(cudaMemcpyAsync(roots.p, rt.data(), L * sizeof(longlong2), cudaMemcpyHostToDevice, ctx->st));
+  CKR(dalloc(ctx, &ctx->d_dm_tw, tw.size()));
+  CKR(dalloc(ctx, &ctx->d_dm_tscale, 2));  // and the largest density
+  CK(cudaMemsetAsync(ctx->d_dm_tscale, 0, 2 * sizeof(int2), ctx->st));
+  CKR(dalloc(ctx, &table, (size_t)NG * L));
+  CK(cudaMemcpyAsync(ctx->d_dm_tw, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
+  CK(cudaMemsetAsync(ctx->d_dm_ut, 0, nu * sizeof(int4), ctx->st));
+  CK(launch_dm_table(NG, NK, ctx->d_kern_fx, reinterpret_cast<const fx::lc*>(ctx->d_tw_fx),
+                     reinterpret_cast<const fx::cx*>(roots.p), reinterpret_cast<fx::cx*>(v.p),
+                     reinterpret_cast<fx::cx*>(raw.p), reinterpret_cast<int*>(mx.p), reinterpret_cast<fx::lc*>(table),
+                     ctx->d_dm_tscale, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  ctx->d_dm_table = table;
+  return MATTOHF_OK;
+}
+
+// W and the buffers for ncols columns of w.  Where there is no memory for them,
+// opt_dm = 0 afterwards.
+int ensure_dm(mattohf_ctx* ctx, int ncols) {
+  const int NG = ctx->NG, NK = ctx->NK;
+  CKR(ensure_dm_tables(ctx));
+  if (!ctx->d_dm_W) {
+    if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
+    if (dalloc(ctx, &ctx->d_dm_W, (size_t)NG * (NG + 1) / 2 * NK)) return dm_no_room(ctx);
   }
   if ((size_t)ncols > ctx->dm_cols) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
@@ -515,7 +523,7 @@ int ensure_dm(mattohf_ctx* ctx, int ncols) {
   return MATTOHF_OK;
 }
 
-int enq_fock_dm(mattohf_ctx* ctx, Block u, Block w, bool same_u, bool have_sizes) {
+FockDmArgs dm_args(const mattohf_ctx* ctx, Block u, Block w) {
   FockDmArgs a;
   a.u = u;
   a.w = w;
@@ -534,6 +542,11 @@ int enq_fock_dm(mattohf_ctx* ctx, Block u, Block w, bool same_u, bool have_sizes
   a.W = reinterpret_cast<fx::lc*>(ctx->d_dm_W);
   a.acc = ctx->d_dm_acc;
   a.wscale = ctx->d_dm_wscale;
+  return a;
+}
+
+int enq_fock_dm(mattohf_ctx* ctx, Block u, Block w, bool same_u, bool have_sizes) {
+  const FockDmArgs a = dm_args(ctx, u, w);
   if (!have_sizes && !same_u) CK(launch_fx_sizes(ctx->NG, fx_args(ctx, u, 1), ctx->st));
   CK(launch_dm_convert(ctx->NG, a, same_u, ctx->st));
   if (!same_u) CK(launch_dm_build(ctx->NG, a, ctx->nsm, ctx->st));
@@ -2612,6 +2625,16 @@ struct mattohf_batch {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int opt_df = 0;  // exchange transforms in double-float arithmetic
   int opt_tile = 0;  // symmetric-exchange tile of every run (0 = the CTA's teams)
+  // Runs whose exchange goes through the density matrix, one after the other: each
+  // fills the GPU by itself.  W and the converted functions are shared.
+  struct DmRun {
+    int r;
+    int4* acc;
+    double2* wscale;
+  };
+  std::vector<DmRun> dm;
+  int4 *dm_W = nullptr, *dm_wt = nullptr;
+  bool opt_dm = true;  // false: a tile was asked for, or no room
   ObsReduceArgs* d_obs = nullptr;
   int *d_tile_pre = nullptr, *d_elem_pre = nullptr, *d_col_pre = nullptr;
   int total_tiles = 0, total_elems = 0, total_cols = 0;
@@ -2657,8 +2680,65 @@ cudaError_t batch_exchange(mattohf_batch* b, int v) {
   if (b->opt_df)
     return launch_fock_sym_df_batch(b->NG, b->d_fsym[v], b->d_fsym_df[v], b->d_tile_pre, b->R, b->total_tiles,
                                     b->d_elem_pre, b->total_elems, b->st);
-  return launch_fock_sym_fx_batch(b->NG, b->d_fsym_fx[v], b->d_tile_pre, b->R, batch_tile(b), b->total_tiles,
-                                  b->d_elem_pre, b->total_elems, b->st);
+  cudaError_t e = launch_fock_sym_fx_batch(b->NG, b->d_fsym_fx[v], b->d_tile_pre, b->R, batch_tile(b), b->total_tiles,
+                                           b->d_elem_pre, b->total_elems, b->st);
+  for (const auto& d : b->dm) {
+    const mattohf_ctx* ctx = b->runs[d.r];
+    const Block u = blk(v >= 1 && v <= 3 ? ctx->d_us : ctx->d_u, ctx->NB, b->NG, ctx->NB);
+    FockDmArgs a = dm_args(ctx, u, u);
+    a.W = reinterpret_cast<fx::lc*>(b->dm_W);
+    a.wt = reinterpret_cast<fx::lc*>(b->dm_wt);
+    a.acc = reinterpret_cast<unsigned long long*>(d.acc);
+    a.wscale = d.wscale;
+    if (e == cudaSuccess) e = launch_dm_convert(b->NG, a, false, b->st);
+    if (e == cudaSuccess) e = launch_dm_build(b->NG, a, ctx->nsm, b->st);
+    if (e == cudaSuccess) e = launch_dm_apply(b->NG, a, ctx->nsm, b->st);
+  }
+  return e;
+}
+
+void batch_free_dm(mattohf_batch* b) {
+  for (auto& d : b->dm) {
+    cudaFree(d.acc);
+    cudaFree(d.wscale);
+  }
+  b->dm.clear();
+  cudaFree(b->dm_W);
+  cudaFree(b->dm_wt);
+  b->dm_W = b->dm_wt = nullptr;
+}
+
+// The runs that go through the density matrix and their buffers.  The line is that of
+// a run alone with twice the launches' time, since pairs of many runs share theirs.
+// Run-steps/s, all by pairs and so: 32 runs of 512/128/8 41 and 176, 256 runs of
+// 128 / 8 to 64 / 1 to 4 14.9 and 17.0 thousand.
+int batch_ensure_dm(mattohf_batch* b) {
+  batch_free_dm(b);
+  if (b->opt_df || !b->opt_dm) return MATTOHF_OK;
+  size_t nW = 0, nw = 0;
+  bool room = true;
+  for (int r = 0; r < b->R && room; ++r) {
+    mattohf_ctx* ctx = b->runs[r];
+    if (!ctx->hf || !fock_dm_wins(ctx, ctx->NB, true, 1.3e8)) continue;
+    const int rc = ensure_dm_tables(ctx);
+    if (rc != MATTOHF_OK && rc != MATTOHF_ERR_ALLOC) return bfail(b, rc, ctx->err);
+    const size_t cols = (size_t)ctx->NK * ctx->NB;
+    mattohf_batch::DmRun d{r, nullptr, nullptr};
+    room = rc == MATTOHF_OK && cudaMalloc((void**)&d.acc, cols * b->NG * 4 * sizeof(unsigned long long)) == cudaSuccess &&
+           cudaMalloc((void**)&d.wscale, cols * sizeof(double2)) == cudaSuccess;
+    b->dm.push_back(d);
+    nW = std::max(nW, (size_t)b->NG * (b->NG + 1) / 2 * ctx->NK);
+    nw = std::max(nw, cols * b->NG);
+  }
+  if (!b->dm.empty())
+    room = room && cudaMalloc((void**)&b->dm_W, nW * sizeof(int4)) == cudaSuccess &&
+           cudaMalloc((void**)&b->dm_wt, nw * sizeof(int4)) == cudaSuccess;
+  if (!room) {  // the pair kernels need none of it
+    cudaGetLastError();
+    batch_free_dm(b);
+    b->opt_dm = false;
+  }
+  return MATTOHF_OK;
 }
 
 // (Re)build every per-run argument array for runs of `nt` steps.
@@ -2680,8 +2760,12 @@ int batch_prepare(mattohf_batch* b, int nt) {
   // one launch shape (a CTA's teams) for every run; a smaller tile leaves
   // teams idle but gives small runs more CTAs
   const int S = batch_tile(b);
+  if (const int rc = batch_ensure_dm(b)) return rc;
   for (int r = 0; r < R; ++r) {
     mattohf_ctx* ctx = b->runs[r];
+    const mattohf_batch::DmRun* dm = nullptr;
+    for (const auto& d : b->dm)
+      if (d.r == r) dm = &d;
     int rc;
     if ((rc = ensure_series(ctx, nt)) || (rc = ensure_scratch(ctx, ctx->NK * ctx->NB)))
       return bfail(b, rc, ctx->err);
@@ -2690,7 +2774,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
     if (b->opt_df && (rc = ensure_sym(ctx, sym_partials(M, S, NG)))) return bfail(b, rc, ctx->err);
     if ((rc = ensure_fx(ctx))) return bfail(b, rc, ctx->err);
     if (!ctx->d_udf && (rc = dalloc(ctx, &ctx->d_udf, (size_t)M * NG))) return bfail(b, rc, ctx->err);
-    tile_pre[r + 1] = tile_pre[r] + T * (T + 1) / 2;
+    tile_pre[r + 1] = tile_pre[r] + (dm ? 0 : T * (T + 1) / 2);
     elem_pre[r + 1] = elem_pre[r] + M * NG;
     col_pre[r + 1] = col_pre[r] + ctx->NK * ctx->NB;
     AField fld[4];
@@ -2739,7 +2823,12 @@ int batch_prepare(mattohf_batch* b, int nt) {
       fp.b0 = ctx->NBocc;
       const AField af = v < 4 ? fld[v] : fld[3];
       CombineArgs c = combine_base(ctx, ub, af, v < 4 ? modes[v] : CM_OBS, fp);
-      if (ctx->hf) c.occ_ex = occ_source(ctx, b->opt_df);
+      if (ctx->hf && !dm) c.occ_ex = occ_source(ctx, b->opt_df);
+      if (dm) {
+        c.occ_ex = ExSource{nullptr, nullptr, nullptr, nullptr, 0, 0};
+        c.row_ex = ExSource{nullptr, dm->wscale, nullptr, reinterpret_cast<const unsigned long long*>(dm->acc), ctx->NB, ctx->NK};
+        c.row_b0 = 0;
+      }
       if (v == 4) c.af.mode = APREV;
       c.out = blko(ctx->d_us, ctx->NB, NG, ctx->NB);
       c.dt = b->dts[r];
@@ -2866,6 +2955,7 @@ int mattohf_batch_destroy(mattohf_batch* b) {
   void* ptrs[] = {b->d_obs, b->d_tile_pre, b->d_elem_pre, b->d_col_pre, b->d_int};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  batch_free_dm(b);
   for (auto* c : b->runs) mattohf_destroy(c);
   for (int v = 0; v < 4; ++v) cudaFree(b->d_comb_pre[v]);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -2956,6 +3046,7 @@ int mattohf_batch_set_option(mattohf_batch* b, int option, long long value) {
     if (value < 0 || value > fock_sym_teams(b->NG) || (value & (value - 1)))
       return bfail(b, MATTOHF_ERR_ARG, "tile size must be 0 or a power of two up to the CTA's teams");
     b->opt_tile = (int)value;
+    b->opt_dm = value == 0;
   } else {
     return bfail(b, MATTOHF_ERR_ARG, "unsupported batch option");
   }

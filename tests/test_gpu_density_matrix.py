@@ -73,3 +73,30 @@ def test_density_matrix_scales(built_lib):
             got[5, 1] = Fw[5, 1]
             assert np.array_equal(got, Fw)
         assert np.array_equal(ctx.ubkwbk_vFwbk(u, u), F)
+
+
+# the runs through the density matrix (no tile pairs) first, between and last, alone, and
+# all of them; two roundings a stage each way on top of the steps' own: 2^-52 times
+# 4 stages times the tolerance of one apply
+@pytest.mark.parametrize("shapes", [[(64, 8), (3, 2), (33, 9)], [(3, 2), (33, 9), (5, 1)], [(33, 9), (64, 8)], [(4, 3)]])
+def test_batch_members_through_the_density_matrix(built_lib, shapes):
+    """A batch of runs either way against the runs by pairs, twice (graph replay), and after a tile is asked for."""
+    from mattohf_gb300 import Batch, _capi
+    nt, dt = 3, 0.003
+    A = 0.02 * np.random.default_rng(8).standard_normal((len(shapes), nt))
+    u0 = [_functions(64, NK, nb, NK) for NK, nb in shapes]
+    tol = 4 * nt * _tol(64)
+    with Batch([_cfg(64, NK, nb) for NK, nb in shapes]) as b:
+        def run():
+            for r, u in enumerate(u0):
+                b[r].set_orbitals(u)
+            return b.rk4_run(A, A, dt), [b[r].get_orbitals() for r in range(len(u0))]
+        first, again = run(), run()
+        b.set_option(_capi.OPT_SYM_TILE, 2)  # pairs
+        pairs = run()
+    for x, y in zip(first[0], again[0]):
+        assert np.array_equal(x, y)
+    for x, y in zip(first[0], pairs[0]):
+        assert np.max(np.abs(np.asarray(x) - np.asarray(y))) <= tol * max(1.0, np.max(np.abs(np.asarray(y))))
+    for a, p in zip(first[1], pairs[1]):
+        assert _rel(a, p) <= tol
