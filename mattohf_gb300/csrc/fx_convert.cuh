@@ -66,7 +66,7 @@ __device__ __forceinline__ i64 fx_convert(double v, Scale s) {
 }
 
 // bounds of the converted orbitals, with a margin for the FP32 arithmetic:
-// 2^60.2 for the norm, 2^58.4 for a component
+// 2^60.2 for the norm, 2^58.4 for a component (2^58.9 for a modulus)
 constexpr float kNorm = 1.3241e18f, kPeak = 3.803e17f;
 
 // s of a set of size z (largest component, largest squared norm; both short of the

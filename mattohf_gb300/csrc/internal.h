@@ -118,7 +118,7 @@ cudaError_t launch_to_df_tables(const double* kern, int nkern, float2* kern_df, 
                                 float4* tw_df, cudaStream_t s);
 
 // Fixed-point exchange (k_fock_fx.cu).
-constexpr int kFxTerms = 16;   // terms that a fixed-point accumulator takes
+constexpr int kFxTerms = 12;   // terms of at most 2^59.3 that a fixed-point accumulator takes
 constexpr int kFxMaxTile = 8;  // largest tile (a row and a column accumulator take one term per round)
 constexpr int kRowsThreads = 128;   // CTA of the exchange on other functions
 constexpr int kRowsCtasPerSm = 12;  // its CTAs per SM to aim at

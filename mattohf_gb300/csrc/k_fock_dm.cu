@@ -18,8 +18,8 @@
 // Scales.  u^ = u s with s^2 n(x) <= 2^119.4 for n(x) = sum |u_kj(x)|^2, so
 // sum_k |D^_k| <= 2^59.4; the kernel's transform
 // is scaled so that its absolute sum over t is below 2^60 for every r, so |W^| <=
-// 2^60.4; w^ = w s_w with components up to 2^57.4, so kDmTerms products / 2^60 stay
-// below 2^63 and are then added to two words in global memory.
+// 2^59.4; w^ = w s_w with components up to 2^57.4 (moduli to 2^57.9), so the kDmTerms = 32
+// products / 2^60 of a sum stay below 2^62.3 and are then added to two words in global memory.
 #include "fx_convert.cuh"
 #include "internal.h"
 

@@ -4,8 +4,13 @@
 // Scales.  Orbitals are converted once per apply to u^ = u s 2^d with one
 // scale s for all of them (k_fx_stats, k_fx_convert): a short factor times a
 // power of two, so that u^ keeps every bit of u, with
-//     |u^|_2 <= 2^60.2      (a pair density's absolute sum stays below 2^60.4)
-//     max |u^| <= 2^58.4    (16 terms phi^ u^ / 2^60 stay below 2^63).
+//     |u^|_2 <= 2^60.2      (a pair density's absolute sum stays below 2^60.4, and
+//                            so does |phi^|, the kernel's being at most 2^60)
+//     each component of u^ <= 2^58.4, its modulus <= 2^58.9.
+// A term phi^ u^ / 2^60 is at most 2^59.3, all of which may fall on one component of the
+// sum: kFxTerms = 12 of them stay below 2^62.9 and the 8 of a tile below 2^62.3 (16, as
+// counted with 2^58.4 and |phi^| <= 2^60, reached 1.19 times 2^63 with equal functions
+// that are flat on a few points).
 // d = 0 except for an orbital whose norm is under half the largest one: d
 // then brings it up to that, and a term that it enters twice is shifted back.
 // The kernel table is K^ = kern s_k with sum_G |K^(G)| <= 2^60 for every k - k'.

@@ -206,8 +206,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
     sw = binary_scale(fx_scale(team_size<T>(wv), 1e30f, 1.0f, kSquareMax));
     asm volatile("bar.sync 4, %0;" ::"r"(32 * workers) : "memory");
     for (int w = 0; w < workers; ++w) zu = fx_larger(zu, size_s[w]);
-    // sums of n terms below 2^62.4
-    su = binary_scale(fx_scale(zu, kPeak * fminf(1.0f, 16.0f / (float)n), 1.0f, kSquareMax));
+    // sums of n terms, at most 2^59.3 each at the full peak (k_fock_fx.cu), below 2^62.9
+    su = binary_scale(fx_scale(zu, kPeak * fminf(1.0f, (float)kFxTerms / (float)n), 1.0f, kSquareMax));
     i64 rr[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) rr[e] = 0;
