@@ -214,6 +214,7 @@ int dalloc(mattohf_ctx* ctx, T** p, size_t n) {
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // or the next launch would report it
     return fail(ctx, MATTOHF_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
   return MATTOHF_OK;
@@ -423,8 +424,8 @@ int ensure_fock_buffers(mattohf_ctx* ctx) {
   const int M = ctx->NK * ctx->NBocc;
   if (ctx->opt_df) CKR(ensure_sym(ctx, sym_partials(M, sym_tile(ctx), ctx->NG)));
   CKR(ensure_fx(ctx));
-  if (use_dm(ctx, ctx->NB, true)) CKR(ensure_dm(ctx, ctx->NK * ctx->NB));  // or to the pairs
   if (!ctx->d_udf) CKR(dalloc(ctx, &ctx->d_udf, (size_t)M * ctx->NG));
+  if (use_dm(ctx, ctx->NB, true)) CKR(ensure_dm(ctx, ctx->NK * ctx->NB));  // or to the pairs
   return MATTOHF_OK;
 }
 
@@ -453,7 +454,7 @@ bool use_dm(const mattohf_ctx* c, int nbw, bool same) {
   return fock_dm_wins(c, nbw, same);
 }
 
-// No memory for W or the sums: the pair kernels take over, which need none of it.
+// No memory for the tables, W or the sums: the pair kernels take over, which need none of it.
 int dm_no_room(mattohf_ctx* ctx) {
   cudaGetLastError();
   destroy_graph(ctx);
@@ -467,8 +468,7 @@ int dm_no_room(mattohf_ctx* ctx) {
 }
 
 // Its tables and the orbitals' place, once per context.
-int ensure_dm_tables(mattohf_ctx* ctx) {
-  if (ctx->d_dm_table) return MATTOHF_OK;
+int make_dm_tables(mattohf_ctx* ctx) {
   const int NG = ctx->NG, NK = ctx->NK, L = dm_length(NK);
   if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "density-matrix tables during capture");
   const std::vector<int4> tw = fx_twiddles_host(L);
@@ -477,10 +477,9 @@ int ensure_dm_tables(mattohf_ctx* ctx) {
     ~Tmp() {
       if (p) cudaFree(p);
     }
-  } v, raw, mx, roots;
+  } v, raw, mx, roots, table;
   const std::vector<longlong2> rt = fx_roots(L);
   const size_t nu = (size_t)NG * ctx->NBocc * (L / 2);
-  int4* table = nullptr;
   CKR(dalloc(ctx, &ctx->d_dm_ut, nu));
   CKR(dalloc(ctx, &v.p, (size_t)(2 * NK - 1) * NG));
   CKR(dalloc(ctx, &raw.p, (size_t)NG * L));
@@ -490,23 +489,36 @@ int ensure_dm_tables(mattohf_ctx* ctx) {
   CKR(dalloc(ctx, &ctx->d_dm_tw, tw.size()));
   CKR(dalloc(ctx, &ctx->d_dm_tscale, 2));  // and the largest density
   CK(cudaMemsetAsync(ctx->d_dm_tscale, 0, 2 * sizeof(int2), ctx->st));
-  CKR(dalloc(ctx, &table, (size_t)NG * L));
+  CKR(dalloc(ctx, &table.p, (size_t)NG * L));
   CK(cudaMemcpyAsync(ctx->d_dm_tw, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemsetAsync(ctx->d_dm_ut, 0, nu * sizeof(int4), ctx->st));
   CK(launch_dm_table(NG, NK, ctx->d_kern_fx, reinterpret_cast<const fx::lc*>(ctx->d_tw_fx),
                      reinterpret_cast<const fx::cx*>(roots.p), reinterpret_cast<fx::cx*>(v.p),
-                     reinterpret_cast<fx::cx*>(raw.p), reinterpret_cast<int*>(mx.p), reinterpret_cast<fx::lc*>(table),
+                     reinterpret_cast<fx::cx*>(raw.p), reinterpret_cast<int*>(mx.p), reinterpret_cast<fx::lc*>(table.p),
                      ctx->d_dm_tscale, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
-  ctx->d_dm_table = table;
+  ctx->d_dm_table = table.p;
+  table.p = nullptr;
   return MATTOHF_OK;
 }
+int ensure_dm_tables(mattohf_ctx* ctx) {
+  if (ctx->d_dm_table) return MATTOHF_OK;
+  const int rc = make_dm_tables(ctx);
+  if (rc != MATTOHF_OK) {  // nothing is left of half a set
+    dalloc(ctx, &ctx->d_dm_ut, 0);
+    dalloc(ctx, &ctx->d_dm_tw, 0);
+    dalloc(ctx, &ctx->d_dm_tscale, 0);
+  }
+  return rc;
+}
 
-// W and the buffers for ncols columns of w.  Where there is no memory for them,
-// opt_dm = 0 afterwards.
+// The tables, W and the buffers for ncols columns of w.  Where there is no memory for
+// them, opt_dm = 0 afterwards.
 int ensure_dm(mattohf_ctx* ctx, int ncols) {
   const int NG = ctx->NG, NK = ctx->NK;
-  CKR(ensure_dm_tables(ctx));
+  const int rc = ensure_dm_tables(ctx);
+  if (rc == MATTOHF_ERR_ALLOC) return dm_no_room(ctx);
+  CKR(rc);
   if (!ctx->d_dm_W) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
     if (dalloc(ctx, &ctx->d_dm_W, (size_t)NG * (NG + 1) / 2 * NK)) return dm_no_room(ctx);
@@ -2364,6 +2376,11 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   const int nseg = (nt + phase) / C;
   const int s_last = nt - C;                 // start of the last segment (0 when C == nt)
   const size_t need = sizeof(double2) * elems * ((size_t)nseg + 4 * (size_t)C + 10);
+  if (need > freeb && ctx->d_dm_W) {  // the exchange by pairs leaves its room
+    CKR(dm_no_room(ctx));
+    CK(cudaMemGetInfo(&freeb, &totalb));
+    freeb += sizeof(double2) * (ctx->ckpt_cap + ctx->store_cap);
+  }
   if (need > freeb) return fail(ctx, MATTOHF_ERR_ALLOC, "checkpoint storage exceeds free device memory; lower ckpt_every");
   CKR(ensure_series(ctx, nt));
   CKR(ensure_scratch(ctx, NK * NB));
@@ -2760,20 +2777,22 @@ int batch_prepare(mattohf_batch* b, int nt) {
   // one launch shape (a CTA's teams) for every run; a smaller tile leaves
   // teams idle but gives small runs more CTAs
   const int S = batch_tile(b);
-  if (const int rc = batch_ensure_dm(b)) return rc;
+  for (auto* ctx : b->runs) {
+    const int M = ctx->NK * ctx->NBocc;
+    int rc;
+    if ((rc = ensure_series(ctx, nt)) || (rc = ensure_scratch(ctx, ctx->NK * ctx->NB)) ||
+        (b->opt_df && (rc = ensure_sym(ctx, sym_partials(M, S, NG)))) || (rc = ensure_fx(ctx)) ||
+        (!ctx->d_udf && (rc = dalloc(ctx, &ctx->d_udf, (size_t)M * NG))))
+      return bfail(b, rc, ctx->err);
+  }
+  if (const int rc = batch_ensure_dm(b)) return rc;  // last: the runs go on without it
   for (int r = 0; r < R; ++r) {
     mattohf_ctx* ctx = b->runs[r];
     const mattohf_batch::DmRun* dm = nullptr;
     for (const auto& d : b->dm)
       if (d.r == r) dm = &d;
-    int rc;
-    if ((rc = ensure_series(ctx, nt)) || (rc = ensure_scratch(ctx, ctx->NK * ctx->NB)))
-      return bfail(b, rc, ctx->err);
     const int M = ctx->NK * ctx->NBocc;
     const int T = (M + S - 1) / S;
-    if (b->opt_df && (rc = ensure_sym(ctx, sym_partials(M, S, NG)))) return bfail(b, rc, ctx->err);
-    if ((rc = ensure_fx(ctx))) return bfail(b, rc, ctx->err);
-    if (!ctx->d_udf && (rc = dalloc(ctx, &ctx->d_udf, (size_t)M * NG))) return bfail(b, rc, ctx->err);
     tile_pre[r + 1] = tile_pre[r] + (dm ? 0 : T * (T + 1) / 2);
     elem_pre[r + 1] = elem_pre[r] + M * NG;
     col_pre[r + 1] = col_pre[r] + ctx->NK * ctx->NB;

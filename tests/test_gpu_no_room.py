@@ -1,0 +1,74 @@
+"""Calls on a device with next to no free memory (needs a GB300): what has a form that needs
+less takes it, what has none reports it, and the context stays usable."""
+from __future__ import annotations
+
+import contextlib
+
+import numpy as np
+import pytest
+
+from test_gpu_fixed_point import _cfg, _functions, _rel
+
+pytestmark = pytest.mark.gpu
+OPT_CHUNKS, OPT_TILE, OPT_GRAPH = 2, 7, 1
+LEFT = 24 << 20
+SHAPE = (512, 128, 32)  # 33 MB of orbitals in the density matrix's layout
+
+
+@contextlib.contextmanager
+def _no_room():
+    """All but LEFT bytes of the device's memory taken (nothing is written to them)."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - LEFT, dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] <= LEFT
+        yield
+    finally:
+        del held
+        torch.cuda.empty_cache()
+
+
+@pytest.fixture(scope="module")
+def orbitals(built_lib):
+    from mattohf_gb300 import Context
+    with Context(_cfg(64, 64, 4)) as ctx:  # every kernel is loaded before the memory goes
+        u = _functions(64, 64, 4, 1)
+        ctx.ubkwbk_vFwbk(u, u)
+        ctx.ubkwbk_hwbk(u, u[:, :2], 0.1)
+    NG, NK, nb = SHAPE
+    return _functions(NG, 4, nb, 2).repeat(NK // 4, axis=0)
+
+
+def test_density_matrix_tables_without_room(orbitals):
+    """No room for the density matrix's tables: the pairs, which were there, and the
+    density matrix again once there is."""
+    from mattohf_gb300 import Context
+    u = orbitals
+    with Context(_cfg(*SHAPE)) as ctx:
+        ctx.set_option(OPT_CHUNKS, 1)  # pairs
+        pairs = ctx.ubkwbk_vFwbk(u, u)
+        ctx.set_option(OPT_CHUNKS, 0)
+        with _no_room():
+            assert np.array_equal(ctx.ubkwbk_vFwbk(u, u), pairs)
+        ctx.set_option(OPT_TILE, 0)
+        dm = ctx.ubkwbk_vFwbk(u, u)
+        assert not np.array_equal(dm, pairs) and _rel(dm, pairs) <= 2.0 ** -45
+
+
+def test_step_without_room(orbitals):
+    """The same for a propagation."""
+    from mattohf_gb300 import Context
+    A = np.full(1, 0.01)
+    out = []
+    with Context(_cfg(*SHAPE)) as ctx:
+        ctx.set_option(OPT_GRAPH, 0)
+        for chunks in (1, 0):
+            ctx.set_option(OPT_CHUNKS, chunks)
+            ctx.set_orbitals(orbitals)
+            with _no_room() if chunks == 0 else contextlib.nullcontext():
+                obs = ctx.rk4_run(A, A, 1e-4)
+            out.append((ctx.get_orbitals(), *obs))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
