@@ -286,20 +286,46 @@ int enq_density(mattohf_ctx* ctx, Block u, cudaStream_t st = nullptr, bool scala
   return MATTOHF_OK;
 }
 
+// A side stream's work between its fork from the main stream and its join.  Where an
+// error leaves before the join, the main stream joins all the same: what waits for it
+// (mattohf_synchronize, the next call) then also waits for the side stream, which may
+// read buffers of the caller.
+struct Branch {
+  mattohf_ctx* ctx = nullptr;
+  cudaStream_t side = nullptr;
+  cudaEvent_t done = nullptr;
+  int fork(mattohf_ctx* c, cudaStream_t s, cudaEvent_t e) {  // after ev_fork was recorded
+    mattohf_ctx* const ctx = c;
+    CK(cudaStreamWaitEvent(s, ctx->ev_fork, 0));
+    this->ctx = c;
+    side = s;
+    done = e;
+    return MATTOHF_OK;
+  }
+  int end() {  // its last launch that the join waits for
+    CK(cudaEventRecord(done, side));
+    return MATTOHF_OK;
+  }
+  int join() {
+    mattohf_ctx* const c = ctx;
+    ctx = nullptr;
+    if (c && cudaStreamWaitEvent(c->st, done, 0) != cudaSuccess) return fail(c, MATTOHF_ERR_CUDA, "stream join failed");
+    return MATTOHF_OK;
+  }
+  ~Branch() {
+    if (ctx && cudaEventRecord(done, side) == cudaSuccess) cudaStreamWaitEvent(ctx->st, done, 0);
+  }
+};
+
 // The density and local potential of u on a stream of its own, beside the exchange
 // that follows on the main one (without exchange: on the main one); the main stream
-// has them after join_density.
-int fork_density(mattohf_ctx* ctx, Block u) {
+// has them after the branch's join.
+int fork_density(mattohf_ctx* ctx, Block u, Branch* b) {
   if (!ctx->hf) return enq_density(ctx, u);
   CK(cudaEventRecord(ctx->ev_fork, ctx->st));
-  CK(cudaStreamWaitEvent(ctx->st_dens, ctx->ev_fork, 0));
+  CKR(b->fork(ctx, ctx->st_dens, ctx->ev_dens));
   CKR(enq_density(ctx, u, ctx->st_dens));
-  CK(cudaEventRecord(ctx->ev_dens, ctx->st_dens));
-  return MATTOHF_OK;
-}
-int join_density(mattohf_ctx* ctx) {
-  if (ctx->hf) CK(cudaStreamWaitEvent(ctx->st, ctx->ev_dens, 0));
-  return MATTOHF_OK;
+  return b->end();
 }
 
 // Which exchange partials a combine launch reads.
@@ -675,7 +701,8 @@ int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mo
   CKR(ensure_scratch(ctx, ctx->NK * w.nb));
   FockPlan fp;
   const bool dens = mode == CM_H && !same_u;
-  if (dens) CKR(fork_density(ctx, u));
+  Branch db;
+  if (dens) CKR(fork_density(ctx, u, &db));
   if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp, same_u));
   else if (mode == CM_F) {
     CK(cudaMemsetAsync(out.p, 0, sizeof(double2) * (size_t)ctx->NK * out.kstride, ctx->st));
@@ -683,7 +710,7 @@ int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mo
   }
   CombineArgs a = combine_base(ctx, w, af, mode, fp);
   a.out = out;
-  if (dens) CKR(join_density(ctx));
+  CKR(db.join());
   CK(launch_combine(ctx->NG, a, ctx->NK * w.nb, ctx->st));
   return MATTOHF_OK;
 }
@@ -732,7 +759,8 @@ ObsReduceArgs obs_args(mattohf_ctx* ctx, int advance) {
 int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, int advance, FockPlan* plan_out = nullptr) {
   const int NG = ctx->NG, NB = ctx->NB;
   Block ub = blk(u, NB, NG, NB);
-  CKR(fork_density(ctx, ub));
+  Branch db;
+  CKR(fork_density(ctx, ub, &db));
   FockPlan fp;
   fp.any = false;
   if (ctx->hf) CKR(enq_fock(ctx, ub, ub, &fp));
@@ -740,7 +768,7 @@ int enq_observables(mattohf_ctx* ctx, const double2* u, AField af, int advance, 
   if (plan_out) *plan_out = fp;
   CombineArgs a = combine_base(ctx, ub, af, CM_OBS, fp);
   CK(launch_combine(NG, a, ctx->NK * NB, ctx->st));
-  CKR(join_density(ctx));
+  CKR(db.join());
   CK(launch_obs_reduce(obs_args(ctx, advance), ctx->st));
   return MATTOHF_OK;
 }
@@ -769,15 +797,16 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
     FockPlan fp;
     const bool side = ctx->hf != 0;
     const bool obs = run && side && s == 0;
+    Branch db, kb;
     if (side) {
       // The density and the kinetic part of h w need only the stage input: each
       // has a stream beside the exchange (one after the other on one stream, their
       // 22 us were a small problem's longest chain).
       CK(cudaEventRecord(ctx->ev_fork, ctx->st));
-      CK(cudaStreamWaitEvent(ctx->st_side, ctx->ev_fork, 0));
-      CK(cudaStreamWaitEvent(ctx->st_dens, ctx->ev_fork, 0));
+      CKR(kb.fork(ctx, ctx->st_side, ctx->ev_join));
+      CKR(db.fork(ctx, ctx->st_dens, ctx->ev_dens));
       CKR(enq_density(ctx, ub, ctx->st_dens, !run || obs));
-      CK(cudaEventRecord(ctx->ev_dens, ctx->st_dens));
+      CKR(db.end());
       CombineArgs pre = combine_base(ctx, ub, fs[s], modes[s], FockPlan());
       pre.split = 1;
       pre.hpre = ctx->d_hpre;
@@ -787,11 +816,11 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
         pre.af_obs.mode = APREV;
       }
       CK(launch_combine(NG, pre, ctx->NK * NB, ctx->st_side));
-      CK(cudaEventRecord(ctx->ev_join, ctx->st_side));
+      CKR(kb.end());
       if (run && s == 1) CK(launch_obs_reduce(obs_args(ctx, 3), ctx->st_side));  // joined by stage 2
       CKR(enq_fock(ctx, ub, ub, &fp, false, run || s > 0));
-      CK(cudaStreamWaitEvent(ctx->st, ctx->ev_dens, 0));
-      CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
+      CKR(db.join());
+      CKR(kb.join());
     } else {
       CKR(enq_density(ctx, ub));
     }
@@ -1336,7 +1365,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
                   ctx->d_colbuf, ctx->d_int, ctx->d_A, ctx->d_Aave, ctx->d_sE,
                   ctx->d_sJ, ctx->d_sN, ctx->d_work, ctx->d_hwork, ctx->d_M, ctx->d_V, ctx->d_evals,
                   ctx->d_eps, ctx->d_err, ctx->d_sym, ctx->d_symF, ctx->d_dpart,
-                  ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale,
+                  ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale, 
                   ctx->d_wfx, ctx->d_wscale, ctx->d_fx_acc, ctx->d_wacc, ctx->d_kern_fx, ctx->d_kscale,
                   ctx->d_tw_fx, ctx->d_tw_small, ctx->d_dm_ut, ctx->d_dm_wt, ctx->d_dm_table, ctx->d_dm_tw, ctx->d_dm_W,
                   ctx->d_dm_tscale, ctx->d_dm_acc, ctx->d_dm_wscale, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
@@ -1558,7 +1587,8 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   const int ncols = nkl * nbw;
   CKR(ensure_scratch(ctx, ncols));
   const bool dens = mode == CM_H || mode == CM_OBS;
-  if (dens) CKR(fork_density(ctx, u));
+  Branch db;
+  if (dens) CKR(fork_density(ctx, u, &db));
   FockPlan fp;
   if (ctx->hf && mode != CM_T) {
     CKR(ensure_fx(ctx));
@@ -1578,7 +1608,7 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
   c.kx = ctx->d_kx + k0;
   c.nk = nkl;
   c.out = out;
-  if (dens) CKR(join_density(ctx));
+  CKR(db.join());
   CK(launch_combine(NG, c, ncols, ctx->st));
   return MATTOHF_OK;
 }

@@ -72,3 +72,30 @@ def test_step_without_room(orbitals):
             out.append((ctx.get_orbitals(), *obs))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_apply_that_runs_out_of_room(orbitals):
+    """An apply whose exchange finds no memory after its density was started: an error; once
+    the streams are synchronised the caller's buffers are free, and the context works."""
+    import torch
+    from mattohf_gb300 import Context, _capi
+    NG, NK, nb = SHAPE
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x).view(np.float64)).cuda()
+    with Context(_cfg(*SHAPE)) as ctx:
+        u, w = dev(orbitals), dev(orbitals[:, :2])
+        ctx.ubk_tubk(orbitals[:, :2], 0.1)  # the buffers that every apply takes
+        out = torch.empty_like(w)
+        torch.empty_like(u).zero_()  # its kernel is loaded too
+        call = lambda: ctx.lib.mattohf_hpsi_device(ctx.h, u.data_ptr(), w.data_ptr(), 2, 0.1, out.data_ptr())
+        torch.cuda.synchronize()
+        with _no_room():
+            assert call() == _capi.ERR_ALLOC
+            ctx.synchronize()
+            u.zero_()
+            torch.cuda.synchronize()
+        u.copy_(dev(orbitals))
+        torch.cuda.synchronize()
+        assert call() == _capi.OK
+        ctx.synchronize()
+        got = out.cpu().numpy().view(np.complex128)
+        assert np.array_equal(got, ctx.ubkwbk_hwbk(orbitals, orbitals[:, :2], 0.1))
