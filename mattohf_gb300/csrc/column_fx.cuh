@@ -78,7 +78,14 @@ __device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, in
     x = fma((double)hx, 4294967296.0, (double)lx);
     y = fma((double)hy, 4294967296.0, (double)ly);
   }
-  return make_double2(fma(x, f.x, x * f.y), fma(y, f.x, y * f.y));
+  x = fma(x, f.x, x * f.y);
+  y = fma(y, f.x, y * f.y);
+  if (s.pexp != nullptr) {
+    const double p = pow2(-s.pexp[q]);
+    x *= p;
+    y *= p;
+  }
+  return make_double2(x, y);
 }
 // Sum over a CTA, result in every thread of warp 0 (fixed order).
 template <int NW>

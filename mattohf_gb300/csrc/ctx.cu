@@ -105,6 +105,8 @@ struct mattohf_ctx {
   int* d_fx_shift = nullptr;
   double2* d_fx_fscale = nullptr;
   int2* d_uscale = nullptr;
+  int4* d_uprod = nullptr;    // of the exchange by itself: orbitals with a scale per grid
+  int* d_points = nullptr;    // point and its exponents
   int4* d_wfx = nullptr;      // other functions in limbs and their scales
   double2* d_wscale = nullptr;
   unsigned long long *d_fx_acc = nullptr, *d_wacc = nullptr;  // exchange sums
@@ -335,6 +337,7 @@ struct FockPlan {
   bool rows = false;          // bands >= b0 by the exchange on rows
   bool dm = false;            // all bands through the density matrix
   bool any = false;           // exchange present at all
+  bool points = false;        // its sums carry a scale per grid point
 };
 
 int ensure_sym(mattohf_ctx* ctx, size_t need) {
@@ -411,7 +414,8 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   a.S = S;
   a.T = (ctx->NK * ctx->NBocc + S - 1) / S;
   a.sizes = ctx->d_fx_sizes;
-  a.ufx = reinterpret_cast<fx::lc*>(ctx->d_ufx);
+  a.ufx = a.uprod = reinterpret_cast<fx::lc*>(ctx->d_ufx);
+  a.pexp = nullptr;
   a.shift = ctx->d_fx_shift;
   a.fscale = ctx->d_fx_fscale;
   a.uscale = ctx->d_uscale;
@@ -422,6 +426,15 @@ FockFxArgs fx_args(const mattohf_ctx* ctx, Block u, int S) {
   a.lift = 1;
   a.halve = 0;
   return a;
+}
+
+// A scale for every grid point (k_fx_points) in the arguments.
+int point_scales(mattohf_ctx* ctx, FockFxArgs* a) {
+  if (!ctx->d_points) CKR(dalloc(ctx, &ctx->d_points, (size_t)ctx->NG));
+  if (!ctx->d_uprod) CKR(dalloc(ctx, &ctx->d_uprod, (size_t)ctx->NK * ctx->NBocc * ctx->NG));
+  a->uprod = reinterpret_cast<fx::lc*>(ctx->d_uprod);
+  a->pexp = ctx->d_points;
+  return MATTOHF_OK;
 }
 
 std::vector<int4> fx_twiddles_host(int NG, bool latency = false);
@@ -595,14 +608,18 @@ int enq_fock_dm(mattohf_ctx* ctx, Block u, Block w, bool same_u, bool have_sizes
 // Exchange of h[u] w.  When w is u itself (all RK4 stages, Ex, Subspace_diag,
 // eps) the occupied rows use the symmetric pair kernel and only the unoccupied
 // rows (if any) the kernel for other functions.  have_sizes: the orbitals' sizes
-// are there (left by the kernel that made them).
-int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = false, bool have_sizes = false) {
+// are there (left by the kernel that made them).  points: for the exchange by itself, by
+// pairs with a scale for every grid point (k_fx_points); the density matrix's W would need
+// one too and still be 1e-14 off where few orbitals reach.
+int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = false, bool have_sizes = false,
+             bool points = false) {
   *plan = FockPlan();
   plan->any = true;
+  plan->points = points;
   const bool same = (w.p == u.p) && (w.kstride == u.kstride) && (w.nb == u.nb);
   const int NG = ctx->NG;
   const int M = ctx->NK * ctx->NBocc;
-  bool dm = use_dm(ctx, w.nb, same);
+  bool dm = !points && use_dm(ctx, w.nb, same);
   if (dm) {
     CKR(ensure_fx(ctx));
     CKR(ensure_dm(ctx, ctx->NK * w.nb));
@@ -625,8 +642,9 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = f
   plan->rows = w.nb > plan->b0;
   CKR(ensure_fx(ctx));
   const int S = fx_tile(ctx);
-  const FockFxArgs a = fx_args(ctx, u, S);
+  FockFxArgs a = fx_args(ctx, u, S);
   FockFxRows r;
+  if (points) CKR(point_scales(ctx, &a));
   if (plan->rows) {
     Block wr = w;
     wr.p = w.p + (size_t)plan->b0 * NG;
@@ -642,6 +660,7 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = f
   CKR(timed_begin(ctx));
   if (plan->rows || !df)
     CK(launch_fx_convert(NG, a, plan->rows ? &r : nullptr, have_sizes, same_u && !plan->occ, ctx->st));
+  if (points && (plan->rows || !df)) CK(launch_fx_points(NG, a, ctx->st));
   if (df) {
     FockSymDfArgs d;
     d.u = ctx->d_udf;
@@ -678,6 +697,7 @@ CombineArgs combine_base(mattohf_ctx* ctx, Block w, AField af, int mode, const F
   if (ex && fp.dm)
     a.row_ex = ExSource{nullptr, ctx->d_dm_wscale, nullptr, ctx->d_dm_acc, w.nb, ctx->NK};
   a.row_b0 = fp.b0;
+  if (fp.points) a.occ_ex.pexp = a.row_ex.pexp = ctx->d_points;
   a.vloc = ctx->d_vloc;
   a.Gx = ctx->d_Gx;
   a.kx = ctx->d_kx;
@@ -703,7 +723,7 @@ int enq_hpsi(mattohf_ctx* ctx, Block u, Block w, BlockOut out, AField af, int mo
   const bool dens = mode == CM_H && !same_u;
   Branch db;
   if (dens) CKR(fork_density(ctx, u, &db));
-  if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp, same_u));
+  if (ctx->hf && mode != CM_T) CKR(enq_fock(ctx, u, w, &fp, same_u, false, mode == CM_F));
   else if (mode == CM_F) {
     CK(cudaMemsetAsync(out.p, 0, sizeof(double2) * (size_t)ctx->NK * out.kstride, ctx->st));
     return MATTOHF_OK;
@@ -1365,7 +1385,7 @@ int mattohf_destroy(mattohf_ctx* ctx) {
                   ctx->d_colbuf, ctx->d_int, ctx->d_A, ctx->d_Aave, ctx->d_sE,
                   ctx->d_sJ, ctx->d_sN, ctx->d_work, ctx->d_hwork, ctx->d_M, ctx->d_V, ctx->d_evals,
                   ctx->d_eps, ctx->d_err, ctx->d_sym, ctx->d_symF, ctx->d_dpart,
-                  ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale, 
+                  ctx->d_ufx, ctx->d_fx_sizes, ctx->d_fx_shift, ctx->d_fx_fscale, ctx->d_uscale, ctx->d_uprod, ctx->d_points,
                   ctx->d_wfx, ctx->d_wscale, ctx->d_fx_acc, ctx->d_wacc, ctx->d_kern_fx, ctx->d_kscale,
                   ctx->d_tw_fx, ctx->d_tw_small, ctx->d_dm_ut, ctx->d_dm_wt, ctx->d_dm_table, ctx->d_dm_tw, ctx->d_dm_W,
                   ctx->d_dm_tscale, ctx->d_dm_acc, ctx->d_dm_wscale, ctx->d_udf, ctx->d_kern_df, ctx->d_tw_df, ctx->d_hpre, ctx->d_ticket,
@@ -1596,7 +1616,10 @@ static int enq_kslice(mattohf_ctx* ctx, const double* d_uocc, int k0, int nkl, c
     a.kern += (size_t)k0 * NG;
     FockFxRows r;
     CKR(fx_rows_args(ctx, w, nkl, &r));
+    fp.points = mode == CM_F;
+    if (fp.points) CKR(point_scales(ctx, &a));
     CK(launch_fx_convert(NG, a, &r, false, false, ctx->st));
+    if (fp.points) CK(launch_fx_points(NG, a, ctx->st));
     CK(launch_fock_fx(NG, a, r, ctx->st));
     fp.any = true;
     fp.rows = true;

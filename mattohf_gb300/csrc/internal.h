@@ -129,6 +129,10 @@ struct FockFxArgs {
   int2* sizes;          // [NK*nbocc]: largest |component| and squared norm (fx_size)
   fx::lc* ufx;          // [NK*nbocc][NG] fixed-point orbitals in limbs
   int* shift;           // [NK*nbocc] extra scale 2^d of an orbital with a small norm
+  // what the pair potentials multiply: ufx, or (pexp not null, launch_fx_points) the
+  // orbitals with a scale for every grid point, u s 2^(pexp - d); F^ then carries 2^pexp
+  fx::lc* uprod;        // [NK*nbocc][NG]
+  int* pexp;            // [NG]
   double2* fscale;      // [NK*nbocc] F = F^ * (x + y)
   int2* uscale;         // the orbitals' common scale (c, k)
   const int2* kern;     // kernel table in limbs
@@ -188,6 +192,8 @@ struct FockFxRows {
 // to fixed point, before either exchange; have_sizes: a.sizes holds.
 cudaError_t launch_fx_convert(int NG, const FockFxArgs& a, const FockFxRows* r, bool have_sizes, bool have_orbitals,
                               cudaStream_t s);
+// a.uprod and a.pexp, after the orbitals' conversion
+cudaError_t launch_fx_points(int NG, const FockFxArgs& a, cudaStream_t s);
 cudaError_t launch_fx_sizes(int NG, const FockFxArgs& a, cudaStream_t s);
 cudaError_t launch_fx_sizes_batch(int NG, const FockFxArgs* d_args, const int* d_elem_pre, int nruns, int total_elems,
                                   cudaStream_t s);
@@ -274,6 +280,7 @@ struct ExSource {
   // or sums with k fastest, [NG][dm_nb][4][dm_nk] (k_fock_dm.cu), and scale
   const unsigned long long* dm;
   int dm_nb, dm_nk;
+  const int* pexp;  // sums that carry 2^pexp at every grid point, or null
 };
 
 struct CombineArgs {

@@ -2,8 +2,9 @@
 // transforms (fft_fx.cuh).
 //
 // Scales.  Orbitals are converted once per apply to u^ = u s 2^d with one
-// scale s for all of them (k_fx_stats, k_fx_convert): a short factor times a
-// power of two, so that u^ keeps every bit of u, with
+// scale s for all of them (k_fx_sizes, k_fx_convert): a short factor times a
+// power of two, so that u^ keeps every bit of the components from 2^-6 of the
+// largest on and 2^-59 of the largest at the others, with
 //     |u^|_2 <= 2^60.2      (a pair density's absolute sum stays below 2^60.4, and
 //                            so does |phi^|, the kernel's being at most 2^60)
 //     each component of u^ <= 2^58.4, its modulus <= 2^58.9.
@@ -11,8 +12,9 @@
 // sum: kFxTerms = 12 of them stay below 2^62.9 and the 8 of a tile below 2^62.3 (16, as
 // counted with 2^58.4 and |phi^| <= 2^60, reached 1.19 times 2^63 with equal functions
 // that are flat on a few points).
-// d = 0 except for an orbital whose norm is under half the largest one: d
-// then brings it up to that, and a term that it enters twice is shifted back.
+// d = 0 except for an orbital whose norm is half the largest one or less: d then
+// brings it to the upper half, and a term that it enters twice is shifted back by 2 d
+// (its components may pass 2^58.4, as a modulus up to 2^60.2; 2 d >= 2 makes up for it).
 // The kernel table is K^ = kern s_k with sum_G |K^(G)| <= 2^60 for every k - k'.
 // A pair's chain is then
 //     p^ = u_a^ conj(u_b^) / 2^60,  phi^ = IFFT(K^ FFT(p^) / 2^60),
@@ -79,15 +81,17 @@ __device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, const FockF
   else __syncthreads();
   g = fx_larger(fx_larger(red[0], red[1]), fx_larger(red[2], red[3]));
   if (!row) own = own_s;
-  Scale s = fx_scale(g, kPeak, 1.0f, kSquareMax);
+  // with a scale per point the sums' terms are uprod's, and u^ is bounded by its norm alone
+  Scale s = fx_scale(g, a.pexp != nullptr ? 1e30f : kPeak, 1.0f, kSquareMax);
   s.k -= a.halve;
   Scale sd = s;
   int d = 0;
   if (row) {
     sd = fx_scale(own, 1e30f, 1.0f, kSquareMax);
-  } else if (a.lift && own.y > 0) {  // a column with less than half the largest norm is lifted by 2^d
-    const int lg = (g.y >> 18) - (own.y >> 18);  // log2 of the squared norms' ratio, to 1
-    if (lg > 2) d = min(60, (lg - 1) >> 1);
+  } else if (a.lift && own.y > 0) {
+    // a column with half the largest norm or less is lifted by 2^d to the upper half: the
+    // largest d with own^2 4^d up to the largest square (keys order like these)
+    d = min(1000, (g.y - own.y) >> 19);
     sd.k += d;
   }
   const bool ok = sd.c != 0;
@@ -145,6 +149,41 @@ __global__ void __launch_bounds__(128) k_fx_convert_batch(const FockFxArgs* __re
                                                           const int* __restrict__ pre, int nruns, int N) {
   const int r = find_run(pre, nruns, blockIdx.x * N);
   fx_convert_body(args[r], FockFxRows{}, N, blockIdx.x - pre[r] / N, false);
+}
+
+// The exchange by itself (mattohf_fock) is accurate at every grid point, as with FP64
+// values, where h[u] w has the kinetic transform's error of one size everywhere.  A
+// pair's density may have one scale, its transform mixing all points; but the product
+// phi_ab(x) u_b(x) then loses what |u_b(x)| is below the peak (a Gaussian's value of 1e-8
+// of it came out 5e-11 off).  So it takes the orbitals again, with a scale 2^pexp(x)
+// that brings the largest of |u_b(x)| 2^-d_b over b (the size of its term: phi_ab^
+// carries 2^d_b) to 2^57 or more.  A CTA takes eight points; it reads the orbitals twice.
+__global__ void __launch_bounds__(512) k_fx_points(FockFxArgs a, int N) {
+  __shared__ int part[16][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, x = blockIdx.x * 8 + (lane & 7);
+  const int M = a.nk * a.nbocc;
+  const Scale s{a.uscale->x, a.uscale->y};
+  constexpr int kNone = -8192;
+  int m = kNone;
+  for (int c = threadIdx.x >> 3; c < M; c += 64) {
+    const double2 z = fx_column(a.u, a.nbocc, c, N)[x];
+    const int e = max((__double2hiint(z.x) & 0x7fffffff) >> 20, (__double2hiint(z.y) & 0x7fffffff) >> 20);
+    if (z.x != 0.0 || z.y != 0.0) m = max(m, max(e, 1) - a.shift[c]);
+  }
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+  if (lane < 8) part[warp][lane] = m;
+  __syncthreads();
+  for (int w = 0; w < 16; ++w) m = max(m, part[w][lane & 7]);
+  // a component with exponent field e is below 2^(e - 1022), s below 2^(k + 4); where all
+  // are zero (2^-2000 = 0), so is the sum of the products' roundings
+  const int pe = s.c == 0 ? 0 : m == kNone ? 2000 : min(1000, 1076 - s.k - m);
+  if (warp == 0 && lane < 8) a.pexp[x] = pe;
+  for (int c = threadIdx.x >> 3; c < M; c += 64) {
+    const double2 z = fx_column(a.u, a.nbocc, c, N)[x];
+    const Scale sx{s.c, s.k + pe - a.shift[c]};
+    a.uprod[(size_t)c * N + x] = s.c ? fx::limbs(cx{fx_convert(z.x, sx), fx_convert(z.y, sx)}) : lc{0, 0, 0, 0};
+  }
 }
 
 // t / 2^s for s > 0, rounded (a floor would be biased by half a place per term)
@@ -247,8 +286,9 @@ __device__ __forceinline__ void fock_sym_fx_body(const FockFxArgs& a, const int 
   const bool va = tw_ < S && ia < M;
   const int oa = va ? ia : 0;
   const int ka = oa / a.nbocc;
-  const lc* ua = a.ufx + (size_t)oa * N;
-  const int sa = 2 * a.shift[oa];
+  const lc *ua = a.ufx + (size_t)oa * N, *uam = a.uprod + (size_t)oa * N;
+  const bool points = a.pexp != nullptr;  // the orbitals' 2^d are in uprod
+  const int sa = points ? 0 : 2 * a.shift[oa];
   cx racc[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) racc[e] = cx{0, 0};
@@ -263,20 +303,20 @@ __device__ __forceinline__ void fock_sym_fx_body(const FockFxArgs& a, const int 
     const bool self = diag && r == 0;
     const int ob = ib < M ? ib : 0;
     const int kb = ob / a.nbocc;
-    const lc* ub = a.ufx + (size_t)ob * N;
+    const lc *ub = a.ufx + (size_t)ob * N, *ubm = a.uprod + (size_t)ob * N;
     const int2* kab = a.kern + (size_t)(ka - kb + a.nk - 1) * N;
     cx x[E];
     const cx rn = pair_potential<N>(x, ua, ub, kab, buf, tw_s, twn_s, tl, tw_);
     if (valid) {
-      const int sb = 2 * a.shift[ob];
+      const int sb = points ? 0 : 2 * a.shift[ob];
       // phi u_b = conj(x) u_b
       if (sb == 0) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) racc[e] = fx::add(racc[e], fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])));
+        for (int e = 0; e < E; ++e) racc[e] = fx::add(racc[e], fx::cmulc(ubm[TM::pos(tl, e)], fx::limbs(x[e])));
       } else {
 #pragma unroll
         for (int e = 0; e < E; ++e)
-          racc[e] = fx::add(racc[e], fx_shift(fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])), sb));
+          racc[e] = fx::add(racc[e], fx_shift(fx::cmulc(ubm[TM::pos(tl, e)], fx::limbs(x[e])), sb));
       }
       if (!self) {
         // phi_ba = conj(phi_ab + c (-1)^x), c = (K_ba - K_ab)(N/2) R_ab(N/2)
@@ -288,13 +328,13 @@ __device__ __forceinline__ void fock_sym_fx_body(const FockFxArgs& a, const int 
 #pragma unroll
           for (int e = 0; e < E; ++e) {
             const int q = TM::pos(tl, e);
-            col[q] = fx::add(col[q], fx::cmul(fx::limbs(fx::add(x[e], c)), ua[q]));
+            col[q] = fx::add(col[q], fx::cmul(fx::limbs(fx::add(x[e], c)), uam[q]));
           }
         } else {
 #pragma unroll
           for (int e = 0; e < E; ++e) {
             const int q = TM::pos(tl, e);
-            col[q] = fx::add(col[q], fx_shift(fx::cmul(fx::limbs(fx::add(x[e], c)), ua[q]), sa));
+            col[q] = fx::add(col[q], fx_shift(fx::cmul(fx::limbs(fx::add(x[e], c)), uam[q]), sa));
           }
         }
       }
@@ -368,18 +408,18 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_fock_fx(FockFxArgs a, FockF
         acc[e] = cx{0, 0};
       }
     }
-    const lc* ub = a.ufx + (size_t)p * N;
+    const lc *ub = a.ufx + (size_t)p * N, *ubm = a.uprod + (size_t)p * N;
     const int2* kab = a.kern + (size_t)(kr - p / a.nbocc + a.nk - 1) * N;
     cx x[E];
     pair_potential<N>(x, wa, ub, kab, buf, tw_s, twn_s, tl, team);
-    const int sb = 2 * a.shift[p];
+    const int sb = a.pexp != nullptr ? 0 : 2 * a.shift[p];
     if (sb == 0) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) acc[e] = fx::add(acc[e], fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])));
+      for (int e = 0; e < E; ++e) acc[e] = fx::add(acc[e], fx::cmulc(ubm[TM::pos(tl, e)], fx::limbs(x[e])));
     } else {
 #pragma unroll
       for (int e = 0; e < E; ++e)
-        acc[e] = fx::add(acc[e], fx_shift(fx::cmulc(ub[TM::pos(tl, e)], fx::limbs(x[e])), sb));
+        acc[e] = fx::add(acc[e], fx_shift(fx::cmulc(ubm[TM::pos(tl, e)], fx::limbs(x[e])), sb));
     }
   }
   if (!valid) return;
@@ -626,6 +666,11 @@ cudaError_t launch_fx_convert(int NG, const FockFxArgs& a, const FockFxRows* r, 
   const int n = (have_orbitals ? 0 : M) + (r ? r->ncols : 0);
   if (n == 0) return cudaSuccess;
   k_fx_convert<<<n, 128, 0, s>>>(a, r ? *r : FockFxRows{}, NG, have_orbitals ? M : 0, scan);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_points(int NG, const FockFxArgs& a, cudaStream_t s) {
+  k_fx_points<<<NG / 8, 512, 0, s>>>(a, NG);
   return cudaGetLastError();
 }
 

@@ -35,7 +35,7 @@ def orbitals(built_lib):
     from mattohf_gb300 import Context
     with Context(_cfg(64, 64, 4)) as ctx:  # every kernel is loaded before the memory goes
         u = _functions(64, 64, 4, 1)
-        ctx.ubkwbk_vFwbk(u, u)
+        ctx.ubkwbk_hwbk(u, u, 0.1)
         ctx.ubkwbk_hwbk(u, u[:, :2], 0.1)
     NG, NK, nb = SHAPE
     return _functions(NG, 4, nb, 2).repeat(NK // 4, axis=0)
@@ -48,12 +48,12 @@ def test_density_matrix_tables_without_room(orbitals):
     u = orbitals
     with Context(_cfg(*SHAPE)) as ctx:
         ctx.set_option(OPT_CHUNKS, 1)  # pairs
-        pairs = ctx.ubkwbk_vFwbk(u, u)
+        pairs = ctx.ubkwbk_hwbk(u, u, 0.1)
         ctx.set_option(OPT_CHUNKS, 0)
         with _no_room():
-            assert np.array_equal(ctx.ubkwbk_vFwbk(u, u), pairs)
+            assert np.array_equal(ctx.ubkwbk_hwbk(u, u, 0.1), pairs)
         ctx.set_option(OPT_TILE, 0)
-        dm = ctx.ubkwbk_vFwbk(u, u)
+        dm = ctx.ubkwbk_hwbk(u, u, 0.1)
         assert not np.array_equal(dm, pairs) and _rel(dm, pairs) <= 2.0 ** -45
 
 
