@@ -54,32 +54,33 @@ __device__ __forceinline__ int2 team_size(const double2 (&v)[E]) {
 // Scales are powers of two here, so that nothing has to be divided by them.
 __device__ __forceinline__ Scale binary_scale(Scale s) { return Scale{s.c ? 8 : 0, s.k}; }
 
-// x <- conj(x k) 2^r for the real factors k (real_limbs, below 2^60), ready for the
-// way back, with r from the product's norm: its N values' partial sums stay below
-// 2^60.5 whatever the factors' range (a kinetic energy's is 2^12 and more between the
-// frequencies that carry a function and the largest).  Returns r.
+// x <- conj(x k 2^-g) 2^r for the real factors k 2^-g (real_limbs; 2^58 <= |k| < 2^60 or
+// zero, 0 <= g <= kMaxShift), ready for the way back, with r from the product's norm:
+// its N values' partial sums stay below 2^60.5 whatever the factors' range (a kinetic
+// energy's is 2^12 and more between the frequencies that carry a function and the
+// largest).  The factors being normalised, the rounding of a product to a place is
+// no larger than what the transform has left in x.  Returns r.
+constexpr int kMaxShift = 100;
 template <int N, int T, int E>
-__device__ __forceinline__ int multiply_back(cx (&x)[E], const int2 (&k)[E]) {
+__device__ __forceinline__ int multiply_back(cx (&x)[E], const int2 (&k)[E], const int (&g)[E]) {
   constexpr int kLog2N = N == 64 ? 6 : N == 128 ? 7 : 8;
   float s = 0.0f;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    const float f = fmaf((float)k[e].x, 0x1p-30f, (float)k[e].y * 0x1p-60f);
-    const float p = __ll2float_rn(x[e].x) * f, q = __ll2float_rn(x[e].y) * f;
+    x[e] = cx{fx::rmul(x[e].x, k[e]), -fx::rmul(x[e].y, k[e])};
+    const float f = __int_as_float((127 - g[e]) << 23), p = __ll2float_rn(x[e].x) * f, q = __ll2float_rn(x[e].y) * f;
     s = fmaf(p, p, fmaf(q, q, s));
   }
 #pragma unroll
   for (int o = T / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   // N s < 2^(log2 N + e + 1) for the exponent e of s; at most 2^120
   const int r = min(29, max(-8, (119 - kLog2N - ((__float_as_int(s) >> 23) - 127)) >> 1));
-  auto mul = [&](i64 a, int2 b) -> i64 {
-    const int ah = fx::hi_limb(a), al = fx::lo_limb(a);
-    const i64 hh = fx::mw(ah, b.x), m = fx::mw(ah, b.y, fx::mw(al, b.x)) + (fx::mw(al, b.y) >> fx::kLimb);
-    if (r >= 0) return (hh << r) + ((m + (1ll << (fx::kLimb - 1 - r))) >> (fx::kLimb - r));
-    return (hh + (m >> fx::kLimb) + (1ll << (-r - 1))) >> -r;
-  };
 #pragma unroll
-  for (int e = 0; e < E; ++e) x[e] = cx{mul(x[e].x, k[e]), -mul(x[e].y, k[e])};
+  for (int e = 0; e < E; ++e) {
+    const int q = r - g[e], left = max(q, 0), right = min(62, max(-q, 0));
+    const i64 half = (1ll << right) >> 1;
+    x[e] = cx{((x[e].x << left) + half) >> right, ((x[e].y << left) + half) >> right};
+  }
   return r;
 }
 
@@ -150,15 +151,19 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
     escale_s[0] = make_int2(0, 1);
   }
   const bool hartree = chunk == 0 && warp == kSmallWarps - 1;
-  int2 vg[E];  // the Hartree warp: vCG 2^kv < 2^60
-  int kv = 0;
+  int2 vg[E];  // the Hartree warp: vCG 2^kv = vg 2^-gg, vg < 2^60
+  int gg[E], kv = 0;
   if (hartree) {
     int m = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) m = max(m, __double2hiint(a.vCG[TM::pos(tl, e)]) & 0x7fffffff);
     kv = 1082 - max(1, __reduce_max_sync(0xffffffffu, m) >> 20);
 #pragma unroll
-    for (int e = 0; e < E; ++e) vg[e] = fx::real_limbs(fx_convert(a.vCG[TM::pos(tl, e)], Scale{8, kv - 3}));
+    for (int e = 0; e < E; ++e) {
+      const double v = a.vCG[TM::pos(tl, e)];
+      gg[e] = min(kMaxShift, 1082 - kv - max(1, (__double2hiint(v) & 0x7fffffff) >> 20));
+      vg[e] = fx::real_limbs(fx_convert(v, Scale{8, kv - 3 + gg[e]}));
+    }
   }
   __syncthreads();
   // Launched as a programmatic dependent of the previous stage: everything
@@ -297,7 +302,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = cx{fx_convert(wv[e].x, s), 0};
     fx::forward<N, false, 1>(x, buf, tw_s, twn_s, tl, team);
-    const int r = multiply_back<N, T>(x, vg);
+    const int r = multiply_back<N, T>(x, vg, gg);
     fx::forward<N, false, 1>(x, buf, tw_s, twn_s, tl, team);
     if (lane < T) {
 #pragma unroll
@@ -319,13 +324,20 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
       m = max(1, __reduce_max_sync(0xffffffffu, m) >> 20);
       const Scale st{8, 1077 - m};  // |G|, |k + A| < 2^(m - 1022): their sum below 2^59
       const i64 kf = fx_convert(kA, st);
+      // every factor with an exponent of its own: with one for all, those of the low
+      // frequencies, which carry the orbital, were off by 2^-57 of the largest (3e-14
+      // Hartree at NG = 256 and a cell of 10), the same way in every step
       int2 t2[E];
+      int g[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const i64 t = fx_convert(a.Gx[TM::pos(tl, e)], st) + kf;
+        i64 t = fx_convert(a.Gx[TM::pos(tl, e)], st) + kf;
+        const int h = min(29, max(0, __clzll(t < 0 ? -t : t) - 4));  // to 2^59 and more
+        t <<= h;
+        g[e] = 2 * h;
         t2[e] = fx::real_limbs(fx::rmul(t, fx::real_limbs(t)));
       }
-      const int r = multiply_back<N, T>(x, t2);
+      const int r = multiply_back<N, T>(x, t2, g);
       fx::forward<N, false, 1>(x, buf, tw_s, twn_s, tl, team);
       if (lane < T) {
 #pragma unroll
