@@ -168,9 +168,10 @@ int mattohf_last_run_timing(mattohf_ctx* ctx, double* run_ms, double* fock_ms, i
  * size for one h[u]u exchange apply, (2) the CTAs per column of the fused
  * small-problem stages and (3) fused stages against the tiled step, with
  * `steps` graph-replayed mattohf_rk4_run steps (dt = 1e-4, A = 0) per
- * candidate, then keeps the fastest as MATTOHF_OPT_SYM_TILE,
- * MATTOHF_OPT_SMALL_CTAS and MATTOHF_OPT_SMALL_STAGES (0 or 1).  The orbitals
- * are restored.  out[3] (may be NULL): tile, CTAs per column (0 if the fused
+ * candidate, then keeps the fastest for h[u]u and the RK4 steps until
+ * MATTOHF_OPT_SYM_TILE, MATTOHF_OPT_SMALL_CTAS or MATTOHF_OPT_SMALL_STAGES is set
+ * again; what it did not time (other functions, the reverse stages of a
+ * gradient) goes by the options and the automatic rules.  The orbitals are restored.  out[3] (may be NULL): tile, CTAs per column (0 if the fused
  * stages do not apply), 1 if the fused stages won; us[3] (may be NULL):
  * microseconds of the exchange apply, of a tiled step and of a fused step. */
 int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* us);

@@ -118,7 +118,7 @@ struct mattohf_ctx {
   double2* d_dm_wscale = nullptr;
   size_t dm_cols = 0;         // columns of d_dm_wt and d_dm_acc
   bool dm_last = false;       // the last exchange went through it
-  int opt_dm = -1;            // 1 / 0: the autotuner's choice; -1: by rule
+  bool dm_room = true;        // false: there was no memory for it
   int2* d_kern_fx = nullptr;  // kernel table in limbs, its scale, the twiddles
   int2* d_kscale = nullptr;
   int4* d_tw_fx = nullptr;
@@ -129,6 +129,9 @@ struct mattohf_ctx {
   int opt_df = 0;             // exchange transforms in double-float arithmetic
   int opt_tile = 0;           // symmetric-exchange tile size (0 = automatic)
   int opt_small = 2;          // fused small-problem RK4 stages: 0 off, 1 on, 2 automatic
+  // the autotuner's choices for what it timed, h[u]u and the RK4 step (0 and -1: none).
+  // Other shapes (Krylov blocks, the reverse stages) keep their rules and the options.
+  int tuned_tile = 0, tuned_dm = -1, tuned_small = -1;
   int opt_small_ctas = 0;     // CTAs per column of the fused stages (0 = automatic)
   bool step_small = false;    // the captured step graph uses the fused stages
   unsigned* d_ticket = nullptr;  // completion counters of the fused stages [1 + NK*NB]
@@ -381,15 +384,13 @@ int timed_end(mattohf_ctx* ctx) {
 // RK4 steps captured in one graph for mattohf_rk4_run (divides 256)
 constexpr int kGraphSteps = 8;
 
-// Tile of the fixed-point exchange.
-int fx_tile(const mattohf_ctx* ctx) {
-  return std::min(kFxMaxTile, ctx->opt_tile > 0 ? ctx->opt_tile : choose_sym_tile(ctx->NG, ctx->NK * ctx->NBocc, ctx->nsm));
-}
-
-// Tile of the adjoint's and the double-float exchange.
+// Tile of the double-float exchange, and of the fixed-point exchange and its adjoint.
 int sym_tile(const mattohf_ctx* ctx) {
-  return ctx->opt_tile > 0 ? ctx->opt_tile : choose_sym_tile(ctx->NG, ctx->NK * ctx->NBocc, ctx->nsm);
+  return ctx->tuned_tile > 0 ? ctx->tuned_tile
+         : ctx->opt_tile > 0 ? ctx->opt_tile
+                             : choose_sym_tile(ctx->NG, ctx->NK * ctx->NBocc, ctx->nsm);
 }
+int fx_tile(const mattohf_ctx* ctx) { return std::min(kFxMaxTile, sym_tile(ctx)); }
 
 // Every buffer the RK4 step's exchange applies need, allocated up front so a
 // graph capture never has to grow one.
@@ -488,8 +489,9 @@ bool fock_dm_wins(const mattohf_ctx* c, int nbw, bool same, double launches = 6.
   return 0.75 * dm + launches < pairs;
 }
 bool use_dm(const mattohf_ctx* c, int nbw, bool same) {
-  if (!c->opt_sym || c->opt_df || c->opt_chunks > 0 || c->opt_dm == 0) return false;
-  if (c->opt_dm < 0 && c->opt_tile > 0) return false;  // a tile asked for: pairs
+  if (!c->opt_sym || c->opt_df || c->opt_chunks > 0 || !c->dm_room) return false;
+  if (c->opt_tile > 0) return false;  // a tile asked for: pairs
+  if (same && nbw == c->NB && c->tuned_dm == 0) return false;
   return fock_dm_wins(c, nbw, same);
 }
 
@@ -501,7 +503,7 @@ int dm_no_room(mattohf_ctx* ctx) {
   CKR(dalloc(ctx, &ctx->d_dm_wt, 0));
   CKR(dalloc(ctx, &ctx->d_dm_acc, 0));
   ctx->dm_cols = 0;
-  ctx->opt_dm = 0;
+  ctx->dm_room = false;
   ctx->err.clear();
   return MATTOHF_OK;
 }
@@ -552,7 +554,7 @@ int ensure_dm_tables(mattohf_ctx* ctx) {
 }
 
 // The tables, W and the buffers for ncols columns of w.  Where there is no memory for
-// them, opt_dm = 0 afterwards.
+// them, dm_room is false afterwards.
 int ensure_dm(mattohf_ctx* ctx, int ncols) {
   const int NG = ctx->NG, NK = ctx->NK;
   const int rc = ensure_dm_tables(ctx);
@@ -623,7 +625,7 @@ int enq_fock(mattohf_ctx* ctx, Block u, Block w, FockPlan* plan, bool same_u = f
   if (dm) {
     CKR(ensure_fx(ctx));
     CKR(ensure_dm(ctx, ctx->NK * w.nb));
-    dm = ctx->opt_dm != 0;
+    dm = ctx->dm_room;
   }
   if (dm) {
     plan->dm = true;
@@ -866,8 +868,9 @@ int enq_rk4(mattohf_ctx* ctx, AField f_m, AField f_ave, AField f_cur, double dt,
 // Fused small-problem stages: is this context's RK loop better served by
 // one launch per stage (one CTA per column) than by the tiled exchange?
 bool use_small(const mattohf_ctx* ctx) {
-  if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
-  if (ctx->opt_small == 1) return true;
+  const int opt = ctx->tuned_small >= 0 ? ctx->tuned_small : ctx->opt_small;
+  if (opt == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
+  if (opt == 1) return true;
   // us per RK4 step, fused against tiled, NG / NK / occupied bands, in fixed point
   // (k_small_fx.cu): 64/8/4 44 61, 128/8/2 65 68, 256/4/2 70 83, 256/8/2 77 85, but
   // 64/16/3 (M^2 NG = 2^17.2) 83 73, 128/8/3 (2^16.2) 76 68, 128/16/2 81 69, 256/8/4 150
@@ -879,10 +882,12 @@ bool use_small(const mattohf_ctx* ctx) {
 // The adjoint's reverse stages, which are in FP64 (k_small_adj.cu): us per reverse
 // step, fused against separate launches, 16/4/2 52 74, 32/16/2 76 91, 64/12/2 96 115,
 // 128/8/2 102 112; 64/8/4 120 108, 128/8/3 138 130, 128/16/2 161 131, 256/4/2 132 126,
-// 256/8/2 228 132.
+// 256/8/2 228 132.  The autotuner times the forward step, so its choice says nothing here.
 bool use_small_reverse(const mattohf_ctx* ctx) {
+  if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
+  if (ctx->opt_small == 1) return true;
   const size_t M = (size_t)ctx->NK * ctx->NBocc;
-  return use_small(ctx) && (ctx->opt_small == 1 || M * M * ctx->NG <= (ctx->NG < 256 ? (size_t)3 << 14 : (size_t)1 << 13));
+  return ctx->NK * ctx->NB <= 64 && M * M * ctx->NG <= (ctx->NG < 256 ? (size_t)3 << 14 : (size_t)1 << 13);
 }
 
 // CTAs per column.  A warp issues at most one FP64 instruction per ~64
@@ -1417,13 +1422,16 @@ int mattohf_set_option(mattohf_ctx* ctx, int option, long long value) {
       if (value < 0 || value > fock_sym_teams(ctx->NG) || (value & (value - 1)))
         return fail(ctx, MATTOHF_ERR_ARG, "tile size must be 0 or a power of two up to the CTA's teams");
       ctx->opt_tile = (int)value;
-      ctx->opt_dm = -1;
+      ctx->tuned_tile = 0;
+      ctx->tuned_dm = -1;
+      ctx->dm_room = true;
       break;
     case MATTOHF_OPT_SMALL_STAGES:
       if (value < 0 || value > 2) return fail(ctx, MATTOHF_ERR_ARG, "small-stage option must be 0, 1 or 2");
       if (value == 1 && !small_stage_supported(ctx->NG))
         return fail(ctx, MATTOHF_ERR_ARG, "fused small stages need NG <= 256");
       ctx->opt_small = (int)value;
+      ctx->tuned_small = -1;
       break;
     case MATTOHF_OPT_L2_FLUSH:
       if (value < 0 || value > (4LL << 30)) return fail(ctx, MATTOHF_ERR_ARG, "flush bytes out of range");
@@ -1928,6 +1936,23 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
     CK(cudaMemsetAsync(ctx->d_int, 0, 2 * sizeof(int), ctx->st));
     return MATTOHF_OK;
   };
+  // the choices as they were, unless all of it succeeds
+  struct Choices {
+    mattohf_ctx* c;
+    int opt_tile, tuned_tile, tuned_dm, tuned_small, ctas;
+    bool keep = false;
+    explicit Choices(mattohf_ctx* c_)
+        : c(c_), opt_tile(c_->opt_tile), tuned_tile(c_->tuned_tile), tuned_dm(c_->tuned_dm), tuned_small(c_->tuned_small),
+          ctas(c_->opt_small_ctas) {}
+    ~Choices() {
+      if (keep) return;
+      c->opt_tile = opt_tile;
+      c->tuned_tile = tuned_tile;
+      c->tuned_dm = tuned_dm;
+      c->tuned_small = tuned_small;
+      c->opt_small_ctas = ctas;
+    }
+  } before(ctx);
   // ---- exchange tile
   int bestS = ctx->opt_df ? sym_tile(ctx) : fx_tile(ctx);
   double tS = 0.0;
@@ -1949,12 +1974,13 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
       return MATTOHF_OK;
     };
     const int M = NK * ctx->NBocc, Smax = ctx->opt_df ? fock_sym_teams(NG) : std::min(kFxMaxTile, fock_sym_teams(NG));
-    ctx->opt_dm = 0;
+    ctx->opt_tile = 0;
+    ctx->tuned_dm = 0;
     for (int S = 1; S <= Smax; S <<= 1) {
       // tiles far beyond a few waves only add partial-sum traffic (and scratch)
       const long long T = (M + S - 1) / S;
       if (S < Smax && T * (T + 1) / 2 > 32LL * ctx->nsm) continue;
-      ctx->opt_tile = S;
+      ctx->tuned_tile = S;
       double t = 0.0;
       CKR(time_exchange(&t));
       if (t < best) {
@@ -1962,14 +1988,13 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
         bestS = S;
       }
     }
-    ctx->opt_tile = bestS;
+    ctx->tuned_tile = bestS;
     // the density-matrix form, where it is in question, against the best tile
-    ctx->opt_dm = -1;
-    if (!ctx->opt_df && ctx->opt_chunks == 0 && fock_dm_wins(ctx, NB, true)) {
-      ctx->opt_dm = 1;
+    ctx->tuned_dm = -1;
+    if (use_dm(ctx, NB, true)) {
       double t = 0.0;
       CKR(time_exchange(&t));
-      ctx->opt_dm = t < best ? 1 : 0;
+      ctx->tuned_dm = t < best ? 1 : 0;
       best = std::min(best, t);
     }
     tS = best;
@@ -1987,17 +2012,16 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
     *t_us = 1e3 * ctx->last_run_ms / steps;
     return MATTOHF_OK;
   };
-  const int opt_small0 = ctx->opt_small, opt_ctas0 = ctx->opt_small_ctas;
   double t_tiled = 0.0, t_fused = 0.0;
   int bestP = 0;
-  ctx->opt_small = 0;
+  ctx->tuned_small = 0;
   int rc = time_steps(&t_tiled);
   const bool fused_ok = small_stage_supported(NG) && !ctx->opt_df && !ctx->opt_timing && ctx->NBocc > 0;
   if (rc == MATTOHF_OK && fused_ok) {
     const int ncols = NK * NB, M = NK * ctx->NBocc;
     const int lo = std::min(kSmallMaxCtas, std::max(1, (M + small_pair_teams(NG) - 1) / small_pair_teams(NG)));
     const int hi = std::min(kSmallMaxCtas, std::max(lo, std::min(M, std::max(1, 2 * ctx->nsm / ncols))));
-    ctx->opt_small = 1;
+    ctx->tuned_small = 1;
     ctx->opt_small_ctas = 0;
     std::vector<int> cand{small_ctas_per_column(ctx)};
     for (int P = lo; P <= hi; ++P)
@@ -2017,15 +2041,12 @@ extern "C" int mattohf_autotune(mattohf_ctx* ctx, int steps, int* out, double* u
   // restore the state whatever happened, then keep the winners
   const int rr = restore();
   destroy_graph(ctx);
-  if (rc != MATTOHF_OK) {
-    ctx->opt_small = opt_small0;
-    ctx->opt_small_ctas = opt_ctas0;
-    return rc;
-  }
-  if (rr != MATTOHF_OK) return rr;
+  CKR(rc);
+  CKR(rr);
   const bool fused_wins = bestP > 0 && t_fused < t_tiled;
-  ctx->opt_small = fused_wins ? 1 : 0;
+  ctx->tuned_small = fused_wins ? 1 : 0;
   ctx->opt_small_ctas = bestP;
+  before.keep = true;
   CK(cudaStreamSynchronize(ctx->st));
   if (out) {
     out[0] = bestS;
@@ -2523,8 +2544,8 @@ extern "C" int mattohf_adjoint(mattohf_ctx* ctx, int objective, int nt, double d
   };
   // stage-store base step: the store slot of step it is (it - seg0)
   CK(cudaMemsetAsync(ctx->d_adj_int, 0, 4 * sizeof(int), ctx->st));
-  // small problems run their forward steps through the fused stages
-  if (use_small(ctx)) CKR(ensure_small_buffers(ctx));
+  // small problems run their steps through the fused stages
+  if (use_small(ctx) || use_small_reverse(ctx)) CKR(ensure_small_buffers(ctx));
   CK(cudaMemsetAsync(ctx->d_ticket, 0, sizeof(unsigned) * (1 + (size_t)NK * NB), ctx->st));
   // gfwd: a step that keeps the segment checkpoint; grec: a step that stores
   // its stage inputs (the last segment in the forward pass, and every
