@@ -884,6 +884,7 @@ bool use_small(const mattohf_ctx* ctx) {
 // 128/8/2 102 112; 64/8/4 120 108, 128/8/3 138 130, 128/16/2 161 131, 256/4/2 132 126,
 // 256/8/2 228 132.  The autotuner times the forward step, so its choice says nothing here.
 bool use_small_reverse(const mattohf_ctx* ctx) {
+  if (!ctx->hf) return false;  // k_small_adj.cu has the exchange in it
   if (ctx->opt_small == 0 || ctx->opt_df || ctx->opt_timing || !small_stage_supported(ctx->NG)) return false;
   if (ctx->opt_small == 1) return true;
   const size_t M = (size_t)ctx->NK * ctx->NBocc;
