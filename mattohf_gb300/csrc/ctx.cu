@@ -229,6 +229,7 @@ size_t orb_elems(const mattohf_ctx* c, int nb) { return (size_t)c->NK * nb * c->
 
 int ensure_stage(mattohf_ctx* ctx, size_t elems) {
   if (elems <= ctx->stage_cap) return MATTOHF_OK;
+  ctx->stage_cap = 0;  // until all three are there, as in the functions below
   CKR(dalloc(ctx, &ctx->d_a, elems));
   CKR(dalloc(ctx, &ctx->d_b, elems));
   CKR(dalloc(ctx, &ctx->d_c, elems));
@@ -244,6 +245,7 @@ int ensure_scratch(mattohf_ctx* ctx, int ncols) {
   if ((size_t)ncols > ctx->wfx_cap) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "scratch growth during capture");
     destroy_graph(ctx);  // the captured step holds the old pointers
+    ctx->wfx_cap = 0;
     CKR(dalloc(ctx, &ctx->d_wfx, (size_t)ncols * ctx->NG));
     CKR(dalloc(ctx, &ctx->d_wacc, (size_t)ncols * 4 * ctx->NG));
     CKR(dalloc(ctx, &ctx->d_wscale, (size_t)ncols));
@@ -253,6 +255,7 @@ int ensure_scratch(mattohf_ctx* ctx, int ncols) {
   if (cb > ctx->colbuf_cap) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "colbuf growth during capture");
     destroy_graph(ctx);
+    ctx->colbuf_cap = 0;
     CKR(dalloc(ctx, &ctx->d_colbuf, cb));
     ctx->colbuf_cap = cb;
   }
@@ -347,6 +350,7 @@ int ensure_sym(mattohf_ctx* ctx, size_t need) {
   if (need <= ctx->sym_cap) return MATTOHF_OK;
   if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "sym scratch growth during capture");
   destroy_graph(ctx);
+  ctx->sym_cap = 0;
   CKR(dalloc(ctx, &ctx->d_sym, need));
   ctx->sym_cap = need;
   return MATTOHF_OK;
@@ -942,6 +946,7 @@ int ensure_small_buffers(mattohf_ctx* ctx) {
   if (need > ctx->small_part_cap) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "fused-stage scratch growth during capture");
     destroy_graph(ctx);  // a captured step holds the old pointer
+    ctx->small_part_cap = 0;
     CKR(dalloc(ctx, &ctx->d_small_part, need));
     ctx->small_part_cap = need;
   }
@@ -1225,6 +1230,7 @@ void release_adjoint_storage(mattohf_ctx* ctx) {
 int ensure_series(mattohf_ctx* ctx, int nt) {
   if (nt <= ctx->series_cap) return MATTOHF_OK;
   destroy_graph(ctx);  // graph holds the old pointers
+  ctx->series_cap = 0;
   CKR(dalloc(ctx, &ctx->d_A, nt));
   CKR(dalloc(ctx, &ctx->d_Aave, nt));
   CKR(dalloc(ctx, &ctx->d_sE, nt));
@@ -1794,6 +1800,7 @@ int mattohf_rk4_run(mattohf_ctx* ctx, int nt, double dt, const double* A, const 
     if ((size_t)ctx->opt_flush > ctx->flush_cap) {
       if (ctx->d_flush) cudaFree(ctx->d_flush);
       ctx->d_flush = nullptr;
+      ctx->flush_cap = 0;
       CK(cudaMalloc(&ctx->d_flush, (size_t)ctx->opt_flush));
       ctx->flush_cap = (size_t)ctx->opt_flush;
     }
@@ -2073,6 +2080,7 @@ int mattohf_last_run_timing(mattohf_ctx* ctx, double* run_ms, double* fock_ms, i
 static int ensure_gs(mattohf_ctx* ctx, int m) {
   const size_t need = orb_elems(ctx, m);
   if (need <= ctx->gs_cap) return MATTOHF_OK;
+  ctx->gs_cap = 0;
   CKR(dalloc(ctx, &ctx->d_work, need));
   CKR(dalloc(ctx, &ctx->d_hwork, need));
   CKR(dalloc(ctx, &ctx->d_M, (size_t)ctx->NK * m * m));

@@ -99,3 +99,27 @@ def test_apply_that_runs_out_of_room(orbitals):
         ctx.synchronize()
         got = out.cpu().numpy().view(np.complex128)
         assert np.array_equal(got, ctx.ubkwbk_hwbk(orbitals, orbitals[:, :2], 0.1))
+
+
+def test_smaller_calls_after_one_that_found_no_room(orbitals):
+    """A call that fails to enlarge the work buffers leaves none of them half made: smaller
+    calls, which the old ones served, make them again and give the same bits."""
+    from mattohf_gb300 import Context, MattohfError, _capi
+    NG, NK, nb = SHAPE
+    A = np.full(3, 0.01)
+    with Context(_cfg(NG, NK, 2)) as ctx:
+        u = np.ascontiguousarray(orbitals[:, :2])
+
+        def small():
+            ctx.set_orbitals(u)
+            return [ctx.ubkwbk_hwbk(u, u[:, :1], 0.1), *ctx.rk4_run(A, A, 1e-4), ctx.GS_calculation(1, 2)["Etot"]]
+
+        before = small()
+        with _no_room():
+            for call in (lambda: ctx.ubkwbk_hwbk(u, orbitals, 0.1), lambda: ctx.rk4_run(np.zeros(1 << 21), np.zeros(1 << 21), 1e-4),
+                         lambda: ctx.GS_calculation(1, 32)):
+                with pytest.raises(MattohfError) as e:
+                    call()
+                assert e.value.status == _capi.ERR_ALLOC
+        for a, b in zip(small(), before):
+            assert np.array_equal(a, b)
