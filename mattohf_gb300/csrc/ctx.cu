@@ -184,6 +184,8 @@ struct mattohf_ctx {
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> fock_events;
   size_t fock_event_used = 0;
   bool capturing = false;
+  // counts the growths of buffers that an ensemble's argument arrays and graph point to
+  unsigned long long moved = 0;
   std::string err;
 };
 
@@ -256,6 +258,7 @@ int ensure_scratch(mattohf_ctx* ctx, int ncols) {
     if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "colbuf growth during capture");
     destroy_graph(ctx);
     ctx->colbuf_cap = 0;
+    ++ctx->moved;
     CKR(dalloc(ctx, &ctx->d_colbuf, cb));
     ctx->colbuf_cap = cb;
   }
@@ -351,6 +354,7 @@ int ensure_sym(mattohf_ctx* ctx, size_t need) {
   if (ctx->capturing) return fail(ctx, MATTOHF_ERR_STATE, "sym scratch growth during capture");
   destroy_graph(ctx);
   ctx->sym_cap = 0;
+  ++ctx->moved;
   CKR(dalloc(ctx, &ctx->d_sym, need));
   ctx->sym_cap = need;
   return MATTOHF_OK;
@@ -1231,6 +1235,7 @@ int ensure_series(mattohf_ctx* ctx, int nt) {
   if (nt <= ctx->series_cap) return MATTOHF_OK;
   destroy_graph(ctx);  // graph holds the old pointers
   ctx->series_cap = 0;
+  ++ctx->moved;
   CKR(dalloc(ctx, &ctx->d_A, nt));
   CKR(dalloc(ctx, &ctx->d_Aave, nt));
   CKR(dalloc(ctx, &ctx->d_sE, nt));
@@ -2740,6 +2745,7 @@ struct mattohf_batch {
   int total_tiles = 0, total_elems = 0, total_cols = 0;
   cudaGraphExec_t exec = nullptr;
   int built_nt = -1;
+  unsigned long long built_moved = 0;  // the runs' `moved` then: a run is also a context of its own
   std::vector<double> dts;
   double last_ms = 0;
   std::string err;
@@ -2839,6 +2845,12 @@ int batch_ensure_dm(mattohf_batch* b) {
     b->opt_dm = false;
   }
   return MATTOHF_OK;
+}
+
+unsigned long long batch_moved(const mattohf_batch* b) {
+  unsigned long long n = 0;
+  for (const auto* c : b->runs) n += c->moved;
+  return n;
 }
 
 // (Re)build every per-run argument array for runs of `nt` steps.
@@ -3000,6 +3012,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
   cudaGraphDestroy(g);
   BCK(ei);
   b->built_nt = nt;
+  b->built_moved = batch_moved(b);
   return MATTOHF_OK;
 }
 
@@ -3086,7 +3099,7 @@ int mattohf_batch_rk4_run(mattohf_batch* b, int nt, const double* dt, const doub
     if (b->dts[r] != dt[r]) dt_changed = true;
     b->dts[r] = dt[r];
   }
-  if (dt_changed || b->built_nt < nt) {
+  if (dt_changed || b->built_nt < nt || b->built_moved != batch_moved(b)) {
     b->built_nt = -1;
     int rc = batch_prepare(b, nt);
     if (rc != MATTOHF_OK) return rc;
