@@ -80,10 +80,14 @@ __device__ __forceinline__ double2 exchange_value(const ExSource& s, int col, in
   }
   x = fma(x, f.x, x * f.y);
   y = fma(y, f.x, y * f.y);
+  if (__double2hiint(f.x) < 0) {  // fx_output_scale: 2^kTiny too large
+    x = fx_times_pow2(-x, -kTiny);
+    y = fx_times_pow2(-y, -kTiny);
+  }
   if (s.pexp != nullptr) {
-    const double p = pow2(-s.pexp[q]);
-    x *= p;
-    y *= p;
+    const int e = -s.pexp[q];
+    x = fx_times_pow2(x, e);
+    y = fx_times_pow2(y, e);
   }
   return make_double2(x, y);
 }

@@ -88,8 +88,15 @@ __device__ __forceinline__ double pow2(int e) {  // 2^e, 0 or infinity outside t
   return e > 1023 ? __longlong_as_double(0x7ff0000000000000ll) : e < -1022 ? 0.0 : __hiloint2double((e + 1023) << 20, 0);
 }
 
+// v 2^e for any e, to denormal numbers.  Not inlined: what is rare stays a branch, not
+// an FP64 product of every value.
+static __device__ __noinline__ double fx_times_pow2(double v, int e) { return v * pow2(e / 2) * pow2(e - e / 2); }
+
 // 2^180 / (s^2 sd sk) as factor + correction: the product of the short factors
-// is exact, its reciprocal is good to twice the precision
+// is exact, its reciprocal is good to twice the precision.  Where a sum of 2^62 times the
+// factor may leave the normal range downwards, both are 2^kTiny larger and negative
+// (exchange_value takes that back).
+constexpr int kTiny = 512;
 __device__ __forceinline__ double2 fx_output_scale(Scale s, Scale sd, Scale sk) {
   if (s.c == 0 || sd.c == 0) return make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
   const int q = s.c * s.c * sd.c * sk.c;  // below 2^16
@@ -98,8 +105,8 @@ __device__ __forceinline__ double2 fx_output_scale(Scale s, Scale sd, Scale sk) 
   r = fma(fma(-r, dq, 1.0), r, r);
   r = fma(fma(-r, dq, 1.0), r, r);
   const double lo = fma(-r, dq, 1.0) * r;
-  const int e = 180 - 2 * s.k - sd.k - sk.k, h = e / 2;
-  const double p = pow2(h), p2 = pow2(e - h);
+  const int e0 = 180 - 2 * s.k - sd.k - sk.k, e = e0 < -800 ? e0 + kTiny : e0, h = e / 2;
+  const double p = e0 < -800 ? -pow2(h) : pow2(h), p2 = pow2(e - h);
   return make_double2(r * p * p2, lo * p * p2);
 }
 
@@ -110,7 +117,19 @@ __device__ __forceinline__ Scale fx_fft_scale(int2 z, int N) {
   if (s.c) s.c = 8;
   return s;
 }
-__device__ __forceinline__ double fx_unscale(Scale s) { return s.c ? pow2(-(s.k + 3)) : __longlong_as_double(0x7ff8000000000000ll); }
+// Back from such a scale: times 2^-(k + 3), which need not be a normal number, by the
+// exponent field in integer work
+struct Unscale {
+  int e;
+  bool ok;
+  __device__ __forceinline__ double operator()(i64 v) const {
+    const double d = (double)v;
+    const int hi = __double2hiint(d), x = ((hi >> 20) & 0x7ff) + e;
+    if (ok && hi != 0 && x > 0 && x < 0x7ff) return __hiloint2double(hi + (e << 20), __double2loint(d));
+    return fx_times_pow2(ok ? d : __longlong_as_double(0x7ff8000000000000ll), e);
+  }
+};
+__device__ __forceinline__ Unscale fx_unscale(Scale s) { return Unscale{-(s.k + 3), s.c != 0}; }
 
 // Size of the values that a CTA's threads hold; red: two words per warp.  Two barriers.
 template <int PER, int NWARP>

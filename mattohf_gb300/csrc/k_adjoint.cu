@@ -73,15 +73,15 @@ __global__ void __launch_bounds__(ColumnCta<N>::TH) k_adj_combine(AdjCombineArgs
       for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(mu[p].x, s1), fx_convert(mu[p].y, s1)};
     }
     fx_block_forward<N>(buf, tw_s);
-    const double u1 = fx_unscale(s1), uv = fx_unscale(sv);
+    const Unscale u1 = fx_unscale(s1), uv = fx_unscale(sv);
     double gp = 0.0;
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
       if (!in) continue;
       const int q = tid + TH * p;
       const double G = a.Gx[q];
-      const double mx = (double)buf[q].x * u1, my = (double)buf[q].y * u1;
-      gp += (G + a.kx[ik] + A) * (mx * ((double)vf[p].y * uv) - my * ((double)vf[p].x * uv));
+      const double mx = u1(buf[q].x), my = u1(buf[q].y);
+      gp += (G + a.kx[ik] + A) * (mx * uv(vf[p].y) - my * uv(vf[p].x));
       const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2) * (1.0 / N);
       lu[p] = make_double2(m * mx, -m * my);  // conjugate: backward next
     }
@@ -94,13 +94,13 @@ __global__ void __launch_bounds__(ColumnCta<N>::TH) k_adj_combine(AdjCombineArgs
       for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(lu[p].x, s2), fx_convert(lu[p].y, s2)};
     }
     fx_block_forward<N>(buf, tw_s);
-    const double u2 = fx_unscale(s2);
+    const Unscale u2 = fx_unscale(s2);
     if (!in) return;
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
       const int q = tid + TH * p;
       const double vl = a.vloc[q];
-      lu[p] = mul_i(make_double2((double)buf[q].x * u2 + vl * mu[p].x, (double)buf[q].y * -u2 + vl * mu[p].y));
+      lu[p] = mul_i(make_double2(vl * mu[p].x + u2(buf[q].x), vl * mu[p].y - u2(buf[q].y)));
       if (a.split == 1) a.lpre[o + q] = lu[p];
     }
     if (a.split == 1) return;

@@ -121,9 +121,8 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
     if (in) buf[tid] = cx{fx_convert(v[0].x, sb), fx_convert(v[0].y, sb)};
     fx_block_forward<N>(buf, tw_s);
     if (in) {
-      const double u = fx_unscale(sb);
-      a.vloc[tid] = (double)buf[tid].x * u * fx_unscale(sr) + a.vion[tid];
-      a.psi[tid] = (double)buf[tid].y * -u * fx_unscale(ss);
+      a.vloc[tid] = Unscale{-(sb.k + sr.k + 6), sb.c != 0 && sr.c != 0}(buf[tid].x) + a.vion[tid];
+      a.psi[tid] = -Unscale{-(sb.k + ss.k + 6), sb.c != 0 && ss.c != 0}(buf[tid].y);
       a.gvion[tid] += sig;
     }
     return;
@@ -132,14 +131,15 @@ __device__ __forceinline__ void density_body(const DensArgs& a) {
   if (in) buf[tid] = cx{fx_convert(v[0].x, s1), 0};
   fx_block_forward<N>(buf, tw_s);
   if (in) {
-    const double f = a.vCG[tid] * fx_unscale(s1) * (1.0 / N);
-    v[0] = make_double2(f * (double)buf[tid].x, -f * (double)buf[tid].y);  // conjugate: backward next
+    const Unscale u = fx_unscale(s1);
+    const double f = a.vCG[tid] * (1.0 / N);
+    v[0] = make_double2(f * u(buf[tid].x), -f * u(buf[tid].y));  // conjugate: backward next
   }
   z = fx_block_size<1, NW>(v, red);
   const Scale s2 = fx_fft_scale(z, N);
   if (in) buf[tid] = cx{fx_convert(v[0].x, s2), fx_convert(v[0].y, s2)};
   fx_block_forward<N>(buf, tw_s);
-  if (in) vh_s[tid] = (double)buf[tid].x * fx_unscale(s2);
+  if (in) vh_s[tid] = fx_unscale(s2)(buf[tid].x);
   __syncthreads();
   for (int ig = tid; ig < N; ig += blockDim.x) a.vloc[ig] = vh_s[ig] + a.vion[ig];
   if (a.scal != nullptr && tid < 64) {
@@ -296,7 +296,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(wv[p].x, s1), fx_convert(wv[p].y, s1)};
     }
     fx_block_forward<N>(buf, tw_s);
-    const double u1 = fx_unscale(s1);
+    const Unscale u1 = fx_unscale(s1);
     if (a.mode == CM_OBS || a.obs) {
       // Ekin and Je of this column by Parseval on FFT(u):
       //   sum_x conj(u) IFFT(f * FFT(u)) = sum_G f(G) |FFT(u)(G)|^2
@@ -308,7 +308,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
         for (int p = 0; p < PER; ++p) {
           const int q = tid + TH * p;
           const double G = a.Gx[q];
-          const double xr = (double)buf[q].x * u1, xi = (double)buf[q].y * u1;
+          const double xr = u1(buf[q].x), xi = u1(buf[q].y);
           const double m2 = xr * xr + xi * xi;
           ek += 0.5 * (G * G + 2.0 * G * kAo + kAo2) * m2;
           je += (G + a.kx[ik] + Ao) * m2;
@@ -343,8 +343,8 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       kin[p] = make_double2(0.0, 0.0);
       if (in) {
         const double G = a.Gx[q];
-        const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2) * (u1 * (1.0 / N));
-        kin[p] = make_double2(m * (double)buf[q].x, -m * (double)buf[q].y);  // conjugate: backward next
+        const double m = 0.5 * (G * G + 2.0 * G * kAx + kA2) * (1.0 / N);
+        kin[p] = make_double2(m * u1(buf[q].x), -m * u1(buf[q].y));  // conjugate: backward next
       }
     }
     z = fx_block_size<PER, NW>(kin, red);
@@ -354,10 +354,10 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, const int c) 
       for (int p = 0; p < PER; ++p) buf[tid + TH * p] = cx{fx_convert(kin[p].x, s2), fx_convert(kin[p].y, s2)};
     }
     fx_block_forward<N>(buf, tw_s);
-    const double u2 = fx_unscale(s2);
+    const Unscale u2 = fx_unscale(s2);
     if (in) {
 #pragma unroll
-      for (int p = 0; p < PER; ++p) kin[p] = make_double2((double)buf[tid + TH * p].x * u2, (double)buf[tid + TH * p].y * -u2);
+      for (int p = 0; p < PER; ++p) kin[p] = make_double2(u2(buf[tid + TH * p].x), -u2(buf[tid + TH * p].y));
     }
   }
   const size_t ocol = (size_t)ik * a.w.nb * N + (size_t)ib * N;  // [NK][NB][NG]

@@ -258,11 +258,12 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
   auto parseval = [&](const cx (&X)[E], Scale s) {
     const int itn = *a.it;
     const double Ao = (itn >= 1 && a.Aobs) ? a.Aobs[itn - 1] : 0.0;
-    const double kAx = a.kx[kr] + Ao, kA2 = kAx * kAx, un = fx_unscale(s);
+    const double kAx = a.kx[kr] + Ao, kA2 = kAx * kAx;
+    const Unscale un = fx_unscale(s);
     double ek = 0.0, je = 0.0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      const double G = a.Gx[TM::pos(tl, e)], xr = (double)X[e].x * un, xi = (double)X[e].y * un;
+      const double G = a.Gx[TM::pos(tl, e)], xr = un(X[e].x), xi = un(X[e].y);
       const double m2 = xr * xr + xi * xi;
       ek += 0.5 * (G * G + 2.0 * G * kAx + kA2) * m2;
       je += (G + a.kx[kr] + Ao) * m2;
