@@ -71,18 +71,17 @@ constexpr float kNorm = 1.3241e18f, kPeak = 3.803e17f;
 
 // s of a set of size z (largest component, largest squared norm; both short of the
 // true ones by less than 2^-17).  Not a number when the set holds a value that is
-// not finite or has an exponent field from emax on; for a set of zeros (or
+// not finite; for a set of zeros (or
 // denormal numbers), so large that every result scales back to zero.  peak: the
 // bound of a component, n: further factor under the norm's.
-__device__ __forceinline__ Scale fx_scale(int2 z, float peak, float n, int emax) {
+__device__ __forceinline__ Scale fx_scale(int2 z, float peak, float n) {
   const int e = z.x >> 20;
-  if (e >= emax) return Scale{0, 0};
+  if (e >= 2047) return Scale{0, 0};
   if (z.x < 0x100000) return Scale{8, 2000};
   // norm^2 = g 2^(2 (e - 1023)); the key's exponent is within a few units of 2 e
   const float g = __int_as_float(((z.y >> 18) - 2 * e + 127) << 23 | (z.y & 0x3ffff) << 5);
   return fx_short_scale(fminf(kNorm * rsqrtf(g * n), peak / fx_mantissa(z.x, e)) * (1.0f - 1.0f / 16384.0f), 1023 - e);
 }
-constexpr int kSquareMax = 1023 + 510;  // the squared norm overflows
 
 __device__ __forceinline__ double pow2(int e) {  // 2^e, 0 or infinity outside the normal range
   return e > 1023 ? __longlong_as_double(0x7ff0000000000000ll) : e < -1022 ? 0.0 : __hiloint2double((e + 1023) << 20, 0);
@@ -113,7 +112,7 @@ __device__ __forceinline__ double2 fx_output_scale(Scale s, Scale sd, Scale sk) 
 // Scale of N values of size z (fx_block_size) that a transform takes: every partial sum is below sqrt(N) |v|_2 <= 2^60.2.  A power
 // of two, so that scaling back is exact.
 __device__ __forceinline__ Scale fx_fft_scale(int2 z, int N) {
-  Scale s = fx_scale(z, 1e30f, (float)N, 2047);
+  Scale s = fx_scale(z, 1e30f, (float)N);
   if (s.c) s.c = 8;
   return s;
 }

@@ -170,12 +170,12 @@ __global__ void __launch_bounds__(128) k_dm_convert(FockDmArgs a, int N, int nbu
   const int m = dm_largest(a.sizes, M, red);
   // n(x) s^2 <= 2^119.4: the sums over a band's pairs keep a bit for their middle words
   const int2 us = nbu == 0 ? *a.uscale : make_int2(0, 0);  // no orbitals to convert: W's scale
-  const Scale su = nbu == 0 ? Scale{us.x, us.y} : fx_scale(fx_size(m, __int_as_float(*a.nmax) * 1.0002f), 1e30f, 2.0f, kSquareMax);
+  const Scale su = nbu == 0 ? Scale{us.x, us.y} : fx_scale(fx_size(m, __int_as_float(*a.nmax) * 1.0002f), 1e30f, 2.0f);
   if (row) {
     for (int j = warp; j < 8 && k0 + j < a.nk; j += 4) {
       const double2* p = src.p + (size_t)(k0 + j) * src.kstride + (size_t)b * N;
       const int2 z = same && b < a.nbocc ? a.sizes[(k0 + j) * a.nbocc + b] : fx_column_size(p, N, lane);
-      if (lane == 0) sw[j] = fx_scale(z, kDmPeak, 1e-6f, kSquareMax);
+      if (lane == 0) sw[j] = fx_scale(z, kDmPeak, 1e-6f);
     }
     __syncthreads();
   }

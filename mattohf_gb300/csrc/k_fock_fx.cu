@@ -20,7 +20,7 @@
 //     p^ = u_a^ conj(u_b^) / 2^60,  phi^ = IFFT(K^ FFT(p^) / 2^60),
 //     F_a^ += phi^ u_b^ / 2^60,     F = F^ 2^180 / (s^3 s_k 2^d_a),
 // every sum exact in integers, so the order of summation does not matter.
-// Orbitals that are not finite, or whose squared norm overflows, give NaN.
+// Orbitals that are not finite give NaN.
 //
 // What bounds it and what it measured.  k_fock_sym_fx at NG = 256, NK = 64,
 // Nocc = 4 (32896 pairs): 165 us, against 918 us of the same pairs in FP64 (89 % FP64
@@ -82,12 +82,12 @@ __device__ __forceinline__ void fx_convert_body(const FockFxArgs& a, const FockF
   g = fx_larger(fx_larger(red[0], red[1]), fx_larger(red[2], red[3]));
   if (!row) own = own_s;
   // with a scale per point the sums' terms are uprod's, and u^ is bounded by its norm alone
-  Scale s = fx_scale(g, a.pexp != nullptr ? 1e30f : kPeak, 1.0f, kSquareMax);
+  Scale s = fx_scale(g, a.pexp != nullptr ? 1e30f : kPeak, 1.0f);
   s.k -= a.halve;
   Scale sd = s;
   int d = 0;
   if (row) {
-    sd = fx_scale(own, 1e30f, 1.0f, kSquareMax);
+    sd = fx_scale(own, 1e30f, 1.0f);
   } else if (a.lift && own.y > 0) {
     // a column with half the largest norm or less is lifted by 2^d to the upper half: the
     // largest d with own^2 4^d up to the largest square (keys order like these)

@@ -208,11 +208,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_stage_fx(SmallStageArgs
     if (lane == 0) size_s[warp] = zu;
 #pragma unroll
     for (int e = 0; e < E; ++e) wv[e] = wcol[TM::pos(tl, e)];
-    sw = binary_scale(fx_scale(team_size<T>(wv), 1e30f, 1.0f, kSquareMax));
+    sw = binary_scale(fx_scale(team_size<T>(wv), 1e30f, 1.0f));
     asm volatile("bar.sync 4, %0;" ::"r"(32 * workers) : "memory");
     for (int w = 0; w < workers; ++w) zu = fx_larger(zu, size_s[w]);
     // sums of n terms, at most 2^59.3 each at the full peak (k_fock_fx.cu), below 2^62.9
-    su = binary_scale(fx_scale(zu, kPeak * fminf(1.0f, (float)kFxTerms / (float)n), 1.0f, kSquareMax));
+    su = binary_scale(fx_scale(zu, kPeak * fminf(1.0f, (float)kFxTerms / (float)n), 1.0f));
     i64 rr[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) rr[e] = 0;

@@ -46,3 +46,18 @@ def test_small_orbitals(built_lib, NG, NK, nb):
             us = u * 2.0 ** e
             for got, ref in ((ctx.dns_vH_of(us), vH), (ctx.ubkwbk_vFwbk(us, w).view(float), F.view(float))):
                 assert np.max(np.abs(np.ldexp(got, -2 * e) - ref)) <= 2.0 ** -60 * np.max(np.abs(ref)), e
+
+
+@pytest.mark.parametrize("NG,NK,nocc,nbw", SHAPES)
+def test_large_functions(built_lib, NG, NK, nocc, nbw):
+    """Beyond 2^510 the square of w is no number, but nothing in h[u] w needs it, and the
+    exchange alone needs no square of u."""
+    from mattohf_gb300 import Context
+    u, w = _functions(NG, NK, nocc, 1), _functions(NG, NK, nbw, 2)
+    with Context(_cfg(NG, NK, nocc)) as ctx:
+        F = ctx.ubkwbk_vFwbk(u, w)
+        for f in (lambda x: ctx.ubk_tubk(x, 0.1), lambda x: ctx.ubkwbk_vFwbk(u, x), lambda x: ctx.ubkwbk_hwbk(u, x, 0.1)):
+            ref = f(w)
+            for e in (505, 515, 900):
+                assert np.array_equal(f(w * 2.0 ** e), ref * 2.0 ** e), e
+        assert np.array_equal(ctx.ubkwbk_vFwbk(u * 2.0 ** 520, w * 2.0 ** -100), F * 2.0 ** 940)
