@@ -89,7 +89,7 @@ struct mattohf_ctx {
   double* d_dpart = nullptr;  // [kDensChunks][NG] density partials
   // state
   double2 *d_u = nullptr, *d_us = nullptr, *d_k[4] = {nullptr, nullptr, nullptr, nullptr};
-  double2* d_hpre = nullptr;  // T_A w + vloc w of an RK4 stage, made beside the exchange
+  double2* d_hpre = nullptr;  // T_A w of an RK4 stage, made beside the exchange
   // staging for host-array entry points
   double2 *d_a = nullptr, *d_b = nullptr, *d_c = nullptr;
   size_t stage_cap = 0;
@@ -105,8 +105,8 @@ struct mattohf_ctx {
   int* d_fx_shift = nullptr;
   double2* d_fx_fscale = nullptr;
   int2* d_uscale = nullptr;
-  int4* d_uprod = nullptr;    // of the exchange by itself: orbitals with a scale per grid
-  int* d_points = nullptr;    // point and its exponents
+  int4* d_uprod = nullptr;    // of the exchange by itself: orbitals with a scale per grid point,
+  int* d_points = nullptr;    // and the points' exponents
   int4* d_wfx = nullptr;      // other functions in limbs and their scales
   double2* d_wscale = nullptr;
   unsigned long long *d_fx_acc = nullptr, *d_wacc = nullptr;  // exchange sums
@@ -2725,7 +2725,7 @@ struct mattohf_batch {
   FockSymDfArgs* d_fsym_df[kVariants] = {};
   FockFxArgs* d_fsym_fx[kVariants] = {};
   CombineArgs* d_comb[kVariants] = {};
-  CombineArgs* d_comb_pre[4] = {};  // stages' kinetic + local-potential pass (beside the exchange)
+  CombineArgs* d_comb_pre[4] = {};  // stages' kinetic pass (beside the exchange)
   cudaStream_t st_side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int opt_df = 0;  // exchange transforms in double-float arithmetic
@@ -2989,7 +2989,7 @@ int batch_prepare(mattohf_batch* b, int nt) {
   BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
   for (int s = 0; s < 4 && e == cudaSuccess; ++s) {
-    // density and the kinetic + local-potential pass beside the exchange
+    // density and the kinetic pass beside the exchange
     e = cudaEventRecord(b->ev_fork, b->st);
     if (e != cudaSuccess) break;
     cudaError_t es = cudaStreamWaitEvent(b->st_side, b->ev_fork, 0);
@@ -3249,7 +3249,7 @@ int mattohf_batch_last_run_ms(mattohf_batch* b, double* ms) {
 
 // The adjoint of every member, one member at a time.  A member of the largest
 // shapes (NG = 512, NK = 128, Nocc = 8: half a million exchange pairs per
-// apply) fills the FP64 pipe by itself, so members side by side would gain no
+// apply) fills the GPU by itself, so members side by side would gain no
 // throughput and would split the device memory that the checkpoint segments
 // use; in turn, each member gets all of it (its segment is fitted to the free
 // memory when ckpt_every <= 0) and releases it before the next one starts.

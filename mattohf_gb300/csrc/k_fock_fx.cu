@@ -25,9 +25,10 @@
 // What bounds it and what it measured.  k_fock_sym_fx at NG = 256, NK = 64,
 // Nocc = 4 (32896 pairs): 165 us, against 918 us of the same pairs in FP64 (89 % FP64
 // pipe).  It issues about 390 instructions per point and pair, 87 of them
-// 32 x 32 + 64-bit multiply-adds at half the rate of the others; the multiplier
-// pipe is 69 % busy, the adder pipe 53 %, shared memory 39 %.  Two CTAs of 128
-// threads a SM at least (a register limit for four of them spills: 183 us).
+// 32 x 32 + 64-bit multiply-adds at half the rate of the others; at NK = 32 (51 us, tiles
+// of 2) the heavy FMA pipe that has these is 55 % busy, the ALU 44 %, the issue slots
+// 48 %.  Two CTAs of 128 threads a SM at least (a register limit for four of them spills:
+// 183 us).
 // Error of one apply against long double, same table, smooth orthonormal
 // orbitals, here / FP64: NG = 64 0.7e-16 / 1.2e-16, NG = 256 1.0e-16 / 1.8e-16,
 // NG = 512 1.3e-16 / 1.9e-16.

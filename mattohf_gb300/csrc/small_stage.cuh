@@ -1,8 +1,8 @@
 // The parts of the fused fixed-point RK4 stages (k_small_fx.cu) outside the transforms:
 // the observables, the staged copies for the adjoint, the exchange of partial results
 // within a column's cluster and the RK4 update.  k_small.cu has the same steps written
-// out in its kernel: with these functions its stages were about 0.8 % slower (50 steps
-// at 64 / 8 / 2: 1.005 against 0.993 of the same earlier build's time), a difference of
+// out in its kernel: with these functions its stages were 1.2 % slower (50 steps at
+// 64 / 8 / 2: 1.005 against 0.993 of the same earlier build's time), a difference of
 // register allocation.
 #pragma once
 #include <cooperative_groups.h>
