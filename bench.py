@@ -114,19 +114,20 @@ class ClockSampler:
         self.device = device
         self.proc = None
         self.lines = []
+        self.before = []  # the last sample before the region: for the maximum clock
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.Q}", "--format=csv,noheader,nounits",
-                 "-lms", "50"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                 "-lms", "5"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
             # nvidia-smi takes a moment to start: the timed region begins after its first sample
             t0 = time.time()
             while not self.lines and time.time() - t0 < 3.0 and self.proc.poll() is None:
                 time.sleep(0.01)
-            self.lines.clear()
+            self.before, self.lines = self.lines[-1:], []
         except (OSError, FileNotFoundError):
             self.proc = None
         return self
@@ -146,20 +147,31 @@ class ClockSampler:
     def summary(self):
         sm, mx, reasons = [], None, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ln in self.lines:
+        for i, ln in enumerate(self.before + self.lines):
             f = [x.strip() for x in ln.split(",")]
             if len(f) < 9:
                 continue
             try:
-                sm.append(float(f[1]))
-                mx = float(f[2])
+                clock, mx = float(f[1]), float(f[2])
             except ValueError:
                 continue
+            if i < len(self.before):
+                continue
+            sm.append(clock)
             for n, v in zip(names, f[5:9]):
                 if v.lower().startswith("active"):
                     reasons.add(n)
         return {"sm_mhz": statistics.median(sm) if sm else None, "sm_max_mhz": mx,
                 "reasons": sorted(reasons), "samples": len(sm)}
+
+
+def multiprocessors(device: int) -> int:
+    import ctypes as C
+    cu = C.CDLL("libcuda.so.1")
+    n = C.c_int()
+    if cu.cuDeviceGetAttribute(C.byref(n), 16, device):  # CU_DEVICE_ATTRIBUTE_MULTIPROCESSOR_COUNT
+        raise RuntimeError("cuDeviceGetAttribute failed")
+    return n.value
 
 
 def bench_config(cfg):
@@ -302,8 +314,11 @@ def run_gpu(args, dist):
     ctx.set_option(_capi.OPT_KERNEL_TIMING, 0)
     mads = exchange_multiply_adds(cfg.NG, cfg.NK, cfg.NB, cfg.NBocc)
     achieved = mads / (fock_ms / nf * 1e-3) / 1e12
-    # 32 a clock and multiprocessor with three different registers each
-    peak_mads = 32 * 152 * (clocks.get("sm_mhz") or 1920.0) * 1e6 / 1e12
+    # 32 a clock and multiprocessor with three different registers each, at the clock sampled
+    # in the region or (the region may be shorter than a sample takes) the largest
+    clock_name, clock = next((n, c) for n, c in (("sampled", clocks["sm_mhz"]), ("largest", clocks["sm_max_mhz"]),
+                                                 ("assumed", 1920.0)) if c)
+    peak_mads = 32 * multiprocessors(dev) * clock * 1e6 / 1e12
     peak = C.c_double()
     lib.mattohf_diag_fp64_peak(dev, C.byref(peak))
     dmma = C.c_double()
@@ -374,7 +389,7 @@ def run_gpu(args, dist):
                          "kernel": "k_dm_build + k_dm_apply",
                          "mads_per_apply": mads, "apply_ms": fock_ms / nf,
                          "peak_source": "32 multiply-adds (32 x 32 + 64 bits) a clock and multiprocessor, measured, "
-                                        "x 152 x the sampled SM clock",
+                                        f"x {multiprocessors(dev)} x the SM clock ({clock_name}, {clock:.0f} MHz)",
                          "fp64_peak_tflops": peak.value, "fp64_tensor_peak": dmma.value,
                          "fp64_tensor_peak_source": "measured DMMA (mma.sync m8n8k4 f64) throughput, "
                                                     "mattohf_diag_dmma_peak",
