@@ -80,3 +80,20 @@ def test_gradient_whose_forward_uses_the_density_matrix(built_lib):
     (_, g0, v0, u0), (_, g1, v1, u1) = out
     assert not np.array_equal(u0, u1) and _rel(u0, u1) <= 8 * _tol(NK)
     assert _rel(g0, g1) <= 2.0 ** 6 * 16 * _tol(NK) and _rel(v0, v1) <= 2.0 ** 6 * 16 * _tol(NK)
+
+
+def test_batch_members_take_their_form(built_lib):
+    """Large members go through the density matrix, whose roundings are others than the
+    pairs'; small ones by pairs, whose sums are exact at any tile."""
+    from mattohf_gb300 import Batch
+    shapes, nt = [(64, 8), (3, 2), (33, 9)], 2
+    u0 = [_functions(64, NK, nb, NK) for NK, nb in shapes]
+    out = []
+    with Batch([_cfg(64, NK, nb) for NK, nb in shapes]) as b:
+        for tile in (0, 2):
+            b.set_option(OPT_TILE, tile)
+            for r, u in enumerate(u0):
+                b[r].set_orbitals(u)
+            b.rk4_run(np.zeros((3, nt)), np.zeros((3, nt)), 0.003)
+            out.append([b[r].get_orbitals() for r in range(3)])
+    assert [np.array_equal(x, y) for x, y in zip(*out)] == [False, True, False]
